@@ -32,6 +32,7 @@
 #include "tlr_dense.h"
 #include "tlr_internal.h"
 #include "tlr_lu.h"
+#include "tlr_pipe.h"
 
 namespace tlr {
 namespace {
@@ -98,6 +99,7 @@ struct Workspace {  // device buffers of the Krylov driver, owned by the context
   float2 *blk32 = nullptr;
   double *bnd = nullptr;       // 2 norms per vector (device)
   double *bnh = nullptr;       // the same, pinned
+  Pipe pipe;                   // pipelined applications (mixed form), on first use
 };
 
 struct Solver {
@@ -206,6 +208,7 @@ struct Solver {
     for (cudaEvent_t e : brev)
       if (e) cudaEventDestroy(e);
     if (ref_exec) cudaGraphExecDestroy(ref_exec);
+    if (pipe_exec) cudaGraphExecDestroy(pipe_exec);
     if (bref_exec) cudaGraphExecDestroy(bref_exec);
   }
 
@@ -558,6 +561,93 @@ struct Solver {
     return TLR_OK;
   }
 
+  // Pipelined applications (tlr_pipe.h): one graph per round -- the residuals
+  // of x and y, one triangular solve of three right-hand sides, the
+  // corrections, the acceptance residual of x -- with one synchronisation.
+  Pipe *pipe = nullptr;
+  cudaGraphExec_t pipe_exec = nullptr;
+  long long pipe_kernels = 0;
+  float2 *pipe_rhs() const { return static_cast<float2 *>(F->vec_m); }
+
+  int build_pipe_graph(double2 *x) {
+    cudaStream_t st = ctx->stream;
+    for (int q = 0; q < 2; ++q)
+      if (!rev[q]) TLR_CUDA(ctx, cudaEventCreate(&rev[q]));
+    TLR_CUDA(ctx, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+    int rc;
+    {
+      CaptureScope cs;
+      rc = pipe_residuals(ctx, *pipe, pipe_rhs());
+      if (!rc) rc = F->enqueue_multi(ctx, 3, rev[0], rev[1]);
+      if (!rc) rc = pipe_targets(ctx, *pipe, sr, si, x, pipe_rhs(), true);
+      if (!rc) rc = pipe_accept(ctx, *pipe, hnorm);
+    }
+    cudaGraph_t g = nullptr;
+    const cudaError_t e = cudaStreamEndCapture(st, &g);
+    if (rc) {
+      if (g) cudaGraphDestroy(g);
+      return rc;
+    }
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaStreamEndCapture (pipelined round)");
+    size_t nn = 0;
+    pipe_kernels = 0;
+    if (cudaGraphGetNodes(g, nullptr, &nn) == cudaSuccess && nn > 0) {
+      std::vector<cudaGraphNode_t> nodes(nn);
+      if (cudaGraphGetNodes(g, nodes.data(), &nn) == cudaSuccess)
+        for (size_t i = 0; i < nn; ++i) {
+          cudaGraphNodeType t;
+          if (cudaGraphNodeGetType(nodes[i], &t) == cudaSuccess && t == cudaGraphNodeTypeKernel)
+            ++pipe_kernels;
+        }
+    }
+    const cudaError_t e2 = cudaGraphInstantiate(&pipe_exec, g, 0);
+    cudaGraphDestroy(g);
+    if (e2 != cudaSuccess) return cuda_fail(ctx, e2, "cudaGraphInstantiate (pipelined round)");
+    return TLR_OK;
+  }
+
+  // allocate what the rounds need (outside any capture) and begin at v
+  int pipe_begin(const double2 *v, double2 *x) {
+    int rc = prepare_ff(ctx);
+    if (!rc) rc = F->solve_multi_prepare(ctx);
+    if (!rc) rc = pipe_start(ctx, *pipe, v, x);
+    if (!rc && !pipe_exec) rc = build_pipe_graph(x);
+    return rc;
+  }
+
+  // x = OP v_j for the current basis vector: rounds until x is accepted
+  // (three for the first vector, then mostly one)
+  int pipe_op(double2 *x) {
+    double prev = INFINITY;
+    for (int round = 0;; ++round) {
+      TLR_CUDA(ctx, cudaGraphLaunch(pipe_exec, ctx->stream));
+      count_launches(pipe_kernels);
+      solves += 3;
+      ++refine;
+      if (round == 0) host_work();
+      TLR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+      float ms = 0.f;
+      if (cudaEventElapsedTime(&ms, rev[0], rev[1]) == cudaSuccess) {
+        tri_ms += ms;
+        ++tri_n;
+      } else {
+        cudaGetLastError();  // not a failure of the solve: no timing this time
+      }
+      const double nr = hnorm[0], ny = hnorm[1];
+      if (nr <= refine_tol * ny) {
+        refine_res[2] = std::max(refine_res[2], nr / ny);
+        return TLR_OK;
+      }
+      // no longer contracting (the float-float residual's floor), or not a
+      // number: the classic loop with its FP64 residuals decides
+      if (round >= 7 || !(nr <= 0.5 * prev)) {
+        const int rc = refine_loop(pipe->b, x, ny);
+        return rc ? rc : pipe_targets(ctx, *pipe, sr, si, x, nullptr, false);
+      }
+      prev = nr;
+    }
+  }
+
   // out = OP in = K^-1 B in
   int op(const double2 *in, double2 *out) {
     int rc = run_spmv(ctx, TLR_MAT_B, in, y);
@@ -598,6 +688,7 @@ void free_workspace(tlr_ctx *ctx) {
     cudaFree(ws->ybuf); cudaFree(ws->rnd); cudaFreeHost(ws->hpin); cudaFreeHost(ws->ypin);
     cudaFreeHost(ws->rnh); cudaFree(ws->blk); cudaFree(ws->blk32); cudaFree(ws->bnd);
     cudaFreeHost(ws->bnh);
+    pipe_free(ws->pipe);
     delete ws;
     ctx->kws = nullptr;
   }
@@ -845,6 +936,18 @@ int run_solve(tlr_ctx *ctx, const tlr_solve_opts *opts, double *lambda,
     }
   }
   ws->prev_ritz = 0;  // tmp is reused below
+  // the mixed form's single-vector applications are pipelined (tlr_pipe.h);
+  // GMRES refinement, the cooperative solve, FP64 acceptance and 512-row
+  // solve blocks (no multi-vector kernels) refine each application by itself
+  const bool piped = prec == 1 && bsz == 1 && !S.gmres && !S.fp64_accept && !F->persistent &&
+                     sblock != 512;
+  if (piped) {
+    int rc = TLR_OK;
+    if (!ws->pipe.vff) rc = pipe_alloc(ctx, ws->pipe, ws->ncv);
+    S.pipe = &ws->pipe;
+    if (!rc) rc = S.pipe_begin(S.V, S.w);
+    if (rc) return rc;
+  }
   double maxerr = 0.0;
   const int nout = nev;
   // Ritz vectors x_i = V Q y_i, lambda_i = sigma + 1/theta_i and explicit
@@ -1026,8 +1129,9 @@ int run_solve(tlr_ctx *ctx, const tlr_solve_opts *opts, double *lambda,
           ++checks;
         };
       }
-      int rc = bsz == 1 ? S.op(S.V + (size_t)j0 * n, S.w)
-                        : S.op_block(S.V + (size_t)j0 * n);
+      int rc = piped      ? S.pipe_op(S.w)
+               : bsz == 1 ? S.op(S.V + (size_t)j0 * n, S.w)
+                          : S.op_block(S.V + (size_t)j0 * n);
       S.host_work();  // operator paths that did not run it
       if (rc) return rc;
       if (prc) return prc;
@@ -1049,7 +1153,14 @@ int run_solve(tlr_ctx *ctx, const tlr_solve_opts *opts, double *lambda,
             rc = kv_update(ctx, n, S.V, n, nk, hcol(pass, j), w, S.npart,
                            pass ? ws->betad + j : nullptr);
         }
-        if (!rc) rc = kv_scale(ctx, n, w, ws->betad + j, 1.0, S.V + (size_t)nk * n);
+        if (!rc && piped) {  // the next vector and its pipelined guesses
+          rc = pipe_coefficients(ctx, ws->pipe, j, hcol(0, j), hcol(1, j), ws->betad + j);
+          if (!rc)
+            rc = pipe_shift(ctx, ws->pipe, j, ws->betad + j, S.sr, S.si, w,
+                            S.V + (size_t)nk * n, S.pipe_rhs());
+        } else if (!rc) {
+          rc = kv_scale(ctx, n, w, ws->betad + j, 1.0, S.V + (size_t)nk * n);
+        }
       }
       if (rc) return rc;
       ortho_ms += ms_since(to);
@@ -1135,6 +1246,16 @@ int run_solve(tlr_ctx *ctx, const tlr_solve_opts *opts, double *lambda,
     }
     H = Hn;
     k = l;
+    if (piped) {  // the rotated basis and projected matrix; x, y, u stand
+      for (int j = 0; j < l; ++j)
+        for (int i = 0; i < ws->pipe.ldh; ++i) {
+          const cd v = i <= l ? H(i, j) : cd(0.0);
+          ws->pipe.hup[(size_t)j * ws->pipe.ldh + i] = make_double2(v.real(), v.imag());
+        }
+      int rc = pipe_upload_h(ctx, ws->pipe, l);
+      if (!rc) rc = pipe_split_basis(ctx, ws->pipe, S.V, l + 1);
+      if (rc) return rc;
+    }
   }
   ws->prev_ritz = nout;  // tmp holds the normalised Ritz vectors
   const auto t2 = clock::now();

@@ -2764,14 +2764,16 @@ int Factor::solve_impl_m(tlr_ctx *ctx) {
 int Factor::solve_impl_m_dispatch(tlr_ctx *ctx, int nr) {
   switch (sw * 16 + nr) {
     case 128 * 16 + 2: return solve_impl_m<128, 2>(ctx);
+    case 128 * 16 + 3: return solve_impl_m<128, 3>(ctx);
     case 128 * 16 + 4: return solve_impl_m<128, 4>(ctx);
     case 128 * 16 + 8: return solve_impl_m<128, 8>(ctx);
     case 256 * 16 + 2: return solve_impl_m<256, 2>(ctx);
+    case 256 * 16 + 3: return solve_impl_m<256, 3>(ctx);
     case 256 * 16 + 4: return solve_impl_m<256, 4>(ctx);
     case 256 * 16 + 8: return solve_impl_m<256, 8>(ctx);
     default:
       return fail(ctx, TLR_ERR_ARG,
-                  "multi-vector solves need 2, 4 or 8 vectors and diagonal blocks of 128 or 256");
+                  "multi-vector solves need 2, 3, 4 or 8 vectors and diagonal blocks of 128 or 256");
   }
 }
 
@@ -2849,6 +2851,22 @@ int Factor::solve_multi(tlr_ctx *ctx, void *x, int nr, cudaEvent_t a, cudaEvent_
     count_launches(graph_m_kernels[nr]);
   }
   TLR_CUDA(ctx, cudaMemcpyAsync(x, vec_m, bytes, cudaMemcpyDeviceToDevice, st));
+  return TLR_OK;
+}
+
+int Factor::enqueue_multi(tlr_ctx *ctx, int nr, cudaEvent_t a, cudaEvent_t b) {
+  cudaStream_t st = ctx->stream;
+  const size_t n = (size_t)sym.nn * 5;
+  int rc = TLR_OK;
+  if (a) TLR_CUDA(ctx, cudaEventRecordWithFlags(a, st, cudaEventRecordExternal));
+  if (wave) {
+    for (int v = 0; v < nr && !rc; ++v)
+      rc = enqueue_solve(ctx, static_cast<float2 *>(vec_m) + v * n, nullptr, nullptr);
+  } else {
+    rc = solve_impl_m_dispatch(ctx, nr);
+  }
+  if (rc) return rc;
+  if (b) TLR_CUDA(ctx, cudaEventRecordWithFlags(b, st, cudaEventRecordExternal));
   return TLR_OK;
 }
 

@@ -131,6 +131,11 @@ struct Factor {
                   cudaEvent_t b = nullptr, bool capture = false);
   // allocate the multi-vector buffers (outside any stream capture)
   int solve_multi_prepare(tlr_ctx *ctx);
+  // Enqueue the solve of the nr right-hand sides in vec_m, in place, for
+  // capture into a caller's graph (solve_multi_prepare first).  With the
+  // dependency-driven level launches (wave) the vectors go one at a time;
+  // the bits are the same.
+  int enqueue_multi(tlr_ctx *ctx, int nr, cudaEvent_t a, cudaEvent_t b);
   template <int SW, int NR> int solve_impl_m(tlr_ctx *ctx);
   int solve_impl_m_dispatch(tlr_ctx *ctx, int nr);
 

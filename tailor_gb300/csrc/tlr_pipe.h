@@ -1,0 +1,64 @@
+// tlr_pipe.h -- pipelined refined operator applications of the mixed form.
+//
+// Shift-and-invert Arnoldi needs x = OP v_j, OP = K^-1 B, to a residual of
+// 1e-12 from a factor that contracts an error by 1e-5 or so per triangular
+// solve: three dependent solves per application when each starts from
+// nothing.  The applications are not independent, though: v_{j+1} is a
+// combination of OP v_j and the basis, so OP v_{j+1} is one of OP^2 v_j and
+// the (known) images of the basis.  The driver therefore carries
+//   x ~ OP v_j,  y ~ OP^2 v_j,  u ~ OP^3 v_j
+// and every triangular solve takes three right-hand sides at once -- the
+// residuals of x and of y, and B y -- reading the factor once.  When x is
+// accepted and v_{j+1} known, the same combination that made v_{j+1} out of
+// x makes the next x out of y and the next y out of u; the new x usually
+// needs one correction only.  x is accepted on the same residual as before
+// (||B v - K x|| <= 1e-12 ||B v||, A x in float-float), so a poor guess
+// costs another round and no accuracy.  Measured rounds per application:
+// 1.13 (60 x 32) to 1.51 (200 x 128, complex target; its factor contracts by
+// 3e-5 only), against three dependent solves.  A pass of a point, before and
+// after: 221 -> 161 ms at 60 x 32, 227 -> 173 ms at 100 x 50, 643 -> 594 ms at
+// 200 x 128, 1465 -> 1231 ms at 300 x 192.
+#pragma once
+
+#include "tlr_internal.h"
+
+namespace tlr {
+
+struct Pipe {
+  long long n = 0;        // scalar unknowns, 5 nn
+  int nn = 0, ncv = 0, ldh = 0;
+  float4 *vff = nullptr;  // the basis as FP32 hi/lo pairs, (ncv + 1) x n
+  float4 *xyff = nullptr; // x and y the same way, interleaved [n][2]
+  double2 *y = nullptr, *b = nullptr, *tx = nullptr, *ty = nullptr;
+  float2 *by32 = nullptr; // B y, the right-hand side of u
+  double2 *H = nullptr;   // (ncv + 1) x ncv projected matrix, ld ldh
+  float4 *g = nullptr;    // combination coefficients, 2 x ldh
+  double *bpart = nullptr, *rpart = nullptr;  // per-CTA partial sums of squares
+  double2 *hup = nullptr; // pinned stage of H
+};
+
+int pipe_alloc(tlr_ctx *ctx, Pipe &p, int ncv);
+void pipe_free(Pipe &p);
+// Begin with v (= basis vector 0): x = y = u = 0.
+int pipe_start(tlr_ctx *ctx, Pipe &p, const double2 *v, double2 *x);
+// basis columns 0 .. nk-1 into p.vff (after a restart)
+int pipe_split_basis(tlr_ctx *ctx, Pipe &p, const double2 *V, int nk);
+// upload the leading l columns of the restarted projected matrix
+int pipe_upload_h(tlr_ctx *ctx, Pipe &p, int l);
+// column j of H from the Gram-Schmidt passes, and the coefficients of the
+// shift: g1 = H h, g2 = H g1(0:j+1)
+int pipe_coefficients(tlr_ctx *ctx, Pipe &p, int j, const double2 *h1, const double2 *h2,
+                      const double *beta);
+// x (holding the orthogonalised w) -> v_{j+1} = w / beta and the next x, y,
+// targets and right-hand side; rhs: 3 x n, its third vector holds u
+int pipe_shift(tlr_ctx *ctx, Pipe &p, int j, const double *beta, double sr, double si,
+               double2 *x, double2 *vnew, const float2 *rhs);
+// rhs = the residuals of x and y, and B y
+int pipe_residuals(tlr_ctx *ctx, Pipe &p, float2 *rhs);
+// x += rhs(0), y += rhs(1) (correct), and the targets of the new x and y
+int pipe_targets(tlr_ctx *ctx, Pipe &p, double sr, double si, double2 *x, const float2 *rhs,
+                 bool correct);
+// out[0] = ||B v - K x||, out[1] = ||B v|| (out: pinned host memory)
+int pipe_accept(tlr_ctx *ctx, Pipe &p, double *out);
+
+}  // namespace tlr

@@ -10,6 +10,7 @@
 // loads; x stays L2-resident.
 #include <atomic>
 
+#include "tlr_ff.cuh"
 #include "tlr_internal.h"
 
 namespace tlr {
@@ -117,32 +118,10 @@ int run_spmv(tlr_ctx *ctx, int which, const double2 *x, double2 *y) {
 
 namespace {
 
-// float-float helpers (Dekker/Knuth error-free transformations on FP32):
-// (hi, lo) += a * x with a = ah + al, x = xh + xl
-__device__ __forceinline__ void ff_mac(float &hi, float &lo, float ah, float al, float xh,
-                                       float xl) {
-  const float p = ah * xh;
-  const float e = fmaf(ah, xh, -p) + fmaf(ah, xl, al * xh);
-  const float s = hi + p;
-  const float bb = s - hi;
-  lo += ((hi - (s - bb)) + (p - bb)) + e;
-  hi = s;
-}
-
-__device__ __forceinline__ void ff_add(float &hi, float &lo, float h2, float l2) {
-  const float s = hi + h2;
-  const float bb = s - hi;
-  lo = lo + l2 + ((hi - (s - bb)) + (h2 - bb));
-  hi = s;
-}
-
 __global__ void k_split_ff(long long n, const double2 *__restrict__ a, float4 *__restrict__ out) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const double2 v = a[i];
-  const float rh = __double2float_rn(v.x), ih = __double2float_rn(v.y);
-  out[i] = make_float4(rh, __double2float_rn(v.x - (double)rh), ih,
-                       __double2float_rn(v.y - (double)ih));
+  out[i] = ff_split(a[i]);
 }
 
 // r = y - (A w - sigma B w): warp per block row, lane (r, c) = 5 r + c
