@@ -490,8 +490,10 @@ int tlr_factor_solve(tlr_ctx *ctx, int nvec, const double *rhs, double *out, int
                    cudaSuccess ? TLR_OK : TLR_ERR_CUDA;
   if (!rc && multi) rc = F->solve_multi(ctx, d, nvec);
   for (int v = 0; v < nvec && !rc && !multi; ++v) rc = F->solve(ctx, d + (size_t)v * n);
-  if (!rc && cudaMemcpy(h.data(), d, h.size() * sizeof(float2), cudaMemcpyDeviceToHost) !=
-                 cudaSuccess)
+  // the solves run on the context's (non-blocking) stream
+  if (!rc && (cudaStreamSynchronize(ctx->stream) != cudaSuccess ||
+              cudaMemcpy(h.data(), d, h.size() * sizeof(float2), cudaMemcpyDeviceToHost) !=
+                  cudaSuccess))
     rc = TLR_ERR_CUDA;
   cudaFree(d);
   if (rc) return rc == TLR_ERR_CUDA ? fail(ctx, rc, "tlr_factor_solve: CUDA error") : rc;
