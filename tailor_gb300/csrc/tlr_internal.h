@@ -198,6 +198,17 @@ struct CaptureScope {  // suppresses counting on this thread during capture
 };
 
 struct DevFront;
+struct TcJob;
+// A batch of products C(rows, cols) -= F(rows, K) F(K, cols), K <= 256, over
+// fronts of the pool: operand planes split once per batch (planes: (atiles +
+// btiles) x 32 chunk images), then the persistent kernel.
+int launch_tc_jobs(tlr_ctx *ctx, const TcJob *jobs, int nj, const int *prefix, const int *pa,
+                   const int *pb, int tiles, int atiles, int btiles, float2 *pool,
+                   unsigned char *planes, int *err, cudaStream_t st);
+// Left products by the dense D_b over 64-column tiles, in place and negated:
+// tiles {front, block, first column, -}, columns [0, 256 block).
+int launch_scale_g(tlr_ctx *ctx, const int4 *tiles, long long nt, float2 *pool, const DevFront *fr,
+                   const long long *inv_off, const float2 *dmat, int *err, cudaStream_t st);
 // Tensor-core Schur update of one panel step (tlr_tc.cu).
 // The same update with the operands converted once per panel step into
 // TF32 plane images (planes: (atiles + btiles) x ceil(w / 8) x 16 KB of
@@ -215,11 +226,12 @@ int launch_gemm_tc(tlr_ctx *ctx, const int *fl, const int *prefix, int nf, int s
 // The complex64 factor rewrite of the block-scaled solves (256-row diagonal
 // blocks) on the tensor cores: U' and D_b from utiles {front, block, first
 // column, kind} (64 columns each), then L' from ltiles {front, block, first
-// row, -} (128 rows each), in place.
+// row, -} (128 rows each), in place.  place: D_b also goes into the pivot
+// block's diagonal position.
 int launch_rewrite_tc(tlr_ctx *ctx, const int4 *ltiles, long long nl, const int4 *utiles,
                       long long nu, float2 *pool, const DevFront *fr, const long long *inv_off,
                       const float2 *Linv, const float2 *Uinv, float2 *dmat, int *err,
-                      cudaStream_t st);
+                      cudaStream_t st, bool place = false);
 
 inline int blocks_for(long long n, int threads) {
   return static_cast<int>((n + threads - 1) / threads);

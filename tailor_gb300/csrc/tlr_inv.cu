@@ -1,0 +1,426 @@
+// tlr_inv.cu -- inverse form of the complex64 factor and its solves.
+//
+// The block-scaled factor (tlr_lu.cu) has identity diagonal blocks: L' and
+// U' of a front's pivot block, D_b on its diagonal.  A front with nb
+// diagonal blocks needs nb dependent steps each way, and the top of the
+// tree is a chain of such steps with little work in each (19 at the root of
+// a 300 x 192 grid).  Here the unit block triangles are inverted in place,
+//   inv(L') = I - N_L,  inv(U') = I - N_U,  X = L'21 inv(L'),
+//   Y = inv(U') U'12,
+// and the rows of N_L are scaled by D, so that with t the gathered
+// right-hand side a front needs one product each way:
+//   forward:  z = [-D N_L | D] t (rows of the pivots), t_b -= X t;
+//   backward: x = z - [N_U | Y] [z; x_b].
+// The storage is that of the factor, p (p + 2 b) entries read once per
+// solve; a solve is three launches per level (gather, forward, backward).
+//
+// The inversion is right-looking, block d from the last down:
+//   F(rows below d, columns left of d)  -= F(rows below d, d) F(d, columns)
+//   F(rows above d, columns right of d) -= F(rows above d, d) F(d, columns)
+// (rows below include the border, columns right of d too): products of
+// inner dimension 256 in the persistent tcgen05 kernel of the Schur updates
+// (3xTF32, FP32 accumulation), step d of every front of the tree in one
+// batch.
+#include <algorithm>
+#include <vector>
+
+#include "tlr_complex.cuh"
+#include "tlr_internal.h"
+#include "tlr_lu.h"
+#include "tlr_pdl.cuh"
+
+namespace tlr {
+namespace {
+
+constexpr int kSW = 256;           // diagonal block
+constexpr int kBatchTiles = 2048;  // operand tiles per batch: 1 GB of planes
+constexpr int kMaxCols = 1024;     // columns of a work item at most
+
+// t = right-hand side of the pivot rows plus the children's border rows
+template <int NR>
+__global__ void k_inv_gather(const int *__restrict__ fl, const DevFront *__restrict__ fr,
+                             const int *__restrict__ gsrc, const int2 *__restrict__ cinv,
+                             const float2 *__restrict__ b, long long xs, float2 *__restrict__ work,
+                             long long ws) {
+  pdl_launch_dependents();
+  const DevFront f = fr[fl[blockIdx.y]];
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool ok = i < f.m;
+  int src = -1;
+  int2 c = make_int2(-1, -1);
+  if (ok) {
+    src = gsrc[f.toff + i];
+    c = cinv[f.toff + i];
+  }
+  pdl_wait();
+  if (!ok) return;
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    float2 *wr = work + r * ws;
+    float2 v = src >= 0 ? b[r * xs + src] : czero<float2>();
+    if (c.x >= 0) v = cadd(v, wr[c.x]);
+    if (c.y >= 0) v = cadd(v, wr[c.y]);
+    wr[f.toff + i] = v;
+  }
+}
+
+// One work item per CTA: 32 rows (lane = row) times a range of columns (8
+// warps, consecutive shares).  Bound by reading the factor: each thread
+// streams its columns 8 at a time, the next 8 in flight while the present
+// ones are applied to all NR vectors, and the first 8 go out before the
+// programmatic-launch wait.  Eight columns keep a thread within 64 registers,
+// four CTAs per SM: 2.11 ms per three-vector solve at 300 x 192 (10 GB, 4.8
+// TB/s) against 2.20 with 16 columns and three CTAs, 2.40 with 16 warps per
+// CTA and 2.5 with four; the block steps it replaces took 3.39 ms (200 x 128:
+// 0.93 against 1.49 ms, 100 x 50: 0.21 against 0.32).  Row tiles split over several items add their
+// partial sums in item order in the item that finishes last, so results do
+// not depend on timing; per vector the arithmetic does not depend on NR.
+constexpr int kW = 8;  // warps per CTA
+constexpr int kQ = 8;  // columns a thread loads at a time
+
+template <int NR>
+__global__ void __launch_bounds__(32 * kW, NR <= 4 ? 4 : 2)
+    k_inv_apply(const SvItem *__restrict__ items, const float2 *__restrict__ pool,
+                const int *__restrict__ uidx, float2 *__restrict__ W, float2 *__restrict__ W2,
+                long long ws, float2 *__restrict__ x, long long xs, float2 *__restrict__ part,
+                int max_split, int *__restrict__ ctr) {
+  using C = float2;
+  constexpr int kT = 32 * kW, kU = kMaxCols / kT;
+  extern __shared__ __align__(16) C sm[];
+  C(*red)[kW][32] = reinterpret_cast<C(*)[kW][32]>(sm);  // [NR][kW][32]
+  C *vs = sm + NR * kW * 32;  // (column k, vector v) at ((k / 2) NR + v) 2 + k % 2
+  __shared__ int s_last;
+  pdl_launch_dependents();
+  const SvItem it = items[blockIdx.x];
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const bool rowok = lane < it.rows;
+  const int cw = (it.cols + 2 * kW - 1) / (2 * kW) * 2;  // columns per warp, even
+  const int q0 = wp * cw, q1 = min(it.cols, q0 + cw);
+  const C *A = pool + it.a + lane;
+  const long long ld = it.ld;
+  auto load = [&](C(&f)[kQ], int k0) {
+    if (rowok && k0 + kQ <= q1) {
+      const C *p = A + k0 * ld;
+#pragma unroll
+      for (int k = 0; k < kQ; ++k, p += ld) f[k] = __ldcs(p);
+    } else {
+#pragma unroll
+      for (int k = 0; k < kQ; ++k)
+        f[k] = (rowok && k0 + k < q1) ? __ldcs(A + (k0 + k) * ld) : czero<C>();
+    }
+  };
+  C cur[kQ];
+  load(cur, q0);
+  int id[kU];
+  if (it.kind == 2)
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int k = threadIdx.x + kT * u;
+      id[u] = (k >= it.piv && k < it.cols) ? uidx[it.vec + k] : 0;
+    }
+  pdl_wait();
+  // this warp finishes vector wp: its rows' own values go out with the rest
+  C base = czero<C>();
+  if (wp < NR && rowok && it.kind != 0)
+    base = (it.kind == 1 ? W : W2)[wp * ws + it.out + lane];
+  const int kend = kW * cw + kQ;
+#pragma unroll
+  for (int u = 0; u < kU; ++u) {
+    const int k = threadIdx.x + kT * u;
+    if (k < it.cols) {
+#pragma unroll
+      for (int v = 0; v < NR; ++v) {
+        C t;
+        if (it.kind == 2)
+          t = k < it.piv ? W2[v * ws + it.vec + k] : x[v * xs + id[u]];
+        else
+          t = W[v * ws + it.vec + k];
+        vs[((k >> 1) * NR + v) * 2 + (k & 1)] = t;
+      }
+    }
+  }
+  for (int k = it.cols + threadIdx.x; k < kend; k += kT)
+#pragma unroll
+    for (int v = 0; v < NR; ++v) vs[((k >> 1) * NR + v) * 2 + (k & 1)] = czero<C>();
+  __syncthreads();
+  C acc[NR];
+#pragma unroll
+  for (int v = 0; v < NR; ++v) acc[v] = czero<C>();
+  const float4 *v4 = reinterpret_cast<const float4 *>(vs);
+  for (int k0 = q0; k0 < q1; k0 += kQ) {
+    C nxt[kQ];
+    load(nxt, k0 + kQ);
+    const float4 *p = v4 + (k0 >> 1) * NR;
+#pragma unroll
+    for (int k = 0; k < kQ; k += 2)
+#pragma unroll
+      for (int v = 0; v < NR; ++v) {
+        const float4 pv = p[(k >> 1) * NR + v];
+        acc[v] = cfma(acc[v], cur[k], make_float2(pv.x, pv.y));
+        acc[v] = cfma(acc[v], cur[k + 1], make_float2(pv.z, pv.w));
+      }
+#pragma unroll
+    for (int k = 0; k < kQ; ++k) cur[k] = nxt[k];
+  }
+#pragma unroll
+  for (int v = 0; v < NR; ++v) red[v][wp][lane] = acc[v];
+  __syncthreads();
+  if (it.nsplit == 1 && wp >= NR) return;
+  C s = czero<C>();
+  if (wp < NR) {
+#pragma unroll
+    for (int k = 0; k < kW; ++k) s = cadd(s, red[wp][k][lane]);
+  }
+  if (it.nsplit > 1) {
+    C *pt = part + (long long)it.tile * max_split * NR * 32;
+    if (wp < NR) pt[(it.split * NR + wp) * 32 + lane] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();  // the CTA's partial sums, ordered by the barrier above
+      const int done = atomicAdd(ctr + it.tile, 1);
+      s_last = done == it.nsplit - 1;
+      if (s_last) ctr[it.tile] = 0;
+      __threadfence();
+    }
+    __syncthreads();
+    if (!s_last || wp >= NR) return;
+    s = czero<C>();
+    for (int q = 0; q < it.nsplit; ++q) s = cadd(s, __ldcg(pt + (q * NR + wp) * 32 + lane));
+  }
+  if (rowok) {
+    if (it.kind == 0)
+      W2[wp * ws + it.out + lane] = s;
+    else if (it.kind == 1)
+      W[wp * ws + it.out + lane] = csub(base, s);
+    else
+      x[wp * xs + uidx[it.out + lane]] = csub(base, s);
+  }
+}
+
+}  // namespace
+
+int Factor::build_inverse(tlr_ctx *ctx) {
+  inverse_ok = false;
+  if (prec != 1 || sw != kSW) return TLR_OK;
+  const int nf = (int)sym.fronts.size();
+  auto blocks_of = [&](int t) { return (sym.fronts[t].p + kSW - 1) / kSW; };
+  // inversion batches: step s takes block nblk - 1 - s of every front
+  std::vector<TcJob> jobs;
+  std::vector<int> pre;
+  inv_batches.clear();
+  long long max_tiles = 0;
+  int maxblk = 0;
+  for (int t = 0; t < nf; ++t) maxblk = std::max(maxblk, blocks_of(t));
+  std::vector<TcJob> cur;
+  auto flush = [&]() {
+    if (cur.empty()) return;
+    TcBatch b;
+    b.job_off = (int)jobs.size();
+    b.jobs = (int)cur.size();
+    std::vector<int> p1, p2, p3;
+    for (const TcJob &j : cur) {
+      p1.push_back(b.tiles);
+      p2.push_back(b.atiles);
+      p3.push_back(b.btiles);
+      const int nr = (j.r1 - j.r0 + 127) / 128, nc = (j.c1 - j.c0 + 63) / 64;
+      b.tiles += nr * nc;
+      b.atiles += nr;
+      b.btiles += nc;
+    }
+    p1.push_back(b.tiles);
+    p2.push_back(b.atiles);
+    p3.push_back(b.btiles);
+    b.prefix_off = (int)pre.size();
+    pre.insert(pre.end(), p1.begin(), p1.end());
+    b.pa_off = (int)pre.size();
+    pre.insert(pre.end(), p2.begin(), p2.end());
+    b.pb_off = (int)pre.size();
+    pre.insert(pre.end(), p3.begin(), p3.end());
+    jobs.insert(jobs.end(), cur.begin(), cur.end());
+    inv_batches.push_back(b);
+    max_tiles = std::max(max_tiles, (long long)b.atiles + b.btiles);
+    cur.clear();
+  };
+  for (int s = 0; s + 1 < maxblk; ++s) {
+    int tiles = 0;
+    for (int t = 0; t < nf; ++t) {
+      const FrontInfo &f = sym.fronts[t];
+      const int d = blocks_of(t) - 1 - s;
+      if (d < 1) continue;
+      const int k0 = d * kSW, kw = std::min(kSW, f.p - k0), k1 = k0 + kw;
+      if (k1 >= f.m) continue;
+      const int n = (f.m - k1 + 127) / 128 + (k0 + 63) / 64 + (k0 + 127) / 128 +
+                    (f.m - k1 + 63) / 64;
+      if (tiles + n > kBatchTiles) {
+        flush();
+        tiles = 0;
+      }
+      tiles += n;
+      cur.push_back({f.off, f.m, k0, kw, k1, f.m, 0, k0, 0});
+      cur.push_back({f.off, f.m, k0, kw, 0, k0, k1, f.m, 0});
+    }
+    flush();
+  }
+  std::vector<int4> gt;
+  for (int t = 0; t < nf; ++t)
+    for (int b = 1; b < blocks_of(t); ++b)
+      for (int c = 0; c < b * kSW; c += 64) gt.push_back(make_int4(t, b, c, 0));
+  n_gtiles = (long long)gt.size();
+  // unknown of every front row
+  std::vector<int> uidx(std::max<long long>(sym.work_elems, 1), 0);
+  for (int t = 0; t < nf; ++t) {
+    const FrontInfo &f = sym.fronts[t];
+    long long a = f.toff;
+    for (int u : f.piv)
+      for (int c = 0; c < 5; ++c) uidx[a++] = u * 5 + c;
+    for (int u : f.border)
+      for (int c = 0; c < 5; ++c) uidx[a++] = u * 5 + c;
+  }
+  // work items of every launch, the longest first
+  std::vector<SvItem> items;
+  item_cols = 64;
+  max_split_tiles = 0;
+  max_split = 1;
+  struct Row {
+    int t, r0, rows, c0, c1, kind;
+  };
+  auto emit = [&](std::vector<Row> &rows, int &off, int &count) {
+    // three items per SM where the level has the work for them, of 256 (a
+    // shorter share per warp is all start-up: 0.22 ms per solve at 100 x 50
+    // against 0.25 with 128) to kMaxCols columns
+    long long total = 0;
+    for (const Row &r : rows) total += r.c1 - r.c0;
+    const int kc = (int)std::min<long long>(
+        kMaxCols, std::max<long long>(256, (total / 456 + 63) / 64 * 64));
+    off = (int)items.size();
+    int tile = 0;
+    for (const Row &r : rows) {
+      const FrontInfo &f = sym.fronts[r.t];
+      const int n = r.c1 - r.c0, ns = std::max(1, (n + kc - 1) / kc);
+      const int chunk = std::max(16, ((n + ns - 1) / ns + 15) / 16 * 16);
+      const int cnt = std::max(1, (n + chunk - 1) / chunk);
+      for (int q = 0; q < cnt; ++q) {
+        const int c0 = r.c0 + q * chunk, c1 = std::min(r.c1, c0 + chunk);
+        SvItem it{};
+        it.a = f.off + (long long)c0 * f.m + r.r0;
+        it.ld = f.m;
+        it.rows = r.rows;
+        it.cols = c1 - c0;
+        it.vec = (int)f.toff + c0;
+        it.piv = r.kind == 2 ? std::max(0, std::min(c1, f.p) - c0) : it.cols;
+        it.out = (int)f.toff + r.r0;
+        it.tile = cnt > 1 ? tile : 0;
+        it.split = q;
+        it.nsplit = cnt;
+        it.kind = r.kind;
+        item_cols = std::max(item_cols, it.cols);
+        items.push_back(it);
+      }
+      if (cnt > 1) ++tile;
+      max_split = std::max(max_split, cnt);
+    }
+    max_split_tiles = std::max(max_split_tiles, tile);
+    count = (int)items.size() - off;
+    std::stable_sort(items.begin() + off, items.end(),
+                     [](const SvItem &a, const SvItem &b) { return a.cols > b.cols; });
+  };
+  for (size_t h = 0; h < levels.size(); ++h) {
+    Level &L = levels[h];
+    std::vector<Row> fw, bw;
+    for (int t : sym.levels[h]) {
+      const FrontInfo &f = sym.fronts[t];
+      for (int b = 0; b < blocks_of(t); ++b) {
+        const int b0 = b * kSW, b1 = std::min(f.p, b0 + kSW);
+        for (int r = b0; r < b1; r += 32) {
+          fw.push_back({t, r, std::min(32, b1 - r), 0, b1, 0});
+          bw.push_back({t, r, std::min(32, b1 - r), b1, f.m, 2});
+        }
+      }
+      for (int r = f.p; r < f.m; r += 32) fw.push_back({t, r, std::min(32, f.m - r), 0, f.p, 1});
+    }
+    emit(fw, L.if_off, L.if_n);
+    emit(bw, L.ib_off, L.ib_n);
+  }
+  auto up = [&](void **p, const void *src, size_t bytes) -> int {
+    const cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 16));
+    if (e != cudaSuccess) {
+      *p = nullptr;
+      return fail(ctx, TLR_ERR_NOMEM,
+                  std::string("factor allocation failed: ") + cudaGetErrorString(e));
+    }
+    if (src && bytes) TLR_CUDA(ctx, cudaMemcpy(*p, src, bytes, cudaMemcpyHostToDevice));
+    return TLR_OK;
+  };
+  const size_t parts = (size_t)std::max(1, max_split_tiles) * max_split * kMaxRhs * 32;
+  int rc;
+  if ((rc = up((void **)&d_inv_jobs, jobs.data(), jobs.size() * sizeof(TcJob))) ||
+      (rc = up((void **)&d_inv_prefix, pre.data(), pre.size() * sizeof(int))) ||
+      (rc = up((void **)&d_gtiles, gt.data(), gt.size() * sizeof(int4))) ||
+      (rc = up((void **)&d_uidx, uidx.data(), uidx.size() * sizeof(int))) ||
+      (rc = up((void **)&d_gsrc, nullptr, uidx.size() * sizeof(int))) ||
+      (rc = up((void **)&d_items, items.data(), items.size() * sizeof(SvItem))) ||
+      (rc = up((void **)&split_part, nullptr, parts * sizeof(float2))) ||
+      (rc = up((void **)&split_ctr, nullptr, std::max(1, max_split_tiles) * sizeof(int))) ||
+      (rc = up((void **)&inv_planes, nullptr,
+               (size_t)max_tiles * (kSW / 8) * tc_chunk_image_bytes())))
+    return rc;
+  TLR_CUDA(ctx, cudaMemset(split_ctr, 0, std::max(1, max_split_tiles) * sizeof(int)));
+  inverse_ok = true;
+  return TLR_OK;
+}
+
+int Factor::invert_pivots(tlr_ctx *ctx) {
+  float2 *P = static_cast<float2 *>(pool);
+  for (const TcBatch &b : inv_batches) {
+    const int rc = launch_tc_jobs(ctx, d_inv_jobs + b.job_off, b.jobs, d_inv_prefix + b.prefix_off,
+                                  d_inv_prefix + b.pa_off, d_inv_prefix + b.pb_off, b.tiles,
+                                  b.atiles, b.btiles, P, inv_planes, d_tc_err, ctx->stream);
+    if (rc) return rc;
+  }
+  return launch_scale_g(ctx, d_gtiles, n_gtiles, P, d_fronts, d_inv_off,
+                        static_cast<const float2 *>(dmat), d_tc_err, ctx->stream);
+}
+
+template <int NR>
+int Factor::solve_inverse(tlr_ctx *ctx, float2 *x, float2 *W, float2 *W2) {
+  cudaStream_t st = ctx->stream;
+  const float2 *P = static_cast<const float2 *>(pool);
+  const long long xs = (long long)sym.nn * 5, ws = sym.work_elems;
+  const size_t sm = ((size_t)(item_cols + 2 * kW - 1) / (2 * kW) * (2 * kW) + kQ + kW * 32) * NR *
+                    sizeof(float2);
+  if (sm > 47 * 1024)
+    TLR_CUDA(ctx, cudaFuncSetAttribute(k_inv_apply<NR>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  auto apply = [&](int off, int n) -> int {
+    if (n <= 0) return TLR_OK;
+    TLR_CUDA(ctx, launch_pdl_smem(true, k_inv_apply<NR>, dim3(n), dim3(32 * kW), sm, st,
+                                  (const SvItem *)(d_items + off), P, (const int *)d_uidx, W, W2,
+                                  ws, x, xs, split_part, max_split, split_ctr));
+    count_launches();
+    return TLR_OK;
+  };
+  int rc = TLR_OK;
+  for (size_t h = 0; h < levels.size() && !rc; ++h) {
+    const Level &L = levels[h];
+    // the first kernel follows a copy or another kernel that does not
+    // trigger early: no programmatic edge for it
+    TLR_CUDA(ctx, launch_pdl(h > 0, k_inv_gather<NR>,
+                             dim3(blocks_for(L.max_m, 128), L.nfronts), dim3(128), st,
+                             (const int *)(d_sched + L.fronts_off), (const DevFront *)d_fronts,
+                             (const int *)d_gsrc, (const int2 *)d_cinv, (const float2 *)x, xs, W,
+                             ws));
+    count_launches();
+    rc = apply(L.if_off, L.if_n);
+  }
+  for (int h = (int)levels.size() - 1; h >= 0 && !rc; --h) 
+    rc = apply(levels[h].ib_off, levels[h].ib_n);
+  return rc;
+}
+
+template int Factor::solve_inverse<1>(tlr_ctx *, float2 *, float2 *, float2 *);
+template int Factor::solve_inverse<2>(tlr_ctx *, float2 *, float2 *, float2 *);
+template int Factor::solve_inverse<3>(tlr_ctx *, float2 *, float2 *, float2 *);
+template int Factor::solve_inverse<4>(tlr_ctx *, float2 *, float2 *, float2 *);
+template int Factor::solve_inverse<8>(tlr_ctx *, float2 *, float2 *, float2 *);
+
+}  // namespace tlr

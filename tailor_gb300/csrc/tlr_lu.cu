@@ -27,6 +27,7 @@
 #include "tlr_complex.cuh"
 #include "tlr_internal.h"
 #include "tlr_lu.h"
+#include "tlr_pdl.cuh"
 
 namespace tlr {
 namespace {
@@ -872,15 +873,6 @@ __global__ void __launch_bounds__(256)
 }
 
 // ------------------------------------------------------------------ solves
-
-// Programmatic dependent launch: a solve kernel lets the next one launch
-// right away (launch_dependents) and waits for its predecessor's results
-// only where it reads them (wait); loads of factor data go out before the
-// wait.  Both are no-ops for a kernel launched without the attribute.
-__device__ __forceinline__ void pdl_launch_dependents() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Forward gather of one level: t[i] = b[unknown of front row perm[i]] for
 // pivot rows (0 for border rows), plus the children's updated border rows
@@ -1912,24 +1904,6 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// launch, with programmatic stream serialisation when pdl (captured into
-// the graph as a programmatic dependency on the previous kernel)
-template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t st,
-                       Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
-}
-
 }  // namespace
 
 // ------------------------------------------------------------------- host
@@ -2230,6 +2204,7 @@ int Factor::setup(tlr_ctx *ctx, int precision, int leaf, int solve_block, int pa
                            cudaMemcpyHostToDevice));
   TLR_CUDA(ctx, cudaMemcpy(d_sched, sched.data(), sched.size() * sizeof(int),
                            cudaMemcpyHostToDevice));
+  if ((rc = build_inverse(ctx))) return rc;
   return build_phases(ctx);
 }
 
@@ -2334,6 +2309,15 @@ void Factor::release() {
   cudaFree(d_inv_off); cudaFree(d_inv_blocks); cudaFree(d_ltiles); cudaFree(d_utiles);
   cudaFree(d_phases); cudaFree(d_barrier); cudaFree(d_solve_err); cudaFree(tc_planes);
   cudaFree(d_wave_tiles); cudaFree(d_wave_ctr); cudaFree(d_ltiles_tc); cudaFree(d_utiles_tc);
+  cudaFree(d_inv_jobs); cudaFree(d_inv_prefix); cudaFree(inv_planes); cudaFree(d_gtiles);
+  cudaFree(d_items); cudaFree(d_uidx); cudaFree(d_gsrc); cudaFree(split_part); cudaFree(split_ctr);
+  d_inv_jobs = nullptr;
+  d_inv_prefix = d_uidx = d_gsrc = split_ctr = nullptr;
+  inv_planes = nullptr;
+  d_gtiles = nullptr;
+  d_items = nullptr;
+  split_part = nullptr;
+  inverse = inverse_ok = false;
   d_ltiles_tc = d_utiles_tc = nullptr;
   d_wave_tiles = nullptr;
   d_wave_ctr = nullptr;
@@ -2366,12 +2350,14 @@ int Factor::rewrite_factors(tlr_ctx *ctx) {
   { k_tri_inv<C, SW><<<dim3(n_inv_blocks, 2), SW, 0, st>>>(d_inv_blocks, P, d_fronts, d_inv_off,
                                                           Li, Ui); count_launches(); }
   if constexpr (sizeof(C) == sizeof(float2) && SW == 256) {
-    if (tensor_cores)  // the products on the tensor cores, like the Schur updates
-      return launch_rewrite_tc(ctx, d_ltiles_tc, n_ltiles_tc, d_utiles_tc, n_utiles_tc,
-                               reinterpret_cast<float2 *>(P), d_fronts, d_inv_off,
-                               reinterpret_cast<const float2 *>(Li),
-                               reinterpret_cast<const float2 *>(Ui),
-                               static_cast<float2 *>(dmat), d_tc_err, st);
+    if (tensor_cores) {  // the products on the tensor cores, like the Schur updates
+      const int rc = launch_rewrite_tc(ctx, d_ltiles_tc, n_ltiles_tc, d_utiles_tc, n_utiles_tc,
+                                       reinterpret_cast<float2 *>(P), d_fronts, d_inv_off,
+                                       reinterpret_cast<const float2 *>(Li),
+                                       reinterpret_cast<const float2 *>(Ui),
+                                       static_cast<float2 *>(dmat), d_tc_err, st, inverse);
+      return rc || !inverse ? rc : invert_pivots(ctx);
+    }
   }
   const size_t ssm = sizeof(C) * SW * kRT;
   TLR_CUDA(ctx, cudaFuncSetAttribute(k_scale_u<C, SW>,
@@ -2482,6 +2468,15 @@ int Factor::factor_impl(tlr_ctx *ctx, double sr, double si, double tiny) {
 }
 
 int Factor::factor(tlr_ctx *ctx, double sr, double si, double tiny) {
+  if (inverse != use_inverse()) {  // captured solves are of the other form
+    inverse = use_inverse();
+    if (graph_exec) cudaGraphExecDestroy(graph_exec);
+    graph_exec = nullptr;
+    for (auto &g : graph_m) {
+      if (g) cudaGraphExecDestroy(g);
+      g = nullptr;
+    }
+  }
   int rc = prec == 0 ? factor_impl<double2>(ctx, sr, si, tiny)
                      : factor_impl<float2>(ctx, sr, si, tiny);
   if (rc) return rc;
@@ -2535,6 +2530,19 @@ int Factor::factor(tlr_ctx *ctx, double sr, double si, double tiny) {
   }
   TLR_CUDA(ctx, cudaMemcpyAsync(d_cinv, cinv.data(), cinv.size() * sizeof(int2),
                                 cudaMemcpyHostToDevice, ctx->stream));
+  std::vector<int> gsrc;
+  if (inverse) {  // right-hand side entry of every pivot row (-1: border row)
+    gsrc.assign(sym.work_elems, -1);
+    for (int t = 0; t < nf; ++t) {
+      const FrontInfo &f = sym.fronts[t];
+      for (int i = 0; i < f.p; ++i) {
+        const int q = perm[f.toff + i];
+        gsrc[f.toff + i] = f.piv[q / 5] * 5 + q % 5;
+      }
+    }
+    TLR_CUDA(ctx, cudaMemcpyAsync(d_gsrc, gsrc.data(), gsrc.size() * sizeof(int),
+                                  cudaMemcpyHostToDevice, ctx->stream));
+  }
   TLR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   factored = true;
   return TLR_OK;
@@ -2627,7 +2635,10 @@ int Factor::enqueue_solve(tlr_ctx *ctx, void *x, cudaEvent_t a, cudaEvent_t b) {
   // external event nodes: the events are recorded (with time stamps) on
   // every replay of the caller's graph
   if (a) TLR_CUDA(ctx, cudaEventRecordWithFlags(a, st, cudaEventRecordExternal));
-  const int rc = prec == 0 ? solve_impl<double2, 128>(ctx, vec_a)
+  const int rc = inverse   ? solve_inverse<1>(ctx, static_cast<float2 *>(vec_a),
+                                              static_cast<float2 *>(work),
+                                              static_cast<float2 *>(work2))
+                 : prec == 0 ? solve_impl<double2, 128>(ctx, vec_a)
                            : (sw == 512   ? solve_impl<float2, 512>(ctx, vec_a)
                               : sw == 256 ? solve_impl<float2, 256>(ctx, vec_a)
                                           : solve_impl<float2, 128>(ctx, vec_a));
@@ -2665,7 +2676,9 @@ int Factor::solve(tlr_ctx *ctx, void *x) {
     int rc;
     {
       CaptureScope cs;
-      rc = prec == 0 ? solve_impl<double2, 128>(ctx, vec_a)
+      rc = inverse   ? solve_inverse<1>(ctx, static_cast<float2 *>(vec_a),
+                                        static_cast<float2 *>(work), static_cast<float2 *>(work2))
+           : prec == 0 ? solve_impl<double2, 128>(ctx, vec_a)
                      : (sw == 512   ? solve_impl<float2, 512>(ctx, vec_a)
                         : sw == 256 ? solve_impl<float2, 256>(ctx, vec_a)
                                     : solve_impl<float2, 128>(ctx, vec_a));
@@ -2762,6 +2775,17 @@ int Factor::solve_impl_m(tlr_ctx *ctx) {
 }
 
 int Factor::solve_impl_m_dispatch(tlr_ctx *ctx, int nr) {
+  if (inverse) {
+    float2 *x = static_cast<float2 *>(vec_m);
+    float2 *W = static_cast<float2 *>(work_m), *W2 = static_cast<float2 *>(work2_m);
+    switch (nr) {
+      case 2: return solve_inverse<2>(ctx, x, W, W2);
+      case 3: return solve_inverse<3>(ctx, x, W, W2);
+      case 4: return solve_inverse<4>(ctx, x, W, W2);
+      case 8: return solve_inverse<8>(ctx, x, W, W2);
+      default: break;
+    }
+  }
   switch (sw * 16 + nr) {
     case 128 * 16 + 2: return solve_impl_m<128, 2>(ctx);
     case 128 * 16 + 3: return solve_impl_m<128, 3>(ctx);
@@ -2859,7 +2883,7 @@ int Factor::enqueue_multi(tlr_ctx *ctx, int nr, cudaEvent_t a, cudaEvent_t b) {
   const size_t n = (size_t)sym.nn * 5;
   int rc = TLR_OK;
   if (a) TLR_CUDA(ctx, cudaEventRecordWithFlags(a, st, cudaEventRecordExternal));
-  if (wave) {
+  if (wave && !inverse) {
     for (int v = 0; v < nr && !rc; ++v)
       rc = enqueue_solve(ctx, static_cast<float2 *>(vec_m) + v * n, nullptr, nullptr);
   } else {

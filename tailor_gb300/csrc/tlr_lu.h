@@ -17,6 +17,35 @@ struct DevFront {
 // Default of Factor::cluster_rows (the automatic cluster-panel choice).
 constexpr int kClusterPanelRows = 256;
 
+// One tensor-core product C(rows, cols) -= F(rows, K) F(K, cols) inside a
+// front (m x m at off in the pool): rows [r0, r1), columns [c0, c1), inner
+// range [k0, k0 + kw).
+struct TcJob {
+  long long off;
+  int m, k0, kw, r0, r1, c0, c1, pad;
+};
+
+// A batch of such products run by one launch: offsets of its jobs and of
+// the per-job prefixes (jobs + 1 each) of its output tiles and of the
+// operand tiles.
+struct TcBatch {
+  int job_off = 0, jobs = 0, prefix_off = 0, pa_off = 0, pb_off = 0;
+  int tiles = 0, atiles = 0, btiles = 0;
+};
+
+// Work item of the inverse-form solves (tlr_inv.cu): up to 32 rows of a
+// front times a range of columns.
+struct SvItem {
+  long long a;     // pool offset of the item's first entry
+  int ld, rows, cols;
+  int vec;         // work index of the first vector entry
+  int piv;         // leading columns whose vector entries are pivot rows' values
+  int out;         // work index of the first row
+  int tile;        // row tile of the launch (partial sums and counter)
+  int split, nsplit;
+  int kind;        // 0 forward pivot rows, 1 forward border rows, 2 backward
+};
+
 struct Step {  // one panel step of one level
   int nf, max_m, max_b, max_ext, prefix_off, tiles;
   // complex64: per-front prefixes (nf + 1 each, in the schedule) of the
@@ -41,6 +70,8 @@ struct Level {
   int wf_n = 0, wb_n = 0;
   long long wcf_off = 0, wcb_off = 0;
   int wctr_n = 0;
+  // inverse-form solve: items of the forward and of the backward launch
+  int if_off = 0, if_n = 0, ib_off = 0, ib_n = 0;
 };
 
 // One phase of the persistent solve: a kind of work item over a level's
@@ -88,6 +119,28 @@ struct Factor {
   int4 *d_ltiles_tc = nullptr, *d_utiles_tc = nullptr;
   long long n_ltiles_tc = 0, n_utiles_tc = 0;
   int n_inv_blocks = 0;
+  // Inverse form (complex64, 256-row blocks, tensor cores): the pivot
+  // blocks are inverted past the diagonal blocks, so a front needs one
+  // product each way (tlr_inv.cu) instead of one step per diagonal block.
+  bool inverse = false;            // the form of the present factor
+  bool inverse_ok = false;         // structures of the form exist
+  std::vector<TcBatch> inv_batches;
+  TcJob *d_inv_jobs = nullptr;
+  int *d_inv_prefix = nullptr;
+  unsigned char *inv_planes = nullptr;
+  int4 *d_gtiles = nullptr;        // 64-column tiles of the D_b row scaling
+  long long n_gtiles = 0;
+  SvItem *d_items = nullptr;
+  int item_cols = 0;               // largest column range of an item
+  int *d_uidx = nullptr;           // unknown of every front row (border: ancestors')
+  int *d_gsrc = nullptr;           // right-hand side entry of every pivot row
+  int max_split_tiles = 0, max_split = 1;
+  float2 *split_part = nullptr;    // partial sums of split row tiles
+  int *split_ctr = nullptr;
+  bool use_inverse() const { return inverse_ok && tensor_cores && !persistent; }
+  int build_inverse(tlr_ctx *ctx); // host structures, called by setup
+  int invert_pivots(tlr_ctx *ctx);
+  template <int NR> int solve_inverse(tlr_ctx *ctx, float2 *x, float2 *W, float2 *W2);
   long long inv_elems = 0, n_ltiles = 0, n_utiles = 0;
   cudaGraphExec_t graph_exec = nullptr;  // captured solve, replayed per call
   // persistent solve: one cooperative launch per solve over a phase table
@@ -132,9 +185,9 @@ struct Factor {
   // allocate the multi-vector buffers (outside any stream capture)
   int solve_multi_prepare(tlr_ctx *ctx);
   // Enqueue the solve of the nr right-hand sides in vec_m, in place, for
-  // capture into a caller's graph (solve_multi_prepare first).  With the
-  // dependency-driven level launches (wave) the vectors go one at a time;
-  // the bits are the same.
+  // capture into a caller's graph (solve_multi_prepare first).  Block steps
+  // with the dependency-driven level launches (wave) take one vector at a
+  // time; the bits are the same.
   int enqueue_multi(tlr_ctx *ctx, int nr, cudaEvent_t a, cudaEvent_t b);
   template <int SW, int NR> int solve_impl_m(tlr_ctx *ctx);
   int solve_impl_m_dispatch(tlr_ctx *ctx, int nr);

@@ -107,8 +107,9 @@ int autotune(tlr_ctx *ctx, ClassState &cs, int ring_slack) {
       cs.sym.reset(new Symbolic(F->sym));
       ctx->shared_sym = cs.sym.get();
     }
-    const int ntc = bi == 0 ? 2 : 1;
-    for (int k = 0; k < ntc && !rc; ++k) {
+    // the tensor-core factor last: its (inverse) form is what the solves of
+    // the 256 block are timed on
+    for (int k = bi == 0 ? 1 : 0; k >= 0 && !rc; --k) {
       F->tensor_cores = bi == 0 ? k == 0 : !cs.cuda_core_schur;
       cudaEventRecord(ctx->ev0, ctx->stream);
       if ((rc = F->factor(ctx, sr, si, tiny))) break;

@@ -328,6 +328,61 @@ __device__ __forceinline__ int find_front(const int *__restrict__ prefix, int nf
   return lo;
 }
 
+__device__ __forceinline__ void split4_tf32(const float *x, uint4 &hi4, uint4 &lo4) {
+  uint32_t h[4], l[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    h[j] = to_tf32(x[j]);
+    l[j] = to_tf32(x[j] - __uint_as_float(h[j]));
+  }
+  hi4 = make_uint4(h[0], h[1], h[2], h[3]);
+  lo4 = make_uint4(l[0], l[1], l[2], l[3]);
+}
+
+// A-operand row `row` of a 128-row plane pair: K' 4 q4 .. +3 real parts and
+// 8 + 4 q4 .. +3 imaginary parts of four complex K entries
+__device__ __forceinline__ void stage_a4(unsigned char *hi, int row, int q4, const float2 *v) {
+  float re[4], im[4];
+  uint4 h, l;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    re[j] = v[j].x;
+    im[j] = v[j].y;
+  }
+  split4_tf32(re, h, l);
+  *reinterpret_cast<uint4 *>(hi + plane_off(row, 4 * q4)) = h;
+  *reinterpret_cast<uint4 *>(hi + kPlane + plane_off(row, 4 * q4)) = l;
+  split4_tf32(im, h, l);
+  *reinterpret_cast<uint4 *>(hi + plane_off(row, 8 + 4 * q4)) = h;
+  *reinterpret_cast<uint4 *>(hi + kPlane + plane_off(row, 8 + 4 * q4)) = l;
+}
+
+// B-operand column bn of a 64-column output tile (planes of 128 "rows":
+// Cr row bn = [Br ; -Bi], Ci row 64 + bn = [Bi ; Br]) for four complex K
+// entries 4 q4 .. +3
+__device__ __forceinline__ void stage_b4(unsigned char *hi, int bn, int q4, const float2 *v) {
+  float br[4], bi[4], nbi[4];
+  uint4 h, l;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    br[j] = v[j].x;
+    bi[j] = v[j].y;
+    nbi[j] = -v[j].y;
+  }
+  unsigned char *lo = hi + kPlane;
+  split4_tf32(br, h, l);
+  *reinterpret_cast<uint4 *>(hi + plane_off(bn, 4 * q4)) = h;
+  *reinterpret_cast<uint4 *>(lo + plane_off(bn, 4 * q4)) = l;
+  *reinterpret_cast<uint4 *>(hi + plane_off(64 + bn, 8 + 4 * q4)) = h;
+  *reinterpret_cast<uint4 *>(lo + plane_off(64 + bn, 8 + 4 * q4)) = l;
+  split4_tf32(nbi, h, l);
+  *reinterpret_cast<uint4 *>(hi + plane_off(bn, 8 + 4 * q4)) = h;
+  *reinterpret_cast<uint4 *>(lo + plane_off(bn, 8 + 4 * q4)) = l;
+  split4_tf32(bi, h, l);
+  *reinterpret_cast<uint4 *>(hi + plane_off(64 + bn, 4 * q4)) = h;
+  *reinterpret_cast<uint4 *>(lo + plane_off(64 + bn, 4 * q4)) = l;
+}
+
 // grid (atiles + btiles, nchmax): blockIdx.x < atiles is A tile
 // (front, 128-row tile), else B tile (front, 64-column tile); blockIdx.y is
 // the K chunk.  pa / pb: per-front prefix of A / B tiles (nf + 1 each).
@@ -403,6 +458,41 @@ __global__ void __launch_bounds__(256)
     split4(ui, h, l);
     *reinterpret_cast<uint4 *>(bh + plane_off(64 + bn, 4 * bq)) = h;
     *reinterpret_cast<uint4 *>(bl + plane_off(64 + bn, 4 * bq)) = l;
+  }
+}
+
+// The same conversion for a batch of jobs (TcJob): A tiles are 128 rows of
+// [r0, r1), B tiles 64 columns of [c0, c1), K chunks of [k0, k0 + kw).
+__global__ void __launch_bounds__(256)
+    k_tc_split_jobs(const TcJob *__restrict__ jobs, const int *__restrict__ pa,
+                    const int *__restrict__ pb, int nj, const float2 *__restrict__ pool,
+                    unsigned char *__restrict__ planes, int atiles, int nchmax) {
+  const int tid = threadIdx.x, c = blockIdx.y;
+  const bool is_a = (int)blockIdx.x < atiles;
+  const int t = is_a ? blockIdx.x : blockIdx.x - atiles;
+  const int lo = find_front(is_a ? pa : pb, nj, t);
+  const TcJob jb = jobs[lo];
+  if (c * kTcKC >= jb.kw) return;
+  const long long m = jb.m;
+  const float2 *F = pool + jb.off;
+  unsigned char *img = planes + ((long long)blockIdx.x * nchmax + c) * kChunkImg;
+  float2 v[4];
+  if (is_a) {
+    const int row = jb.r0 + (t - pa[lo]) * kTcM + (tid & (kTcM - 1)), aq = tid >> 7;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int kc = c * kTcKC + 4 * aq + j;
+      v[j] = (row < jb.r1 && kc < jb.kw) ? F[(jb.k0 + kc) * m + row] : make_float2(0.f, 0.f);
+    }
+    stage_a4(img, tid & (kTcM - 1), aq, v);
+  } else if (tid < 128) {
+    const int bn = tid & 63, bq = tid >> 6, col = jb.c0 + (t - pb[lo]) * kTcN + bn;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int kb = c * kTcKC + 4 * bq + j;
+      v[j] = (col < jb.c1 && kb < jb.kw) ? F[col * m + jb.k0 + kb] : make_float2(0.f, 0.f);
+    }
+    stage_b4(img, bn, bq, v);
   }
 }
 
@@ -605,13 +695,16 @@ __global__ void __launch_bounds__(256, MINB)
 // out raises the error flag and the CTA's abort word, every role stops
 // waiting, and the copies and MMAs already issued are awaited (bounded)
 // before TMEM is released.
+// With jobs (JOB) the tiles are those of a batch of TcJobs instead of the
+// trailing blocks of one panel step.
 constexpr int kPersistThreads = 320;
 
-template <int S>
+template <int S, bool JOB>
 __global__ void __launch_bounds__(kPersistThreads, 1)
-    k_gemm_tc_persist(const int *__restrict__ fl, const int *__restrict__ prefix,
-                      const int *__restrict__ pa, const int *__restrict__ pb, int nf, int s, int w,
-                      int tiles, float2 *__restrict__ pool, const DevFront *__restrict__ fr,
+    k_gemm_tc_persist(const TcJob *__restrict__ jobs, const int *__restrict__ fl,
+                      const int *__restrict__ prefix, const int *__restrict__ pa,
+                      const int *__restrict__ pb, int nf, int s, int w, int tiles,
+                      float2 *__restrict__ pool, const DevFront *__restrict__ fr,
                       const unsigned char *__restrict__ planes_a,
                       const unsigned char *__restrict__ planes_b, int nchmax,
                       int *__restrict__ err) {
@@ -650,23 +743,36 @@ __global__ void __launch_bounds__(kPersistThreads, 1)
   // tile t -> front, its first row / column and the operand images
   struct Tile {
     float2 *F;
-    int m, R0, C0, nch;
+    int m, R0, C0, r1, c1, nch;  // leading dimension, origin, ends
     const unsigned char *ga, *gb;
   };
   auto decode = [&](int t) {
     Tile d;
     const int lo = find_front(prefix, nf, t);
-    const DevFront f = fr[fl[lo]];
-    const int k0 = s * w, ww = min(w, f.p - k0);
-    const int base = k0 + ww, ext = f.m - base;
-    const int ntm = (ext + kTcM - 1) / kTcM;
+    int r0, c0, kw;
+    if constexpr (JOB) {
+      const TcJob jb = jobs[lo];
+      d.F = pool + jb.off;
+      d.m = jb.m;
+      d.r1 = jb.r1;
+      d.c1 = jb.c1;
+      r0 = jb.r0;
+      c0 = jb.c0;
+      kw = jb.kw;
+    } else {
+      const DevFront f = fr[fl[lo]];
+      const int k0 = s * w;
+      kw = min(w, f.p - k0);
+      d.F = pool + f.off;
+      d.m = d.r1 = d.c1 = f.m;
+      r0 = c0 = k0 + kw;
+    }
+    const int ntm = (d.r1 - r0 + kTcM - 1) / kTcM;
     const int lt = t - prefix[lo];
     const int rt = lt % ntm, ct = lt / ntm;
-    d.F = pool + f.off;
-    d.m = f.m;
-    d.R0 = base + rt * kTcM;
-    d.C0 = base + ct * kTcN;
-    d.nch = (ww + kTcKC - 1) / kTcKC;
+    d.R0 = r0 + rt * kTcM;
+    d.C0 = c0 + ct * kTcN;
+    d.nch = (kw + kTcKC - 1) / kTcKC;
     d.ga = planes_a + (long long)(pa[lo] + rt) * nchmax * kChunkImg;
     d.gb = planes_b + (long long)(pb[lo] + ct) * nchmax * kChunkImg;
     return d;
@@ -741,13 +847,13 @@ __global__ void __launch_bounds__(kPersistThreads, 1)
     for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++ti) {
       const Tile d = decode(t);
       const int acc = ti & 1;
-      const bool row_ok = d.R0 + row < d.m;
+      const bool row_ok = d.R0 + row < d.r1;
       // this tile's F22 entries, fetched while its MMAs run
       float2 f22[32];
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
         const int n = 32 * h2 + j;
-        f22[j] = (row_ok && d.C0 + n < d.m) ? d.F[(long long)(d.C0 + n) * d.m + d.R0 + row]
+        f22[j] = (row_ok && d.C0 + n < d.c1) ? d.F[(long long)(d.C0 + n) * d.m + d.R0 + row]
                                             : make_float2(0.f, 0.f);
       }
       bool ok = true;
@@ -767,7 +873,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1)
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const int n = n0 + j;
-            if (d.C0 + n < d.m) {
+            if (d.C0 + n < d.c1) {
               float2 v = f22[8 * part + j];
               v.x -= __uint_as_float(cr[j]);
               v.y -= __uint_as_float(ci[j]);
@@ -826,61 +932,6 @@ namespace {
 constexpr int kRwSW = 256;                          // diagonal-block size
 constexpr int kRwLStage = 10 * kPlane;              // A hi/lo + four B tiles hi/lo
 constexpr int kRwUStage = 6 * kPlane;               // two A tiles hi/lo + B hi/lo
-
-__device__ __forceinline__ void split4_tf32(const float *x, uint4 &hi4, uint4 &lo4) {
-  uint32_t h[4], l[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    h[j] = to_tf32(x[j]);
-    l[j] = to_tf32(x[j] - __uint_as_float(h[j]));
-  }
-  hi4 = make_uint4(h[0], h[1], h[2], h[3]);
-  lo4 = make_uint4(l[0], l[1], l[2], l[3]);
-}
-
-// A-operand row `row` of a 128-row plane pair: K' 4 q4 .. +3 real parts and
-// 8 + 4 q4 .. +3 imaginary parts of four complex K entries
-__device__ __forceinline__ void stage_a4(unsigned char *hi, int row, int q4, const float2 *v) {
-  float re[4], im[4];
-  uint4 h, l;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    re[j] = v[j].x;
-    im[j] = v[j].y;
-  }
-  split4_tf32(re, h, l);
-  *reinterpret_cast<uint4 *>(hi + plane_off(row, 4 * q4)) = h;
-  *reinterpret_cast<uint4 *>(hi + kPlane + plane_off(row, 4 * q4)) = l;
-  split4_tf32(im, h, l);
-  *reinterpret_cast<uint4 *>(hi + plane_off(row, 8 + 4 * q4)) = h;
-  *reinterpret_cast<uint4 *>(hi + kPlane + plane_off(row, 8 + 4 * q4)) = l;
-}
-
-// B-operand column bn of a 64-column output tile (planes of 128 "rows":
-// Cr row bn = [Br ; -Bi], Ci row 64 + bn = [Bi ; Br]) for four complex K
-// entries 4 q4 .. +3
-__device__ __forceinline__ void stage_b4(unsigned char *hi, int bn, int q4, const float2 *v) {
-  float br[4], bi[4], nbi[4];
-  uint4 h, l;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    br[j] = v[j].x;
-    bi[j] = v[j].y;
-    nbi[j] = -v[j].y;
-  }
-  unsigned char *lo = hi + kPlane;
-  split4_tf32(br, h, l);
-  *reinterpret_cast<uint4 *>(hi + plane_off(bn, 4 * q4)) = h;
-  *reinterpret_cast<uint4 *>(lo + plane_off(bn, 4 * q4)) = l;
-  *reinterpret_cast<uint4 *>(hi + plane_off(64 + bn, 8 + 4 * q4)) = h;
-  *reinterpret_cast<uint4 *>(lo + plane_off(64 + bn, 8 + 4 * q4)) = l;
-  split4_tf32(nbi, h, l);
-  *reinterpret_cast<uint4 *>(hi + plane_off(bn, 8 + 4 * q4)) = h;
-  *reinterpret_cast<uint4 *>(lo + plane_off(bn, 8 + 4 * q4)) = l;
-  split4_tf32(bi, h, l);
-  *reinterpret_cast<uint4 *>(hi + plane_off(64 + bn, 4 * q4)) = h;
-  *reinterpret_cast<uint4 *>(lo + plane_off(64 + bn, 4 * q4)) = l;
-}
 
 // the three MMAs of one K step (A_lo B_hi + A_hi B_lo + A_hi B_hi)
 __device__ __forceinline__ void mma3(uint32_t tmem, uint32_t a_hi, uint32_t b_hi, uint32_t acc0) {
@@ -1036,11 +1087,14 @@ __global__ void __launch_bounds__(256, 1)
   tc_teardown<512>(tmem);
 }
 
+// DENSE (k_scale_g): the left factor is the dense D_b, the tile 64 columns
+// left of block b, and the product is negated.
+template <bool DENSE>
 __global__ void __launch_bounds__(256, 2)
     k_scale_u_tc(const int4 *__restrict__ tiles, float2 *__restrict__ pool,
                  const DevFront *__restrict__ fr, const long long *__restrict__ inv_off,
                  const float2 *__restrict__ Linv, const float2 *__restrict__ Uinv,
-                 float2 *__restrict__ dmat, int *__restrict__ err) {
+                 float2 *__restrict__ dmat, int *__restrict__ err, int place) {
   extern __shared__ __align__(1024) unsigned char tc_smem[];
   __shared__ __align__(8) uint64_t bars[2];
   __shared__ uint32_t tmem_slot;
@@ -1056,11 +1110,11 @@ __global__ void __launch_bounds__(256, 2)
   const float2 *src;
   float2 *dst;
   long long ld, ncol;
-  if (tl.w == 0) {
+  if (DENSE || tl.w == 0) {
     dst = pool + f.off + b0;
     src = dst;
     ld = f.m;
-    ncol = f.m;
+    ncol = DENSE ? b0 : f.m;
   } else {
     src = Linv + io;
     dst = dmat + io;
@@ -1081,7 +1135,7 @@ __global__ void __launch_bounds__(256, 2)
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const int q = c * kTcKC + k;
-      va[k] = (ai < nb && q < nb && q >= ai) ? Ui[(long long)q * nb + ai] : make_float2(0.f, 0.f);
+      va[k] = (ai < nb && q < nb && (DENSE || q >= ai)) ? Ui[(long long)q * nb + ai] : make_float2(0.f, 0.f);
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -1105,7 +1159,7 @@ __global__ void __launch_bounds__(256, 2)
     }
     {
       const int mt = ai >> 7;
-      if (mt < nmt && (mt == 0 || c >= 16)) {  // tile mt reads this chunk
+      if (mt < nmt && (DENSE || mt == 0 || c >= 16)) {  // tile mt reads this chunk
         unsigned char *ah = st + 2 * mt * kPlane;
         stage_a4(ah, ai & 127, 0, va);
         stage_a4(ah, ai & 127, 1, va + 4);
@@ -1118,7 +1172,7 @@ __global__ void __launch_bounds__(256, 2)
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t base = smem_addr(st), b_hi = base + 4 * kPlane;
       for (int mt = 0; mt < nmt; ++mt) {
-        const int cfirst = mt == 0 ? 0 : 16;  // inv(U_bb)(i, q) = 0 for q < i
+        const int cfirst = DENSE || mt == 0 ? 0 : 16;  // inv(U_bb)(i, q) = 0 for q < i
         if (c < cfirst) continue;
 #pragma unroll
         for (int j = 0; j < 2; ++j)
@@ -1146,9 +1200,14 @@ __global__ void __launch_bounds__(256, 2)
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const int col = col0 + n0 + j;
-            if (col < ncol)
-              dst[(long long)col * ld + row] =
-                  make_float2(__uint_as_float(cr[j]), __uint_as_float(ci[j]));
+            if (col < ncol) {
+              const float sgn = DENSE ? -1.f : 1.f;
+              const float2 v =
+                  make_float2(sgn * __uint_as_float(cr[j]), sgn * __uint_as_float(ci[j]));
+              dst[(long long)col * ld + row] = v;
+              if (!DENSE && place && tl.w)  // D_b over the pivot block's diagonal block
+                pool[f.off + (long long)(b0 + col) * f.m + b0 + row] = v;
+            }
           }
         }
       }
@@ -1169,13 +1228,13 @@ int launch_gemm_tc_bulk(tlr_ctx *ctx, const int *fl, const int *prefix, const in
                                                                planes, atiles, nchmax); count_launches(); }
   const unsigned char *pbp = planes + (long long)atiles * nchmax * kChunkImg;
   if (variant == 2) {  // persistent, warp-specialised: one CTA per SM, four stages
-    auto k = k_gemm_tc_persist<4>;
+    auto k = k_gemm_tc_persist<4, false>;
     const int smem = (int)gemm_tc_bulk_smem(4);
     TLR_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
     const int grid = std::max(1, std::min(tiles, std::max(sms, 1)));
-    { k<<<grid, kPersistThreads, smem, st>>>(fl, prefix, pa, pb, nf, s, w, tiles, pool, fr,
+    { k<<<grid, kPersistThreads, smem, st>>>(nullptr, fl, prefix, pa, pb, nf, s, w, tiles, pool, fr,
                                              planes, pbp, nchmax, err); count_launches(); }
   } else if (variant == 1) {  // two stages, three CTAs per SM, half the F22 prefetched
     auto k = k_gemm_tc_bulk<2, 3, 16>;
@@ -1206,17 +1265,50 @@ int launch_gemm_tc(tlr_ctx *ctx, const int *fl, const int *prefix, int nf, int s
 int launch_rewrite_tc(tlr_ctx *ctx, const int4 *ltiles, long long nl, const int4 *utiles,
                       long long nu, float2 *pool, const DevFront *fr, const long long *inv_off,
                       const float2 *Linv, const float2 *Uinv, float2 *dmat, int *err,
-                      cudaStream_t st) {
+                      cudaStream_t st, bool place) {
   const size_t lsm = 2 * kRwLStage + 1024, usm = 2 * kRwUStage + 1024;
   TLR_CUDA(ctx, cudaFuncSetAttribute(k_scale_l_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)lsm));
-  TLR_CUDA(ctx, cudaFuncSetAttribute(k_scale_u_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)usm));
+  TLR_CUDA(ctx, cudaFuncSetAttribute(k_scale_u_tc<false>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)usm));
   if (nu > 0)
-    { k_scale_u_tc<<<(unsigned)nu, 256, usm, st>>>(utiles, pool, fr, inv_off, Linv, Uinv, dmat,
-                                                  err); count_launches(); }
+    { k_scale_u_tc<false><<<(unsigned)nu, 256, usm, st>>>(utiles, pool, fr, inv_off, Linv, Uinv,
+                                                         dmat, err, place ? 1 : 0); count_launches(); }
   if (nl > 0)
     { k_scale_l_tc<<<(unsigned)nl, 256, lsm, st>>>(ltiles, pool, fr, inv_off, Linv, err); count_launches(); }
+  TLR_CUDA(ctx, cudaGetLastError());
+  return TLR_OK;
+}
+
+int launch_tc_jobs(tlr_ctx *ctx, const TcJob *jobs, int nj, const int *prefix, const int *pa,
+                   const int *pb, int tiles, int atiles, int btiles, float2 *pool,
+                   unsigned char *planes, int *err, cudaStream_t st) {
+  constexpr int nchmax = kRwSW / kTcKC;
+  if (tiles <= 0) return TLR_OK;
+  { k_tc_split_jobs<<<dim3(atiles + btiles, nchmax), 256, 0, st>>>(jobs, pa, pb, nj, pool, planes,
+                                                                  atiles, nchmax); count_launches(); }
+  auto k = k_gemm_tc_persist<4, true>;
+  const int smem = (int)gemm_tc_bulk_smem(4);
+  TLR_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  int sms = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+  const int grid = std::max(1, std::min(tiles, std::max(sms, 1)));
+  { k<<<grid, kPersistThreads, smem, st>>>(jobs, nullptr, prefix, pa, pb, nj, 0, 0, tiles, pool,
+                                           nullptr, planes,
+                                           planes + (long long)atiles * nchmax * kChunkImg, nchmax,
+                                           err); count_launches(); }
+  TLR_CUDA(ctx, cudaGetLastError());
+  return TLR_OK;
+}
+
+int launch_scale_g(tlr_ctx *ctx, const int4 *tiles, long long nt, float2 *pool, const DevFront *fr,
+                   const long long *inv_off, const float2 *dmat, int *err, cudaStream_t st) {
+  if (nt <= 0) return TLR_OK;
+  const size_t usm = 2 * kRwUStage + 1024;
+  TLR_CUDA(ctx, cudaFuncSetAttribute(k_scale_u_tc<true>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)usm));
+  { k_scale_u_tc<true><<<(unsigned)nt, 256, usm, st>>>(tiles, pool, fr, inv_off, nullptr, dmat,
+                                                      nullptr, err, 0); count_launches(); }
   TLR_CUDA(ctx, cudaGetLastError());
   return TLR_OK;
 }
