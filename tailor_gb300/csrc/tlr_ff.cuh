@@ -6,13 +6,17 @@
 
 namespace tlr {
 
-// (hi, lo) += a * x with a = ah + al, x = xh + xl
+// (hi, lo) += a * x with a = ah + al, x = xh + xl: the leading product is
+// exact in p + e, its sum exact in s and the two-sum's rest; twelve
+// instructions
 __device__ __forceinline__ void ff_mac(float &hi, float &lo, float ah, float al, float xh,
                                        float xl) {
-  const float p = ah * xh;
-  const float e = fmaf(ah, xh, -p) + fmaf(ah, xl, al * xh);
-  const float s = hi + p;
-  const float bb = s - hi;
+  const float p = __fmul_rn(ah, xh);
+  const float e = fmaf(ah, xh, -p);
+  lo = fmaf(ah, xl, lo);
+  lo = fmaf(al, xh, lo);
+  const float s = __fadd_rn(hi, p);
+  const float bb = __fadd_rn(s, -hi);
   lo += ((hi - (s - bb)) + (p - bb)) + e;
   hi = s;
 }
@@ -42,6 +46,38 @@ __device__ __forceinline__ void ffc_mac(FFC &s, const float4 &a, const float4 &x
   ff_mac(s.rh, s.rl, -a.z, -a.w, x.z, x.w);
   ff_mac(s.ih, s.il, a.x, a.y, x.z, x.w);
   ff_mac(s.ih, s.il, a.z, a.w, x.x, x.y);
+}
+
+// (h, l) with h + l renormalised so that h carries the leading bits
+__device__ __forceinline__ void ff_norm(float &h, float &l) {
+  const float s = h + l;
+  l = l - (s - h);
+  h = s;
+}
+
+// a - b of two complex float-float values
+__device__ __forceinline__ float4 ffc_sub(float4 a, const FFC &b) {
+  ff_add(a.x, a.y, -b.rh, -b.rl);
+  ff_add(a.z, a.w, -b.ih, -b.il);
+  ff_norm(a.x, a.y);
+  ff_norm(a.z, a.w);
+  return a;
+}
+
+// a * f, f = fh + fl real
+__device__ __forceinline__ float4 ffc_scale(float4 a, float fh, float fl) {
+  float4 r;
+  r.x = a.x * fh;
+  r.y = fmaf(a.x, fh, -r.x) + fmaf(a.x, fl, a.y * fh);
+  r.z = a.z * fh;
+  r.w = fmaf(a.z, fh, -r.z) + fmaf(a.z, fl, a.w * fh);
+  ff_norm(r.x, r.y);
+  ff_norm(r.z, r.w);
+  return r;
+}
+
+__device__ __forceinline__ double2 ff_value(const float4 &a) {
+  return make_double2((double)a.x + (double)a.y, (double)a.z + (double)a.w);
 }
 
 __device__ __forceinline__ double2 ffc_value(const FFC &s) {

@@ -108,6 +108,8 @@ struct tlr_ctx {
   double *red = nullptr;     // [RD_COUNT]
   double *partial = nullptr; // per-block partial sums for norms
   int partial_blocks = 0;
+  int *kv_ctr = nullptr;     // arrival counters of the basis reductions
+  int kv_ctr_n = 0;
   int *bc_modes = nullptr;   // [nz][2]: incoming and neutral counts
   double *bc_cond = nullptr; // [nz]: cond(R) per far-field node
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -162,9 +164,19 @@ int vec_norm_async(tlr_ctx *ctx, const double2 *v, long long count, double *scra
 // h = V(:, 0:nk)^H w
 int kv_dot(tlr_ctx *ctx, long long n, const double2 *V, long long ldv, int nk,
            const double2 *w, double2 *part, double2 *h);
-// w -= V(:, 0:nk) h; with norm, also *norm = ||w|| of the result
+// w -= V(:, 0:nk) h; with norm, also *norm = ||w|| of the result and, with a
+// column, the projected matrix's column j (its Gram-Schmidt passes h1, h2 and
+// the norm) and the coefficients g = [H h | H (H h)(0:j+1)] of the pipelined
+// applications' shift
+struct KvColumn {
+  const double2 *h1 = nullptr, *h2 = nullptr;
+  double2 *H = nullptr;  // ldh x columns
+  float4 *g = nullptr;   // 2 x ldh
+  int j = 0, ldh = 0;
+};
 int kv_update(tlr_ctx *ctx, long long n, const double2 *V, long long ldv, int nk,
-              const double2 *h, double2 *w, double *npart, double *norm);
+              const double2 *h, double2 *w, double *npart, double *norm,
+              const KvColumn *column = nullptr);
 // out(:, 0:nl) = V(:, 0:nq) Y(0:nq, 0:nl); out must not overlap V
 int kv_combine(tlr_ctx *ctx, long long n, const double2 *V, long long ldv, int nq,
                const double2 *Y, int ldy, int nl, double2 *out, long long ldo);

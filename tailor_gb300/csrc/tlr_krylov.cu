@@ -577,10 +577,10 @@ struct Solver {
     int rc;
     {
       CaptureScope cs;
-      rc = pipe_residuals(ctx, *pipe, pipe_rhs());
+      rc = pipe_residuals(ctx, *pipe, pipe_rhs(), F->d_solve_err);
       if (!rc) rc = F->enqueue_multi(ctx, 3, rev[0], rev[1]);
       if (!rc) rc = pipe_targets(ctx, *pipe, sr, si, x, pipe_rhs(), true);
-      if (!rc) rc = pipe_accept(ctx, *pipe, hnorm);
+      if (!rc) rc = pipe_accept(ctx, *pipe, hnorm, F->d_solve_err);
     }
     cudaGraph_t g = nullptr;
     const cudaError_t e = cudaStreamEndCapture(st, &g);
@@ -1148,17 +1148,17 @@ int run_solve(tlr_ctx *ctx, const tlr_solve_opts *opts, double *lambda,
       for (int i = 0; i < bsz && !rc; ++i) {
         const int j = j0 + i, nk = j + bsz;
         double2 *w = bsz == 1 ? S.w : S.Wb + (size_t)i * n;
+        const Pipe &pp = ws->pipe;
+        const KvColumn column{hcol(0, j), hcol(1, j), pp.H, pp.g, j, pp.ldh};
         for (int pass = 0; pass < 2 && !rc; ++pass) {
           rc = kv_dot(ctx, n, S.V, n, nk, w, S.kpart, hcol(pass, j));
           if (!rc)
             rc = kv_update(ctx, n, S.V, n, nk, hcol(pass, j), w, S.npart,
-                           pass ? ws->betad + j : nullptr);
+                           pass ? ws->betad + j : nullptr, pass && piped ? &column : nullptr);
         }
         if (!rc && piped) {  // the next vector and its pipelined guesses
-          rc = pipe_coefficients(ctx, ws->pipe, j, hcol(0, j), hcol(1, j), ws->betad + j);
-          if (!rc)
-            rc = pipe_shift(ctx, ws->pipe, j, ws->betad + j, S.sr, S.si, w,
-                            S.V + (size_t)nk * n, S.pipe_rhs());
+          rc = pipe_shift(ctx, ws->pipe, j, ws->betad + j, S.sr, S.si, w,
+                          S.V + (size_t)nk * n, S.pipe_rhs());
         } else if (!rc) {
           rc = kv_scale(ctx, n, w, ws->betad + j, 1.0, S.V + (size_t)nk * n);
         }

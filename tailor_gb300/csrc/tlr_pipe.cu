@@ -4,6 +4,7 @@
 // application (EigenSolver.cpp:61-71).
 #include <algorithm>
 
+#include "tlr_async.cuh"
 #include "tlr_complex.cuh"
 #include "tlr_ff.cuh"
 #include "tlr_pipe.h"
@@ -12,11 +13,19 @@ namespace tlr {
 namespace {
 
 // The element-wise kernels own whole grid nodes (five unknowns), because
-// they end in a product with the block-diagonal B: 51 nodes per CTA.
-constexpr int kNodes = 51, kRows = 5 * kNodes, kThreads = 256;
-constexpr int kWarpRows = 8;  // block rows (warps) per CTA of the A products
+// they end in a product with the block-diagonal B: 12 nodes per CTA of 64
+// threads, so that the smallest grids still fill the SMs.
+constexpr int kNodes = 12, kRows = 5 * kNodes, kThreads = 64;
+// the shift: 10 nodes per CTA, five threads per row sharing the basis
+// vectors (one thread per row left 38 CTAs of 20 dependent steps at 60 x 32:
+// 15 us)
+constexpr int kSNodes = 10, kSRows = 5 * kSNodes, kSGroups = 5, kSThreads = 256;
+// A products: one CTA of 16 warps per SM, each warp with a ring of five
+// stages of six blocks in shared memory (192 KB)
+constexpr int kRWarps = 16, kRStages = 5, kRBlocks = 6, kRStage = 25 * kRBlocks;
+constexpr size_t kRSmem = sizeof(float4) * kRWarps * kRStages * kRStage;
 
-__device__ __forceinline__ double2 block_row(const double2 *__restrict__ Bb, const double2 *s) {
+__device__ __forceinline__ double2 block_row(const double2 *Bb, const double2 *s) {
   double2 acc = make_double2(0.0, 0.0);
 #pragma unroll
   for (int q = 0; q < 5; ++q) acc = cfma(acc, Bb[q], s[q]);
@@ -24,45 +33,62 @@ __device__ __forceinline__ double2 block_row(const double2 *__restrict__ Bb, con
 }
 
 // Targets of x and y and the right-hand side of u, for this thread's row:
-// tx = b + sigma B x, ty = B x + sigma B y, u's right-hand side B y.
-__device__ __forceinline__ void targets(long long i, const double2 *__restrict__ Bb,
-                                        const double2 *xs, const double2 *ys, double2 b,
+// tx = b + sigma B x, ty = B x + sigma B y, u's right-hand side B y (FP32, the
+// factor's precision; FP64 only where sigma needs it: the FP64 pipe is what
+// these kernels are short of).  xs: x of the node, ys: y of the node as
+// float-float.
+__device__ __forceinline__ void targets(long long i, const double2 *Bb, const float2 *B32,
+                                        const double2 *xs, const float4 *ys, double2 b,
                                         double2 sg, double2 *__restrict__ tx,
                                         double2 *__restrict__ ty, float2 *__restrict__ by32) {
-  const double2 bx = block_row(Bb, xs), by = block_row(Bb, ys);
-  tx[i] = cfma(b, sg, bx);
-  ty[i] = cfma(bx, sg, by);
-  by32[i] = make_float2((float)by.x, (float)by.y);
+  const double2 bx = block_row(Bb, xs);
+  if (sg.x == 0.0 && sg.y == 0.0) {
+    float2 by = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int q = 0; q < 5; ++q) by = cfma(by, B32[q], make_float2(ys[q].x, ys[q].z));
+    tx[i] = b;
+    ty[i] = bx;
+    by32[i] = by;
+  } else {
+    double2 yd[5];
+#pragma unroll
+    for (int q = 0; q < 5; ++q) yd[q] = ff_value(ys[q]);
+    const double2 by = block_row(Bb, yd);
+    tx[i] = cfma(b, sg, bx);
+    ty[i] = cfma(bx, sg, by);
+    by32[i] = make_float2((float)by.x, (float)by.y);
+  }
 }
 
 // this CTA's sum of |b|^2
+template <int THREADS>
 __device__ __forceinline__ void block_sum_sq(double s, double *out) {
-  __shared__ double red[kThreads / 32];
+  __shared__ double red[THREADS / 32];
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
   __syncthreads();
   if (threadIdx.x == 0) {
     double t = 0.0;
-    for (int p = 0; p < kThreads / 32; ++p) t += red[p];
+    for (int p = 0; p < THREADS / 32; ++p) t += red[p];
     *out = t;
   }
 }
 
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kSThreads)
     k_pipe_start(long long n, const double2 *__restrict__ v, const double2 *__restrict__ B,
-                 float4 *__restrict__ vff, double2 *__restrict__ x, double2 *__restrict__ y,
+                 float4 *__restrict__ vff, double2 *__restrict__ x,
                  float4 *__restrict__ xyff, double2 *__restrict__ b, double2 *__restrict__ tx,
                  double2 *__restrict__ ty, float2 *__restrict__ by32, double *__restrict__ bpart) {
-  __shared__ double2 vs[kRows];
+  __shared__ double2 vs[kSRows];
   const int t = threadIdx.x;
-  const long long i = (long long)blockIdx.x * kRows + t;
-  const bool ok = t < kRows && i < n;
+  const long long i = (long long)blockIdx.x * kSRows + t;
+  const bool ok = t < kSRows && i < n;
   double2 vi = make_double2(0.0, 0.0);
   if (ok) {
     vi = v[i];
     vs[t] = vi;
     vff[i] = ff_split(vi);
-    x[i] = y[i] = make_double2(0.0, 0.0);
+    x[i] = make_double2(0.0, 0.0);
     xyff[2 * i] = xyff[2 * i + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   __syncthreads();
@@ -75,55 +101,17 @@ __global__ void __launch_bounds__(kThreads)
     by32[i] = make_float2(0.f, 0.f);
     s2 = bi.x * bi.x + bi.y * bi.y;
   }
-  block_sum_sq(s2, bpart + blockIdx.x);
+  block_sum_sq<kSThreads>(s2, bpart + blockIdx.x);
+}
+
+__global__ void k_pipe_b32(long long n, const double2 *__restrict__ B, float2 *__restrict__ B32) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) B32[i] = make_float2((float)B[i].x, (float)B[i].y);
 }
 
 __global__ void k_pipe_split(long long n, const double2 *__restrict__ a, float4 *__restrict__ out) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] = ff_split(a[i]);
-}
-
-// Column j of H = the two Gram-Schmidt passes and beta, then g1 = H h and
-// g2 = H g1(0 : j+1) (OP V h = V g1; OP V g1 = V g2 + g1(j+1) OP v_{j+1}).
-// One CTA: four lanes per row.
-__global__ void __launch_bounds__(kThreads)
-    k_pipe_coef(int j, int ldh, const double2 *__restrict__ h1, const double2 *__restrict__ h2,
-                const double *__restrict__ beta, double2 *__restrict__ H,
-                float4 *__restrict__ g) {
-  extern __shared__ double2 sh[];  // [2][ldh]: h, then g1
-  double2 *gs = sh + ldh;
-  const int m = j + 2;  // rows of the column
-  for (int i = threadIdx.x; i < ldh; i += kThreads) {
-    double2 v = make_double2(0.0, 0.0);
-    if (i <= j) {
-      v = cadd(h1[i], h2[i]);
-      sh[i] = v;
-    } else if (i == j + 1) {
-      v.x = *beta;
-    }
-    H[(long long)j * ldh + i] = v;
-  }
-  __syncthreads();
-  const int part = threadIdx.x & 3;
-  for (int pass = 0; pass < 2; ++pass) {
-    const double2 *c = pass ? gs : sh;
-    for (int r0 = 0; r0 < m; r0 += kThreads / 4) {
-      const int i = r0 + threadIdx.x / 4;
-      double2 acc = make_double2(0.0, 0.0);
-      if (i < m)
-        for (int q = part; q <= j; q += 4) acc = cfma(acc, H[(long long)q * ldh + i], c[q]);
-#pragma unroll
-      for (int o = 1; o < 4; o <<= 1) {
-        acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
-        acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
-      }
-      if (part == 0 && i < m) {
-        if (!pass) gs[i] = acc;
-        g[pass * ldh + i] = ff_split(acc);
-      }
-    }
-    __syncthreads();
-  }
 }
 
 // v_{j+1} = w / beta, x' = (y - V g1) / beta, y' = (u - V g2 - g1(j+1) x') /
@@ -132,219 +120,332 @@ __global__ void __launch_bounds__(kThreads)
 // run in float-float on the FP32 pipe (they only make the guesses that the
 // refinement corrects; FP64 FMAs would take ten times the reading).  The
 // new basis vector itself is formed in FP64.
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kSThreads, 3)
     k_pipe_shift(long long n, int nk, int ldh, const float4 *__restrict__ vff,
                  const float4 *__restrict__ g, const double *__restrict__ beta,
-                 const double2 *__restrict__ B, double2 sg, double2 *__restrict__ x,
-                 double2 *__restrict__ y, double2 *__restrict__ vnew,
+                 const double2 *__restrict__ B, const float2 *__restrict__ B32, double2 sg,
+                 double2 *__restrict__ x, double2 *__restrict__ vnew,
                  float4 *__restrict__ vffnew, float4 *__restrict__ xyff,
                  double2 *__restrict__ b, double2 *__restrict__ tx, double2 *__restrict__ ty,
                  const float2 *__restrict__ u, float2 *__restrict__ by32,
                  double *__restrict__ bpart) {
   extern __shared__ float4 gsh[];  // [2][nk + 1]
-  __shared__ double2 vs[kRows], xs[kRows], ys[kRows];
+  __shared__ double2 vs[kSRows], xs[kSRows];
+  __shared__ float4 ys[kSRows];
+  __shared__ FFC part[kSGroups - 1][2][kSRows];
   float4 *g1 = gsh, *g2 = gsh + nk + 1;
   const int t = threadIdx.x;
-  for (int k = t; k <= nk; k += kThreads) {
+  for (int k = t; k <= nk; k += kSThreads) {
     g1[k] = g[k];
     g2[k] = g[ldh + k];
   }
+  const int grp = t / kSRows, r = t - grp * kSRows;
+  const long long i = (long long)blockIdx.x * kSRows + r;
+  const bool ok = grp < kSGroups && i < n;
+  const bool own = ok && grp == 0;
+  // the owner's operands go out before the basis products
+  double2 w = make_double2(0.0, 0.0), bl[5];
+  float4 yi = make_float4(0.f, 0.f, 0.f, 0.f);
+  float2 ui = make_float2(0.f, 0.f), b32[5];
+  const double d = *beta;
+  if (own) {
+    w = x[i];
+    yi = xyff[2 * i + 1];
+    ui = u[i];
+    const long long bo = (i / 5) * 25 + (r % 5) * 5;
+#pragma unroll
+    for (int q = 0; q < 5; ++q) {
+      bl[q] = B[bo + q];
+      b32[q] = B32[bo + q];
+    }
+  }
   __syncthreads();
-  const long long i = (long long)blockIdx.x * kRows + t;
-  const bool ok = t < kRows && i < n;
-  if (ok) {
-    FFC a1{0.f, 0.f, 0.f, 0.f}, a2{0.f, 0.f, 0.f, 0.f};
+  FFC a1{0.f, 0.f, 0.f, 0.f}, a2{0.f, 0.f, 0.f, 0.f};
+  if (ok) {  // basis vectors grp, grp + 5, ...
     const float4 *Vi = vff + i;
-    int k = 0;
-    for (; k + 4 <= nk; k += 4) {
+    int k = grp;
+    for (; k + 3 * kSGroups < nk; k += 4 * kSGroups) {
       float4 v[4];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) v[q] = Vi[(long long)(k + q) * n];
+      for (int q = 0; q < 4; ++q) v[q] = Vi[(long long)(k + q * kSGroups) * n];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        ffc_mac(a1, v[q], g1[k + q]);
-        ffc_mac(a2, v[q], g2[k + q]);
+        ffc_mac(a1, v[q], g1[k + q * kSGroups]);
+        ffc_mac(a2, v[q], g2[k + q * kSGroups]);
       }
     }
-    for (; k < nk; ++k) {
+    for (; k < nk; k += kSGroups) {
       const float4 v = Vi[(long long)k * n];
       ffc_mac(a1, v, g1[k]);
       ffc_mac(a2, v, g2[k]);
     }
-    const double d = *beta;
+    if (grp > 0) {
+      part[grp - 1][0][r] = a1;
+      part[grp - 1][1][r] = a2;
+    }
+  }
+  __syncthreads();
+  if (own) {
+#pragma unroll
+    for (int q = 0; q < kSGroups - 1; ++q) {
+      const FFC p1 = part[q][0][r], p2 = part[q][1][r];
+      ff_add(a1.rh, a1.rl, p1.rh, p1.rl);
+      ff_add(a1.ih, a1.il, p1.ih, p1.il);
+      ff_add(a2.rh, a2.rl, p2.rh, p2.rl);
+      ff_add(a2.ih, a2.il, p2.ih, p2.il);
+    }
     const double f = (d > 0.0 && d < INFINITY) ? 1.0 / d : 0.0;
-    const double2 w = x[i];
     const double2 v = make_double2(w.x * f, w.y * f);
     const float4 vf = ff_split(v);
     ffc_mac(a1, vf, g1[nk]);
     ffc_mac(a2, vf, g2[nk]);
-    const double2 s1 = ffc_value(a1), s2 = ffc_value(a2), yi = y[i];
-    const float2 ui = u[i];
-    const float4 gn = g1[nk];
-    const double2 gd = make_double2((double)gn.x + (double)gn.y, (double)gn.z + (double)gn.w);
-    const double2 xn = make_double2((yi.x - s1.x) * f, (yi.y - s1.y) * f);
-    double2 yn = cfms(make_double2((double)ui.x - s2.x, (double)ui.y - s2.y), gd, xn);
-    yn.x *= f;
-    yn.y *= f;
+    // the guesses stay on the FP32 pipe (float-float)
+    const float fh = (float)f, fl = (float)(f - (double)fh);
+    const float4 xn = ffc_scale(ffc_sub(yi, a1), fh, fl);
+    ffc_mac(a2, xn, g1[nk]);
+    const float4 yn =
+        ffc_scale(ffc_sub(make_float4(ui.x, 0.f, ui.y, 0.f), a2), fh, fl);
+    const double2 xd = ff_value(xn);
     vnew[i] = v;
     vffnew[i] = vf;
-    x[i] = xn;
-    y[i] = yn;
-    xyff[2 * i] = ff_split(xn);
-    xyff[2 * i + 1] = ff_split(yn);
-    vs[t] = v;
-    xs[t] = xn;
-    ys[t] = yn;
+    x[i] = xd;
+    xyff[2 * i] = xn;
+    xyff[2 * i + 1] = yn;
+    vs[r] = v;
+    xs[r] = xd;
+    ys[r] = yn;
   }
   __syncthreads();
   double s2 = 0.0;
-  if (ok) {
-    const double2 *Bb = B + (i / 5) * 25 + (t % 5) * 5;
-    const int q = t / 5 * 5;
-    const double2 bi = block_row(Bb, vs + q);
+  if (own) {
+    const int q = r / 5 * 5;
+    const double2 bi = block_row(bl, vs + q);
     b[i] = bi;
     s2 = bi.x * bi.x + bi.y * bi.y;
-    targets(i, Bb, xs + q, ys + q, bi, sg, tx, ty, by32);
+    targets(i, bl, b32, xs + q, ys + q, bi, sg, tx, ty, by32);
   }
-  block_sum_sq(s2, bpart + blockIdx.x);
+  block_sum_sq<kSThreads>(s2, bpart + blockIdx.x);
 }
 
 // x += c_x, y += c_y (with corrections), their splits and targets.
 __global__ void __launch_bounds__(kThreads)
-    k_pipe_targets(long long n, int correct, const double2 *__restrict__ B, double2 sg,
-                   double2 *__restrict__ x, double2 *__restrict__ y, float4 *__restrict__ xyff,
+    k_pipe_targets(long long n, int correct, const double2 *__restrict__ B,
+                   const float2 *__restrict__ B32, double2 sg, double2 *__restrict__ x,
+                   float4 *__restrict__ xyff,
                    const double2 *__restrict__ b, double2 *__restrict__ tx,
                    double2 *__restrict__ ty, const float2 *__restrict__ rhs,
                    float2 *__restrict__ by32) {
-  __shared__ double2 xs[kRows], ys[kRows];
+  __shared__ double2 xs[kRows];
+  __shared__ float4 ys[kRows];
   const int t = threadIdx.x;
   const long long i = (long long)blockIdx.x * kRows + t;
   const bool ok = t < kRows && i < n;
+  double2 bl[5], bi = make_double2(0.0, 0.0);
+  float2 b32[5];
   if (ok) {
-    double2 xi = x[i], yi = y[i];
+    double2 xi = x[i];
+    float4 yi = xyff[2 * i + 1];
+    const long long bo = (i / 5) * 25 + (t % 5) * 5;
+#pragma unroll
+    for (int q = 0; q < 5; ++q) {
+      bl[q] = B[bo + q];
+      b32[q] = B32[bo + q];
+    }
+    bi = b[i];
     if (correct) {
       const float2 cx = rhs[i], cy = rhs[n + i];
       xi.x += cx.x;
       xi.y += cx.y;
-      yi.x += cy.x;
-      yi.y += cy.y;
+      ff_add(yi.x, yi.y, cy.x, 0.f);
+      ff_add(yi.z, yi.w, cy.y, 0.f);
+      ff_norm(yi.x, yi.y);
+      ff_norm(yi.z, yi.w);
       x[i] = xi;
-      y[i] = yi;
+      xyff[2 * i + 1] = yi;
     }
     xyff[2 * i] = ff_split(xi);
-    xyff[2 * i + 1] = ff_split(yi);
     xs[t] = xi;
     ys[t] = yi;
   }
   __syncthreads();
   if (ok) {
-    const double2 *Bb = B + (i / 5) * 25 + (t % 5) * 5;
     const int q = t / 5 * 5;
-    targets(i, Bb, xs + q, ys + q, b[i], sg, tx, ty, by32);
+    targets(i, bl, b32, xs + q, ys + q, bi, sg, tx, ty, by32);
   }
 }
 
 // A times x (NV = 1) or x and y (NV = 2) in float-float, subtracted from
-// the targets.  Warp per block row, lane 5 r + c holds entry (r, c) of each
-// block; the operator is read once for both vectors.  NV = 2 writes the
-// three right-hand sides, NV = 1 this CTA's sum of |r|^2.
+// the targets.  Bound by reading the operator (NV = 1) and by the float-float
+// arithmetic on the FP32 pipe (NV = 2, 96 instructions per entry).  A block
+// row's blocks are contiguous, so each warp streams its rows (row gw, gw + W,
+// ...) through its own ring with bulk copies of six blocks, issued by its
+// first lane five stages ahead and across rows.  Lane 5 b + r multiplies row r
+// of block b: 30 of 32 lanes work (25 with a lane per entry of one block), a
+// lane's five entries are 80 consecutive bytes (no bank conflicts), and a row
+// is summed over six lanes at its end.  Every wait is bounded: on a timeout
+// the warp raises the error flag, waits once more for its copies in flight
+// and stops.  NV = 2 writes the three right-hand sides, NV = 1 the norms
+// out[0] = |r|, out[1] = |b| (b's partial sums: bpart).
 template <int NV>
-__global__ void __launch_bounds__(32 * kWarpRows)
+__global__ void __launch_bounds__(32 * kRWarps, 1)
     k_pipe_residual(int nrows, const int *__restrict__ row_ptr, const int *__restrict__ col,
                     const float4 *__restrict__ aff, const float4 *__restrict__ xyff,
                     const double2 *__restrict__ tx, const double2 *__restrict__ ty,
                     const float2 *__restrict__ by32, float2 *__restrict__ rhs, long long n,
-                    double *__restrict__ rpart) {
-  __shared__ double red[kWarpRows];
+                    double *__restrict__ rpart, int nb, const double *__restrict__ bpart,
+                    int *__restrict__ arrived, double *__restrict__ out, int *__restrict__ err) {
+  extern __shared__ __align__(128) float4 ring_all[];
+  __shared__ __align__(8) uint64_t full_all[kRWarps][kRStages];
+  __shared__ double red[2][kRWarps];
+  __shared__ int last;
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-  const int row = blockIdx.x * kWarpRows + wp;
-  const int c = lane % 5;
-  const bool active = lane < 25;
+  float4 *ring = ring_all + wp * kRStages * kRStage;
+  uint64_t *full = full_all[wp];
+  const int W = gridDim.x * kRWarps, gw = wp * gridDim.x + blockIdx.x;
+  if (lane == 0) {
+    for (int q = 0; q < kRStages; ++q) mbar_init(&full[q], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncwarp();
+  // producer cursor (first lane): the next blocks [pk, pe) of row prow
+  int prow = gw - W, pk = 0, pe = 0, issued = 0;
+  auto issue = [&]() {
+    while (pk >= pe) {
+      prow += W;
+      if (prow >= nrows) {
+        prow -= W;  // stay here: nothing left
+        return;
+      }
+      pk = row_ptr[prow];
+      pe = row_ptr[prow + 1];
+    }
+    const int nb = min(kRBlocks, pe - pk), st = issued % kRStages;
+    mbar_expect_tx(&full[st], nb * 400);
+    bulk_g2s(ring + st * kRStage, aff + (size_t)pk * 25, nb * 400, &full[st]);
+    pk += nb;
+    ++issued;
+  };
+  if (lane == 0)
+    for (int q = 0; q < kRStages; ++q) issue();
+  const int l = min(lane, 29), bl = l / 5, rr = l % 5;
+  int consumed = 0;
+  bool fine = true;
   double s2 = 0.0;
-  if (row < nrows) {
+  for (int row = gw; row < nrows && fine; row += W) {
+    const int k0 = row_ptr[row], k1 = row_ptr[row + 1];
     FFC s[NV];
 #pragma unroll
     for (int v = 0; v < NV; ++v) s[v] = FFC{0.f, 0.f, 0.f, 0.f};
-    const int k0 = row_ptr[row], k1 = row_ptr[row + 1];
-    constexpr int kU = NV == 1 ? 8 : 5;
-    for (int k = k0; k < k1; k += kU) {
-      float4 a[kU], xv[kU][NV];
+    // the columns of 30 blocks at a time, x one stage ahead
+    int mycol = lane < 30 && k0 + lane < k1 ? col[k0 + lane] : 0;
+    for (int kb = k0; kb < k1 && fine; kb += 30) {
+      const int nxcol = lane < 30 && kb + 30 + lane < k1 ? col[kb + 30 + lane] : 0;
+      float4 xv[NV][5];
+      auto load_x = [&](int j) {  // stage j of this group of 30 blocks
+        const int c = __shfl_sync(0xffffffffu, mycol, min(j * kRBlocks + bl, 29));
+        const float4 *p = xyff + (size_t)c * 10;
 #pragma unroll
-      for (int u = 0; u < kU; ++u) {
-        const bool ok = active && k + u < k1;
-        a[u] = ok ? __ldcs(aff + (size_t)(k + u) * 25 + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float4 *p = xyff + (ok ? 2 * ((size_t)col[k + u] * 5 + c) : 0);
+        for (int q = 0; q < 5; ++q)
 #pragma unroll
-        for (int v = 0; v < NV; ++v) xv[u][v] = ok ? p[v] : make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int v = 0; v < NV; ++v) xv[v][q] = p[2 * q + v];
+      };
+      load_x(0);
+      for (int j = 0; j < 5 && kb + j * kRBlocks < k1; ++j) {
+        const int st = consumed % kRStages;
+        if (!mbar_wait(&full[st], (consumed / kRStages) & 1)) fine = false;
+        fine = __all_sync(0xffffffffu, fine);
+        if (!fine) break;
+        if (kb + j * kRBlocks + bl < k1) {
+          const float4 *ap = ring + st * kRStage + l * 5;
+#pragma unroll
+          for (int q = 0; q < 5; ++q) {
+            const float4 av = ap[q];
+#pragma unroll
+            for (int v = 0; v < NV; ++v) ffc_mac(s[v], av, xv[v][q]);
+          }
+        }
+        __syncwarp();
+        ++consumed;
+        if (lane == 0) issue();
+        if (j < 4) load_x(j + 1);
       }
-#pragma unroll
-      for (int u = 0; u < kU; ++u)
-#pragma unroll
-        for (int v = 0; v < NV; ++v) ffc_mac(s[v], a[u], xv[u][v]);
+      mycol = nxcol;
     }
+    // lanes r, r + 5, ..., r + 25 hold row r
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
 #pragma unroll
-      for (int d = 1; d < 5; ++d) {
-        const float h1 = __shfl_down_sync(0xffffffffu, s[v].rh, d);
-        const float l1 = __shfl_down_sync(0xffffffffu, s[v].rl, d);
-        const float h2 = __shfl_down_sync(0xffffffffu, s[v].ih, d);
-        const float l2 = __shfl_down_sync(0xffffffffu, s[v].il, d);
-        if (c == 0) {
+      for (int d = 0; d < 3; ++d) {
+        const int o = d == 0 ? 15 : 5;
+        const float h1 = __shfl_down_sync(0xffffffffu, s[v].rh, o * (d == 2 ? 2 : 1));
+        const float l1 = __shfl_down_sync(0xffffffffu, s[v].rl, o * (d == 2 ? 2 : 1));
+        const float h2 = __shfl_down_sync(0xffffffffu, s[v].ih, o * (d == 2 ? 2 : 1));
+        const float l2 = __shfl_down_sync(0xffffffffu, s[v].il, o * (d == 2 ? 2 : 1));
+        if (d == 0 ? lane < 15 : lane < 5) {
           ff_add(s[v].rh, s[v].rl, h1, l1);
           ff_add(s[v].ih, s[v].il, h2, l2);
         }
       }
     }
-    if (active && c == 0) {
-      const size_t i = (size_t)row * 5 + lane / 5;
+    if (lane < 5) {
+      const size_t i = (size_t)row * 5 + rr;
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
-        const double2 a = ffc_value(s[v]), tg = v ? ty[i] : tx[i];
-        const double2 r = make_double2(tg.x - a.x, tg.y - a.y);
-        if (NV == 1)
-          s2 = r.x * r.x + r.y * r.y;
-        else
+        const double2 av = ffc_value(s[v]), tg = v ? ty[i] : tx[i];
+        const double2 r = make_double2(tg.x - av.x, tg.y - av.y);
+        if (NV == 1) {
+          s2 = fma(r.x, r.x, s2);
+          s2 = fma(r.y, r.y, s2);
+        } else {
           rhs[v * n + i] = make_float2((float)r.x, (float)r.y);
+        }
       }
       if (NV == 2) rhs[2 * n + i] = by32[i];
     }
   }
+  if (!fine && lane == 0) {
+    atomicExch(err, 1);
+    for (int q = consumed; q < issued; ++q) mbar_wait(&full[q % kRStages], (q / kRStages) & 1);
+  }
   if (NV == 1) {
-    for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-    if (lane == 0) red[wp] = s2;
+    for (int o = 4; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);  // lanes 0 .. 4
+    if (lane == 0) red[0][wp] = s2;
     __syncthreads();
     if (threadIdx.x == 0) {
       double t = 0.0;
-      for (int p = 0; p < kWarpRows; ++p) t += red[p];
+      for (int p = 0; p < kRWarps; ++p) t += red[0][p];
       rpart[blockIdx.x] = t;
+      __threadfence();
+      last = atomicAdd(arrived, 1) == (int)gridDim.x - 1;
+      if (last) *arrived = 0;
+      __threadfence();
+    }
+    __syncthreads();
+    if (!last) return;
+    // the last CTA: both norms, the partial sums added in a fixed order
+    double a = 0.0, b = 0.0;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += 32 * kRWarps) a += __ldcg(rpart + i);
+    for (int i = threadIdx.x; i < nb; i += 32 * kRWarps) b += bpart[i];
+    for (int o = 16; o > 0; o >>= 1) {
+      a += __shfl_xor_sync(0xffffffffu, a, o);
+      b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+    if (lane == 0) {
+      red[0][wp] = a;
+      red[1][wp] = b;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+      double t = 0.0;
+      for (int p = 0; p < kRWarps; ++p) t += red[threadIdx.x][p];
+      out[threadIdx.x] = sqrt(t);
     }
   }
 }
 
-// out = sqrt of the two partial sums, summed in a fixed order
-__global__ void __launch_bounds__(512)
-    k_pipe_norms(int nr, const double *__restrict__ rpart, int nb,
-                 const double *__restrict__ bpart, double *__restrict__ out) {
-  __shared__ double red[2][16];
-  double s[2] = {0.0, 0.0};
-  for (int i = threadIdx.x; i < nr; i += 512) s[0] += rpart[i];
-  for (int i = threadIdx.x; i < nb; i += 512) s[1] += bpart[i];
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    for (int o = 16; o > 0; o >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
-    if ((threadIdx.x & 31) == 0) red[k][threadIdx.x >> 5] = s[k];
-  }
-  __syncthreads();
-  if (threadIdx.x < 2) {
-    double t = 0.0;
-    for (int p = 0; p < 16; ++p) t += red[threadIdx.x][p];
-    out[threadIdx.x] = sqrt(t);
-  }
-}
-
 int node_blocks(const Pipe &p) { return blocks_for(p.nn, kNodes); }
-int row_blocks(const Pipe &p) { return blocks_for(p.nn, kWarpRows); }
+int shift_blocks(const Pipe &p) { return blocks_for(p.nn, kSNodes); }
+int row_blocks(const Pipe &p) { return std::min(p.sms, blocks_for(p.nn, kRWarps)); }
 
 }  // namespace
 
@@ -353,32 +454,42 @@ int pipe_alloc(tlr_ctx *ctx, Pipe &p, int ncv) {
   p.n = 5LL * ctx->nn;
   p.ncv = ncv;
   p.ldh = ncv + 2;
+  p.sms = 1;
+  cudaDeviceGetAttribute(&p.sms, cudaDevAttrMultiProcessorCount, ctx->device);
+  TLR_CUDA(ctx, cudaFuncSetAttribute(k_pipe_residual<1>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRSmem));
+  TLR_CUDA(ctx, cudaFuncSetAttribute(k_pipe_residual<2>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRSmem));
   const size_t n = (size_t)p.n;
   TLR_CUDA(ctx, cudaMalloc(&p.vff, sizeof(float4) * n * (ncv + 1)));
   TLR_CUDA(ctx, cudaMalloc(&p.xyff, sizeof(float4) * 2 * n));
-  TLR_CUDA(ctx, cudaMalloc(&p.y, sizeof(double2) * n));
+  TLR_CUDA(ctx, cudaMalloc(&p.B32, sizeof(float2) * 5 * n));
   TLR_CUDA(ctx, cudaMalloc(&p.b, sizeof(double2) * n));
   TLR_CUDA(ctx, cudaMalloc(&p.tx, sizeof(double2) * n));
   TLR_CUDA(ctx, cudaMalloc(&p.ty, sizeof(double2) * n));
   TLR_CUDA(ctx, cudaMalloc(&p.by32, sizeof(float2) * n));
   TLR_CUDA(ctx, cudaMalloc(&p.H, sizeof(double2) * p.ldh * ncv));
   TLR_CUDA(ctx, cudaMalloc(&p.g, sizeof(float4) * 2 * p.ldh));
-  TLR_CUDA(ctx, cudaMalloc(&p.bpart, sizeof(double) * node_blocks(p)));
+  TLR_CUDA(ctx, cudaMalloc(&p.bpart, sizeof(double) * shift_blocks(p)));
   TLR_CUDA(ctx, cudaMalloc(&p.rpart, sizeof(double) * row_blocks(p)));
+  TLR_CUDA(ctx, cudaMalloc(&p.arrived, sizeof(int)));
+  TLR_CUDA(ctx, cudaMemsetAsync(p.arrived, 0, sizeof(int), ctx->stream));
   TLR_CUDA(ctx, cudaHostAlloc(&p.hup, sizeof(double2) * p.ldh * ncv, cudaHostAllocDefault));
   return TLR_OK;
 }
 
 void pipe_free(Pipe &p) {
-  cudaFree(p.vff); cudaFree(p.xyff); cudaFree(p.y); cudaFree(p.b); cudaFree(p.tx);
+  cudaFree(p.vff); cudaFree(p.xyff); cudaFree(p.B32); cudaFree(p.b); cudaFree(p.tx);
   cudaFree(p.ty); cudaFree(p.by32); cudaFree(p.H); cudaFree(p.g); cudaFree(p.bpart); cudaFree(p.rpart);
+  cudaFree(p.arrived);
   cudaFreeHost(p.hup);
   p = Pipe();
 }
 
 int pipe_start(tlr_ctx *ctx, Pipe &p, const double2 *v, double2 *x) {
-  { k_pipe_start<<<node_blocks(p), kThreads, 0, ctx->stream>>>(
-      p.n, v, ctx->B, p.vff, x, p.y, p.xyff, p.b, p.tx, p.ty, p.by32, p.bpart); count_launches(); }
+  { k_pipe_b32<<<blocks_for(5 * p.n, 256), 256, 0, ctx->stream>>>(5 * p.n, ctx->B, p.B32); count_launches(); }
+  { k_pipe_start<<<shift_blocks(p), kSThreads, 0, ctx->stream>>>(
+      p.n, v, ctx->B, p.vff, x, p.xyff, p.b, p.tx, p.ty, p.by32, p.bpart); count_launches(); }
   TLR_CUDA(ctx, cudaGetLastError());
   return TLR_OK;
 }
@@ -396,34 +507,24 @@ int pipe_upload_h(tlr_ctx *ctx, Pipe &p, int l) {
   return TLR_OK;
 }
 
-int pipe_coefficients(tlr_ctx *ctx, Pipe &p, int j, const double2 *h1, const double2 *h2,
-                      const double *beta) {
-  const size_t sm = sizeof(double2) * 2 * p.ldh;
-  if (sm > 48 * 1024)
-    TLR_CUDA(ctx, cudaFuncSetAttribute(k_pipe_coef, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)sm));
-  { k_pipe_coef<<<1, kThreads, sm, ctx->stream>>>(j, p.ldh, h1, h2, beta, p.H, p.g); count_launches(); }
-  TLR_CUDA(ctx, cudaGetLastError());
-  return TLR_OK;
-}
-
 int pipe_shift(tlr_ctx *ctx, Pipe &p, int j, const double *beta, double sr, double si,
                double2 *x, double2 *vnew, const float2 *rhs) {
   const size_t sm = sizeof(float4) * 2 * (j + 2);
-  if (sm > 32 * 1024)  // the static arrays take 12 KB of the 48 KB
+  if (sm > 38 * 1024)  // the static arrays take 9 KB of the 48 KB
     TLR_CUDA(ctx, cudaFuncSetAttribute(k_pipe_shift, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)sm));
-  { k_pipe_shift<<<node_blocks(p), kThreads, sm, ctx->stream>>>(
-      p.n, j + 1, p.ldh, p.vff, p.g, beta, ctx->B, make_double2(sr, si), x, p.y, vnew,
+  { k_pipe_shift<<<shift_blocks(p), kSThreads, sm, ctx->stream>>>(
+      p.n, j + 1, p.ldh, p.vff, p.g, beta, ctx->B, p.B32, make_double2(sr, si), x, vnew,
       p.vff + (size_t)(j + 1) * p.n, p.xyff, p.b, p.tx, p.ty, rhs + 2 * p.n,
       p.by32, p.bpart); count_launches(); }
   TLR_CUDA(ctx, cudaGetLastError());
   return TLR_OK;
 }
 
-int pipe_residuals(tlr_ctx *ctx, Pipe &p, float2 *rhs) {
-  { k_pipe_residual<2><<<row_blocks(p), 32 * kWarpRows, 0, ctx->stream>>>(
-      p.nn, ctx->row_ptr, ctx->col, ctx->aff, p.xyff, p.tx, p.ty, p.by32, rhs, p.n, nullptr); count_launches(); }
+int pipe_residuals(tlr_ctx *ctx, Pipe &p, float2 *rhs, int *err) {
+  { k_pipe_residual<2><<<row_blocks(p), 32 * kRWarps, kRSmem, ctx->stream>>>(
+      p.nn, ctx->row_ptr, ctx->col, ctx->aff, p.xyff, p.tx, p.ty, p.by32, rhs, p.n, nullptr, 0,
+      nullptr, nullptr, nullptr, err); count_launches(); }
   TLR_CUDA(ctx, cudaGetLastError());
   return TLR_OK;
 }
@@ -431,16 +532,16 @@ int pipe_residuals(tlr_ctx *ctx, Pipe &p, float2 *rhs) {
 int pipe_targets(tlr_ctx *ctx, Pipe &p, double sr, double si, double2 *x, const float2 *rhs,
                  bool correct) {
   { k_pipe_targets<<<node_blocks(p), kThreads, 0, ctx->stream>>>(
-      p.n, correct ? 1 : 0, ctx->B, make_double2(sr, si), x, p.y, p.xyff, p.b, p.tx, p.ty, rhs,
+      p.n, correct ? 1 : 0, ctx->B, p.B32, make_double2(sr, si), x, p.xyff, p.b, p.tx, p.ty, rhs,
       p.by32); count_launches(); }
   TLR_CUDA(ctx, cudaGetLastError());
   return TLR_OK;
 }
 
-int pipe_accept(tlr_ctx *ctx, Pipe &p, double *out) {
-  { k_pipe_residual<1><<<row_blocks(p), 32 * kWarpRows, 0, ctx->stream>>>(
-      p.nn, ctx->row_ptr, ctx->col, ctx->aff, p.xyff, p.tx, p.ty, p.by32, nullptr, p.n, p.rpart); count_launches(); }
-  { k_pipe_norms<<<1, 512, 0, ctx->stream>>>(row_blocks(p), p.rpart, node_blocks(p), p.bpart, out); count_launches(); }
+int pipe_accept(tlr_ctx *ctx, Pipe &p, double *out, int *err) {
+  { k_pipe_residual<1><<<row_blocks(p), 32 * kRWarps, kRSmem, ctx->stream>>>(
+      p.nn, ctx->row_ptr, ctx->col, ctx->aff, p.xyff, p.tx, p.ty, p.by32, nullptr, p.n, p.rpart,
+      shift_blocks(p), p.bpart, p.arrived, out, err); count_launches(); }
   TLR_CUDA(ctx, cudaGetLastError());
   return TLR_OK;
 }

@@ -26,14 +26,17 @@ namespace tlr {
 
 struct Pipe {
   long long n = 0;        // scalar unknowns, 5 nn
-  int nn = 0, ncv = 0, ldh = 0;
+  int nn = 0, ncv = 0, ldh = 0, sms = 1;
   float4 *vff = nullptr;  // the basis as FP32 hi/lo pairs, (ncv + 1) x n
-  float4 *xyff = nullptr; // x and y the same way, interleaved [n][2]
-  double2 *y = nullptr, *b = nullptr, *tx = nullptr, *ty = nullptr;
+  // x (held in FP64 too, by the caller) and y the same way, interleaved [n][2]
+  float4 *xyff = nullptr;
+  float2 *B32 = nullptr;  // B in FP32
+  double2 *b = nullptr, *tx = nullptr, *ty = nullptr;
   float2 *by32 = nullptr; // B y, the right-hand side of u
   double2 *H = nullptr;   // (ncv + 1) x ncv projected matrix, ld ldh
   float4 *g = nullptr;    // combination coefficients, 2 x ldh
   double *bpart = nullptr, *rpart = nullptr;  // per-CTA partial sums of squares
+  int *arrived = nullptr; // CTAs done with the acceptance residual
   double2 *hup = nullptr; // pinned stage of H
 };
 
@@ -45,20 +48,17 @@ int pipe_start(tlr_ctx *ctx, Pipe &p, const double2 *v, double2 *x);
 int pipe_split_basis(tlr_ctx *ctx, Pipe &p, const double2 *V, int nk);
 // upload the leading l columns of the restarted projected matrix
 int pipe_upload_h(tlr_ctx *ctx, Pipe &p, int l);
-// column j of H from the Gram-Schmidt passes, and the coefficients of the
-// shift: g1 = H h, g2 = H g1(0:j+1)
-int pipe_coefficients(tlr_ctx *ctx, Pipe &p, int j, const double2 *h1, const double2 *h2,
-                      const double *beta);
 // x (holding the orthogonalised w) -> v_{j+1} = w / beta and the next x, y,
 // targets and right-hand side; rhs: 3 x n, its third vector holds u
 int pipe_shift(tlr_ctx *ctx, Pipe &p, int j, const double *beta, double sr, double si,
                double2 *x, double2 *vnew, const float2 *rhs);
 // rhs = the residuals of x and y, and B y
-int pipe_residuals(tlr_ctx *ctx, Pipe &p, float2 *rhs);
+// (err: set when a bounded wait of the kernel ran out)
+int pipe_residuals(tlr_ctx *ctx, Pipe &p, float2 *rhs, int *err);
 // x += rhs(0), y += rhs(1) (correct), and the targets of the new x and y
 int pipe_targets(tlr_ctx *ctx, Pipe &p, double sr, double si, double2 *x, const float2 *rhs,
                  bool correct);
 // out[0] = ||B v - K x||, out[1] = ||B v|| (out: pinned host memory)
-int pipe_accept(tlr_ctx *ctx, Pipe &p, double *out);
+int pipe_accept(tlr_ctx *ctx, Pipe &p, double *out, int *err);
 
 }  // namespace tlr

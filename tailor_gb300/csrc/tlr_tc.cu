@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <cstdint>
 
+#include "tlr_async.cuh"
 #include "tlr_complex.cuh"
 #include "tlr_internal.h"
 #include "tlr_lu.h"
@@ -34,11 +35,6 @@ constexpr int kTcKC = 8;       // complex K columns per stage (16 real: re | im)
 constexpr int kPlane = 8192;   // bytes of one 128 x 16 TF32 operand plane
 constexpr int kStage = 4 * kPlane;  // A_hi, A_lo, B_hi, B_lo
 constexpr int kTmemCols = 128;
-constexpr unsigned kWaitLimit = 1u << 22;
-
-__device__ __forceinline__ uint32_t smem_addr(const void *p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
 
 __device__ __forceinline__ uint32_t to_tf32(float x) {
   uint32_t r;
@@ -74,25 +70,6 @@ __device__ __forceinline__ void mma_commit(uint64_t *bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                    smem_addr(bar))
                : "memory");
-}
-
-__device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}\n"
-      : "=r"(ok)
-      : "r"(smem_addr(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-// bounded wait; false on timeout
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity,
-                                          unsigned limit = kWaitLimit) {
-  for (unsigned it = 0; it < limit; ++it)
-    if (mbar_test(bar, parity)) return true;
-  return false;
 }
 
 // Bounded-wait check: one thread waits on an mbarrier that nothing will
@@ -494,23 +471,6 @@ __global__ void __launch_bounds__(256)
     }
     stage_b4(img, bn, bq, v);
   }
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)),
-               "r"(bytes)
-               : "memory");
-}
-
-// global -> shared bulk copy of `bytes` (16-byte aligned addresses, size a
-// multiple of 16), completing `bytes` transactions on bar
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes,
-                                         uint64_t *bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
-          "r"(smem_addr(dst)),
-      "l"(src), "r"(bytes), "r"(smem_addr(bar))
-      : "memory");
 }
 
 // S: ring stages (shared memory S x 32 KB), MINB: CTAs per SM the register
