@@ -200,7 +200,10 @@ typedef struct {
                              kernel (one CTA per SM: a copy thread, an MMA
                              thread and eight epilogue warps, two TMEM
                              accumulators, so a tile's F22 update overlaps
-                             the next tile's MMAs); FP64 form: CUDA-core
+                             the next tile's MMAs); FP64 form with panels of
+                             32 columns (its default): tcgen05 on exact
+                             integer slices of 56 bits, one FP64 rounding per
+                             entry and panel; other panel widths: CUDA-core
                              FP64 FMA.
                              1: CUDA cores (FP32 / FP64 FMA).  2: mixed form
                              on tcgen05 with every tile staging its own
@@ -431,6 +434,12 @@ int tlr_factor_solve(tlr_ctx *ctx, int nvec, const double *rhs, double *out, int
 
 int tlr_schur_update_c64(const float *front, int m, int p, int k0, int w, unsigned lbo,
                          unsigned sbo, float *out);
+
+/* Test hook, no counterpart in the reference: the same update of a
+ * complex128 front (w must be 32) by exact integer slices on the tensor
+ * cores (sliced = 1) or by FP64 FMAs on the CUDA cores (0). */
+int tlr_schur_update_c128(const double *front, int m, int p, int k0, int w, int sliced,
+                          double *out);
 
 /* An explicit generalized pencil A x = lambda B x as a solver context
  * (EigenSolver::solve(recipe, eigenMatrix, massMatrix, ...),

@@ -210,6 +210,17 @@ struct CaptureScope {  // suppresses counting on this thread during capture
 };
 
 struct DevFront;
+// FP64 Schur update of one panel step (32 columns) of complex128 fronts by
+// exact integer slices on the tensor cores (tlr_oz.cu): prefix of the 128 x 32
+// output tiles, pa / pb of the 128-row L21 and 32-column U12 tiles; planes:
+// atiles x oz_a_image_bytes() + btiles x oz_b_image_bytes(), rexp: 32 ints per
+// front.
+int launch_gemm_oz(tlr_ctx *ctx, const int *fl, const int *prefix, const int *pa, const int *pb,
+                   int nf, int s, int w, int max_ext, double2 *pool, const DevFront *fr, int tiles,
+                   int atiles, int btiles, unsigned char *planes, int *rexp, int *err,
+                   cudaStream_t st);
+size_t oz_a_image_bytes();
+size_t oz_b_image_bytes();
 struct TcJob;
 // A batch of products C(rows, cols) -= F(rows, K) F(K, cols), K <= 256, over
 // fronts of the pool: operand planes split once per batch (planes: (atiles +

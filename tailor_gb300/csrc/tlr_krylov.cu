@@ -729,15 +729,14 @@ int run_solve(tlr_ctx *ctx, const tlr_solve_opts *opts, double *lambda,
   const cd target(rcp.omega_im, -rcp.omega_re);
   const cd sigma = o.use_sigma ? cd(o.sigma_re, o.sigma_im) : target;
   const int prec = o.precision == 1 ? 1 : 0;
-  // Schur updates on the tensor cores: tcgen05 (3xTF32) for complex64
-  // fronts, DMMA (FP64 mma.sync) for complex128 fronts
   // Schur-update kernel: 0 = the fastest measured one (complex64: tcgen05
-  // fed by bulk copies of pre-split operand planes; complex128: CUDA-core
-  // FP64, since GB300's DMMA rate is no higher and measured 13% slower);
+  // 3xTF32 fed by bulk copies of pre-split operand planes; complex128, with
+  // its default 32-column panels: exact integer slices on tcgen05, tlr_oz.cu);
   // 1 = CUDA cores; 2 = the other tensor-core variant (complex64: tiles
   // staging their own operands; complex128: DMMA)
   const bool tc = prec == 1 ? o.cuda_core_schur != 1 : o.cuda_core_schur == 2;
   const bool tc_bulk = o.cuda_core_schur != 2;
+  const bool sliced = prec == 0 && o.cuda_core_schur == 0;
   // bulk-copy kernels: 0 the persistent warp-specialised one (default), 3
   // the two-stage ring at three CTAs per SM, 4 one tile per CTA
   const int tc_variant = o.cuda_core_schur == 3 ? 1 : (o.cuda_core_schur == 4 ? 0 : 2);
@@ -754,7 +753,7 @@ int run_solve(tlr_ctx *ctx, const tlr_solve_opts *opts, double *lambda,
   // factorisation (reused when sigma, precision and Schur kernel are unchanged)
   Factor *F = ctx->factor;
   if (F && (F->prec != prec || F->sigma_re != sigma.real() || F->sigma_im != sigma.imag() ||
-            F->tensor_cores != tc || F->tc_bulk != tc_bulk || F->tc_variant != tc_variant ||
+            F->tensor_cores != tc || F->sliced != sliced || F->tc_bulk != tc_bulk || F->tc_variant != tc_variant ||
             F->sw != sblock || F->w != pwidth || F->ring_slack != rslack || !F->factored)) {
     if (F->prec != prec || F->sw != sblock || F->w != pwidth || F->ring_slack != rslack) {
       free_factor(ctx);
@@ -778,6 +777,7 @@ int run_solve(tlr_ctx *ctx, const tlr_solve_opts *opts, double *lambda,
                     : (o.cluster_panel < 0 ? INT_MAX : kClusterPanelRows);
   if (F->cluster_rows != crows) F->factored = false;
   F->tensor_cores = tc;
+  F->sliced = sliced;
   F->tc_bulk = tc_bulk;
   F->tc_variant = tc_variant;
   F->cluster_rows = crows;

@@ -1960,6 +1960,8 @@ int Factor::setup(tlr_ctx *ctx, int precision, int leaf, int solve_block, int pa
   // schedules: per level, fronts sorted by p descending; per step prefix
   std::vector<int> sched;
   long long max_plane_tiles = 0;  // largest atiles + btiles of a panel step
+  size_t oz_bytes = 0;            // largest operand images of a sliced update
+  int oz_fronts = 1;
   levels.clear();
   for (size_t h = 0; h < sym.levels.size(); ++h) {
     Level L;
@@ -2030,6 +2032,23 @@ int Factor::setup(tlr_ctx *ctx, int precision, int leaf, int solve_block, int pa
           (pass ? st.btiles : st.atiles) = tot;
         }
         max_plane_tiles = std::max(max_plane_tiles, (long long)st.atiles + st.btiles);
+      }
+      if (prec == 0 && w == kOzPanel) {  // the sliced update's tiles
+        for (int pass = 0; pass < 3; ++pass) {
+          (pass == 2 ? st.pb_off : pass ? st.pa_off : st.oz_prefix_off) = (int)sched.size();
+          int tot = 0;
+          for (int q = 0; q < st.nf; ++q) {
+            const FrontInfo &f = sym.fronts[fl[q]];
+            const int ext = f.m - s * w - std::min(w, f.p - s * w);
+            const int na = (ext + 127) / 128, nb = (ext + 31) / 32;
+            sched.push_back(tot);
+            tot += pass == 2 ? nb : pass ? na : na * nb;
+          }
+          sched.push_back(tot);
+          (pass == 2 ? st.btiles : pass ? st.atiles : st.oz_tiles) = tot;
+        }
+        oz_bytes = std::max(oz_bytes, st.atiles * oz_a_image_bytes() + st.btiles * oz_b_image_bytes());
+        oz_fronts = std::max(oz_fronts, st.nf);
       }
       L.steps.push_back(st);
     }
@@ -2180,6 +2199,10 @@ int Factor::setup(tlr_ctx *ctx, int precision, int leaf, int solve_block, int pa
       (rc = alloc((void **)&tc_planes, (size_t)max_plane_tiles * ((w + 7) / 8) *
                                            tc_chunk_image_bytes())))
     return rc;
+  if (prec == 0 && w == kOzPanel &&
+      ((rc = alloc((void **)&tc_planes, oz_bytes)) ||
+       (rc = alloc((void **)&d_rowexp, sizeof(int) * kOzPanel * oz_fronts))))
+    return rc;
   partial_stride = std::max(partial_elems, 1LL);
   TLR_CUDA(ctx, cudaMemcpy(d_inv_off, inv_off.data(), nf * sizeof(long long),
                            cudaMemcpyHostToDevice));
@@ -2309,6 +2332,8 @@ void Factor::release() {
   cudaFree(d_inv_off); cudaFree(d_inv_blocks); cudaFree(d_ltiles); cudaFree(d_utiles);
   cudaFree(d_phases); cudaFree(d_barrier); cudaFree(d_solve_err); cudaFree(tc_planes);
   cudaFree(d_wave_tiles); cudaFree(d_wave_ctr); cudaFree(d_ltiles_tc); cudaFree(d_utiles_tc);
+  cudaFree(d_rowexp);
+  d_rowexp = nullptr;
   cudaFree(d_inv_jobs); cudaFree(d_inv_prefix); cudaFree(inv_planes); cudaFree(d_gtiles);
   cudaFree(d_items); cudaFree(d_uidx); cudaFree(d_gsrc); cudaFree(split_part); cudaFree(split_ctr);
   d_inv_jobs = nullptr;
@@ -2443,7 +2468,13 @@ int Factor::factor_impl(tlr_ctx *ctx, double sr, double si, double tiny) {
               { k_gemm32<<<S.tiles, 256, 0, st>>>(fl, d_sched + S.prefix_off, S.nf, s, w,
                                                 reinterpret_cast<float2 *>(P), d_fronts); count_launches(); }
           }
-          else if (tensor_cores)
+          else if (sliced && w == kOzPanel) {
+            const int rc = launch_gemm_oz(ctx, fl, d_sched + S.oz_prefix_off, d_sched + S.pa_off,
+                                          d_sched + S.pb_off, S.nf, s, w, S.max_ext,
+                                          reinterpret_cast<double2 *>(P), d_fronts, S.oz_tiles,
+                                          S.atiles, S.btiles, tc_planes, d_rowexp, d_tc_err, st);
+            if (rc) return rc;
+          } else if (tensor_cores)
             { k_gemm_dmma<<<S.tiles, 256, 0, st>>>(fl, d_sched + S.prefix_off, S.nf, s, w,
                                                   reinterpret_cast<double2 *>(P), d_fronts); count_launches(); }
           else
@@ -2895,3 +2926,56 @@ int Factor::enqueue_multi(tlr_ctx *ctx, int nr, cudaEvent_t a, cudaEvent_t b) {
 }
 
 }  // namespace tlr
+
+// ---------------------------------------------------------------- test hook
+extern "C" int tlr_schur_update_c128(const double *front, int m, int p, int k0, int w, int sliced,
+                                     double *out) {
+  using namespace tlr;
+  if (!front || !out || m <= 0 || p <= 0 || p > m || k0 < 0 || k0 >= p || w != kOzPanel ||
+      k0 % w != 0)
+    return TLR_ERR_ARG;
+  const int ext = m - k0 - std::min(w, p - k0);
+  const size_t bytes = (size_t)m * m * sizeof(double2);
+  const int na = (ext + 127) / 128, nb = (ext + 31) / 32, nt = (ext + kTile - 1) / kTile;
+  DevFront h{};
+  h.p = p;
+  h.m = m;
+  h.parent = -1;
+  // fl, the prefixes {0, total} of sliced tiles, A and B tiles and 64 x 64
+  // tiles, err, row exponents
+  int hi[10 + kOzPanel] = {0, 0, na * nb, 0, na, 0, nb, 0, nt * nt, 0};
+  double2 *F = nullptr;
+  DevFront *fr = nullptr;
+  int *ints = nullptr;
+  unsigned char *planes = nullptr;
+  tlr_ctx ctx;
+  int rc = TLR_OK, herr = 0;
+  if (cudaGetDevice(&ctx.device) != cudaSuccess || cudaMalloc(&F, bytes) != cudaSuccess ||
+      cudaMalloc(&fr, sizeof(DevFront)) != cudaSuccess ||
+      cudaMalloc(&ints, sizeof(hi)) != cudaSuccess ||
+      cudaMalloc(&planes, na * oz_a_image_bytes() + nb * oz_b_image_bytes() + 16) != cudaSuccess ||
+      cudaStreamCreate(&ctx.stream) != cudaSuccess)
+    rc = TLR_ERR_NOMEM;
+  else if (cudaMemcpy(F, front, bytes, cudaMemcpyHostToDevice) != cudaSuccess ||
+           cudaMemcpy(fr, &h, sizeof(h), cudaMemcpyHostToDevice) != cudaSuccess ||
+           cudaMemcpy(ints, hi, sizeof(hi), cudaMemcpyHostToDevice) != cudaSuccess)
+    rc = TLR_ERR_CUDA;
+  if (!rc && ext > 0) {
+    if (sliced)
+      rc = launch_gemm_oz(&ctx, ints, ints + 1, ints + 3, ints + 5, 1, k0 / w, w, ext, F, fr,
+                          na * nb, na, nb, planes, ints + 10, ints + 9, ctx.stream);
+    else
+      { k_gemm<double2><<<nt * nt, 256, 0, ctx.stream>>>(ints, ints + 7, 1, k0 / w, w, F, fr); count_launches(); }
+  }
+  if (!rc && (cudaStreamSynchronize(ctx.stream) != cudaSuccess ||
+              cudaMemcpy(out, F, bytes, cudaMemcpyDeviceToHost) != cudaSuccess ||
+              cudaMemcpy(&herr, ints + 9, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess ||
+              herr))
+    rc = TLR_ERR_CUDA;
+  cudaFree(F);
+  cudaFree(fr);
+  cudaFree(ints);
+  cudaFree(planes);
+  if (ctx.stream) cudaStreamDestroy(ctx.stream);
+  return rc;
+}

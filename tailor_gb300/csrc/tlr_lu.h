@@ -14,6 +14,8 @@ struct DevFront {
 };
 
 
+constexpr int kOzPanel = 32;  // panel columns of the sliced FP64 Schur update
+
 // Default of Factor::cluster_rows (the automatic cluster-panel choice).
 constexpr int kClusterPanelRows = 256;
 
@@ -50,7 +52,10 @@ struct Step {  // one panel step of one level
   int nf, max_m, max_b, max_ext, prefix_off, tiles;
   // complex64: per-front prefixes (nf + 1 each, in the schedule) of the
   // step's 128-row L21 tiles and 64-column U12 tiles, and their totals
+  // (complex128 in 32-column panels: 128-row and 32-column tiles of the
+  // sliced update, with the prefix of its 128 x 32 output tiles)
   int pa_off = 0, pb_off = 0, atiles = 0, btiles = 0;
+  int oz_prefix_off = 0, oz_tiles = 0;
 };
 
 struct Level {
@@ -98,6 +103,10 @@ struct Factor {
   // with three stages / two CTAs per SM, 1 two stages / three CTAs per SM
   int tc_variant = 2;
   unsigned char *tc_planes = nullptr;
+  // complex128 Schur updates by exact integer slices on the tensor cores
+  // (tlr_oz.cu), with 32-column panels
+  bool sliced = false;
+  int *d_rowexp = nullptr;
   int w = 32;    // panel width
   int sw = 128;  // rows of a diagonal block of the solves (128 or 256)
   int ring_slack = kRingSlackDefault;  // nested-dissection ring slack, percent
