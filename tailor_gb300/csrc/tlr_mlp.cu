@@ -25,6 +25,10 @@ struct tlr_mlp {
   float *act = nullptr, *pre = nullptr, *dact = nullptr;  // [layers+1][batch][maxw]
   int cap = 0, maxw = 0;
   float *xbuf = nullptr, *ybuf = nullptr, *loss = nullptr;
+  float *wpart = nullptr;  // row-split partial parameter gradients: max_split x n_params
+  int max_split = 1;
+  float *lpart = nullptr;  // per-CTA partial losses
+  int *lctr = nullptr;     // CTAs done with the loss
   long long adam_t = 0;
   cudaStream_t stream = nullptr;
 };
@@ -40,29 +44,111 @@ __device__ __forceinline__ float silu_grad(float z) {
   return s * (1.f + z * (1.f - s));
 }
 
-// Y[n][o] = X[n][i] W^T + b (optionally SiLU), pre-activation kept in Z.
-__global__ void k_lin_fwd(int n, int in, int out, const float *__restrict__ X, int ldx,
-                          const float *__restrict__ W, const float *__restrict__ b,
-                          float *__restrict__ Z, float *__restrict__ Y, int ldy, int act) {
-  __shared__ float xs[kT][kT + 1], ws[kT][kT + 1];
-  const int row = blockIdx.y * kT + threadIdx.y, col = blockIdx.x * kT + threadIdx.x;
-  float acc = 0.f;
-  for (int k0 = 0; k0 < in; k0 += kT) {
-    xs[threadIdx.y][threadIdx.x] =
-        (row < n && k0 + threadIdx.x < in) ? X[(long long)row * ldx + k0 + threadIdx.x] : 0.f;
-    const int wr = blockIdx.x * kT + threadIdx.y;
-    ws[threadIdx.y][threadIdx.x] =
-        (wr < out && k0 + threadIdx.x < in) ? W[(long long)wr * in + k0 + threadIdx.x] : 0.f;
-    __syncthreads();
+constexpr int kMaxSplit = 16;   // row ranges of a weight gradient
+constexpr int kLossCtas = 64;
+
+// The three products of a layer in FP32 over 64 x 64 tiles: 256 threads of 4 x
+// 4 results, inner chunks of 16 in shared memory (inner index leading), the
+// next chunk's loads in flight during the present one's FMAs.  32 x 32 tiles
+// with a result per thread were bound by shared-memory reads (two per FMA), and
+// a weight gradient by its 64 CTAs of 2048 serial rows.
+//   kFwd:    Y[r][c] = act(sum_k X[r][k] W[c][k] + b[c]), Z the pre-activation
+//   kData:   dX[r][c] = sum_k dZ[r][k] W[k][c] (times silu'(Z[r][c]) with Z)
+//   kWeight: dW[r][c] = sum_k dZ[k][r] X[k][c], db[r] = sum_k dZ[k][r] over the
+//            rows k of range blockIdx.z
+enum LayerProduct { kFwd, kData, kWeight };
+constexpr int kG = 64, kGK = 16;
+
+template <int MODE>
+__global__ void __launch_bounds__(256)
+    k_layer(int M, int N, int K, const float *__restrict__ A, int lda,
+            const float *__restrict__ B, int ldb, const float *__restrict__ bias,
+            float *__restrict__ Z, float *__restrict__ C, int ldc, int act, int krange,
+            long long zstride, float *__restrict__ db) {
+  __shared__ __align__(16) float as[kGK][kG + 4], bs[kGK][kG + 4];
+  const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+  const int r0 = blockIdx.y * kG, c0 = blockIdx.x * kG;
+  const int ka = MODE == kWeight ? blockIdx.z * krange : 0;
+  const int kb = MODE == kWeight ? min(K, ka + krange) : K;
+  // element (line, k) of an operand whose inner index is contiguous (thread:
+  // one line, four k) or whose lines are (one k, four lines)
+  constexpr bool aInner = MODE != kWeight, bInner = MODE == kFwd;
+  float ra[4], rb[4];
+  auto load = [&](int k0) {
 #pragma unroll
-    for (int k = 0; k < kT; ++k) acc = fmaf(xs[threadIdx.y][k], ws[threadIdx.x][k], acc);
+    for (int q = 0; q < 4; ++q) {
+      const int la = aInner ? tid / 4 : tx * 4 + q, k1 = k0 + (aInner ? (tid % 4) * 4 + q : ty);
+      ra[q] = r0 + la < M && k1 < kb
+                  ? A[aInner ? (long long)(r0 + la) * lda + k1 : (long long)k1 * lda + r0 + la]
+                  : 0.f;
+      const int lb = bInner ? tid / 4 : tx * 4 + q, k2 = k0 + (bInner ? (tid % 4) * 4 + q : ty);
+      rb[q] = c0 + lb < N && k2 < kb
+                  ? B[bInner ? (long long)(c0 + lb) * ldb + k2 : (long long)k2 * ldb + c0 + lb]
+                  : 0.f;
+    }
+  };
+  float acc[4][4] = {};
+  float sb = 0.f;  // kWeight: this thread's share of db (64 threads of the first column)
+  load(ka);
+  for (int k0 = ka; k0 < kb; k0 += kGK) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (aInner) as[(tid % 4) * 4 + q][tid / 4] = ra[q];
+      else as[ty][tx * 4 + q] = ra[q];
+      if (bInner) bs[(tid % 4) * 4 + q][tid / 4] = rb[q];
+      else bs[ty][tx * 4 + q] = rb[q];
+    }
+    __syncthreads();
+    if (k0 + kGK < kb) load(k0 + kGK);
+#pragma unroll
+    for (int k = 0; k < kGK; ++k) {
+      const float4 a = *reinterpret_cast<const float4 *>(&as[k][ty * 4]);
+      const float4 b = *reinterpret_cast<const float4 *>(&bs[k][tx * 4]);
+      const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+    }
+    if (MODE == kWeight && blockIdx.x == 0 && tid < kG)
+#pragma unroll
+      for (int k = 0; k < kGK; ++k) sb += as[k][tid];
     __syncthreads();
   }
-  if (row < n && col < out) {
-    const float z = acc + b[col];
-    if (Z) Z[(long long)row * ldy + col] = z;
-    Y[(long long)row * ldy + col] = act ? silu(z) : z;
+  if (MODE == kWeight) {
+    C += blockIdx.z * zstride;
+    if (blockIdx.x == 0 && tid < kG && r0 + tid < M) db[blockIdx.z * zstride + r0 + tid] = sb;
   }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = r0 + ty * 4 + i;
+    if (r >= M) break;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int c = c0 + tx * 4 + j;
+      if (c >= N) break;
+      const long long o = (long long)r * ldc + c;
+      float v = acc[i][j];
+      if (MODE == kFwd) {
+        v += bias[c];
+        if (Z) Z[o] = v;
+        if (act) v = silu(v);
+      } else if (MODE == kData && Z) {
+        v *= silu_grad(Z[o]);
+      }
+      C[o] = v;
+    }
+  }
+}
+
+// g[x] = the partial gradients of all row ranges, in order
+__global__ void k_sum_splits(long long count, int splits, const float *__restrict__ part,
+                             float *__restrict__ g) {
+  const long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= count) return;
+  float s = 0.f;
+  for (int z = 0; z < splits; ++z) s += part[z * count + x];
+  g[x] = s;
 }
 
 // BF16 inference layer: weights and activations in bf16, FP32 accumulate.
@@ -93,66 +179,19 @@ __global__ void k_lin_fwd16(int n, int in, int out, const __nv_bfloat16 *__restr
   }
 }
 
-// dX[n][i] = dZ[n][o] W[o][i]
-__global__ void k_lin_bwd_data(int n, int in, int out, const float *__restrict__ dZ, int ldz,
-                               const float *__restrict__ W, float *__restrict__ dX, int ldx) {
-  __shared__ float zs[kT][kT + 1], ws[kT][kT + 1];
-  const int row = blockIdx.y * kT + threadIdx.y, col = blockIdx.x * kT + threadIdx.x;
-  float acc = 0.f;
-  for (int k0 = 0; k0 < out; k0 += kT) {
-    zs[threadIdx.y][threadIdx.x] =
-        (row < n && k0 + threadIdx.x < out) ? dZ[(long long)row * ldz + k0 + threadIdx.x] : 0.f;
-    const int wc = blockIdx.x * kT + threadIdx.x;
-    ws[threadIdx.y][threadIdx.x] =
-        (k0 + threadIdx.y < out && wc < in) ? W[(long long)(k0 + threadIdx.y) * in + wc] : 0.f;
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < kT; ++k) acc = fmaf(zs[threadIdx.y][k], ws[k][threadIdx.x], acc);
-    __syncthreads();
-  }
-  if (row < n && col < in) dX[(long long)row * ldx + col] = acc;
-}
-
-// dW[o][i] += sum_n dZ[n][o] X[n][i];  db[o] += sum_n dZ[n][o]
-__global__ void k_lin_bwd_weight(int n, int in, int out, const float *__restrict__ dZ, int ldz,
-                                 const float *__restrict__ X, int ldx, float *__restrict__ dW,
-                                 float *__restrict__ db) {
-  __shared__ float zs[kT][kT + 1], xs[kT][kT + 1];
-  const int o = blockIdx.y * kT + threadIdx.y, i = blockIdx.x * kT + threadIdx.x;
-  float acc = 0.f, accb = 0.f;
-  for (int r0 = 0; r0 < n; r0 += kT) {
-    const int zo = blockIdx.y * kT + threadIdx.x;
-    zs[threadIdx.y][threadIdx.x] =
-        (r0 + threadIdx.y < n && zo < out) ? dZ[(long long)(r0 + threadIdx.y) * ldz + zo] : 0.f;
-    xs[threadIdx.y][threadIdx.x] =
-        (r0 + threadIdx.y < n && i < in) ? X[(long long)(r0 + threadIdx.y) * ldx + i] : 0.f;
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < kT; ++k) {
-      acc = fmaf(zs[k][threadIdx.y], xs[k][threadIdx.x], acc);
-      accb += zs[k][threadIdx.y];
-    }
-    __syncthreads();
-  }
-  if (o < out && i < in) dW[(long long)o * in + i] += acc;
-  if (o < out && blockIdx.x == 0 && threadIdx.x == 0) db[o] += accb;
-}
-
-__global__ void k_silu_bwd(long long count, int cols, int ld, const float *__restrict__ Z,
-                           float *__restrict__ dA) {
-  const long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= count) return;
-  const long long r = x / cols, c = x % cols;
-  dA[r * ld + c] *= silu_grad(Z[r * ld + c]);
-}
-
-// loss = mean((Y - T)^2) over n*o; dY = 2 (Y - T) / (n o)
-__global__ void k_mse(int n, int o, int ld, const float *__restrict__ Y, const float *__restrict__ T,
-                      float *__restrict__ dY, float *__restrict__ loss) {
+// loss = mean((Y - T)^2) over n*o; dY = 2 (Y - T) / (n o).  The CTAs' partial
+// sums are added in CTA order by the CTA that finishes last.
+__global__ void __launch_bounds__(256)
+    k_mse(int n, int o, int ld, const float *__restrict__ Y, const float *__restrict__ T,
+          float *__restrict__ dY, float *__restrict__ loss, float *__restrict__ part,
+          int *__restrict__ ctr) {
   __shared__ float sh[256];
+  __shared__ bool last;
   float s = 0.f;
-  const float scale = 2.f / (float)((long long)n * o);
-  for (long long x = threadIdx.x; x < (long long)n * o; x += blockDim.x) {
+  const long long total = (long long)n * o;
+  const float scale = 2.f / (float)total;
+  for (long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x; x < total;
+       x += (long long)gridDim.x * blockDim.x) {
     const long long r = x / o, c = x % o;
     const float d = Y[r * ld + c] - T[x];
     s += d * d;
@@ -164,7 +203,18 @@ __global__ void k_mse(int n, int o, int ld, const float *__restrict__ Y, const f
     if (threadIdx.x < k) sh[threadIdx.x] += sh[threadIdx.x + k];
     __syncthreads();
   }
-  if (threadIdx.x == 0) *loss = sh[0] / (float)((long long)n * o);
+  if (threadIdx.x == 0) {
+    part[blockIdx.x] = sh[0];
+    __threadfence();
+    last = atomicAdd(ctr, 1) == (int)gridDim.x - 1;
+    if (last) {
+      *ctr = 0;
+      __threadfence();
+      float t = 0.f;
+      for (int b = 0; b < (int)gridDim.x; ++b) t += __ldcg(part + b);
+      *loss = t / (float)total;
+    }
+  }
 }
 
 __global__ void k_adam(long long count, float *__restrict__ p, const float *__restrict__ g,
@@ -205,37 +255,52 @@ void forward(tlr_mlp *m, int n) {
   for (int l = 0; l < m->n_layers; ++l) {
     const int in = m->fan_in[l], out = m->fan_out[l];
     float *Z = m->pre + plane * (l + 1), *Y = m->act + plane * (l + 1);
-    dim3 g((out + kT - 1) / kT, (n + kT - 1) / kT), b(kT, kT);
-    { k_lin_fwd<<<g, b, 0, m->stream>>>(n, in, out, X, ldx, m->params + m->w_off[l],
-                                      m->params + m->b_off[l], Z, Y, m->maxw,
-                                      l + 1 < m->n_layers); count_launches(); }
+    const dim3 g(blocks_for(out, kG), blocks_for(n, kG));
+    { k_layer<kFwd><<<g, 256, 0, m->stream>>>(n, out, in, X, ldx, m->params + m->w_off[l], in,
+                                              m->params + m->b_off[l], Z, Y, m->maxw,
+                                              l + 1 < m->n_layers, 0, 0, nullptr); count_launches(); }
     X = Y;
     ldx = m->maxw;
   }
 }
 
-// backward from dact[last] (dY); accumulates into grads (zeroed by caller)
+// loss and dY of the batch in act[last] / ybuf
+void loss_gradient(tlr_mlp *m, int n) {
+  const size_t plane = (size_t)m->cap * m->maxw;
+  const int ctas = std::min(kLossCtas, blocks_for((long long)n * m->n_out, 1024));
+  { k_mse<<<ctas, 256, 0, m->stream>>>(n, m->n_out, m->maxw, m->act + plane * m->n_layers, m->ybuf,
+                                       m->dact + plane * m->n_layers, m->loss, m->lpart,
+                                       m->lctr); count_launches(); }
+}
+
+// backward from dact[last] (dY) into grads.  The rows of a weight gradient are
+// split into ranges of 128 (up to kMaxSplit), so that the 16 tiles of a 256 x
+// 256 layer fill the SMs; one launch adds the ranges of all layers.
 void backward(tlr_mlp *m, int n) {
   const size_t plane = (size_t)m->cap * m->maxw;
+  const int splits = std::min(m->max_split, std::max(1, n / 128));
+  const int krange = ((n + splits - 1) / splits + kGK - 1) / kGK * kGK;
+  const int nz = (n + krange - 1) / krange;
+  float *dst = nz > 1 ? m->wpart : m->grads;
   for (int l = m->n_layers - 1; l >= 0; --l) {
     const int in = m->fan_in[l], out = m->fan_out[l];
-    float *dZ = m->dact + plane * (l + 1);
-    if (l + 1 < m->n_layers) {
-      const long long cnt = (long long)n * out;
-      { k_silu_bwd<<<blocks_for(cnt, 256), 256, 0, m->stream>>>(cnt, out, m->maxw,
-                                                             m->pre + plane * (l + 1), dZ); count_launches(); }
-    }
+    const float *dZ = m->dact + plane * (l + 1);
     const float *X = l == 0 ? m->xbuf : m->act + plane * l;
     const int ldx = l == 0 ? m->n_in : m->maxw;
-    dim3 gw((in + kT - 1) / kT, (out + kT - 1) / kT), b(kT, kT);
-    { k_lin_bwd_weight<<<gw, b, 0, m->stream>>>(n, in, out, dZ, m->maxw, X, ldx,
-                                              m->grads + m->w_off[l], m->grads + m->b_off[l]); count_launches(); }
-    if (l > 0) {
-      dim3 gd((in + kT - 1) / kT, (n + kT - 1) / kT);
-      { k_lin_bwd_data<<<gd, b, 0, m->stream>>>(n, in, out, dZ, m->maxw, m->params + m->w_off[l],
-                                              m->dact + plane * l, m->maxw); count_launches(); }
+    const dim3 gw(blocks_for(in, kG), blocks_for(out, kG), nz);
+    { k_layer<kWeight><<<gw, 256, 0, m->stream>>>(out, in, n, dZ, m->maxw, X, ldx, nullptr, nullptr,
+                                                  dst + m->w_off[l], in, 0, krange, m->n_params,
+                                                  dst + m->b_off[l]); count_launches(); }
+    if (l > 0) {  // times silu' of the layer below: dZ of that layer
+      const dim3 gd(blocks_for(in, kG), blocks_for(n, kG));
+      { k_layer<kData><<<gd, 256, 0, m->stream>>>(n, in, out, dZ, m->maxw, m->params + m->w_off[l],
+                                                  in, nullptr, m->pre + plane * l,
+                                                  m->dact + plane * l, m->maxw, 0, 0, 0, nullptr); count_launches(); }
     }
   }
+  if (nz > 1)
+    { k_sum_splits<<<blocks_for(m->n_params, 256), 256, 0, m->stream>>>(m->n_params, nz, m->wpart,
+                                                                       m->grads); count_launches(); }
 }
 
 }  // namespace
@@ -275,11 +340,16 @@ int tlr_mlp_create(int n_in, int width, int depth, int n_out, unsigned long long
     for (long long k = 0; k < (long long)m->fan_in[l] * m->fan_out[l]; ++k)
       h[m->w_off[l] + k] = (float)((2.0 * next() - 1.0) * a);
   }
+  // at most 256 MB of partial gradients
+  m->max_split = (int)std::max(1LL, std::min<long long>(kMaxSplit, (64LL << 20) / off));
   if (cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking) ||
       cudaMalloc(&m->params, sizeof(float) * off) || cudaMalloc(&m->grads, sizeof(float) * off) ||
       cudaMalloc(&m->m1, sizeof(float) * off) || cudaMalloc(&m->m2, sizeof(float) * off) ||
       cudaMalloc(&m->params16, sizeof(__nv_bfloat16) * off) ||
       cudaMalloc(&m->loss, sizeof(float)) ||
+      (m->max_split > 1 && cudaMalloc(&m->wpart, sizeof(float) * m->max_split * off)) ||
+      cudaMalloc(&m->lpart, sizeof(float) * kLossCtas) || cudaMalloc(&m->lctr, sizeof(int)) ||
+      cudaMemset(m->lctr, 0, sizeof(int)) ||
       cudaMemcpy(m->params, h.data(), sizeof(float) * off, cudaMemcpyHostToDevice) ||
       cudaMemset(m->m1, 0, sizeof(float) * off) || cudaMemset(m->m2, 0, sizeof(float) * off)) {
     tlr_mlp_destroy(m);
@@ -295,6 +365,7 @@ void tlr_mlp_destroy(tlr_mlp *m) {
   cudaFree(m->params); cudaFree(m->grads); cudaFree(m->m1); cudaFree(m->m2);
   cudaFree(m->params16); cudaFree(m->act); cudaFree(m->pre); cudaFree(m->dact);
   cudaFree(m->xbuf); cudaFree(m->ybuf); cudaFree(m->loss);
+  cudaFree(m->wpart); cudaFree(m->lpart); cudaFree(m->lctr);
   if (m->stream) cudaStreamDestroy(m->stream);
   delete m;
 }
@@ -318,11 +389,8 @@ int tlr_mlp_gradients(tlr_mlp *m, const float *X, const float *Y, int n, float *
   if (rc) return rc;
   cudaMemcpyAsync(m->xbuf, X, sizeof(float) * n * m->n_in, cudaMemcpyHostToDevice, m->stream);
   cudaMemcpyAsync(m->ybuf, Y, sizeof(float) * n * m->n_out, cudaMemcpyHostToDevice, m->stream);
-  cudaMemsetAsync(m->grads, 0, sizeof(float) * m->n_params, m->stream);
   forward(m, n);
-  const size_t plane = (size_t)m->cap * m->maxw;
-  { k_mse<<<1, 256, 0, m->stream>>>(n, m->n_out, m->maxw, m->act + plane * m->n_layers, m->ybuf,
-                                  m->dact + plane * m->n_layers, m->loss); count_launches(); }
+  loss_gradient(m, n);
   backward(m, n);
   if (grads)
     cudaMemcpyAsync(grads, m->grads, sizeof(float) * m->n_params, cudaMemcpyDeviceToHost,
@@ -347,7 +415,6 @@ int tlr_mlp_train(tlr_mlp *m, const float *X, const float *Y, int n, int epochs,
   }
   cudaMemcpy(dX, X, sizeof(float) * (size_t)n * m->n_in, cudaMemcpyHostToDevice);
   cudaMemcpy(dY, Y, sizeof(float) * (size_t)n * m->n_out, cudaMemcpyHostToDevice);
-  const size_t plane = (size_t)m->cap * m->maxw;
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   std::vector<float> hl;
   for (int ep = 0; ep < epochs; ++ep) {
@@ -359,10 +426,8 @@ int tlr_mlp_train(tlr_mlp *m, const float *X, const float *Y, int n, int epochs,
                       cudaMemcpyDeviceToDevice, m->stream);
       cudaMemcpyAsync(m->ybuf, dY + (size_t)r0 * m->n_out, sizeof(float) * nr * m->n_out,
                       cudaMemcpyDeviceToDevice, m->stream);
-      cudaMemsetAsync(m->grads, 0, sizeof(float) * m->n_params, m->stream);
       forward(m, nr);
-      { k_mse<<<1, 256, 0, m->stream>>>(nr, m->n_out, m->maxw, m->act + plane * m->n_layers,
-                                      m->ybuf, m->dact + plane * m->n_layers, m->loss); count_launches(); }
+      loss_gradient(m, nr);
       backward(m, nr);
       ++m->adam_t;
       const float c1 = 1.f - std::pow(b1, (float)m->adam_t), c2 = 1.f - std::pow(b2, (float)m->adam_t);
