@@ -919,62 +919,67 @@ __global__ void k_sgather(const int *__restrict__ fl, const DevFront *__restrict
 // inverse for a chunk of kIC columns in registers; step q publishes the
 // final row q through shared memory and the other rows take its multiple
 // (column-oriented substitution).  Stored column-major, leading dim nb.
-constexpr int kIC = 32;
+// The column chunks are independent: one CTA each (blockIdx.z), 8 columns.  All
+// chunks of 32 columns in one CTA were 128 x 4 serial steps of 128 FP64 FMAs
+// per thread (3.3 ms for the three blocks of a 303 x 303 pencil).
+constexpr int kIC = 8;
 
 template <class C, int SW>
 __global__ void __launch_bounds__(SW)
     k_tri_inv(const int2 *__restrict__ blocks, const C *__restrict__ pool,
               const DevFront *__restrict__ fr, const long long *__restrict__ inv_off,
               C *__restrict__ Linv, C *__restrict__ Uinv) {
-  __shared__ C rowq[kIC];
+  __shared__ C rowq[2][kIC];  // alternate steps, one barrier each
   const int2 fb = blocks[blockIdx.x];
   const DevFront f = fr[fb.x];
   const int b0 = fb.y * SW, nb = min(SW, f.p - b0);
   const C *F = pool + f.off + (long long)b0 * f.m + b0;  // F[c * m + r] = K_bb(r, c)
-  const int m = f.m, r = threadIdx.x;
+  const int r = threadIdx.x;
+  const long long m = f.m;
   const bool lower = blockIdx.y == 0;
   C *out = (lower ? Linv : Uinv) + inv_off[fb.x] + (long long)fb.y * SW * SW;
-  for (int c0 = 0; c0 < nb; c0 += kIC) {
-    C x[kIC];
+  const int c0 = blockIdx.z * kIC;
+  if (c0 >= nb) return;
+  C x[kIC];
 #pragma unroll
-    for (int j = 0; j < kIC; ++j) x[j] = r == c0 + j ? cmake<C>(1, 0) : czero<C>();
-    if (lower) {
-      for (int q = c0; q < nb; ++q) {
-        if (r == q)
+  for (int j = 0; j < kIC; ++j) x[j] = r == c0 + j ? cmake<C>(1, 0) : czero<C>();
+  const bool on = r < nb;
+  if (lower) {
+    C l = on ? F[c0 * m + r] : czero<C>();  // column q, one step ahead
+    for (int q = c0; q < nb; ++q) {
+      const C ln = on && q + 1 < nb ? F[(q + 1) * m + r] : czero<C>();
+      if (r == q)
 #pragma unroll
-          for (int j = 0; j < kIC; ++j) rowq[j] = x[j];
-        __syncthreads();
-        if (r > q && r < nb) {
-          const C l = F[(long long)q * m + r];
+        for (int j = 0; j < kIC; ++j) rowq[q & 1][j] = x[j];
+      __syncthreads();
+      if (r > q && on)
 #pragma unroll
-          for (int j = 0; j < kIC; ++j) x[j] = cfms(x[j], l, rowq[j]);
-        }
-        __syncthreads();
-      }
-    } else {
-      for (int q = min(nb - 1, c0 + kIC - 1); q >= 0; --q) {
-        if (r == q) {
-          const C d = cinv(F[(long long)q * m + q]);
-#pragma unroll
-          for (int j = 0; j < kIC; ++j) {
-            x[j] = cmul(x[j], d);
-            rowq[j] = x[j];
-          }
-        }
-        __syncthreads();
-        if (r < q) {
-          const C u = F[(long long)q * m + r];
-#pragma unroll
-          for (int j = 0; j < kIC; ++j) x[j] = cfms(x[j], u, rowq[j]);
-        }
-        __syncthreads();
-      }
+        for (int j = 0; j < kIC; ++j) x[j] = cfms(x[j], l, rowq[q & 1][j]);
+      l = ln;
     }
-    if (r < nb)
+  } else {
+    const int qs = min(nb - 1, c0 + kIC - 1);
+    const C d = on ? cinv(F[r * m + r]) : czero<C>();
+    C u = on ? F[qs * m + r] : czero<C>();
+    for (int q = qs; q >= 0; --q) {
+      const C un = on && q > 0 ? F[(q - 1) * m + r] : czero<C>();
+      if (r == q)
 #pragma unroll
-      for (int j = 0; j < kIC; ++j)
-        if (c0 + j < nb) out[(long long)(c0 + j) * nb + r] = x[j];
+        for (int j = 0; j < kIC; ++j) {
+          x[j] = cmul(x[j], d);
+          rowq[q & 1][j] = x[j];
+        }
+      __syncthreads();
+      if (r < q)
+#pragma unroll
+        for (int j = 0; j < kIC; ++j) x[j] = cfms(x[j], u, rowq[q & 1][j]);
+      u = un;
+    }
   }
+  if (on)
+#pragma unroll
+    for (int j = 0; j < kIC; ++j)
+      if (c0 + j < nb) out[(long long)(c0 + j) * nb + r] = x[j];
 }
 
 // L'(rows, c) = L(rows, c) inv(L_cc) in place: CTA = 32 rows of block
@@ -2372,7 +2377,7 @@ int Factor::rewrite_factors(tlr_ctx *ctx) {
   cudaStream_t st = ctx->stream;
   C *P = static_cast<C *>(pool);
   C *Li = static_cast<C *>(linv), *Ui = static_cast<C *>(uinv);
-  { k_tri_inv<C, SW><<<dim3(n_inv_blocks, 2), SW, 0, st>>>(d_inv_blocks, P, d_fronts, d_inv_off,
+  { k_tri_inv<C, SW><<<dim3(n_inv_blocks, 2, SW / kIC), SW, 0, st>>>(d_inv_blocks, P, d_fronts, d_inv_off,
                                                           Li, Ui); count_launches(); }
   if constexpr (sizeof(C) == sizeof(float2) && SW == 256) {
     if (tensor_cores) {  // the products on the tensor cores, like the Schur updates
