@@ -142,10 +142,11 @@ class Problem:
         return a
 
     def spmv(self, which: int, x: np.ndarray) -> np.ndarray:
-        xr = np.ascontiguousarray(np.stack([x.real, x.imag], -1), dtype=np.float64)
-        y = np.empty_like(xr)
-        self.check(self.lib.tlr_spmv(self.ctx, which, _ptr(xr), _ptr(y), 0))
-        return y[..., 0] + 1j * y[..., 1]
+        # complex128 is the ABI's interleaved (re, im) layout
+        x = np.ascontiguousarray(x, dtype=np.complex128)
+        y = np.empty_like(x)
+        self.check(self.lib.tlr_spmv(self.ctx, which, _ptr(x), _ptr(y), 0))
+        return y
 
 
 class Metrics:

@@ -12,6 +12,7 @@
 // coalesced 16-byte streaming stores.  Each block entry is accumulated in
 // the reference's ADD order (K0, xi-line combination, eta-line
 // combination, cross term); this file is compiled with --fmad=false.
+#include <algorithm>
 #include <cfloat>
 
 #include "tlr_internal.h"
@@ -279,7 +280,9 @@ struct WriterSharedT {
 template <int SX, int SE>
 __global__ void __launch_bounds__(kWriterThreads)
     k_write_rows_t(int ny, int nz, DevRule xi, DevRule eta, const double *__restrict__ coef,
-                   double2 *__restrict__ L, double2 *__restrict__ Mv) {
+                   double2 *__restrict__ L, double2 *__restrict__ Mv,
+                   double *__restrict__ partial, double *__restrict__ norm,
+                   int *__restrict__ ctr) {
   using SH = WriterSharedT<SX, SE>;
   constexpr int S = SH::S, NL = SH::NL;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -287,6 +290,7 @@ __global__ void __launch_bounds__(kWriterThreads)
   const int nn = ny * nz;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int groups = (nn + kSub - 1) / kSub;
+  double s2 = 0.0;  // this thread's share of |L|^2
   for (int g = blockIdx.x; g < groups; g += gridDim.x) {
     const int n0 = g * kSub;
     const int cnt = min(kSub, nn - n0);
@@ -399,8 +403,42 @@ __global__ void __launch_bounds__(kWriterThreads)
     for (int u = warp; u < cnt; u += kWriterThreads / 32)
       if (lane < 25)
         __stcs(Mv + (long long)(n0 + u) * 25 + lane, make_double2(sh.cf[u][CF_GAMMA + lane], 0.0));
+    // |L|^2 from the staged blocks: the line blocks' entries and the six
+    // nonzeros of every cross block (a pass over the written operator took
+    // as long as half the writing, on the FP64 pipe)
+    for (int x = tid; x < cnt * NL * 25; x += kWriterThreads) {
+      const double2 e = sh.line[x / (NL * 25)][x / 25 % NL][x % 25];
+      s2 = fma(e.x, e.x, fma(e.y, e.y, s2));
+    }
+    for (int x = tid; x < cnt * S; x += kWriterThreads) {
+      const int u = x / S, k = x % S;
+      if (sh.order[u][k / SX] != sh.ce[u] && k % SX != sh.cx[u])
+#pragma unroll
+        for (int p = 0; p < 6; ++p) s2 = fma(sh.cross[u][k][p], sh.cross[u][k][p], s2);
+    }
     __syncthreads();
   }
+  // the CTAs' sums are added in CTA order by the CTA that finishes last
+  __shared__ double red[kWriterThreads / 32];
+  __shared__ bool last;
+  for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+  if (lane == 0) red[warp] = s2;
+  __syncthreads();
+  if (tid == 0) {
+    double t = 0.0;
+    for (int w = 0; w < kWriterThreads / 32; ++w) t += red[w];
+    partial[blockIdx.x] = t;
+    __threadfence();
+    last = atomicAdd(ctr, 1) == (int)gridDim.x - 1;
+    if (last) *ctr = 0;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!last || tid >= 32) return;
+  double t = 0.0;
+  for (int b = tid; b < (int)gridDim.x; b += 32) t += __ldcg(partial + b);
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (tid == 0) *norm = sqrt(t);
 }
 
 template <int SX, int SE>
@@ -413,9 +451,12 @@ int launch_writer_t(tlr_ctx *ctx) {
   TLR_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_write_rows_t<SX, SE>,
                                                               kWriterThreads, smem));
   const int groups = (ctx->nn + kSub - 1) / kSub;
-  const int grid = std::max(1, std::min(groups, sms * std::max(per_sm, 1)));
+  // one partial sum per CTA in ctx->partial (64 x partial_blocks words)
+  const int grid = std::max(1, std::min({groups, sms * std::max(per_sm, 1),
+                                         64 * ctx->partial_blocks}));
   { k_write_rows_t<SX, SE><<<grid, kWriterThreads, smem, ctx->stream>>>(
-      ctx->ny, ctx->nz, ctx->xi, ctx->eta, ctx->coef, ctx->L, ctx->M); count_launches(); }
+      ctx->ny, ctx->nz, ctx->xi, ctx->eta, ctx->coef, ctx->L, ctx->M, ctx->partial,
+      ctx->pin + PIN_NORMS + 1, ctx->kv_ctr); count_launches(); }
   TLR_CUDA(ctx, cudaGetLastError());
   return TLR_OK;
 }
@@ -458,15 +499,19 @@ int run_assemble(tlr_ctx *ctx, tlr_operator_diag *diag) {
   p.a2_re = ar * ar - ai * ai;
   p.a2_im = ar * ai + ai * ar;
   p.alpha_finite = std::isfinite(ar) && std::isfinite(ai);
+  {
+    int rc = pinned_words(ctx);
+    if (!rc) rc = arrival_counters(ctx, 1);
+    if (rc) return rc;
+  }
   TLR_CUDA(ctx, cudaMemsetAsync(ctx->status, 0, sizeof(int) * ST_COUNT, ctx->stream));
   { k_coefficients<<<blocks_for(ctx->nn, 32), 32, 0, ctx->stream>>>(
       p, ctx->base_c, ctx->derivs, ctx->metrics, ctx->coef, ctx->status); count_launches(); }
   TLR_CUDA(ctx, cudaGetLastError());
-  int st[ST_COUNT];
-  TLR_CUDA(ctx, cudaMemcpyAsync(st, ctx->status, sizeof(st), cudaMemcpyDeviceToHost,
-                                ctx->stream));
+  TLR_CUDA(ctx, cudaMemcpyAsync(ctx->pin + PIN_STATUS, ctx->status, sizeof(int) * ST_COUNT,
+                                cudaMemcpyDeviceToHost, ctx->stream));
   TLR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  if (st[ST_COEF])
+  if (reinterpret_cast<const int *>(ctx->pin + PIN_STATUS)[ST_COEF])
     return fail(ctx, TLR_ERR_COEFFICIENTS,
                 "At least one node produced invalid curvilinear LNS coefficients "
                 "during global operator validation");
@@ -493,6 +538,11 @@ int run_assemble(tlr_ctx *ctx, tlr_operator_diag *diag) {
     TLR_CUDA(ctx, cudaGetLastError());
   }
   TLR_CUDA(ctx, cudaEventRecord(ctx->ev1, ctx->stream));
+  if (diag) {  // the specialised writers leave ||L|| themselves
+    int rc = frobenius_async(ctx, ctx->M, (long long)ctx->nn * 25, ctx->pin + PIN_NORMS);
+    if (!rc && wr < 0) rc = frobenius_async(ctx, ctx->L, ctx->nnzb * 25, ctx->pin + PIN_NORMS + 1);
+    if (rc) return rc;
+  }
   TLR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   if (diag) {
     tlr_operator_diag d{};
@@ -501,10 +551,8 @@ int run_assemble(tlr_ctx *ctx, tlr_operator_diag *diag) {
     d.mass_used_blocks = d.mass_allocated_blocks = ctx->nn;
     d.spatial_used_blocks = d.spatial_allocated_blocks = (double)ctx->nnzb;
     cudaEventElapsedTime(&d.assemble_ms, ctx->ev0, ctx->ev1);
-    int rc = frobenius(ctx, ctx->M, (long long)ctx->nn * 25, &d.mass_frobenius_norm);
-    if (rc) return rc;
-    rc = frobenius(ctx, ctx->L, ctx->nnzb * 25, &d.spatial_frobenius_norm);
-    if (rc) return rc;
+    d.mass_frobenius_norm = ctx->pin[PIN_NORMS];
+    d.spatial_frobenius_norm = ctx->pin[PIN_NORMS + 1];
     *diag = d;
   }
   return TLR_OK;

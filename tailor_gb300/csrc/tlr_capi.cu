@@ -275,6 +275,7 @@ void tlr_ctx_destroy(tlr_ctx *ctx) {
   cudaFree(ctx->M); cudaFree(ctx->B); cudaFree(ctx->status); cudaFree(ctx->red);
   cudaFree(ctx->partial); cudaFree(ctx->bc_modes); cudaFree(ctx->bc_cond);
   cudaFree(ctx->aff); cudaFree(ctx->wff); cudaFree(ctx->wff_m); cudaFree(ctx->kv_ctr);
+  cudaFree(ctx->spmv_xy); cudaFree(ctx->bc_part); cudaFreeHost(ctx->pin);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -399,18 +400,16 @@ int tlr_spmv(tlr_ctx *ctx, int which, const double *x, double *y, int device_poi
     TLR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return TLR_OK;
   }
-  double2 *dx = nullptr, *dy = nullptr;
-  TLR_CUDA(ctx, cudaMallocAsync(&dx, bytes, ctx->stream));
-  TLR_CUDA(ctx, cudaMallocAsync(&dy, bytes, ctx->stream));
+  // the two vectors are kept: the pool's memory went back at every
+  // synchronisation, so each call paid for its allocation again
+  if (!ctx->spmv_xy) TLR_CUDA(ctx, cudaMalloc(&ctx->spmv_xy, 2 * bytes));
+  double2 *dx = ctx->spmv_xy, *dy = dx + 5 * (size_t)ctx->nn;
   TLR_CUDA(ctx, cudaMemcpyAsync(dx, x, bytes, cudaMemcpyHostToDevice, ctx->stream));
-  int rc = run_spmv(ctx, which, dx, dy);
-  if (rc == TLR_OK) {
-    TLR_CUDA(ctx, cudaMemcpyAsync(y, dy, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-  }
-  cudaFreeAsync(dx, ctx->stream);
-  cudaFreeAsync(dy, ctx->stream);
+  const int rc = run_spmv(ctx, which, dx, dy);
+  if (rc) return rc;
+  TLR_CUDA(ctx, cudaMemcpyAsync(y, dy, bytes, cudaMemcpyDeviceToHost, ctx->stream));
   TLR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  return rc;
+  return TLR_OK;
 }
 
 size_t tlr_out_bytes(tlr_ctx *ctx, int what) {

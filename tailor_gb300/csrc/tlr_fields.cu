@@ -7,7 +7,9 @@
 // values equal a scalar CPU evaluation of the same expressions bit for bit.
 // Failure flags follow the reference's collective checks; diagnostics use
 // deterministic two-pass reductions (block partials, then one ordered sum).
+#include <algorithm>
 #include <cfloat>
+#include <cstring>
 
 #include "tlr_internal.h"
 
@@ -199,7 +201,9 @@ __global__ void k_baseflow_prep(int nn, const double *__restrict__ base_c,
   if ((threadIdx.x & 31) == 0) atomic_max_d(red + RD_BFIM, imax);
 }
 
-// 25 physical derivatives per node (BaseFlowDerivatives.cpp:100-213).
+// 25 physical derivatives per node (BaseFlowDerivatives.cpp:100-213), a thread
+// per node and field (blockIdx.y): the five fields in one thread were a chain
+// of 500 dependent taps (82 us at 60 x 32).
 __global__ void k_derivatives(int ny, int nz, DevRule xi, DevRule eta,
                               const double *__restrict__ base,
                               const double *__restrict__ met,
@@ -217,7 +221,8 @@ __global__ void k_derivatives(int ny, int nz, DevRule xi, DevRule eta,
   const double *xw1 = xi.w1 + i * xi.s, *xw2 = xi.w2 + i * xi.s;
   const int *eoff = eta.off + j * eta.s;
   const double *ew1 = eta.w1 + j * eta.s, *ew2 = eta.w2 + j * eta.s;
-  for (int f = 0; f < 5; ++f) {
+  {
+    const int f = blockIdx.y;
     const double *v = base + f * (size_t)nn;
     double vx = 0.0, ve = 0.0, vxx = 0.0, vee = 0.0, vxe = 0.0;
     for (int s = 0; s < xi.s; ++s) {
@@ -249,72 +254,80 @@ __global__ void k_derivatives(int ny, int nz, DevRule xi, DevRule eta,
     for (int d = 0; d < 5; ++d) ok = ok && finite(out[d]);
     if (!ok) {
       atomicMax(status + ST_DERIV, 1);
-      continue;
+      return;
     }
 #pragma unroll
     for (int d = 0; d < 5; ++d) der[(d * 5 + f) * (size_t)nn + n] = out[d];
   }
 }
 
-// Sum of squares of ncomp SoA planes: block partials, then ordered sums.
-__global__ void k_sq_partial(int nn, int ncomp, const double *__restrict__ v,
-                             double *__restrict__ partial) {
-  __shared__ double sh[32];
-  for (int c = 0; c < ncomp; ++c) {
-    double s = 0.0;
-    for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < nn;
-         n += gridDim.x * blockDim.x) {
-      const double x = v[c * (size_t)nn + n];
-      s += x * x;
-    }
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double t = 0.0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += sh[w];
-      partial[blockIdx.x * ncomp + c] = t;
-    }
-    __syncthreads();
+// out[c] = the norm of SoA plane c = blockIdx.y: per-CTA partial sums, added
+// in CTA order (one warp, strided) by the plane's last CTA
+__global__ void __launch_bounds__(256)
+    k_plane_norms(int nn, const double *__restrict__ v, double *__restrict__ partial,
+                  double *__restrict__ out, int *__restrict__ ctr) {
+  __shared__ double sh[8];
+  __shared__ bool last;
+  const int c = blockIdx.y;
+  double s = 0.0;
+  for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < nn; n += gridDim.x * blockDim.x) {
+    const double x = v[c * (size_t)nn + n];
+    s = fma(x, x, s);
   }
-}
-
-__global__ void k_sq_final(int nblocks, int ncomp, const double *partial,
-                           double *out) {
-  const int c = threadIdx.x;
-  if (c >= ncomp) return;
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+  __syncthreads();
+  double *part = partial + c * gridDim.x;
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int w = 0; w < 8; ++w) t += sh[w];
+    part[blockIdx.x] = t;
+    __threadfence();
+    last = atomicAdd(ctr + c, 1) == (int)gridDim.x - 1;
+    if (last) ctr[c] = 0;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!last || threadIdx.x >= 32) return;
   double t = 0.0;
-  for (int b = 0; b < nblocks; ++b) t += partial[b * ncomp + c];
-  out[c] = sqrt(t);
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += 32) t += __ldcg(part + b);
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (threadIdx.x == 0) out[c] = sqrt(t);
 }
 
-int norms(tlr_ctx *ctx, const double *planes, int ncomp, double *host_out) {
-  const int blocks = ctx->partial_blocks;
-  { k_sq_partial<<<blocks, 256, 0, ctx->stream>>>(ctx->nn, ncomp, planes,
-                                                ctx->partial); count_launches(); }
-  { k_sq_final<<<1, 32, 0, ctx->stream>>>(blocks, ncomp, ctx->partial,
-                                        ctx->partial + blocks * 32); count_launches(); }
-  TLR_CUDA(ctx, cudaMemcpyAsync(host_out, ctx->partial + blocks * 32,
-                                sizeof(double) * ncomp, cudaMemcpyDeviceToHost,
-                                ctx->stream));
-  TLR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+// the planes' norms into ctx->pin (PIN_NORMS), without a synchronisation
+int norms_async(tlr_ctx *ctx, const double *planes, int ncomp) {
+  int rc = pinned_words(ctx);
+  if (!rc) rc = arrival_counters(ctx, ncomp);
+  if (rc) return rc;
+  // partial sums: ncomp x blocks of the 64 x partial_blocks words
+  const int blocks = std::max(1, std::min(ctx->partial_blocks, blocks_for(ctx->nn, 256)));
+  { k_plane_norms<<<dim3(blocks, ncomp), 256, 0, ctx->stream>>>(
+      ctx->nn, planes, ctx->partial, ctx->pin + PIN_NORMS, ctx->kv_ctr); count_launches(); }
+  TLR_CUDA(ctx, cudaGetLastError());
   return TLR_OK;
 }
 
+// status words and reductions through pinned memory; synchronises
 int read_status(tlr_ctx *ctx, int *st, double *red) {
-  TLR_CUDA(ctx, cudaMemcpyAsync(st, ctx->status, sizeof(int) * ST_COUNT,
+  TLR_CUDA(ctx, cudaMemcpyAsync(ctx->pin + PIN_STATUS, ctx->status, sizeof(int) * ST_COUNT,
                                 cudaMemcpyDeviceToHost, ctx->stream));
-  TLR_CUDA(ctx, cudaMemcpyAsync(red, ctx->red, sizeof(double) * RD_COUNT,
+  TLR_CUDA(ctx, cudaMemcpyAsync(ctx->pin + PIN_RED, ctx->red, sizeof(double) * RD_COUNT,
                                 cudaMemcpyDeviceToHost, ctx->stream));
   TLR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  memcpy(st, ctx->pin + PIN_STATUS, sizeof(int) * ST_COUNT);
+  memcpy(red, ctx->pin + PIN_RED, sizeof(double) * RD_COUNT);
   return TLR_OK;
 }
 
 int reset_status(tlr_ctx *ctx) {
-  double init[RD_COUNT] = {DBL_MAX, -DBL_MAX, 0, 0, 0, 0, 0, 0};
+  const int rc = pinned_words(ctx);
+  if (rc) return rc;
+  const double init[RD_COUNT] = {DBL_MAX, -DBL_MAX, 0, 0, 0, 0, 0, 0};
+  memcpy(ctx->pin + PIN_RED, init, sizeof(init));  // the last stage has synchronised
   TLR_CUDA(ctx, cudaMemsetAsync(ctx->status, 0, sizeof(int) * ST_COUNT,
                                 ctx->stream));
-  TLR_CUDA(ctx, cudaMemcpyAsync(ctx->red, init, sizeof(init),
+  TLR_CUDA(ctx, cudaMemcpyAsync(ctx->red, ctx->pin + PIN_RED, sizeof(init),
                                 cudaMemcpyHostToDevice, ctx->stream));
   return TLR_OK;
 }
@@ -330,6 +343,11 @@ int run_metrics(tlr_ctx *ctx, tlr_metric_diag *diag) {
   { k_metrics_first<<<blocks_for(nn, kNodeThreads), kNodeThreads, 0, ctx->stream>>>(
       ctx->ny, ctx->nz, ctx->span, ctx->xi, ctx->eta, ctx->grid_c,
       ctx->metrics, ctx->status, ctx->red); count_launches(); }
+  // the second-order metrics and the norms follow without waiting: their
+  // results do not count when the first kernel found something wrong
+  { k_metrics_second<<<blocks_for(nn, kNodeThreads), kNodeThreads, 0, ctx->stream>>>(
+      ctx->ny, ctx->nz, ctx->xi, ctx->eta, ctx->metrics, ctx->status); count_launches(); }
+  if ((rc = norms_async(ctx, ctx->metrics, 10))) return rc;
   int st[ST_COUNT];
   double red[RD_COUNT];
   if ((rc = read_status(ctx, st, red))) return rc;
@@ -358,13 +376,10 @@ int run_metrics(tlr_ctx *ctx, tlr_metric_diag *diag) {
              "is %.16g", d.max_grid_imaginary);
     return fail(ctx, TLR_ERR_COMPLEX, buf);
   }
-  { k_metrics_second<<<blocks_for(nn, kNodeThreads), kNodeThreads, 0, ctx->stream>>>(
-      ctx->ny, ctx->nz, ctx->xi, ctx->eta, ctx->metrics, ctx->status); count_launches(); }
-  if ((rc = read_status(ctx, st, red))) return rc;
   if (st[ST_SECOND])
     return fail(ctx, TLR_ERR_NONFINITE,
                 "Computed second-order metrics are not finite");
-  if ((rc = norms(ctx, ctx->metrics, 10, d.norms))) return rc;
+  memcpy(d.norms, ctx->pin + PIN_NORMS, sizeof(d.norms));
   if (diag) *diag = d;
   return TLR_OK;
 }
@@ -377,15 +392,16 @@ int run_derivatives(tlr_ctx *ctx, tlr_deriv_diag *diag) {
                                 ctx->stream));
   { k_baseflow_prep<<<blocks_for(nn, kNodeThreads), kNodeThreads, 0, ctx->stream>>>(
       nn, ctx->base_c, ctx->base, ctx->status, ctx->red); count_launches(); }
-  { k_derivatives<<<blocks_for(nn, kNodeThreads), kNodeThreads, 0, ctx->stream>>>(
+  { k_derivatives<<<dim3(blocks_for(nn, kNodeThreads), 5), kNodeThreads, 0, ctx->stream>>>(
       ctx->ny, ctx->nz, ctx->xi, ctx->eta, ctx->base, ctx->metrics,
       ctx->derivs, ctx->status); count_launches(); }
+  if ((rc = norms_async(ctx, ctx->derivs, 25))) return rc;
   int st[ST_COUNT];
   double red[RD_COUNT];
   if ((rc = read_status(ctx, st, red))) return rc;
   tlr_deriv_diag d{};
   d.max_baseflow_imaginary = red[RD_BFIM];
-  if ((rc = norms(ctx, ctx->derivs, 25, d.norms))) return rc;
+  memcpy(d.norms, ctx->pin + PIN_NORMS, sizeof(d.norms));
   if (diag) *diag = d;
   if (st[ST_STENCIL])
     return fail(ctx, TLR_ERR_STENCIL,

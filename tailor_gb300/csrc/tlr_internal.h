@@ -110,6 +110,9 @@ struct tlr_ctx {
   int partial_blocks = 0;
   int *kv_ctr = nullptr;     // arrival counters of the basis reductions
   int kv_ctr_n = 0;
+  double *pin = nullptr;     // pinned host words that kernels and copies write
+  double *bc_part = nullptr;   // partial sums of the boundary stage's norm
+  double2 *spmv_xy = nullptr;  // operand and result of host-array products
   int *bc_modes = nullptr;   // [nz][2]: incoming and neutral counts
   double *bc_cond = nullptr; // [nz]: cond(R) per far-field node
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -143,6 +146,14 @@ int run_assemble(tlr_ctx *ctx, tlr_operator_diag *diag);
 int run_bc(tlr_ctx *ctx, tlr_bc_diag *diag);
 int run_spmv(tlr_ctx *ctx, int which, const double2 *x, double2 *y);
 int frobenius(tlr_ctx *ctx, const double2 *v, long long count, double *out);
+// The same without a synchronisation: *out in device or pinned memory.
+int frobenius_async(tlr_ctx *ctx, const double2 *v, long long count, double *out);
+// Zeroed counters (at least `count`) of kernels whose last CTA finishes a
+// reduction and clears its counter again.
+int arrival_counters(tlr_ctx *ctx, int count);
+// ctx->pin: kPinWords doubles (PIN_*), allocated on first use
+int pinned_words(tlr_ctx *ctx);
+enum : int { PIN_STATUS = 0, PIN_RED = 8, PIN_NORMS = 16, kPinWords = 64 };
 // r = y - (A_bc - sigma B_bc) w with A_bc w in float-float arithmetic on the
 // FP32 pipe (about 48-bit significands); builds ctx->aff on first use.
 int residual_ff(tlr_ctx *ctx, const double2 *y, const double2 *w, double sr, double si,

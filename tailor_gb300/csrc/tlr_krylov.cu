@@ -750,6 +750,9 @@ int run_solve(tlr_ctx *ctx, const tlr_solve_opts *opts, double *lambda,
     return fail(ctx, TLR_ERR_ARG, "ring_slack_percent must lie in [100, 1000]");
   const int rslack = o.ring_slack_percent ? o.ring_slack_percent : kRingSlackDefault;
 
+  // counters for every basis size, so that captured norms keep their address
+  if (const int rc = arrival_counters(ctx, ncv / 8 + 2)) return rc;
+
   // factorisation (reused when sigma, precision and Schur kernel are unchanged)
   Factor *F = ctx->factor;
   if (F && (F->prec != prec || F->sigma_re != sigma.real() || F->sigma_im != sigma.imag() ||

@@ -269,7 +269,6 @@ int row_blocks(tlr_ctx *ctx, long long n) {
 
 }  // namespace
 
-// arrival counters of the last-CTA reductions, one per column group
 int arrival_counters(tlr_ctx *ctx, int count) {
   if (ctx->kv_ctr && ctx->kv_ctr_n >= count) return TLR_OK;
   TLR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -279,6 +278,12 @@ int arrival_counters(tlr_ctx *ctx, int count) {
   TLR_CUDA(ctx, cudaMalloc(&ctx->kv_ctr, sizeof(int) * cap));
   TLR_CUDA(ctx, cudaMemsetAsync(ctx->kv_ctr, 0, sizeof(int) * cap, ctx->stream));
   ctx->kv_ctr_n = cap;
+  return TLR_OK;
+}
+
+int pinned_words(tlr_ctx *ctx) {
+  if (!ctx->pin)
+    TLR_CUDA(ctx, cudaHostAlloc(&ctx->pin, sizeof(double) * kPinWords, cudaHostAllocDefault));
   return TLR_OK;
 }
 

@@ -65,9 +65,12 @@ __global__ void __launch_bounds__(32 * kRowsPerCta)
   if (active && c == 0) y[(size_t)row * 5 + lane / 5] = make_double2(sr, si);
 }
 
-__global__ void k_sq2_partial(long long n, const double2 *__restrict__ v,
-                              double *__restrict__ partial) {
+// *out = ||v||: per-CTA partial sums, added in CTA order (one warp, strided) by
+// the CTA that finishes last
+__global__ void k_sq2(long long n, const double2 *__restrict__ v, double *__restrict__ partial,
+                      double *__restrict__ out, int *__restrict__ ctr) {
   __shared__ double sh[32];
+  __shared__ bool last;
   double s = 0.0;
   for (long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x; x < n;
        x += (long long)gridDim.x * blockDim.x) {
@@ -81,14 +84,17 @@ __global__ void k_sq2_partial(long long n, const double2 *__restrict__ v,
     double t = 0.0;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += sh[w];
     partial[blockIdx.x] = t;
+    __threadfence();
+    last = atomicAdd(ctr, 1) == (int)gridDim.x - 1;
+    if (last) *ctr = 0;
+    __threadfence();
   }
-}
-
-__global__ void k_sum_sqrt(int n, const double *partial, double *out) {
-  if (threadIdx.x != 0) return;
+  __syncthreads();
+  if (!last || threadIdx.x >= 32) return;
   double t = 0.0;
-  for (int b = 0; b < n; ++b) t += partial[b];
-  *out = sqrt(t);
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += 32) t += __ldcg(partial + b);
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (threadIdx.x == 0) *out = sqrt(t);
 }
 
 }  // namespace
@@ -361,18 +367,22 @@ int residual_ff(tlr_ctx *ctx, const double2 *y, const double2 *w, double sr, dou
 int vec_norm_async(tlr_ctx *ctx, const double2 *v, long long count, double *scratch,
                    double *out) {
   const int blocks = ctx->partial_blocks;
-  { k_sq2_partial<<<blocks, 256, 0, ctx->stream>>>(count, v, scratch); count_launches(); }
-  { k_sum_sqrt<<<1, 32, 0, ctx->stream>>>(blocks, scratch, out); count_launches(); }
+  if (!ctx->kv_ctr) return fail(ctx, TLR_ERR_ARG, "reduction counters not allocated");
+  { k_sq2<<<blocks, 256, 0, ctx->stream>>>(count, v, scratch, out, ctx->kv_ctr); count_launches(); }
   return TLR_OK;
 }
 
+int frobenius_async(tlr_ctx *ctx, const double2 *v, long long count, double *out) {
+  const int rc = arrival_counters(ctx, 1);
+  return rc ? rc : vec_norm_async(ctx, v, count, ctx->partial, out);
+}
+
 int frobenius(tlr_ctx *ctx, const double2 *v, long long count, double *out) {
-  const int blocks = ctx->partial_blocks;
-  { k_sq2_partial<<<blocks, 256, 0, ctx->stream>>>(count, v, ctx->partial); count_launches(); }
-  { k_sum_sqrt<<<1, 32, 0, ctx->stream>>>(blocks, ctx->partial, ctx->partial + blocks); count_launches(); }
-  TLR_CUDA(ctx, cudaMemcpyAsync(out, ctx->partial + blocks, sizeof(double),
-                                cudaMemcpyDeviceToHost, ctx->stream));
+  int rc = pinned_words(ctx);
+  if (!rc) rc = frobenius_async(ctx, v, count, ctx->pin + PIN_NORMS);
+  if (rc) return rc;
   TLR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  *out = ctx->pin[PIN_NORMS];
   return TLR_OK;
 }
 
