@@ -1167,6 +1167,159 @@ __global__ void __launch_bounds__(256, (SW <= 256 && sizeof(C) == 8) ? 3 : 1)
   }
 }
 
+// ---- complex128 steps --------------------------------------------------------
+// A step near the root has little work, so its time is a chain of latencies:
+// with 32-row CTAs (16 K FMAs each at two per cycle and SM, 4 us), sixteen
+// columns in sequence per thread and two dependent loads before the factor's
+// addresses are known, a step took 8 us however few its CTAs.  Here a CTA has
+// eight rows and a thread four columns of one row (row lane % 8, columns 4 g ..
+// 4 g + 3 of group g = 4 warp + lane / 8); the sums are folded as a tree: four
+// groups by two exchanges, eight warps through shared memory.  k_wave sums a
+// complex128 row in the same order.  A solve at 60 x 32: 0.60 -> 0.45 ms; at
+// 150 x 64, bound by the FP64 pipe's rate, 2.04 ms either way.
+constexpr int kDRows = 8;
+
+__device__ __forceinline__ double2 shfl_xor_c(double2 v, int o) {
+  return make_double2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
+}
+__device__ __forceinline__ double2 tree8(const double2 *s, int stride) {
+  return cadd(cadd(cadd(s[0], s[stride]), cadd(s[2 * stride], s[3 * stride])),
+              cadd(cadd(s[4 * stride], s[5 * stride]), cadd(s[6 * stride], s[7 * stride])));
+}
+// this warp's four groups: (s0 + s1) + (s2 + s3) in every lane of the row
+__device__ __forceinline__ double2 tree_groups(double2 s) {
+  s = cadd(s, shfl_xor_c(s, 8));
+  return cadd(s, shfl_xor_c(s, 16));
+}
+
+__global__ void __launch_bounds__(256)
+    k_blk_update_d(const StepFront *__restrict__ sf, int b, int backward,
+                   const double2 *__restrict__ pool, double2 *__restrict__ work,
+                   const int *__restrict__ nodes, double2 *__restrict__ x) {
+  using C = double2;
+  constexpr int SW = 128;
+  __shared__ C red[8][kDRows];
+  pdl_launch_dependents();
+  const StepFront f = sf[blockIdx.y];
+  const int b0 = b * SW, b1 = min(f.p, b0 + SW), nb = b1 - b0;
+  const int lo = backward ? 0 : b1, hi = backward ? b0 : f.m;
+  const int r0 = lo + blockIdx.x * kDRows;
+  if (nb <= 0 || r0 >= hi) return;
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const int lr = lane % kDRows, q0 = 4 * (4 * wp + lane / kDRows), r = r0 + lr;
+  const bool ok = r < hi;
+  const C *F = pool + f.off + (long long)(b0 + q0) * f.m + r;
+  C fv[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    fv[k] = ok && q0 + k < nb ? F[(long long)k * f.m] : czero<C>();
+  pdl_wait();
+  C *t = work + f.toff;
+  C tv[4], v = czero<C>();
+#pragma unroll
+  for (int k = 0; k < 4; ++k) tv[k] = q0 + k < nb ? __ldcg(t + b0 + q0 + k) : czero<C>();
+  if (ok && threadIdx.x < kDRows) v = __ldcg(t + r);
+  C acc = czero<C>();
+#pragma unroll
+  for (int k = 0; k < 4; ++k) acc = cfma(acc, fv[k], tv[k]);
+  acc = tree_groups(acc);
+  if (lane < kDRows) red[wp][lane] = acc;
+  __syncthreads();
+  if (ok && threadIdx.x < kDRows) {
+    v = csub(v, tree8(&red[0][lr], kDRows));
+    t[r] = v;
+    if (backward && r >= b0 - SW) x[(long long)nodes[f.node_off + r / 5] * 5 + r % 5] = v;
+  }
+}
+
+// Border product of the backward pass: partial[front][chunk][i] over 128
+// columns of the border, eight rows per CTA.
+constexpr int kBCD = 128;
+__global__ void __launch_bounds__(256)
+    k_border_gemv_d(const StepFront *__restrict__ sf, const double2 *__restrict__ pool,
+                    const int *__restrict__ nodes, const double2 *__restrict__ x,
+                    double2 *__restrict__ partial, int nck, int pmax) {
+  using C = double2;
+  __shared__ C xs[kBCD];
+  __shared__ C red[8][kDRows];
+  pdl_launch_dependents();
+  const int fq = blockIdx.z;
+  const StepFront f = sf[fq];
+  const int r0 = blockIdx.x * kDRows, c0 = f.p + blockIdx.y * kBCD;
+  if (r0 >= f.p || c0 >= f.m) return;
+  const int nc = min(kBCD, f.m - c0);
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const int lr = lane % kDRows, q0 = 4 * (4 * wp + lane / kDRows), r = r0 + lr;
+  const bool ok = r < f.p;
+  int id = -1;
+  if (threadIdx.x < nc) {
+    const int c = c0 + threadIdx.x;
+    id = nodes[f.node_off + c / 5] * 5 + c % 5;
+  }
+  const C *F = pool + f.off + (long long)(c0 + q0) * f.m + r;
+  C fv[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    fv[k] = ok && q0 + k < nc ? F[(long long)k * f.m] : czero<C>();
+  pdl_wait();
+  if (threadIdx.x < kBCD) xs[threadIdx.x] = id >= 0 ? __ldcg(x + id) : czero<C>();
+  __syncthreads();
+  C acc = czero<C>();
+#pragma unroll
+  for (int k = 0; k < 4; ++k) acc = cfma(acc, fv[k], xs[q0 + k]);
+  acc = tree_groups(acc);
+  if (lane < kDRows) red[wp][lane] = acc;
+  __syncthreads();
+  if (ok && threadIdx.x < kDRows)
+    partial[((long long)fq * nck + blockIdx.y) * pmax + r] = tree8(&red[0][lr], kDRows);
+}
+
+// Start of a front's backward pass (k_bwd_start), eight rows per CTA; a row's
+// border partial sums are shared between its 32 threads.
+__global__ void __launch_bounds__(256)
+    k_bwd_start_d(const StepFront *__restrict__ sf, const double2 *__restrict__ dmat,
+                  const double2 *__restrict__ work, double2 *__restrict__ work2,
+                  const double2 *__restrict__ partial, int nck, int pmax,
+                  const int *__restrict__ nodes, double2 *__restrict__ x) {
+  using C = double2;
+  constexpr int SW = 128;
+  __shared__ C red[8][kDRows];
+  pdl_launch_dependents();
+  const int fq = blockIdx.y;
+  const StepFront f = sf[fq];
+  const int blk = blockIdx.x / (SW / kDRows), part = blockIdx.x % (SW / kDRows);
+  const int b0 = blk * SW, nb = min(SW, f.p - b0);
+  const int rr0 = part * kDRows;
+  if (nb <= 0 || rr0 >= nb) return;
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const int lr = lane % kDRows, g = 4 * wp + lane / kDRows, q0 = 4 * g;
+  const int rr = rr0 + lr, r = b0 + rr;
+  const bool ok = rr < nb;
+  const C *Dm = dmat + f.inv + (long long)blk * SW * SW + (long long)q0 * nb + rr;
+  C dv[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) dv[k] = ok && q0 + k < nb ? Dm[(long long)k * nb] : czero<C>();
+  pdl_wait();
+  const C *z = work + f.toff + b0 + q0;
+  C acc = czero<C>();
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    acc = cfma(acc, dv[k], q0 + k < nb ? __ldcg(z + k) : czero<C>());
+  if (ok && f.m > f.p) {  // chunks g, g + 32, ... of the border
+    const int nchf = (f.m - f.p + kBCD - 1) / kBCD;
+    const C *pp = partial + (long long)fq * nck * pmax + r;
+    for (int k = g; k < nchf; k += 32) acc = csub(acc, __ldcg(pp + (long long)k * pmax));
+  }
+  acc = tree_groups(acc);
+  if (lane < kDRows) red[wp][lane] = acc;
+  __syncthreads();
+  if (ok && threadIdx.x < kDRows) {
+    const C w = tree8(&red[0][lr], kDRows);
+    work2[f.toff + r] = w;
+    if (b0 + SW >= f.p) x[(long long)nodes[f.node_off + r / 5] * 5 + r % 5] = w;
+  }
+}
+
 // ---- dependency-driven level solve ---------------------------------------
 // A level whose fronts have several diagonal blocks needs, step by step,
 // one launch per block, and the top of the elimination tree is a chain of
@@ -1278,12 +1431,28 @@ __global__ void __launch_bounds__(256, (SW <= 256 && sizeof(C) == 8) ? 2 : 1)
       }
       for (int q = threadIdx.x; q < nb; q += blockDim.x) vs[q] = __ldcg(t + b0 + q);
       __syncthreads();
-      const C acc = dot_cols<C, kQ>(fv, vs + q0, full, nb - q0);
-      red[wp][lane] = acc;
+      if constexpr (sizeof(C) == sizeof(double2)) {
+        // k_blk_update_d's order: groups of four columns, then a tree
+        C s4[4];
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          s4[h] = czero<C>();
+#pragma unroll
+          for (int k = 4 * h; k < 4 * h + 4; ++k)
+            s4[h] = cfma(s4[h], fv[k], q0 + k < nb ? vs[q0 + k] : czero<C>());
+        }
+        red[wp][lane] = cadd(cadd(s4[0], s4[1]), cadd(s4[2], s4[3]));
+      } else {
+        red[wp][lane] = dot_cols<C, kQ>(fv, vs + q0, full, nb - q0);
+      }
       __syncthreads();
       if (wp == 0 && rowok) {
+        if constexpr (sizeof(C) == sizeof(double2)) {
+          v = csub(v, tree8(&red[0][lane], 32));
+        } else {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) v = csub(v, red[k][lane]);
+          for (int k = 0; k < 8; ++k) v = csub(v, red[k][lane]);
+        }
       }
       __syncthreads();  // vs and red are reused
     }
@@ -1315,52 +1484,12 @@ __global__ void __launch_bounds__(256, (SW <= 256 && sizeof(C) == 8) ? 2 : 1)
   }
 }
 
-// Backward border product, pass 1: partial[front][chunk][i] = sum over a
-// kBC-column chunk of the border of U'(i, c) x[unknown of border row c],
-// pivot rows i (the border unknowns belong to ancestors, already solved).
-// CTA = 32 rows x 8 warps of kBC/8 columns.
 constexpr int kBC = 256;
 
-template <class C>
-__global__ void __launch_bounds__(256)
-    k_border_gemv(const int *__restrict__ fl, const C *__restrict__ pool,
-                  const DevFront *__restrict__ fr, const int *__restrict__ nodes,
-                  const C *__restrict__ x, double2 *__restrict__ partial, int nck, int pmax) {
-  __shared__ C xs[kBC];
-  __shared__ C red[8][32];
-  pdl_launch_dependents();
-  pdl_wait();
-  const int fq = blockIdx.z;
-  const DevFront f = fr[fl[fq]];
-  const int r0 = blockIdx.x * 32;
-  const int c0 = f.p + blockIdx.y * kBC;
-  if (r0 >= f.p || c0 >= f.m) return;
-  const int nc = min(kBC, f.m - c0);
-  for (int k = threadIdx.x; k < nc; k += blockDim.x) {
-    const int c = c0 + k;
-    xs[k] = x[(long long)nodes[f.node_off + c / 5] * 5 + c % 5];
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-  const int r = r0 + lane;
-  C acc = czero<C>();
-  if (r < f.p) {
-    const int ka = wp * (kBC / 8), kb = min(nc, ka + kBC / 8);
-    const C *F = pool + f.off + (long long)c0 * f.m + r;
-#pragma unroll 8
-    for (int k = ka; k < kb; ++k) acc = cfma(acc, F[(long long)k * f.m], xs[k]);
-  }
-  red[wp][lane] = acc;
-  __syncthreads();
-  if (wp == 0 && r < f.p) {
-    C v = czero<C>();
-#pragma unroll
-    for (int k = 0; k < 8; ++k) v = cadd(v, red[k][lane]);
-    partial[((long long)fq * nck + blockIdx.y) * pmax + r] = to64(v);
-  }
-}
-
-// The same border product for complex64 factors, with the warp's kBC/8
+// Backward border product, pass 1 (complex64): partial[front][chunk][i] = sum
+// over a kBC-column chunk of the border of U'(i, c) x[unknown of border row
+// c], pivot rows i (the border unknowns belong to ancestors, already solved).
+// CTA = 32 rows x 8 warps of kBC/8 columns, with the warp's kBC/8
 // columns loaded before the programmatic-launch wait (the factor does not
 // depend on earlier kernels of the solve) and summed in the same order.
 __global__ void __launch_bounds__(256, 3)
@@ -2068,7 +2197,8 @@ int Factor::setup(tlr_ctx *ctx, int precision, int leaf, int solve_block, int pa
       L.pmax = std::max(L.pmax, f.p);
       L.bmax = std::max(L.bmax, f.m - f.p);
     }
-    L.nck_b = std::max(1, (L.bmax + kBC - 1) / kBC);
+    const int bc = prec == 0 ? kBCD : kBC;
+    L.nck_b = std::max(1, (L.bmax + bc - 1) / bc);
     L.blk_nf.clear();
     L.fwd_rows.clear();
     for (int b = 0; b * sw < L.pmax; ++b) {
@@ -2208,6 +2338,19 @@ int Factor::setup(tlr_ctx *ctx, int precision, int leaf, int solve_block, int pa
       ((rc = alloc((void **)&tc_planes, oz_bytes)) ||
        (rc = alloc((void **)&d_rowexp, sizeof(int) * kOzPanel * oz_fronts))))
     return rc;
+  if (prec == 0) {
+    std::vector<StepFront> sf;
+    for (auto &L : levels) {
+      L.sf_off = (int)sf.size();
+      for (int q = 0; q < L.nfronts; ++q) {
+        const int t = sched[L.fronts_off + q];
+        sf.push_back({df[t].off, df[t].toff, inv_off[t], df[t].p, df[t].m, df[t].node_off, 0});
+      }
+    }
+    if ((rc = alloc((void **)&d_sfronts, sf.size() * sizeof(StepFront)))) return rc;
+    TLR_CUDA(ctx, cudaMemcpy(d_sfronts, sf.data(), sf.size() * sizeof(StepFront),
+                             cudaMemcpyHostToDevice));
+  }
   partial_stride = std::max(partial_elems, 1LL);
   TLR_CUDA(ctx, cudaMemcpy(d_inv_off, inv_off.data(), nf * sizeof(long long),
                            cudaMemcpyHostToDevice));
@@ -2338,7 +2481,9 @@ void Factor::release() {
   cudaFree(d_phases); cudaFree(d_barrier); cudaFree(d_solve_err); cudaFree(tc_planes);
   cudaFree(d_wave_tiles); cudaFree(d_wave_ctr); cudaFree(d_ltiles_tc); cudaFree(d_utiles_tc);
   cudaFree(d_rowexp);
+  cudaFree(d_sfronts);
   d_rowexp = nullptr;
+  d_sfronts = nullptr;
   cudaFree(d_inv_jobs); cudaFree(d_inv_prefix); cudaFree(inv_planes); cudaFree(d_gtiles);
   cudaFree(d_items); cudaFree(d_uidx); cudaFree(d_gsrc); cudaFree(split_part); cudaFree(split_ctr);
   d_inv_jobs = nullptr;
@@ -2587,8 +2732,8 @@ int Factor::factor(tlr_ctx *ctx, double sr, double si, double tiny) {
 template <class C, int SW>
 int Factor::solve_impl(tlr_ctx *ctx, void *xv) {
   cudaStream_t st = ctx->stream;
-  // programmatic dependent launch pays for the complex64 solve (about 7% at
-  // 200 x 128) but not for the register-heavier complex128 kernels
+  // programmatic dependent launch pays for the complex64 block steps (about 7%
+  // at 200 x 128) but not for complex128 (0.50 against 0.45 ms at 60 x 32)
   const bool pdl = sizeof(C) == sizeof(float2);
   const C *P = static_cast<const C *>(pool);
   C *W = static_cast<C *>(work);
@@ -2597,6 +2742,7 @@ int Factor::solve_impl(tlr_ctx *ctx, void *xv) {
   for (size_t h = 0; h < levels.size(); ++h) {
     const Level &L = levels[h];
     const int *fl = d_sched + L.fronts_off;
+    [[maybe_unused]] const StepFront *sf = d_sfronts + L.sf_off;
     // the first kernel follows a copy (or an event) node, not a kernel: no
     // programmatic edge for it
     TLR_CUDA(ctx, launch_pdl(pdl && h > 0, k_sgather<C>, dim3(blocks_for(L.max_m, 128), L.nfronts), dim3(128),
@@ -2615,9 +2761,13 @@ int Factor::solve_impl(tlr_ctx *ctx, void *xv) {
     for (int b = 0; b < (int)L.blk_nf.size(); ++b) {
       const int rows = L.fwd_rows[b];
       if (rows > 0) {
-        TLR_CUDA(ctx, launch_pdl(pdl, k_blk_update<C, SW>, dim3(blocks_for(rows, 32), L.blk_nf[b]),
-                                 dim3(256), st, fl, b, 0, P, (const DevFront *)d_fronts, W,
-                                 (const int *)d_nodes, x));
+        if constexpr (sizeof(C) == sizeof(double2))
+          TLR_CUDA(ctx, launch_pdl(pdl, k_blk_update_d, dim3(blocks_for(rows, kDRows), L.blk_nf[b]),
+                                   dim3(256), st, sf, b, 0, P, W, (const int *)d_nodes, x));
+        else
+          TLR_CUDA(ctx, launch_pdl(pdl, k_blk_update<C, SW>,
+                                   dim3(blocks_for(rows, 32), L.blk_nf[b]), dim3(256), st, fl, b,
+                                   0, P, (const DevFront *)d_fronts, W, (const int *)d_nodes, x));
         count_launches();
       }
     }
@@ -2625,6 +2775,7 @@ int Factor::solve_impl(tlr_ctx *ctx, void *xv) {
   for (int h = (int)levels.size() - 1; h >= 0; --h) {
     const Level &L = levels[h];
     const int *fl = d_sched + L.fronts_off;
+    [[maybe_unused]] const StepFront *sf = d_sfronts + L.sf_off;
     if (L.bmax > 0) {
       const dim3 g(blocks_for(L.pmax, 32), L.nck_b, L.nfronts);
       if constexpr (sizeof(C) == sizeof(float2))
@@ -2632,17 +2783,25 @@ int Factor::solve_impl(tlr_ctx *ctx, void *xv) {
                                  (const DevFront *)d_fronts, (const int *)d_nodes, (const C *)x,
                                  d_partial, L.nck_b, L.pmax));
       else
-        TLR_CUDA(ctx, launch_pdl(pdl, k_border_gemv<C>, g, dim3(256), st, fl, P,
-                                 (const DevFront *)d_fronts, (const int *)d_nodes, (const C *)x,
-                                 d_partial, L.nck_b, L.pmax));
+        TLR_CUDA(ctx, launch_pdl(pdl, k_border_gemv_d,
+                                 dim3(blocks_for(L.pmax, kDRows), L.nck_b, L.nfronts), dim3(256),
+                                 st, sf, P, (const int *)d_nodes, (const C *)x, d_partial, L.nck_b,
+                                 L.pmax));
       count_launches();
     }
-    TLR_CUDA(ctx, launch_pdl(pdl, k_bwd_start<C, SW>,
-                             dim3((unsigned)L.blk_nf.size() * (SW / 32), L.nfronts), dim3(256), st,
-                             fl, (const DevFront *)d_fronts, (const long long *)d_inv_off,
-                             static_cast<const C *>(dmat), (const C *)W, W2,
-                             (const double2 *)d_partial, L.nck_b, L.pmax, (const int *)d_nodes,
-                             x));
+    if constexpr (sizeof(C) == sizeof(double2))
+      TLR_CUDA(ctx, launch_pdl(pdl, k_bwd_start_d,
+                               dim3((unsigned)L.blk_nf.size() * (SW / kDRows), L.nfronts),
+                               dim3(256), st, sf, static_cast<const C *>(dmat), (const C *)W, W2,
+                               (const double2 *)d_partial, L.nck_b, L.pmax, (const int *)d_nodes,
+                               x));
+    else
+      TLR_CUDA(ctx, launch_pdl(pdl, k_bwd_start<C, SW>,
+                               dim3((unsigned)L.blk_nf.size() * (SW / 32), L.nfronts), dim3(256),
+                               st, fl, (const DevFront *)d_fronts, (const long long *)d_inv_off,
+                               static_cast<const C *>(dmat), (const C *)W, W2,
+                               (const double2 *)d_partial, L.nck_b, L.pmax, (const int *)d_nodes,
+                               x));
     count_launches();
     if (wave && L.wave) {
       TLR_CUDA(ctx, launch_pdl(pdl, k_wave<C, SW, true>, dim3(std::min(L.wb_n, wave_grid)),
@@ -2654,9 +2813,13 @@ int Factor::solve_impl(tlr_ctx *ctx, void *xv) {
       continue;
     }
     for (int b = (int)L.blk_nf.size() - 1; b >= 1; --b) {
-      TLR_CUDA(ctx, launch_pdl(pdl, k_blk_update<C, SW>, dim3(blocks_for(b * SW, 32), L.blk_nf[b]),
-                               dim3(256), st, fl, b, 1, P, (const DevFront *)d_fronts, W2,
-                               (const int *)d_nodes, x));
+      if constexpr (sizeof(C) == sizeof(double2))
+        TLR_CUDA(ctx, launch_pdl(pdl, k_blk_update_d, dim3(blocks_for(b * SW, kDRows), L.blk_nf[b]),
+                                 dim3(256), st, sf, b, 1, P, W2, (const int *)d_nodes, x));
+      else
+        TLR_CUDA(ctx, launch_pdl(pdl, k_blk_update<C, SW>,
+                                 dim3(blocks_for(b * SW, 32), L.blk_nf[b]), dim3(256), st, fl, b,
+                                 1, P, (const DevFront *)d_fronts, W2, (const int *)d_nodes, x));
       count_launches();
     }
   }

@@ -13,6 +13,12 @@ struct DevFront {
   int p, m, parent, node_off;
 };
 
+// What a complex128 solve step needs of a front, in the levels' order.
+struct StepFront {
+  long long off, toff, inv;  // pool, work and diagonal-block offsets
+  int p, m, node_off, pad;
+};
+
 
 constexpr int kOzPanel = 32;  // panel columns of the sliced FP64 Schur update
 
@@ -60,6 +66,7 @@ struct Step {  // one panel step of one level
 
 struct Level {
   int nfronts = 0, fronts_off = 0, max_m = 0;
+  int sf_off = 0;  // first entry of the level in Factor::d_sfronts
   int pmax = 0, bmax = 0, nck_b = 1;  // backward border GEMV chunks
   int kids[2] = {0, 0}, kids_off[2] = {0, 0}, kids_maxb[2] = {0, 0};
   long long entry_begin = 0, entry_end = 0, pool_begin = 0, pool_end = 0;
@@ -106,6 +113,7 @@ struct Factor {
   // complex128 Schur updates by exact integer slices on the tensor cores
   // (tlr_oz.cu), with 32-column panels
   bool sliced = false;
+  StepFront *d_sfronts = nullptr;  // complex128: fronts of every level in order
   int *d_rowexp = nullptr;
   int w = 32;    // panel width
   int sw = 128;  // rows of a diagonal block of the solves (128 or 256)
