@@ -208,7 +208,8 @@ struct Solver {
     for (cudaEvent_t e : brev)
       if (e) cudaEventDestroy(e);
     if (ref_exec) cudaGraphExecDestroy(ref_exec);
-    if (pipe_exec) cudaGraphExecDestroy(pipe_exec);
+    for (auto g : pipe_exec)
+      if (g) cudaGraphExecDestroy(g);
     if (bref_exec) cudaGraphExecDestroy(bref_exec);
   }
 
@@ -565,11 +566,11 @@ struct Solver {
   // of x and y, one triangular solve of three right-hand sides, the
   // corrections, the acceptance residual of x -- with one synchronisation.
   Pipe *pipe = nullptr;
-  cudaGraphExec_t pipe_exec = nullptr;
-  long long pipe_kernels = 0;
+  cudaGraphExec_t pipe_exec[2] = {};  // a step's first round, later rounds
+  long long pipe_kernels[2] = {};
   float2 *pipe_rhs() const { return static_cast<float2 *>(F->vec_m); }
 
-  int build_pipe_graph(double2 *x) {
+  int build_pipe_graph(double2 *x, int later) {
     cudaStream_t st = ctx->stream;
     for (int q = 0; q < 2; ++q)
       if (!rev[q]) TLR_CUDA(ctx, cudaEventCreate(&rev[q]));
@@ -577,9 +578,9 @@ struct Solver {
     int rc;
     {
       CaptureScope cs;
-      rc = pipe_residuals(ctx, *pipe, pipe_rhs(), F->d_solve_err);
+      rc = pipe_residuals(ctx, *pipe, pipe_rhs(), later != 0, F->d_solve_err);
       if (!rc) rc = F->enqueue_multi(ctx, 3, rev[0], rev[1]);
-      if (!rc) rc = pipe_targets(ctx, *pipe, sr, si, x, pipe_rhs(), true);
+      if (!rc) rc = pipe_targets(ctx, *pipe, sr, si, x, pipe_rhs(), 1 + later);
       if (!rc) rc = pipe_accept(ctx, *pipe, hnorm, F->d_solve_err);
     }
     cudaGraph_t g = nullptr;
@@ -590,17 +591,17 @@ struct Solver {
     }
     if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaStreamEndCapture (pipelined round)");
     size_t nn = 0;
-    pipe_kernels = 0;
+    pipe_kernels[later] = 0;
     if (cudaGraphGetNodes(g, nullptr, &nn) == cudaSuccess && nn > 0) {
       std::vector<cudaGraphNode_t> nodes(nn);
       if (cudaGraphGetNodes(g, nodes.data(), &nn) == cudaSuccess)
         for (size_t i = 0; i < nn; ++i) {
           cudaGraphNodeType t;
           if (cudaGraphNodeGetType(nodes[i], &t) == cudaSuccess && t == cudaGraphNodeTypeKernel)
-            ++pipe_kernels;
+            ++pipe_kernels[later];
         }
     }
-    const cudaError_t e2 = cudaGraphInstantiate(&pipe_exec, g, 0);
+    const cudaError_t e2 = cudaGraphInstantiate(&pipe_exec[later], g, 0);
     cudaGraphDestroy(g);
     if (e2 != cudaSuccess) return cuda_fail(ctx, e2, "cudaGraphInstantiate (pipelined round)");
     return TLR_OK;
@@ -611,7 +612,8 @@ struct Solver {
     int rc = prepare_ff(ctx);
     if (!rc) rc = F->solve_multi_prepare(ctx);
     if (!rc) rc = pipe_start(ctx, *pipe, v, x);
-    if (!rc && !pipe_exec) rc = build_pipe_graph(x);
+    for (int later = 0; later < 2 && !rc; ++later)
+      if (!pipe_exec[later]) rc = build_pipe_graph(x, later);
     return rc;
   }
 
@@ -620,8 +622,9 @@ struct Solver {
   int pipe_op(double2 *x) {
     double prev = INFINITY;
     for (int round = 0;; ++round) {
-      TLR_CUDA(ctx, cudaGraphLaunch(pipe_exec, ctx->stream));
-      count_launches(pipe_kernels);
+      const int later = round > 0;
+      TLR_CUDA(ctx, cudaGraphLaunch(pipe_exec[later], ctx->stream));
+      count_launches(pipe_kernels[later]);
       solves += 3;
       ++refine;
       if (round == 0) host_work();
@@ -642,7 +645,7 @@ struct Solver {
       // number: the classic loop with its FP64 residuals decides
       if (round >= 7 || !(nr <= 0.5 * prev)) {
         const int rc = refine_loop(pipe->b, x, ny);
-        return rc ? rc : pipe_targets(ctx, *pipe, sr, si, x, nullptr, false);
+        return rc ? rc : pipe_targets(ctx, *pipe, sr, si, x, nullptr, 0);
       }
       prev = nr;
     }

@@ -227,16 +227,20 @@ __global__ void __launch_bounds__(kSThreads, 3)
   block_sum_sq<kSThreads>(s2, bpart + blockIdx.x);
 }
 
-// x += c_x, y += c_y (with corrections), their splits and targets.
+// x += c_x, y += c_y and u = c_u, or u += c_u where the round refined u
+// (correct 1, 2; 0: none), their splits and targets; u's target is B y + sigma
+// B u, in FP32.
 __global__ void __launch_bounds__(kThreads)
     k_pipe_targets(long long n, int correct, const double2 *__restrict__ B,
                    const float2 *__restrict__ B32, double2 sg, double2 *__restrict__ x,
                    float4 *__restrict__ xyff,
                    const double2 *__restrict__ b, double2 *__restrict__ tx,
-                   double2 *__restrict__ ty, const float2 *__restrict__ rhs,
-                   float2 *__restrict__ by32) {
+                   double2 *__restrict__ ty, float2 *__restrict__ rhs,
+                   float2 *__restrict__ by32, float2 *__restrict__ u32,
+                   float2 *__restrict__ tu32) {
   __shared__ double2 xs[kRows];
   __shared__ float4 ys[kRows];
+  __shared__ float2 us[kRows];
   const int t = threadIdx.x;
   const long long i = (long long)blockIdx.x * kRows + t;
   const bool ok = t < kRows && i < n;
@@ -263,20 +267,38 @@ __global__ void __launch_bounds__(kThreads)
       x[i] = xi;
       xyff[2 * i + 1] = yi;
     }
+    float2 ui = correct ? rhs[2 * n + i] : u32[i];
+    if (correct == 2) {
+      const float2 uo = u32[i];
+      ui.x += uo.x;
+      ui.y += uo.y;
+      rhs[2 * n + i] = ui;
+    }
+    if (correct) u32[i] = ui;
     xyff[2 * i] = ff_split(xi);
     xs[t] = xi;
     ys[t] = yi;
+    us[t] = ui;
   }
   __syncthreads();
   if (ok) {
     const int q = t / 5 * 5;
     targets(i, bl, b32, xs + q, ys + q, bi, sg, tx, ty, by32);
+    float2 tu = by32[i];
+    if (sg.x != 0.0 || sg.y != 0.0) {
+      float2 bu = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int k = 0; k < 5; ++k) bu = cfma(bu, b32[k], us[q + k]);
+      tu = cfma(tu, make_float2((float)sg.x, (float)sg.y), bu);
+    }
+    tu32[i] = tu;
   }
 }
 
-// A times x (NV = 1) or x and y (NV = 2) in float-float, subtracted from
-// the targets.  Bound by reading the operator (NV = 1) and by the float-float
-// arithmetic on the FP32 pipe (NV = 2, 96 instructions per entry).  A block
+// A times x (NV = 1), x and y (NV = 2) or x, y and u (NV = 3) in float-float,
+// subtracted from the targets.  Bound by reading the operator (NV = 1) and by
+// the float-float arithmetic on the FP32 pipe (NV = 2, 96 instructions per
+// entry).  A block
 // row's blocks are contiguous, so each warp streams its rows (row gw, gw + W,
 // ...) through its own ring with bulk copies of six blocks, issued by its
 // first lane five stages ahead and across rows.  Lane 5 b + r multiplies row r
@@ -284,15 +306,16 @@ __global__ void __launch_bounds__(kThreads)
 // lane's five entries are 80 consecutive bytes (no bank conflicts), and a row
 // is summed over six lanes at its end.  Every wait is bounded: on a timeout
 // the warp raises the error flag, waits once more for its copies in flight
-// and stops.  NV = 2 writes the three right-hand sides, NV = 1 the norms
+// and stops.  NV = 2 and 3 write the three right-hand sides, NV = 1 the norms
 // out[0] = |r|, out[1] = |b| (b's partial sums: bpart).
 template <int NV>
 __global__ void __launch_bounds__(32 * kRWarps, 1)
     k_pipe_residual(int nrows, const int *__restrict__ row_ptr, const int *__restrict__ col,
                     const float4 *__restrict__ aff, const float4 *__restrict__ xyff,
                     const double2 *__restrict__ tx, const double2 *__restrict__ ty,
-                    const float2 *__restrict__ by32, float2 *__restrict__ rhs, long long n,
-                    double *__restrict__ rpart, int nb, const double *__restrict__ bpart,
+                    const float2 *__restrict__ by32, const float2 *__restrict__ u32,
+                    float2 *__restrict__ rhs, long long n, double *__restrict__ rpart, int nb,
+                    const double *__restrict__ bpart,
                     int *__restrict__ arrived, double *__restrict__ out, int *__restrict__ err) {
   extern __shared__ __align__(128) float4 ring_all[];
   __shared__ __align__(8) uint64_t full_all[kRWarps][kRStages];
@@ -340,14 +363,19 @@ __global__ void __launch_bounds__(32 * kRWarps, 1)
     int mycol = lane < 30 && k0 + lane < k1 ? col[k0 + lane] : 0;
     for (int kb = k0; kb < k1 && fine; kb += 30) {
       const int nxcol = lane < 30 && kb + 30 + lane < k1 ? col[kb + 30 + lane] : 0;
-      float4 xv[NV][5];
+      constexpr int NF = NV < 3 ? NV : 2;  // vectors held as float-float
+      float4 xv[NF][5];
+      float2 uv[NV == 3 ? 5 : 1];
       auto load_x = [&](int j) {  // stage j of this group of 30 blocks
         const int c = __shfl_sync(0xffffffffu, mycol, min(j * kRBlocks + bl, 29));
         const float4 *p = xyff + (size_t)c * 10;
 #pragma unroll
         for (int q = 0; q < 5; ++q)
 #pragma unroll
-          for (int v = 0; v < NV; ++v) xv[v][q] = p[2 * q + v];
+          for (int v = 0; v < NF; ++v) xv[v][q] = p[2 * q + v];
+        if (NV == 3)
+#pragma unroll
+          for (int q = 0; q < 5; ++q) uv[q % (NV == 3 ? 5 : 1)] = u32[(size_t)c * 5 + q];
       };
       load_x(0);
       for (int j = 0; j < 5 && kb + j * kRBlocks < k1; ++j) {
@@ -361,7 +389,11 @@ __global__ void __launch_bounds__(32 * kRWarps, 1)
           for (int q = 0; q < 5; ++q) {
             const float4 av = ap[q];
 #pragma unroll
-            for (int v = 0; v < NV; ++v) ffc_mac(s[v], av, xv[v][q]);
+            for (int v = 0; v < NF; ++v) ffc_mac(s[v], av, xv[v][q]);
+            if (NV == 3) {
+              const float2 ui = uv[q % (NV == 3 ? 5 : 1)];
+              ffc_mac(s[NV - 1], av, make_float4(ui.x, 0.f, ui.y, 0.f));
+            }
           }
         }
         __syncwarp();
@@ -390,7 +422,7 @@ __global__ void __launch_bounds__(32 * kRWarps, 1)
     if (lane < 5) {
       const size_t i = (size_t)row * 5 + rr;
 #pragma unroll
-      for (int v = 0; v < NV; ++v) {
+      for (int v = 0; v < (NV < 3 ? NV : 2); ++v) {
         const double2 av = ffc_value(s[v]), tg = v ? ty[i] : tx[i];
         const double2 r = make_double2(tg.x - av.x, tg.y - av.y);
         if (NV == 1) {
@@ -401,6 +433,11 @@ __global__ void __launch_bounds__(32 * kRWarps, 1)
         }
       }
       if (NV == 2) rhs[2 * n + i] = by32[i];
+      if (NV == 3) {  // by32: the target of u
+        const double2 au = ffc_value(s[NV - 1]);
+        const float2 tu = by32[i];
+        rhs[2 * n + i] = make_float2((float)(tu.x - au.x), (float)(tu.y - au.y));
+      }
     }
   }
   if (!fine && lane == 0) {
@@ -460,6 +497,8 @@ int pipe_alloc(tlr_ctx *ctx, Pipe &p, int ncv) {
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRSmem));
   TLR_CUDA(ctx, cudaFuncSetAttribute(k_pipe_residual<2>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRSmem));
+  TLR_CUDA(ctx, cudaFuncSetAttribute(k_pipe_residual<3>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRSmem));
   const size_t n = (size_t)p.n;
   TLR_CUDA(ctx, cudaMalloc(&p.vff, sizeof(float4) * n * (ncv + 1)));
   TLR_CUDA(ctx, cudaMalloc(&p.xyff, sizeof(float4) * 2 * n));
@@ -468,6 +507,8 @@ int pipe_alloc(tlr_ctx *ctx, Pipe &p, int ncv) {
   TLR_CUDA(ctx, cudaMalloc(&p.tx, sizeof(double2) * n));
   TLR_CUDA(ctx, cudaMalloc(&p.ty, sizeof(double2) * n));
   TLR_CUDA(ctx, cudaMalloc(&p.by32, sizeof(float2) * n));
+  TLR_CUDA(ctx, cudaMalloc(&p.u32, sizeof(float2) * n));
+  TLR_CUDA(ctx, cudaMalloc(&p.tu32, sizeof(float2) * n));
   TLR_CUDA(ctx, cudaMalloc(&p.H, sizeof(double2) * p.ldh * ncv));
   TLR_CUDA(ctx, cudaMalloc(&p.g, sizeof(float4) * 2 * p.ldh));
   TLR_CUDA(ctx, cudaMalloc(&p.bpart, sizeof(double) * shift_blocks(p)));
@@ -480,8 +521,8 @@ int pipe_alloc(tlr_ctx *ctx, Pipe &p, int ncv) {
 
 void pipe_free(Pipe &p) {
   cudaFree(p.vff); cudaFree(p.xyff); cudaFree(p.B32); cudaFree(p.b); cudaFree(p.tx);
-  cudaFree(p.ty); cudaFree(p.by32); cudaFree(p.H); cudaFree(p.g); cudaFree(p.bpart); cudaFree(p.rpart);
-  cudaFree(p.arrived);
+  cudaFree(p.ty); cudaFree(p.by32); cudaFree(p.u32); cudaFree(p.tu32); cudaFree(p.H); cudaFree(p.g);
+  cudaFree(p.bpart); cudaFree(p.rpart); cudaFree(p.arrived);
   cudaFreeHost(p.hup);
   p = Pipe();
 }
@@ -521,27 +562,32 @@ int pipe_shift(tlr_ctx *ctx, Pipe &p, int j, const double *beta, double sr, doub
   return TLR_OK;
 }
 
-int pipe_residuals(tlr_ctx *ctx, Pipe &p, float2 *rhs, int *err) {
-  { k_pipe_residual<2><<<row_blocks(p), 32 * kRWarps, kRSmem, ctx->stream>>>(
-      p.nn, ctx->row_ptr, ctx->col, ctx->aff, p.xyff, p.tx, p.ty, p.by32, rhs, p.n, nullptr, 0,
-      nullptr, nullptr, nullptr, err); count_launches(); }
+int pipe_residuals(tlr_ctx *ctx, Pipe &p, float2 *rhs, bool refine_u, int *err) {
+  if (refine_u)
+    { k_pipe_residual<3><<<row_blocks(p), 32 * kRWarps, kRSmem, ctx->stream>>>(
+        p.nn, ctx->row_ptr, ctx->col, ctx->aff, p.xyff, p.tx, p.ty, p.tu32, p.u32, rhs, p.n,
+        nullptr, 0, nullptr, nullptr, nullptr, err); count_launches(); }
+  else
+    { k_pipe_residual<2><<<row_blocks(p), 32 * kRWarps, kRSmem, ctx->stream>>>(
+        p.nn, ctx->row_ptr, ctx->col, ctx->aff, p.xyff, p.tx, p.ty, p.by32, nullptr, rhs, p.n,
+        nullptr, 0, nullptr, nullptr, nullptr, err); count_launches(); }
   TLR_CUDA(ctx, cudaGetLastError());
   return TLR_OK;
 }
 
-int pipe_targets(tlr_ctx *ctx, Pipe &p, double sr, double si, double2 *x, const float2 *rhs,
-                 bool correct) {
+int pipe_targets(tlr_ctx *ctx, Pipe &p, double sr, double si, double2 *x, float2 *rhs,
+                 int correct) {
   { k_pipe_targets<<<node_blocks(p), kThreads, 0, ctx->stream>>>(
-      p.n, correct ? 1 : 0, ctx->B, p.B32, make_double2(sr, si), x, p.xyff, p.b, p.tx, p.ty, rhs,
-      p.by32); count_launches(); }
+      p.n, correct, ctx->B, p.B32, make_double2(sr, si), x, p.xyff, p.b, p.tx, p.ty, rhs, p.by32,
+      p.u32, p.tu32); count_launches(); }
   TLR_CUDA(ctx, cudaGetLastError());
   return TLR_OK;
 }
 
 int pipe_accept(tlr_ctx *ctx, Pipe &p, double *out, int *err) {
   { k_pipe_residual<1><<<row_blocks(p), 32 * kRWarps, kRSmem, ctx->stream>>>(
-      p.nn, ctx->row_ptr, ctx->col, ctx->aff, p.xyff, p.tx, p.ty, p.by32, nullptr, p.n, p.rpart,
-      shift_blocks(p), p.bpart, p.arrived, out, err); count_launches(); }
+      p.nn, ctx->row_ptr, ctx->col, ctx->aff, p.xyff, p.tx, p.ty, p.by32, nullptr, nullptr, p.n,
+      p.rpart, shift_blocks(p), p.bpart, p.arrived, out, err); count_launches(); }
   TLR_CUDA(ctx, cudaGetLastError());
   return TLR_OK;
 }

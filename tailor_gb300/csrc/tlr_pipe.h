@@ -13,11 +13,15 @@
 // x makes the next x out of y and the next y out of u; the new x usually
 // needs one correction only.  x is accepted on the same residual as before
 // (||B v - K x|| <= 1e-12 ||B v||, A x in float-float), so a poor guess
-// costs another round and no accuracy.  Measured rounds per application:
-// 1.13 (60 x 32) to 1.51 (200 x 128, complex target; its factor contracts by
-// 3e-5 only), against three dependent solves.  A pass of a point, before and
-// after: 221 -> 161 ms at 60 x 32, 227 -> 173 ms at 100 x 50, 643 -> 594 ms at
-// 200 x 128, 1465 -> 1231 ms at 300 x 192.
+// costs another round and no accuracy.  A step's second and later rounds refine
+// u too (against B y + sigma B u in FP32), which makes the next step's y better:
+// 192 -> 175 rounds at 300 x 192, 196 -> 175 at 200 x 128, 353 -> 348 at 60 x 32.
+// Measured rounds per application: 1.12 (60 x 32), 1.16 (100 x 50), 1.32 (300 x
+// 192) and 1.35 (200 x 128, complex target; its factor contracts by 3e-5 only),
+// against three dependent solves.  A pass of a point with these applications
+// alone, before and after: 221 -> 161 ms at 60 x 32, 227 -> 173 ms at 100 x 50,
+// 643 -> 594 ms at 200 x 128, 1465 -> 1231 ms at 300 x 192; refining u took
+// another 30 of 495 ms at 200 x 128 and 50 of 1048 ms at 300 x 192.
 #pragma once
 
 #include "tlr_internal.h"
@@ -33,6 +37,7 @@ struct Pipe {
   float2 *B32 = nullptr;  // B in FP32
   double2 *b = nullptr, *tx = nullptr, *ty = nullptr;
   float2 *by32 = nullptr; // B y, the right-hand side of u
+  float2 *u32 = nullptr, *tu32 = nullptr;  // u and its target B y + sigma B u
   double2 *H = nullptr;   // (ncv + 1) x ncv projected matrix, ld ldh
   float4 *g = nullptr;    // combination coefficients, 2 x ldh
   double *bpart = nullptr, *rpart = nullptr;  // per-CTA partial sums of squares
@@ -52,12 +57,15 @@ int pipe_upload_h(tlr_ctx *ctx, Pipe &p, int l);
 // targets and right-hand side; rhs: 3 x n, its third vector holds u
 int pipe_shift(tlr_ctx *ctx, Pipe &p, int j, const double *beta, double sr, double si,
                double2 *x, double2 *vnew, const float2 *rhs);
-// rhs = the residuals of x and y, and B y
-// (err: set when a bounded wait of the kernel ran out)
-int pipe_residuals(tlr_ctx *ctx, Pipe &p, float2 *rhs, int *err);
-// x += rhs(0), y += rhs(1) (correct), and the targets of the new x and y
-int pipe_targets(tlr_ctx *ctx, Pipe &p, double sr, double si, double2 *x, const float2 *rhs,
-                 bool correct);
+// rhs = the residuals of x and y, and B y or (refine_u, in a step's second and
+// later rounds) the residual of u; err: set when a bounded wait of the kernel
+// ran out
+int pipe_residuals(tlr_ctx *ctx, Pipe &p, float2 *rhs, bool refine_u, int *err);
+// x += rhs(0), y += rhs(1), u = rhs(2) (correct 1) or u += rhs(2) (correct 2,
+// rhs(2) then holds u), and the targets of the new iterates; correct 0: the
+// targets only
+int pipe_targets(tlr_ctx *ctx, Pipe &p, double sr, double si, double2 *x, float2 *rhs,
+                 int correct);
 // out[0] = ||B v - K x||, out[1] = ||B v|| (out: pinned host memory)
 int pipe_accept(tlr_ctx *ctx, Pipe &p, double *out, int *err);
 
