@@ -66,17 +66,19 @@ __global__ void k_inv_gather(const int *__restrict__ fl, const DevFront *__restr
 
 // One work item per CTA: 32 rows (lane = row) times a range of columns (8
 // warps, consecutive shares).  Bound by reading the factor: each thread
-// streams its columns 8 at a time, the next 8 in flight while the present
-// ones are applied to all NR vectors, and the first 8 go out before the
-// programmatic-launch wait.  Eight columns keep a thread within 64 registers,
-// four CTAs per SM: 2.11 ms per three-vector solve at 300 x 192 (10 GB, 4.8
-// TB/s) against 2.20 with 16 columns and three CTAs, 2.40 with 16 warps per
-// CTA and 2.5 with four; the block steps it replaces took 3.39 ms (200 x 128:
-// 0.93 against 1.49 ms, 100 x 50: 0.21 against 0.32).  Row tiles split over several items add their
-// partial sums in item order in the item that finishes last, so results do
-// not depend on timing; per vector the arithmetic does not depend on NR.
-constexpr int kW = 8;  // warps per CTA
-constexpr int kQ = 8;  // columns a thread loads at a time
+// fetches 16 of its columns at a time, applies them to all NR vectors and
+// fetches the next 16; four CTAs per SM keep the reads going meanwhile.  The
+// first 16 go out before the programmatic-launch wait.  A three-vector solve
+// takes 1.98 ms at 300 x 192 (10 GB, 5.1 TB/s) and 0.885 ms at 200 x 128,
+// against 2.07 and 0.912 ms with two buffers of eight columns (the same 64
+// registers); 16 warps or two buffers of 16 per CTA were slower still (2.40,
+// 2.20 ms), and so were tiles copied to consecutive addresses (2.20).  The block
+// steps it replaces took 3.39 ms (200 x 128: 1.49 ms, 100 x 50: 0.32 against
+// 0.21).  Row tiles split over several items add their partial sums in item
+// order in the item that finishes last, so results do not depend on timing;
+// per vector the arithmetic does not depend on NR.
+constexpr int kW = 8;   // warps per CTA
+constexpr int kQ = 16;  // columns a thread loads at a time
 
 template <int NR>
 __global__ void __launch_bounds__(32 * kW, NR <= 4 ? 4 : 2)
@@ -147,9 +149,8 @@ __global__ void __launch_bounds__(32 * kW, NR <= 4 ? 4 : 2)
 #pragma unroll
   for (int v = 0; v < NR; ++v) acc[v] = czero<C>();
   const float4 *v4 = reinterpret_cast<const float4 *>(vs);
+#pragma unroll 1
   for (int k0 = q0; k0 < q1; k0 += kQ) {
-    C nxt[kQ];
-    load(nxt, k0 + kQ);
     const float4 *p = v4 + (k0 >> 1) * NR;
 #pragma unroll
     for (int k = 0; k < kQ; k += 2)
@@ -159,8 +160,7 @@ __global__ void __launch_bounds__(32 * kW, NR <= 4 ? 4 : 2)
         acc[v] = cfma(acc[v], cur[k], make_float2(pv.x, pv.y));
         acc[v] = cfma(acc[v], cur[k + 1], make_float2(pv.z, pv.w));
       }
-#pragma unroll
-    for (int k = 0; k < kQ; ++k) cur[k] = nxt[k];
+    load(cur, k0 + kQ);
   }
 #pragma unroll
   for (int v = 0; v < NR; ++v) red[v][wp][lane] = acc[v];
@@ -412,7 +412,7 @@ int Factor::solve_inverse(tlr_ctx *ctx, float2 *x, float2 *W, float2 *W2) {
     count_launches();
     rc = apply(L.if_off, L.if_n);
   }
-  for (int h = (int)levels.size() - 1; h >= 0 && !rc; --h) 
+  for (int h = (int)levels.size() - 1; h >= 0 && !rc; --h)
     rc = apply(levels[h].ib_off, levels[h].ib_n);
   return rc;
 }
