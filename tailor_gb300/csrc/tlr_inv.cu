@@ -12,7 +12,8 @@
 //   forward:  z = [-D N_L | D] t (rows of the pivots), t_b -= X t;
 //   backward: x = z - [N_U | Y] [z; x_b].
 // The storage is that of the factor, p (p + 2 b) entries read once per
-// solve; a solve is three launches per level (gather, forward, backward).
+// solve; a solve is one forward and one backward launch per level, and a
+// gather launch before the forward one where the level is large.
 //
 // The inversion is right-looking, block d from the last down:
 //   F(rows below d, columns left of d)  -= F(rows below d, d) F(d, columns)
@@ -35,6 +36,7 @@ namespace {
 constexpr int kSW = 256;           // diagonal block
 constexpr int kBatchTiles = 2048;  // operand tiles per batch: 1 GB of planes
 constexpr int kMaxCols = 1024;     // columns of a work item at most
+constexpr long long kSmallCols = 131072;  // columns of all items of a small level at most
 
 // t = right-hand side of the pivot rows plus the children's border rows
 template <int NR>
@@ -77,13 +79,23 @@ __global__ void k_inv_gather(const int *__restrict__ fl, const DevFront *__restr
 // 0.21).  Row tiles split over several items add their partial sums in item
 // order in the item that finishes last, so results do not depend on timing;
 // per vector the arithmetic does not depend on NR.
+//
+// G: the variant of the levels with at most kSmallCols columns of 32 rows (32 MB
+// of factor).  There a launch costs more than its work, so the forward items
+// collect t themselves from the right-hand side and the children, each as many
+// columns as it needs, instead of a gather launch per level; the indices wait in
+// shared memory, read before the programmatic-launch wait.  A solve: 0.128 ->
+// 0.115 ms at 60 x 32, 0.182 -> 0.171 ms at 83 x 47.  Larger levels lose by the
+// repeated gathering: with G everywhere 2.20 instead of 1.98 ms at 300 x 192, and
+// up to 48 MB 0.894 instead of 0.884 ms at 200 x 128.
 constexpr int kW = 8;   // warps per CTA
 constexpr int kQ = 16;  // columns a thread loads at a time
 
-template <int NR>
+template <int NR, bool G>
 __global__ void __launch_bounds__(32 * kW, NR <= 4 ? 4 : 2)
     k_inv_apply(const SvItem *__restrict__ items, const float2 *__restrict__ pool,
-                const int *__restrict__ uidx, float2 *__restrict__ W, float2 *__restrict__ W2,
+                const int *__restrict__ uidx, const int *__restrict__ gsrc,
+                const int2 *__restrict__ cinv, float2 *__restrict__ W, float2 *__restrict__ W2,
                 long long ws, float2 *__restrict__ x, long long xs, float2 *__restrict__ part,
                 int max_split, int *__restrict__ ctr) {
   using C = float2;
@@ -113,31 +125,78 @@ __global__ void __launch_bounds__(32 * kW, NR <= 4 ? 4 : 2)
   };
   C cur[kQ];
   load(cur, q0);
+  // where this thread's vector entries come from: backward, the unknown; G
+  // forward, the right-hand side and the children.  G keeps them in shared
+  // memory (each thread reads back its own).
+  int *src = reinterpret_cast<int *>(vs + (kW * cw + kQ) * NR) + threadIdx.x;
   int id[kU];
-  if (it.kind == 2)
+  int2 bc = make_int2(-1, -1);
+  if constexpr (G) {
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int k = threadIdx.x + kT * u;
+      if (k < it.cols) {
+        if (it.kind == 2) {
+          src[kT * u] = k >= it.piv ? uidx[it.vec + k] : 0;
+        } else {
+          const int2 c = cinv[it.vec + k];
+          src[kT * u] = gsrc[it.vec + k];
+          src[kMaxCols + kT * u] = c.x;
+          src[2 * kMaxCols + kT * u] = c.y;
+        }
+      }
+    }
+    if (wp < NR && rowok && it.kind == 1) bc = cinv[it.out + lane];
+  } else if (it.kind == 2) {
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
       const int k = threadIdx.x + kT * u;
       id[u] = (k >= it.piv && k < it.cols) ? uidx[it.vec + k] : 0;
     }
+  }
   pdl_wait();
   // this warp finishes vector wp: its rows' own values go out with the rest
   C base = czero<C>();
-  if (wp < NR && rowok && it.kind != 0)
-    base = (it.kind == 1 ? W : W2)[wp * ws + it.out + lane];
+  if (wp < NR && rowok && it.kind != 0) {
+    if (!G || it.kind == 2) {
+      base = (it.kind == 1 ? W : W2)[wp * ws + it.out + lane];
+    } else {
+      if (bc.x >= 0) base = cadd(base, W[wp * ws + bc.x]);
+      if (bc.y >= 0) base = cadd(base, W[wp * ws + bc.y]);
+    }
+  }
   const int kend = kW * cw + kQ;
 #pragma unroll
   for (int u = 0; u < kU; ++u) {
     const int k = threadIdx.x + kT * u;
     if (k < it.cols) {
+      if constexpr (G) {
+        if (it.kind == 2) {
+          const int i = src[kT * u];
 #pragma unroll
-      for (int v = 0; v < NR; ++v) {
-        C t;
-        if (it.kind == 2)
-          t = k < it.piv ? W2[v * ws + it.vec + k] : x[v * xs + id[u]];
-        else
-          t = W[v * ws + it.vec + k];
-        vs[((k >> 1) * NR + v) * 2 + (k & 1)] = t;
+          for (int v = 0; v < NR; ++v)
+            vs[((k >> 1) * NR + v) * 2 + (k & 1)] =
+                k < it.piv ? W2[v * ws + it.vec + k] : x[v * xs + i];
+        } else {
+          const int i0 = src[kT * u], i1 = src[kMaxCols + kT * u], i2 = src[2 * kMaxCols + kT * u];
+#pragma unroll
+          for (int v = 0; v < NR; ++v) {
+            C t = i0 >= 0 ? x[v * xs + i0] : czero<C>();
+            if (i1 >= 0) t = cadd(t, W[v * ws + i1]);
+            if (i2 >= 0) t = cadd(t, W[v * ws + i2]);
+            vs[((k >> 1) * NR + v) * 2 + (k & 1)] = t;
+          }
+        }
+      } else {
+#pragma unroll
+        for (int v = 0; v < NR; ++v) {
+          C t;
+          if (it.kind == 2)
+            t = k < it.piv ? W2[v * ws + it.vec + k] : x[v * xs + id[u]];
+          else
+            t = W[v * ws + it.vec + k];
+          vs[((k >> 1) * NR + v) * 2 + (k & 1)] = t;
+        }
       }
     }
   }
@@ -284,7 +343,7 @@ int Factor::build_inverse(tlr_ctx *ctx) {
   struct Row {
     int t, r0, rows, c0, c1, kind;
   };
-  auto emit = [&](std::vector<Row> &rows, int &off, int &count) {
+  auto emit = [&](std::vector<Row> &rows, int &off, int &count, bool &small) {
     // three items per SM where the level has the work for them, of 256 (a
     // shorter share per warp is all start-up: 0.22 ms per solve at 100 x 50
     // against 0.25 with 128) to kMaxCols columns
@@ -321,6 +380,7 @@ int Factor::build_inverse(tlr_ctx *ctx) {
     }
     max_split_tiles = std::max(max_split_tiles, tile);
     count = (int)items.size() - off;
+    small = total <= kSmallCols;
     std::stable_sort(items.begin() + off, items.end(),
                      [](const SvItem &a, const SvItem &b) { return a.cols > b.cols; });
   };
@@ -338,8 +398,8 @@ int Factor::build_inverse(tlr_ctx *ctx) {
       }
       for (int r = f.p; r < f.m; r += 32) fw.push_back({t, r, std::min(32, f.m - r), 0, f.p, 1});
     }
-    emit(fw, L.if_off, L.if_n);
-    emit(bw, L.ib_off, L.ib_n);
+    emit(fw, L.if_off, L.if_n, L.if_small);
+    emit(bw, L.ib_off, L.ib_n, L.ib_small);
   }
   auto up = [&](void **p, const void *src, size_t bytes) -> int {
     const cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 16));
@@ -386,34 +446,39 @@ int Factor::solve_inverse(tlr_ctx *ctx, float2 *x, float2 *W, float2 *W2) {
   cudaStream_t st = ctx->stream;
   const float2 *P = static_cast<const float2 *>(pool);
   const long long xs = (long long)sym.nn * 5, ws = sym.work_elems;
-  const size_t sm = ((size_t)(item_cols + 2 * kW - 1) / (2 * kW) * (2 * kW) + kQ + kW * 32) * NR *
-                    sizeof(float2);
-  if (sm > 47 * 1024)
-    TLR_CUDA(ctx, cudaFuncSetAttribute(k_inv_apply<NR>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  auto apply = [&](int off, int n) -> int {
+  const size_t vec = ((size_t)(item_cols + 2 * kW - 1) / (2 * kW) * (2 * kW) + kQ + kW * 32) * NR *
+                     sizeof(float2);
+  auto apply = [&](bool small, bool pdl, int off, int n) -> int {
     if (n <= 0) return TLR_OK;
-    TLR_CUDA(ctx, launch_pdl_smem(true, k_inv_apply<NR>, dim3(n), dim3(32 * kW), sm, st,
-                                  (const SvItem *)(d_items + off), P, (const int *)d_uidx, W, W2,
-                                  ws, x, xs, split_part, max_split, split_ctr));
+    auto *kernel = small ? k_inv_apply<NR, true> : k_inv_apply<NR, false>;
+    const size_t sm = vec + (small ? 3 * kMaxCols * sizeof(int) : 0);
+    if (sm > 47 * 1024)
+      TLR_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)sm));
+    TLR_CUDA(ctx, launch_pdl_smem(pdl, kernel, dim3(n), dim3(32 * kW), sm, st,
+                                  (const SvItem *)(d_items + off), P, (const int *)d_uidx,
+                                  (const int *)d_gsrc, (const int2 *)d_cinv, W, W2, ws, x, xs,
+                                  split_part, max_split, split_ctr));
     count_launches();
     return TLR_OK;
   };
   int rc = TLR_OK;
+  // the first kernel follows a copy or another kernel that does not trigger
+  // early: no programmatic edge for it
   for (size_t h = 0; h < levels.size() && !rc; ++h) {
     const Level &L = levels[h];
-    // the first kernel follows a copy or another kernel that does not
-    // trigger early: no programmatic edge for it
-    TLR_CUDA(ctx, launch_pdl(h > 0, k_inv_gather<NR>,
-                             dim3(blocks_for(L.max_m, 128), L.nfronts), dim3(128), st,
-                             (const int *)(d_sched + L.fronts_off), (const DevFront *)d_fronts,
-                             (const int *)d_gsrc, (const int2 *)d_cinv, (const float2 *)x, xs, W,
-                             ws));
-    count_launches();
-    rc = apply(L.if_off, L.if_n);
+    if (!L.if_small) {
+      TLR_CUDA(ctx, launch_pdl(h > 0, k_inv_gather<NR>,
+                               dim3(blocks_for(L.max_m, 128), L.nfronts), dim3(128), st,
+                               (const int *)(d_sched + L.fronts_off), (const DevFront *)d_fronts,
+                               (const int *)d_gsrc, (const int2 *)d_cinv, (const float2 *)x, xs, W,
+                               ws));
+      count_launches();
+    }
+    rc = apply(L.if_small, h > 0 || !L.if_small, L.if_off, L.if_n);
   }
   for (int h = (int)levels.size() - 1; h >= 0 && !rc; --h)
-    rc = apply(levels[h].ib_off, levels[h].ib_n);
+    rc = apply(levels[h].ib_small, true, levels[h].ib_off, levels[h].ib_n);
   return rc;
 }
 

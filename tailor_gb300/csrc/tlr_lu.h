@@ -84,6 +84,7 @@ struct Level {
   int wctr_n = 0;
   // inverse-form solve: items of the forward and of the backward launch
   int if_off = 0, if_n = 0, ib_off = 0, ib_n = 0;
+  bool if_small = false, ib_small = false;  // launch-bound (tlr_inv.cu)
 };
 
 // One phase of the persistent solve: a kind of work item over a level's
