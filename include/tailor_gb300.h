@@ -424,6 +424,9 @@ int tlr_sweep(const tlr_grid_class *classes, int nclass, const tlr_sweep_point *
  * k0 must be a multiple of w, w <= 64.  lbo/sbo: shared-memory descriptor
  * strides of the operand planes in bytes (0: the library's values).
  * Writes the updated front to out. */
+int tlr_schur_update_c64(const float *front, int m, int p, int k0, int w, unsigned lbo,
+                         unsigned sbo, float *out);
+
 /* Test hook, no counterpart in the reference: x = K^-1 rhs through the
  * context's complex64 factor (left by a mixed-form tlr_solve) for nvec
  * host vectors rhs [nvec][5N] complex (rounded to complex64), written to
@@ -432,14 +435,19 @@ int tlr_sweep(const tlr_grid_class *classes, int nclass, const tlr_sweep_point *
  * both give the same bits. */
 int tlr_factor_solve(tlr_ctx *ctx, int nvec, const double *rhs, double *out, int multi);
 
-int tlr_schur_update_c64(const float *front, int m, int p, int k0, int w, unsigned lbo,
-                         unsigned sbo, float *out);
-
 /* Test hook, no counterpart in the reference: the same update of a
  * complex128 front (w must be 32) by exact integer slices on the tensor
  * cores (sliced = 1) or by FP64 FMAs on the CUDA cores (0). */
 int tlr_schur_update_c128(const double *front, int m, int p, int k0, int w, int sliced,
                           double *out);
+
+/* Test hook, no counterpart in the reference: the rewrite that ends a
+ * complex128 factorisation, on one factored front (m x m, p pivots, column-
+ * major, L below and U on and above the diagonal): every 128-column block of L
+ * times inv(L_bb), inv(U_bb) times every 128-row block of U, outside the
+ * diagonal blocks, to out; inv(U_bb) inv(L_bb) of every block, nb x nb and one
+ * after the other, to dmat.  sliced as above. */
+int tlr_rewrite_c128(const double *front, int m, int p, int sliced, double *out, double *dmat);
 
 /* An explicit generalized pencil A x = lambda B x as a solver context
  * (EigenSolver::solve(recipe, eigenMatrix, massMatrix, ...),

@@ -158,6 +158,7 @@ SIGNATURES = {
     "tlr_kernel_launches": ([], ctypes.c_longlong),
     "tlr_sweep": ([_P, _I, _P, _I, _P, _P, _P, _P, _P, _P], _I),
     "tlr_schur_update_c128": ([_P, _I, _I, _I, _I, _I, _P], _I),
+    "tlr_rewrite_c128": ([_P, _I, _I, _I, _P, _P], _I),
     "tlr_schur_update_c64": ([_P, _I, _I, _I, _I, ctypes.c_uint, ctypes.c_uint, _P], _I),
     "tlr_factor_solve": ([_P, _I, _P, _P, _I], _I),
     "tlr_wait_selftest": ([_I, ctypes.c_uint, _P], _I),

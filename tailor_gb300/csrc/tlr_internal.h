@@ -224,14 +224,25 @@ struct DevFront;
 // FP64 Schur update of one panel step (32 columns) of complex128 fronts by
 // exact integer slices on the tensor cores (tlr_oz.cu): prefix of the 128 x 32
 // output tiles, pa / pb of the 128-row L21 and 32-column U12 tiles; planes:
-// atiles x oz_a_image_bytes() + btiles x oz_b_image_bytes(), rexp: 32 ints per
+// oz_update_bytes(atiles, btiles), rexp: 32 ints per
 // front.
 int launch_gemm_oz(tlr_ctx *ctx, const int *fl, const int *prefix, const int *pa, const int *pb,
                    int nf, int s, int w, int max_ext, double2 *pool, const DevFront *fr, int tiles,
                    int atiles, int btiles, unsigned char *planes, int *rexp, int *err,
                    cudaStream_t st);
-size_t oz_a_image_bytes();
-size_t oz_b_image_bytes();
+struct OzJob;
+struct OzBatch;
+// One batch of the products that rewrite a complex128 factor (L' = L inv(L_cc)
+// and U' = inv(U_bb) U): the operands of all its passes
+// are split before any pass writes, so the products are in place.  prefix: at
+// prefix_off the batch's jobs + 1 prefixes of output tiles, then of the A and of
+// the B tiles; rexp: 32 ints per job.
+int launch_rewrite_oz(tlr_ctx *ctx, const OzBatch &b, const OzJob *jobs, const int *prefix,
+                      double2 *pool, const double2 *linv, const double2 *uinv,
+                      unsigned char *planes, int *rexp, int *err, cudaStream_t st);
+// bytes of the operand images of so many A and B tiles
+size_t oz_update_bytes(size_t atiles, size_t btiles);
+size_t oz_rewrite_bytes(size_t atiles, size_t btiles);
 struct TcJob;
 // A batch of products C(rows, cols) -= F(rows, K) F(K, cols), K <= 256, over
 // fronts of the pool: operand planes split once per batch (planes: (atiles +

@@ -982,11 +982,14 @@ __global__ void __launch_bounds__(SW)
       if (c0 + j < nb) out[(long long)(c0 + j) * nb + r] = x[j];
 }
 
+// The CUDA-core products of the rewrite (complex128 by default only for the D_b
+// and for blocks of fewer than 32 columns; the rest is sliced, tlr_oz.cu).
 // L'(rows, c) = L(rows, c) inv(L_cc) in place: CTA = 32 rows of block
 // column c (all nb columns, staged in shared memory before any write);
 // thread (row, g) forms columns g, g+8, ... of its row.
 // tiles: {front, block c, first row, -}.
 constexpr int kRT = 32;
+constexpr size_t kOzBatchBytes = (size_t)512 << 20;  // operand images of a sliced rewrite batch
 
 template <class C, int SW>
 __global__ void __launch_bounds__(256)
@@ -2042,6 +2045,65 @@ __global__ void __launch_bounds__(256)
 
 // ------------------------------------------------------------------- host
 
+// The products that rewrite a complex128 factor, cut into batches of at most
+// kOzBatchBytes of operand images; the passes of a diagonal block stay in one
+// batch (its products are in place, so all its operands are split first).
+struct RewriteFront {
+  long long off, inv_off;  // in the pool, in linv / uinv / dmat
+  int p, m;
+};
+
+static void plan_rewrite_oz(const std::vector<RewriteFront> &fronts, std::vector<OzJob> &jobs,
+                            std::vector<int> &prefix, std::vector<OzBatch> &batches) {
+  constexpr int sw = 32 * kOzPasses;
+  std::vector<OzJob> pass[kOzPasses];
+  size_t bytes = 0;
+  auto flush = [&]() {
+    if (pass[0].empty()) return;
+    OzBatch b;
+    b.job_off = (int)jobs.size();
+    b.prefix_off = (int)prefix.size();
+    std::vector<int> pt{0}, pa{0}, pb{0};
+    for (int q = 0; q < kOzPasses; ++q) {
+      b.pass[q] = pt.back();
+      for (const OzJob &j : pass[q]) {
+        const int na = (j.rows + 127) / 128, nb = (j.cols + 31) / 32;
+        pt.push_back(pt.back() + na * nb);
+        pa.push_back(pa.back() + na);
+        pb.push_back(pb.back() + nb);
+        b.max_len = std::max({b.max_len, j.rows, j.cols});
+        jobs.push_back(j);
+      }
+      pass[q].clear();
+    }
+    b.pass[kOzPasses] = pt.back();
+    b.jobs = (int)pt.size() - 1;
+    b.atiles = pa.back();
+    b.btiles = pb.back();
+    for (const auto *v : {&pt, &pa, &pb}) prefix.insert(prefix.end(), v->begin(), v->end());
+    batches.push_back(b);
+    bytes = 0;
+  };
+  for (const RewriteFront &f : fronts)
+    for (int b0 = 0; b0 < f.p; b0 += sw) {
+      const int nb = std::min(sw, f.p - b0), b1 = b0 + nb, ext = f.m - b1;
+      const int passes = (nb + 31) / 32;
+      const long long io = f.inv_off + (long long)b0 * sw, m = f.m;
+      const long long L = f.off + b0 * m + b1, U = f.off + b1 * m + b0;
+      if (ext == 0 || nb < kOzPanel) continue;
+      const size_t need = passes * oz_rewrite_bytes((ext + 127) / 128 + 1, (ext + 31) / 32 + passes);
+      if (bytes + need > kOzBatchBytes) flush();
+      bytes += need;
+      for (int q = 0; q < passes; ++q) {
+        const int k = 32 * q, kw = std::min(32, nb - k);
+        const long long ck = io + (long long)k * nb;  // column k of the inverses
+        pass[q].push_back({L + k * m, io + k, L, f.m, nb, f.m, ext, nb, kw, 0, 0});
+        pass[q].push_back({ck, U + k, U, nb, f.m, f.m, nb, ext, kw, 1, 0});
+      }
+    }
+  flush();
+}
+
 int Factor::setup(tlr_ctx *ctx, int precision, int leaf, int solve_block, int panel_width,
                   int ring_slack_percent) {
   prec = precision;
@@ -2181,7 +2243,7 @@ int Factor::setup(tlr_ctx *ctx, int precision, int leaf, int solve_block, int pa
           sched.push_back(tot);
           (pass == 2 ? st.btiles : pass ? st.atiles : st.oz_tiles) = tot;
         }
-        oz_bytes = std::max(oz_bytes, st.atiles * oz_a_image_bytes() + st.btiles * oz_b_image_bytes());
+        oz_bytes = std::max(oz_bytes, oz_update_bytes(st.atiles, st.btiles));
         oz_fronts = std::max(oz_fronts, st.nf);
       }
       L.steps.push_back(st);
@@ -2260,7 +2322,7 @@ int Factor::setup(tlr_ctx *ctx, int precision, int leaf, int solve_block, int pa
   // tiles of the factor rewrite L' = L Dl^-1, U' = Du^-1 U, D = Du^-1 Dl^-1
   std::vector<long long> inv_off(nf);
   std::vector<int2> inv_blocks;
-  std::vector<int4> ltiles, utiles, ltiles_tc, utiles_tc;
+  std::vector<int4> ltiles, utiles, l64, u64, ltiles_tc, utiles_tc;
   inv_elems = 0;
   for (int t = 0; t < nf; ++t) {
     const int p = sym.fronts[t].p, m = sym.fronts[t].m;
@@ -2269,9 +2331,10 @@ int Factor::setup(tlr_ctx *ctx, int precision, int leaf, int solve_block, int pa
       const int b1 = std::min(p, (b + 1) * sw), nb = b1 - b * sw;
       inv_blocks.push_back(make_int2(t, b));
       inv_elems += (long long)nb * nb;
-      for (int r = b1; r < m; r += kRT) ltiles.push_back(make_int4(t, b, r, 0));
-      for (int c = b1; c < m; c += kRT) utiles.push_back(make_int4(t, b, c, 0));
-      for (int c = 0; c < nb; c += kRT) utiles.push_back(make_int4(t, b, c, 1));
+      const bool fp64 = nb < kOzPanel;
+      for (int r = b1; r < m; r += kRT) (fp64 ? l64 : ltiles).push_back(make_int4(t, b, r, 0));
+      for (int c = b1; c < m; c += kRT) (fp64 ? u64 : utiles).push_back(make_int4(t, b, c, 0));
+      for (int c = 0; c < nb; c += kRT) u64.push_back(make_int4(t, b, c, 1));
       if (prec == 1 && sw == 256) {
         for (int r = b1; r < m; r += 128) ltiles_tc.push_back(make_int4(t, b, r, 0));
         for (int c = b1; c < m; c += 64) utiles_tc.push_back(make_int4(t, b, c, 0));
@@ -2279,6 +2342,23 @@ int Factor::setup(tlr_ctx *ctx, int precision, int leaf, int solve_block, int pa
       }
     }
   }
+  std::vector<OzJob> oz_jobs;
+  std::vector<int> oz_prefix;
+  oz_batches.clear();
+  if (prec == 0 && w == kOzPanel && sw == 32 * kOzPasses) {
+    std::vector<RewriteFront> rf;
+    for (int t = 0; t < nf; ++t)
+      rf.push_back({sym.fronts[t].off, inv_off[t], sym.fronts[t].p, sym.fronts[t].m});
+    plan_rewrite_oz(rf, oz_jobs, oz_prefix, oz_batches);
+    for (const OzBatch &b : oz_batches) {
+      oz_bytes = std::max(oz_bytes, oz_rewrite_bytes(b.atiles, b.btiles));
+      oz_fronts = std::max(oz_fronts, b.jobs);
+    }
+  }
+  n_ltiles64 = (long long)l64.size();
+  n_utiles64 = (long long)u64.size();
+  ltiles.insert(ltiles.begin(), l64.begin(), l64.end());
+  utiles.insert(utiles.begin(), u64.begin(), u64.end());
   n_ltiles = (long long)ltiles.size();
   n_utiles = (long long)utiles.size();
   n_ltiles_tc = (long long)ltiles_tc.size();
@@ -2336,8 +2416,16 @@ int Factor::setup(tlr_ctx *ctx, int precision, int leaf, int solve_block, int pa
     return rc;
   if (prec == 0 && w == kOzPanel &&
       ((rc = alloc((void **)&tc_planes, oz_bytes)) ||
-       (rc = alloc((void **)&d_rowexp, sizeof(int) * kOzPanel * oz_fronts))))
+       (rc = alloc((void **)&d_rowexp, sizeof(int) * kOzPanel * oz_fronts)) ||
+       (rc = alloc((void **)&d_oz_jobs, oz_jobs.size() * sizeof(OzJob))) ||
+       (rc = alloc((void **)&d_oz_prefix, oz_prefix.size() * sizeof(int)))))
     return rc;
+  if (!oz_jobs.empty()) {
+    TLR_CUDA(ctx, cudaMemcpy(d_oz_jobs, oz_jobs.data(), oz_jobs.size() * sizeof(OzJob),
+                             cudaMemcpyHostToDevice));
+    TLR_CUDA(ctx, cudaMemcpy(d_oz_prefix, oz_prefix.data(), oz_prefix.size() * sizeof(int),
+                             cudaMemcpyHostToDevice));
+  }
   if (prec == 0) {
     std::vector<StepFront> sf;
     for (auto &L : levels) {
@@ -2480,9 +2568,10 @@ void Factor::release() {
   cudaFree(d_inv_off); cudaFree(d_inv_blocks); cudaFree(d_ltiles); cudaFree(d_utiles);
   cudaFree(d_phases); cudaFree(d_barrier); cudaFree(d_solve_err); cudaFree(tc_planes);
   cudaFree(d_wave_tiles); cudaFree(d_wave_ctr); cudaFree(d_ltiles_tc); cudaFree(d_utiles_tc);
-  cudaFree(d_rowexp);
+  cudaFree(d_rowexp); cudaFree(d_oz_jobs); cudaFree(d_oz_prefix);
   cudaFree(d_sfronts);
-  d_rowexp = nullptr;
+  d_rowexp = d_oz_prefix = nullptr;
+  d_oz_jobs = nullptr;
   d_sfronts = nullptr;
   cudaFree(d_inv_jobs); cudaFree(d_inv_prefix); cudaFree(inv_planes); cudaFree(d_gtiles);
   cudaFree(d_items); cudaFree(d_uidx); cudaFree(d_gsrc); cudaFree(split_part); cudaFree(split_ctr);
@@ -2534,16 +2623,28 @@ int Factor::rewrite_factors(tlr_ctx *ctx) {
       return rc || !inverse ? rc : invert_pivots(ctx);
     }
   }
+  long long nu = n_utiles, nl = n_ltiles;
+  if constexpr (sizeof(C) == sizeof(double2)) {
+    if (sliced && d_oz_jobs) {  // L' and U' in slices, like the Schur updates
+      for (const OzBatch &b : oz_batches) {
+        const int rc = launch_rewrite_oz(ctx, b, d_oz_jobs, d_oz_prefix, P, Li, Ui, tc_planes,
+                                         d_rowexp, d_tc_err, st);
+        if (rc) return rc;
+      }
+      nu = n_utiles64;
+      nl = n_ltiles64;
+    }
+  }
   const size_t ssm = sizeof(C) * SW * kRT;
   TLR_CUDA(ctx, cudaFuncSetAttribute(k_scale_u<C, SW>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm));
   TLR_CUDA(ctx, cudaFuncSetAttribute(k_scale_l<C, SW>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm));
-  if (n_utiles > 0)
-    { k_scale_u<C, SW><<<(unsigned)n_utiles, SW > 256 ? SW : 256, ssm, st>>>(d_utiles, P, d_fronts, d_inv_off, Li,
+  if (nu > 0)
+    { k_scale_u<C, SW><<<(unsigned)nu, SW > 256 ? SW : 256, ssm, st>>>(d_utiles, P, d_fronts, d_inv_off, Li,
                                                             Ui, static_cast<C *>(dmat)); count_launches(); }
-  if (n_ltiles > 0)
-    { k_scale_l<C, SW><<<(unsigned)n_ltiles, 256, ssm, st>>>(d_ltiles, P, d_fronts, d_inv_off,
+  if (nl > 0)
+    { k_scale_l<C, SW><<<(unsigned)nl, 256, ssm, st>>>(d_ltiles, P, d_fronts, d_inv_off,
                                                             Li); count_launches(); }
   return TLR_OK;
 }
@@ -3121,7 +3222,7 @@ extern "C" int tlr_schur_update_c128(const double *front, int m, int p, int k0, 
   if (cudaGetDevice(&ctx.device) != cudaSuccess || cudaMalloc(&F, bytes) != cudaSuccess ||
       cudaMalloc(&fr, sizeof(DevFront)) != cudaSuccess ||
       cudaMalloc(&ints, sizeof(hi)) != cudaSuccess ||
-      cudaMalloc(&planes, na * oz_a_image_bytes() + nb * oz_b_image_bytes() + 16) != cudaSuccess ||
+      cudaMalloc(&planes, oz_update_bytes(na, nb) + 16) != cudaSuccess ||
       cudaStreamCreate(&ctx.stream) != cudaSuccess)
     rc = TLR_ERR_NOMEM;
   else if (cudaMemcpy(F, front, bytes, cudaMemcpyHostToDevice) != cudaSuccess ||
@@ -3144,6 +3245,88 @@ extern "C" int tlr_schur_update_c128(const double *front, int m, int p, int k0, 
   cudaFree(fr);
   cudaFree(ints);
   cudaFree(planes);
+  if (ctx.stream) cudaStreamDestroy(ctx.stream);
+  return rc;
+}
+
+// ---------------------------------------------------------------- test hook
+extern "C" int tlr_rewrite_c128(const double *front, int m, int p, int sliced, double *out,
+                                double *dmat) {
+  using namespace tlr;
+  if (!front || !out || !dmat || m <= 0 || p <= 0 || p > m) return TLR_ERR_ARG;
+  constexpr int SW = 32 * kOzPasses;
+  const size_t bytes = (size_t)m * m * sizeof(double2);
+  std::vector<OzJob> jobs;
+  std::vector<int> prefix;
+  std::vector<OzBatch> batches;
+  plan_rewrite_oz({{0, 0, p, m}}, jobs, prefix, batches);
+  DevFront h{};
+  h.p = p;
+  h.m = m;
+  h.parent = -1;
+  std::vector<int2> blocks;
+  std::vector<int4> lt, ut, l64, u64;
+  size_t inv = 0, img = 16;
+  int nj = 1;
+  for (int b = 0; b * SW < p; ++b) {
+    const int b1 = std::min(p, (b + 1) * SW), nb = b1 - b * SW;
+    blocks.push_back(make_int2(0, b));
+    inv += (size_t)nb * nb * sizeof(double2);
+    const bool fp64 = nb < kOzPanel;
+    for (int r = b1; r < m; r += kRT) (fp64 ? l64 : lt).push_back(make_int4(0, b, r, 0));
+    for (int c = b1; c < m; c += kRT) (fp64 ? u64 : ut).push_back(make_int4(0, b, c, 0));
+    for (int c = 0; c < nb; c += kRT) u64.push_back(make_int4(0, b, c, 1));
+  }
+  for (const OzBatch &b : batches) {
+    img = std::max(img, oz_rewrite_bytes(b.atiles, b.btiles));
+    nj = std::max(nj, b.jobs);
+  }
+  tlr_ctx ctx;
+  Factor F;
+  F.prec = 0;
+  F.sliced = sliced != 0;
+  F.oz_batches = batches;
+  F.n_inv_blocks = (int)blocks.size();
+  F.n_ltiles64 = (long long)l64.size();
+  F.n_utiles64 = (long long)u64.size();
+  lt.insert(lt.begin(), l64.begin(), l64.end());
+  ut.insert(ut.begin(), u64.begin(), u64.end());
+  F.n_ltiles = (long long)lt.size();
+  F.n_utiles = (long long)ut.size();
+  int rc = TLR_OK, herr = 0;
+  auto up = [&](auto **q, const void *src, size_t n) {
+    if (rc) return;
+    if (cudaMalloc((void **)q, std::max<size_t>(n, 16)) != cudaSuccess)
+      rc = TLR_ERR_NOMEM;
+    else if (src && n && cudaMemcpy(*q, src, n, cudaMemcpyHostToDevice) != cudaSuccess)
+      rc = TLR_ERR_CUDA;
+  };
+  const long long zero = 0;
+  up(&F.pool, front, bytes);
+  up(&F.d_fronts, &h, sizeof(h));
+  up(&F.d_inv_off, &zero, sizeof(zero));
+  up(&F.d_inv_blocks, blocks.data(), blocks.size() * sizeof(int2));
+  up(&F.d_ltiles, lt.data(), lt.size() * sizeof(int4));
+  up(&F.d_utiles, ut.data(), ut.size() * sizeof(int4));
+  up(&F.linv, nullptr, inv);
+  up(&F.uinv, nullptr, inv);
+  up(&F.dmat, nullptr, inv);
+  up(&F.tc_planes, nullptr, img);
+  up(&F.d_rowexp, nullptr, sizeof(int) * kOzPanel * nj);
+  up(&F.d_tc_err, &herr, sizeof(int));
+  up(&F.d_oz_jobs, jobs.data(), jobs.size() * sizeof(OzJob));
+  up(&F.d_oz_prefix, prefix.data(), prefix.size() * sizeof(int));
+  if (!rc && (cudaGetDevice(&ctx.device) != cudaSuccess ||
+              cudaStreamCreate(&ctx.stream) != cudaSuccess))
+    rc = TLR_ERR_CUDA;
+  if (!rc) rc = F.rewrite_factors<double2, SW>(&ctx);
+  if (!rc && (cudaStreamSynchronize(ctx.stream) != cudaSuccess ||
+              cudaMemcpy(out, F.pool, bytes, cudaMemcpyDeviceToHost) != cudaSuccess ||
+              cudaMemcpy(dmat, F.dmat, inv, cudaMemcpyDeviceToHost) != cudaSuccess ||
+              cudaMemcpy(&herr, F.d_tc_err, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess ||
+              herr))
+    rc = TLR_ERR_CUDA;
+  F.release();
   if (ctx.stream) cudaStreamDestroy(ctx.stream);
   return rc;
 }

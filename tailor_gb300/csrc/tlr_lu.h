@@ -22,6 +22,22 @@ struct StepFront {
 
 constexpr int kOzPanel = 32;  // panel columns of the sliced FP64 Schur update
 
+// One 32-column pass of a product of the complex128 rewrite, column-major:
+// kind 0 L' (A in the pool, B in linv), 1 U' (A in uinv, B in the pool).
+struct OzJob {
+  long long a, b, c;
+  int lda, ldb, ldc, rows, cols, kw, kind, pad;
+};
+
+constexpr int kOzPasses = 4;  // 128-row diagonal blocks, 32 columns per pass
+
+// A batch of such passes, ordered by pass; pass[q]: its first output tile
+struct OzBatch {
+  int job_off = 0, jobs = 0, prefix_off = 0, atiles = 0, btiles = 0;
+  int max_len = 0;  // longest side of a product
+  int pass[kOzPasses + 1] = {};
+};
+
 // Default of Factor::cluster_rows (the automatic cluster-panel choice).
 constexpr int kClusterPanelRows = 256;
 
@@ -114,6 +130,10 @@ struct Factor {
   // complex128 Schur updates by exact integer slices on the tensor cores
   // (tlr_oz.cu), with 32-column panels
   bool sliced = false;
+  // its products of the factor rewrite, in batches
+  std::vector<OzBatch> oz_batches;
+  OzJob *d_oz_jobs = nullptr;
+  int *d_oz_prefix = nullptr;
   StepFront *d_sfronts = nullptr;  // complex128: fronts of every level in order
   int *d_rowexp = nullptr;
   int w = 32;    // panel width
@@ -160,6 +180,9 @@ struct Factor {
   int invert_pivots(tlr_ctx *ctx);
   template <int NR> int solve_inverse(tlr_ctx *ctx, float2 *x, float2 *W, float2 *W2);
   long long inv_elems = 0, n_ltiles = 0, n_utiles = 0;
+  // sliced rewrite: leading L and U tiles that stay in FP64 (the D_b, blocks of
+  // fewer than 32 columns)
+  long long n_ltiles64 = 0, n_utiles64 = 0;
   cudaGraphExec_t graph_exec = nullptr;  // captured solve, replayed per call
   // persistent solve: one cooperative launch per solve over a phase table
   bool persistent = false;
