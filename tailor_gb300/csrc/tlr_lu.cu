@@ -2374,7 +2374,8 @@ int Factor::setup(tlr_ctx *ctx, int precision, int leaf, int solve_block, int pa
     }
     return TLR_OK;
   };
-  if ((rc = alloc(&pool, (size_t)sym.pool_elems * csize)) ||
+  // 16 bytes to spare: copies of a front's columns are 16-byte aligned ranges
+  if ((rc = alloc(&pool, (size_t)sym.pool_elems * csize + 16)) ||
       (rc = alloc(&work, (size_t)sym.work_elems * csize)) ||
       (rc = alloc((void **)&d_fronts, nf * sizeof(DevFront))) ||
       (rc = alloc((void **)&d_entries, sym.entries.size() * sizeof(AsmEntry))) ||

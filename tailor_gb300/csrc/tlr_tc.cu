@@ -647,9 +647,19 @@ __global__ void __launch_bounds__(256, MINB)
 //     and, after the tile's last chunk, the accumulator (tfull[]);
 //   warps 0..7: the epilogue.  Warp w owns tile rows 32 (w % 4) + lane
 //     (its TMEM lane quarter) and the 32 complex columns 32 (w / 4) .. +31;
-//     it loads its F22 entries of a tile before that tile's accumulator is
-//     ready, then subtracts the accumulator and releases it (tempty[]),
-//     while the MMAs of the next tile run on the other accumulator.
+//     it subtracts the accumulator from F22 and releases it (tempty[]), while
+//     the MMAs of the next tile run on the other accumulator;
+//   warp 10: bulk copies of the F22 tiles, 16 columns at a time, into four
+//     slots (ffull[] / fempty[]), so the next tile's reads are in flight all
+//     the time.  A column of a tile starts on any 8-byte boundary; its copy is
+//     the 16-byte aligned range around it.
+// Loads of F22 into registers wait for L1 lines and for the epilogue before
+// (DRAM 52% busy, tensor pipe 32%); with the copies the largest update at 150 x
+// 96 takes 445 instead of 511 us (62%, 36%), a factorisation 334 instead of 350
+// ms at 300 x 192 and 126 instead of 131 ms at 200 x 128.  It is now bound by
+// reading 256 KB of operand images per tile from L2 (11 TB/s over all SMs).
+// Three or five ring stages: 342 ms both; keeping a row tile's A images in
+// shared memory instead: 396 ms, its CTAs work on distant parts of F22.
 // The MMAs and the epilogue arithmetic are those of k_gemm_tc_bulk, so the
 // factors are bitwise the same.  Every wait is bounded: a wait that runs
 // out raises the error flag and the CTA's abort word, every role stops
@@ -657,7 +667,9 @@ __global__ void __launch_bounds__(256, MINB)
 // before TMEM is released.
 // With jobs (JOB) the tiles are those of a batch of TcJobs instead of the
 // trailing blocks of one panel step.
-constexpr int kPersistThreads = 320;
+constexpr int kPersistThreads = 352;
+constexpr int kFCols = 16, kFCol = 1040;  // F22 slot: columns, bytes of one
+constexpr int kFSlots = kTcN / kFCols;
 
 template <int S, bool JOB>
 __global__ void __launch_bounds__(kPersistThreads, 1)
@@ -670,10 +682,13 @@ __global__ void __launch_bounds__(kPersistThreads, 1)
                       int *__restrict__ err) {
   extern __shared__ __align__(1024) unsigned char tc_smem[];
   __shared__ __align__(8) uint64_t full[S], empty[S], tfull[2], tempty[2];
+  __shared__ __align__(8) uint64_t ffull[kFSlots], fempty[kFSlots];
   __shared__ uint32_t tmem_slot;
   __shared__ volatile int abort_flag;
   __shared__ int issued_g, consumed_g, committed_g;  // chunk counters at exit
+  __shared__ int issued_f;                           // F22 slots filled at exit
   unsigned char *ring = tc_smem + ((1024 - (smem_addr(tc_smem) & 1023)) & 1023);
+  unsigned char *fbuf = ring + S * kStage;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (warp == 8) {
@@ -691,9 +706,13 @@ __global__ void __launch_bounds__(kPersistThreads, 1)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&tfull[q])));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 8;" ::"r"(smem_addr(&tempty[q])));
     }
+    for (int q = 0; q < kFSlots; ++q) {
+      mbar_init(&ffull[q], 1);
+      mbar_init(&fempty[q], 8);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     abort_flag = 0;
-    issued_g = consumed_g = committed_g = 0;
+    issued_g = consumed_g = committed_g = issued_f = 0;
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -800,6 +819,28 @@ __global__ void __launch_bounds__(kPersistThreads, 1)
       consumed_g = g;
       committed_g = committed;
     }
+  } else if (warp == 10) {  // F22 copies
+    int nf22 = 0;
+    for (int t = blockIdx.x; t < tiles && !abort_flag; t += gridDim.x) {
+      const Tile d = decode(t);
+      const int rows = min(kTcM, d.r1 - d.R0);
+      for (int q = 0; q < kFSlots; ++q, ++nf22) {
+        bool ok = true;
+        if (lane == 0 && nf22 >= kFSlots)
+          ok = wait_bar(&fempty[q], (nf22 / kFSlots - 1) & 1);
+        if (!__shfl_sync(0xffffffffu, ok ? 1 : 0, 0)) break;
+        const int c = d.C0 + kFCols * q + lane;
+        uint32_t bytes = 0;
+        const float2 *src = d.F + (long long)c * d.m + d.R0;
+        const int pad = (int)(reinterpret_cast<uintptr_t>(src) >> 3) & 1;
+        if (lane < kFCols && c < d.c1) bytes = (rows + pad + 1) / 2 * 16;
+        const uint32_t all = __reduce_add_sync(0xffffffffu, bytes);
+        if (lane == 0) mbar_expect_tx(&ffull[q], all);
+        __syncwarp();
+        if (bytes) bulk_g2s(fbuf + (q * kFCols + lane) * kFCol, src - pad, bytes, &ffull[q]);
+      }
+    }
+    if (lane == 0) issued_f = nf22;
   } else {  // epilogue, warps 0..7
     const int q4 = warp & 3, h2 = warp >> 2;
     const int row = 32 * q4 + lane;
@@ -808,14 +849,6 @@ __global__ void __launch_bounds__(kPersistThreads, 1)
       const Tile d = decode(t);
       const int acc = ti & 1;
       const bool row_ok = d.R0 + row < d.r1;
-      // this tile's F22 entries, fetched while its MMAs run
-      float2 f22[32];
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const int n = 32 * h2 + j;
-        f22[j] = (row_ok && d.C0 + n < d.c1) ? d.F[(long long)(d.C0 + n) * d.m + d.R0 + row]
-                                            : make_float2(0.f, 0.f);
-      }
       bool ok = true;
       if (lane == 0) ok = wait_bar(&tfull[acc], (ti >> 1) & 1);
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
@@ -823,25 +856,34 @@ __global__ void __launch_bounds__(kPersistThreads, 1)
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t lane_addr = tmem + 128 * acc + ((uint32_t)(32 * q4) << 16);
 #pragma unroll
-      for (int part = 0; part < 4; ++part) {
+      for (int q = 0; q < kFSlots; ++q) {
         uint32_t cr[8], ci[8];
-        const int n0 = 32 * h2 + 8 * part;
+        const int n0 = kFCols * q + 8 * h2;
         TLR_TC_LD8(lane_addr + n0, cr);
         TLR_TC_LD8(lane_addr + 64 + n0, ci);
+        ok = wait_bar(&ffull[q], ti & 1);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (!__all_sync(0xffffffffu, ok)) break;
         if (row_ok) {
+          float2 *p = d.F + (long long)(d.C0 + n0) * d.m + d.R0;
+          const unsigned char *sp = fbuf + n0 * kFCol + 8 * row;
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int n = n0 + j;
-            if (d.C0 + n < d.c1) {
-              float2 v = f22[8 * part + j];
+          for (int j = 0; j < 8; ++j, p += d.m) {
+            if (d.C0 + n0 + j < d.c1) {
+              const int pad = (int)(reinterpret_cast<uintptr_t>(p) & 8);
+              float2 v = *reinterpret_cast<const float2 *>(sp + j * kFCol + pad);
               v.x -= __uint_as_float(cr[j]);
               v.y -= __uint_as_float(ci[j]);
-              d.F[(long long)(d.C0 + n) * d.m + d.R0 + row] = v;
+              p[row] = v;
             }
           }
         }
+        __syncwarp();
+        if (lane == 0)
+          asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(&fempty[q]))
+                       : "memory");
       }
+      if (!__all_sync(0xffffffffu, ok)) break;
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0)
@@ -854,6 +896,10 @@ __global__ void __launch_bounds__(kPersistThreads, 1)
     // let the copies and MMAs already issued land before TMEM is released
     for (int g = consumed_g; g < issued_g; ++g) mbar_wait(&full[g % S], (g / S) & 1);
     if (committed_g > 0) mbar_wait(&empty[(committed_g - 1) % S], ((committed_g - 1) / S) & 1);
+    for (int q = 0; q < kFSlots; ++q) {  // slot q: fills q, q + kFSlots, ...
+      const int fills = (issued_f - q + kFSlots - 1) / kFSlots;
+      if (issued_f > q) mbar_wait(&ffull[q], (fills - 1) & 1);
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -866,6 +912,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1)
 size_t gemm_tc_smem() { return 2 * kStage + 1024; }
 
 size_t gemm_tc_bulk_smem(int stages) { return stages * kStage + 1024; }
+size_t gemm_tc_persist_smem(int stages) { return gemm_tc_bulk_smem(stages) + kTcN * kFCol; }
 size_t tc_chunk_image_bytes() { return kChunkImg; }
 
 namespace {
@@ -1189,7 +1236,7 @@ int launch_gemm_tc_bulk(tlr_ctx *ctx, const int *fl, const int *prefix, const in
   const unsigned char *pbp = planes + (long long)atiles * nchmax * kChunkImg;
   if (variant == 2) {  // persistent, warp-specialised: one CTA per SM, four stages
     auto k = k_gemm_tc_persist<4, false>;
-    const int smem = (int)gemm_tc_bulk_smem(4);
+    const int smem = (int)gemm_tc_persist_smem(4);
     TLR_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
@@ -1248,7 +1295,7 @@ int launch_tc_jobs(tlr_ctx *ctx, const TcJob *jobs, int nj, const int *prefix, c
   { k_tc_split_jobs<<<dim3(atiles + btiles, nchmax), 256, 0, st>>>(jobs, pa, pb, nj, pool, planes,
                                                                   atiles, nchmax); count_launches(); }
   auto k = k_gemm_tc_persist<4, true>;
-  const int smem = (int)gemm_tc_bulk_smem(4);
+  const int smem = (int)gemm_tc_persist_smem(4);
   TLR_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
