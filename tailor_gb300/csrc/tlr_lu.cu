@@ -77,12 +77,8 @@ __global__ void k_extend(const int *__restrict__ kids, const DevFront *__restric
   }
 }
 
-// Block-wide argmax of (value, row) pairs: largest value, ties to the
-// smaller row; warp shuffles, then one warp over the warp winners.  The
-// result is returned to every thread.
 template <class T>
-__device__ __forceinline__ void block_argmax(T &best, int &bi, T *wval, int *widx) {
-  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+__device__ __forceinline__ void warp_argmax(T &best, int &bi) {  // result in lane 0
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const T a = __shfl_down_sync(0xffffffffu, best, o);
@@ -92,32 +88,25 @@ __device__ __forceinline__ void block_argmax(T &best, int &bi, T *wval, int *wid
       bi = ia;
     }
   }
+}
+
+// Block-wide argmax of (value, row) pairs: largest value, ties to the
+// smaller row; warp shuffles, then every warp over the warp winners, so one
+// barrier is enough.  The result is in lane 0 of every warp (row: all lanes).
+// wval / widx: 32 entries, alternate ones for successive calls.
+template <class T>
+__device__ __forceinline__ void block_argmax(T &best, int &bi, T *wval, int *widx) {
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  warp_argmax(best, bi);
   if (lane == 0) {
     wval[wp] = best;
     widx[wp] = bi;
   }
   __syncthreads();
-  if (wp == 0) {
-    best = lane < nw ? wval[lane] : T(-2);
-    bi = lane < nw ? widx[lane] : 0x7fffffff;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const T a = __shfl_down_sync(0xffffffffu, best, o);
-      const int ia = __shfl_down_sync(0xffffffffu, bi, o);
-      if (a > best || (a == best && ia < bi)) {
-        best = a;
-        bi = ia;
-      }
-    }
-    if (lane == 0) {
-      wval[0] = best;
-      widx[0] = bi;
-    }
-  }
-  __syncthreads();
-  best = wval[0];
-  bi = widx[0];
-  __syncthreads();  // wval/widx are reused by the next call
+  best = lane < nw ? wval[lane] : T(-2);
+  bi = lane < nw ? widx[lane] : 0x7fffffff;
+  warp_argmax(best, bi);
+  bi = __shfl_sync(0xffffffffu, bi, 0);
 }
 
 // Panel factorisation of step s for one front per CTA: columns k0..k0+ww,
@@ -126,8 +115,66 @@ __device__ __forceinline__ void block_argmax(T &best, int &bi, T *wval, int *wid
 // updates stay inside the sub-panel, then the rest of the panel is updated
 // once per sub-panel (a unit-lower solve for its U rows and a rank-kSB
 // update below), so each panel element crosses L2 ww/kSB times instead of
-// ww times.
+// ww times.  Bound by the latency of a column; the update of a column looks for
+// the next pivot on the way, and of the eight barriers per column two are left
+// (complex128: four).
 constexpr int kSB = 8;
+
+// best = the largest |a| (and its row) of one thread's rows in a column
+template <class T>
+__device__ __forceinline__ void take_best(T a, int r, T &best, int &bi) {
+  if (a > best) {
+    best = a;
+    bi = r;
+  }
+}
+
+// One column step on rows [r0, r1) of a sub-panel: `a` is row 0 of the pivot
+// column (leading dimension ld), u(j) the pivot row's entry j columns on, nc the
+// columns after the pivot.  l = a / pivot, a_j -= l u_j, and the candidates of
+// the next column.  complex64: a thread per row.  complex128 is bound by the
+// FP64 pipe, so one warp inverts the pivot and the products are spread evenly
+// over the CTA, at the price of two barriers.
+template <class C, class U, class T>
+__device__ __forceinline__ void column_step(C *a, long long ld, int r0, int r1, int nc, C pv, U u,
+                                            C *sinv, T &best, int &bi) {
+  if constexpr (sizeof(C) == sizeof(float2)) {
+    const C inv = cinv(pv);
+    C uu[kSB - 1];
+#pragma unroll
+    for (int j = 0; j < kSB - 1; ++j) uu[j] = j < nc ? u(j) : czero<C>();
+    for (int r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
+      C *q = a + r;
+      const C l = cmul(*q, inv);
+      *q = l;
+#pragma unroll
+      for (int j = 0; j < kSB - 1; ++j)
+        if (j < nc) {
+          q += ld;
+          const C v = cfms(*q, l, uu[j]);
+          *q = v;
+          if (j == 0) take_best(cabs1(v), r, best, bi);
+        }
+    }
+  } else {
+    if (threadIdx.x < 32) {
+      const C inv = cinv(pv);
+      if (threadIdx.x == 0) *sinv = inv;
+    }
+    __syncthreads();
+    const C inv = *sinv;
+    for (int r = r0 + threadIdx.x; r < r1; r += blockDim.x) a[r] = cmul(a[r], inv);
+    __syncthreads();
+    const int nr = r1 - r0;
+    for (int x = threadIdx.x; x < nr * nc; x += blockDim.x) {
+      const int j = x / nr, r = r0 + x - j * nr;
+      C *q = a + (j + 1) * ld + r;
+      const C v = cfms(*q, a[r], u(j));
+      *q = v;
+      if (j == 0) take_best(cabs1(v), r, best, bi);
+    }
+  }
+}
 
 template <class C>
 __global__ void __launch_bounds__(512)
@@ -135,9 +182,10 @@ __global__ void __launch_bounds__(512)
             const DevFront *__restrict__ fr, int *__restrict__ ipiv,
             int *__restrict__ pert, double tiny) {
   using T = typename Real<C>::T;
-  __shared__ T sval[32];
-  __shared__ int sidx[32];
+  __shared__ T sval[2][32];
+  __shared__ int sidx[2][32];
   __shared__ C lsub[kSB][kSB];
+  __shared__ C sinv;
   const DevFront f = fr[fl[blockIdx.x]];
   C *F = pool + f.off;
   const int m = f.m, p = f.p;
@@ -146,14 +194,11 @@ __global__ void __launch_bounds__(512)
   for (int jb = 0; jb < ww; jb += kSB) {
     const int nb = min(kSB, ww - jb);
     const int c0 = k0 + jb, c1 = c0 + nb;  // sub-panel columns [c0, c1)
+    T best = -1;  // the first column's candidates; later ones come with the update
+    int bi = c0;
+    for (int r = c0 + tid; r < p; r += nt) take_best(cabs1(F[(long long)c0 * m + r]), r, best, bi);
     for (int col = c0; col < c1; ++col) {
-      T best = -1;
-      int bi = col;
-      for (int r = col + tid; r < p; r += nt) {
-        const T a = cabs1(F[(long long)col * m + r]);
-        if (a > best) { best = a; bi = r; }
-      }
-      block_argmax(best, bi, sval, sidx);
+      block_argmax(best, bi, sval[col & 1], sidx[col & 1]);
       if (tid == 0) ipiv[f.toff + col] = bi;
       const int pr = bi;
       if (pr != col)
@@ -171,18 +216,13 @@ __global__ void __launch_bounds__(512)
           atomicAdd(pert, 1);
         }
       }
-      const C inv = cinv(pv);
-      for (int r = col + 1 + tid; r < p; r += nt)
-        F[(long long)col * m + r] = cmul(F[(long long)col * m + r], inv);
-      __syncthreads();
-      const int nr = p - col - 1, nc = c1 - col - 1;
-      for (int x = tid; x < nr * nc; x += nt) {
-        const int r = col + 1 + x % nr, c = col + 1 + x / nr;
-        F[(long long)c * m + r] =
-            cfms(F[(long long)c * m + r], F[(long long)col * m + r], F[(long long)c * m + col]);
-      }
-      __syncthreads();
+      best = -1;
+      bi = col + 1;
+      column_step(
+          F + (long long)col * m, m, col + 1, p, c1 - col - 1, pv,
+          [&](int j) { return F[(long long)(col + 1 + j) * m + col]; }, &sinv, best, bi);
     }
+    __syncthreads();
     if (c1 >= k0 + ww) break;
     // U rows of the sub-panel for the remaining panel columns: unit-lower solve
     for (int x = tid; x < nb * nb; x += nt) lsub[x / nb][x % nb] = F[(long long)(c0 + x % nb) * m + c0 + x / nb];
@@ -267,8 +307,8 @@ __global__ void __cluster_dims__(kPanelCluster, 1, 1) __launch_bounds__(256)
   using T = typename Real<C>::T;
   cg::cluster_group cluster = cg::this_cluster();
   const int q = (int)cluster.block_rank();
-  __shared__ T sval[32];
-  __shared__ int sidx[32];
+  __shared__ T sval[2][32];
+  __shared__ int sidx[2][32];
   __shared__ T cval;
   __shared__ int cidx;
   __shared__ int gsel[1];
@@ -287,24 +327,20 @@ __global__ void __cluster_dims__(kPanelCluster, 1, 1) __launch_bounds__(256)
   for (int jb = 0; jb < ww; jb += kSB) {
     const int nb = min(kSB, ww - jb);
     const int c0 = k0 + jb, c1 = c0 + nb;
+    T best = -1;  // local candidate over owned rows; later columns': with the update
+    int bi = p;
+    for (int r = max(ra, c0) + tid; r < rb; r += nt)
+      take_best(cabs1(__ldcg(F + (long long)c0 * m + r)), r, best, bi);
     for (int col = c0; col < c1; ++col) {
-      // local candidate over owned rows >= col
-      T best = -1;
-      int bi = p;
-      for (int r = max(ra, col) + tid; r < rb; r += nt) {
-        const T a = cabs1(__ldcg(F + (long long)col * m + r));
-        if (a > best) { best = a; bi = r; }
-      }
-      block_argmax(best, bi, sval, sidx);
+      block_argmax(best, bi, sval[col & 1], sidx[col & 1]);
       if (tid == 0) {
         cval = best;
         cidx = bi;
       }
       cluster.sync();
-      // every CTA reads the kPanelCluster candidates and picks the same pivot
-      const int gi = cluster_argmax<T, kPanelCluster>(cluster, &cval, &cidx, p, gsel);
-      const int pr = gi < p ? gi : col;
-      if (q == 0) {
+      if (q == 0) {  // picks the pivot out of the CTAs' candidates
+        const int gi = cluster_argmax<T, kPanelCluster>(cluster, &cval, &cidx, p, gsel);
+        const int pr = gi < p ? gi : col;
         if (tid == 0) ipiv[f.toff + col] = pr;
         if (pr != col)
           for (int c = k0 + tid; c < k0 + ww; c += nt) {
@@ -321,19 +357,27 @@ __global__ void __cluster_dims__(kPanelCluster, 1, 1) __launch_bounds__(256)
       __threadfence();
       cluster.sync();
       const C inv = cinv(__ldcg(F + (long long)col * m + col));
-      const int r0 = max(ra, col + 1);
-      for (int r = r0 + tid; r < rb; r += nt)
-        F[(long long)col * m + r] = cmul(__ldcg(F + (long long)col * m + r), inv);
-      __syncthreads();
-      const int nr = rb - r0, nc = c1 - col - 1;
-      for (int x = tid; x < nr * nc; x += nt) {
-        const int r = r0 + x % nr, c = col + 1 + x / nr;
-        F[(long long)c * m + r] = cfms(__ldcg(F + (long long)c * m + r),
-                                       __ldcg(F + (long long)col * m + r),
-                                       __ldcg(F + (long long)c * m + col));
+      C u[kSB - 1];
+#pragma unroll
+      for (int j = 0; j < kSB - 1; ++j)
+        u[j] = col + 1 + j < c1 ? __ldcg(F + (long long)(col + 1 + j) * m + col) : czero<C>();
+      best = -1;
+      bi = p;
+      for (int r = max(ra, col + 1) + tid; r < rb; r += nt) {
+        C *row = F + (long long)col * m + r;
+        const C l = cmul(__ldcg(row), inv);
+        *row = l;
+#pragma unroll
+        for (int j = 0; j < kSB - 1; ++j)
+          if (col + 1 + j < c1) {
+            row += m;
+            const C v = cfms(__ldcg(row), l, u[j]);
+            *row = v;
+            if (j == 0) take_best(cabs1(v), r, best, bi);
+          }
       }
-      __syncthreads();
     }
+    __syncthreads();
     if (c1 >= k0 + ww) break;
     // CTA 0: U rows of the sub-panel for the remaining panel columns
     if (q == 0) {
@@ -393,15 +437,15 @@ __global__ void __cluster_dims__(kPanelCluster, 1, 1) __launch_bounds__(256)
   const int q = (int)cluster.block_rank();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C *P = reinterpret_cast<C *>(smem_raw);  // P[(c - k0) * ldp + (r - ra)]
-  __shared__ T sval[32];
-  __shared__ int sidx[32];
+  __shared__ T sval[2][32];
+  __shared__ int sidx[2][32];
   __shared__ T cval;
   __shared__ int cidx;
   __shared__ int gsel[1];
   __shared__ C lsub[kSB][kSB];
-  __shared__ C urow[kSB];               // pivot row entries of the sub-panel
+  __shared__ C sinv;
+  __shared__ C urow[2][kSB];            // the pivot and its row in the sub-panel
   __shared__ C ublk[kSB][kPanelW];      // sub-panel U rows for the rank-nb update
-  __shared__ C piv;
   const DevFront f = fr[fl[blockIdx.x / kPanelCluster]];
   C *F = pool + f.off;
   const int m = f.m, p = f.p;
@@ -423,23 +467,21 @@ __global__ void __cluster_dims__(kPanelCluster, 1, 1) __launch_bounds__(256)
   for (int jb = 0; jb < ww; jb += kSB) {
     const int nb = min(kSB, ww - jb);
     const int c0 = k0 + jb, c1 = c0 + nb;
+    T best = -1;  // local candidate over owned rows; later columns': with the update
+    int bi = p;
+    for (int r = max(ra, c0) + tid; r < rb; r += nt)
+      take_best(cabs1(P[(c0 - k0) * ldp + r - ra]), r, best, bi);
     for (int col = c0; col < c1; ++col) {
       const int cc = col - k0;
-      T best = -1;
-      int bi = p;
-      for (int r = max(ra, col) + tid; r < rb; r += nt) {
-        const T a = cabs1(P[cc * ldp + r - ra]);
-        if (a > best) { best = a; bi = r; }
-      }
-      block_argmax(best, bi, sval, sidx);
+      block_argmax(best, bi, sval[col & 1], sidx[col & 1]);
       if (tid == 0) {
         cval = best;
         cidx = bi;
       }
       cluster.sync();
-      const int gi = cluster_argmax<T, kPanelCluster>(cluster, &cval, &cidx, p, gsel);
-      const int pr = gi < p ? gi : col;
-      if (q == 0) {
+      if (q == 0) {  // picks the pivot out of the CTAs' candidates
+        const int gi = cluster_argmax<T, kPanelCluster>(cluster, &cval, &cidx, p, gsel);
+        const int pr = gi < p ? gi : col;
         if (tid == 0) ipiv[f.toff + col] = pr;
         if (pr != col) {
           // owner of row pr and its local row (CTA 0 owns [k0, top_end))
@@ -459,22 +501,16 @@ __global__ void __cluster_dims__(kPanelCluster, 1, 1) __launch_bounds__(256)
         }
       }
       cluster.sync();
-      if (tid == 0) piv = P0[cc * ldp + col - k0];
-      if (tid < c1 - col - 1) urow[tid] = P0[(cc + 1 + tid) * ldp + col - k0];
+      C *ur = urow[col & 1];
+      if (tid < c1 - col) ur[tid] = P0[(cc + tid) * ldp + col - k0];
       __syncthreads();
-      const C inv = cinv(piv);
-      const int r0 = max(ra, col + 1);
-      for (int r = r0 + tid; r < rb; r += nt)
-        P[cc * ldp + r - ra] = cmul(P[cc * ldp + r - ra], inv);
-      __syncthreads();
-      const int nr = rb - r0, nc = c1 - col - 1;
-      for (int x = tid; x < nr * nc; x += nt) {
-        const int r = r0 + x % nr, c = col + 1 + x / nr;
-        P[(c - k0) * ldp + r - ra] =
-            cfms(P[(c - k0) * ldp + r - ra], P[cc * ldp + r - ra], urow[c - col - 1]);
-      }
-      __syncthreads();
+      best = -1;
+      bi = p;
+      column_step(
+          P + cc * ldp - ra, ldp, max(ra, col + 1), rb, c1 - col - 1, ur[0],
+          [&](int j) { return ur[1 + j]; }, &sinv, best, bi);
     }
+    __syncthreads();
     if (c1 >= k0 + ww) break;
     if (q == 0) {
       for (int x = tid; x < nb * nb; x += nt)
@@ -539,55 +575,85 @@ __global__ void k_swap(const int *__restrict__ fl, int s, int w, C *__restrict__
 }
 
 // L21 = F21 U_kk^-1 on the border rows p..m-1 of the panel columns.  CTA =
-// 32 border rows x all ww columns staged in shared memory; column-oriented
-// substitution with all 256 threads: x_c = t_c / U_cc, then t_c' -= x_c U_cc'
-// for every later column c' (one barrier per step).
+// 32 border rows x all ww columns staged in shared memory, in blocks of kTB
+// columns: one warp solves a block with a row per lane in registers (x_c = t_c
+// / U_cc, then t_c' -= x_c U_cc'), then all warps subtract its products from the
+// columns after it, every element in the order c = 0, 1, ... of a column-by-
+// column substitution, so the bits do not depend on kTB.  Bound by latency: 2
+// ww / kTB barriers instead of 2 ww, and products out of registers (60 x 32: 32.7
+// -> 18.5 us per launch on average, k_trsm_urow 24.9 -> 21.9 us; with the
+// panels' fewer barriers a complex64 factorisation takes 10.7 instead of 11.7 ms
+// at 60 x 32, 117 instead of 126 at 200 x 128, 315 instead of 334 at 300 x 192,
+// a complex128 one 38 instead of 42 at 60 x 32, 181 instead of 188 at 150 x 64).
+template <class C>
+constexpr int kTBlock = sizeof(C) == sizeof(float2) ? 16 : 4;  // FP64: one warp is slow
+
 template <class C>
 __global__ void __launch_bounds__(256)
     k_trsm_border(const int *__restrict__ fl, int s, int w, C *__restrict__ pool,
                   const DevFront *__restrict__ fr) {
+  constexpr int kTB = kTBlock<C>;
   extern __shared__ __align__(16) unsigned char sm[];
   C *U = reinterpret_cast<C *>(sm);  // ww x ww, column-major U[c * w + r]
   C *T = U + w * w;                  // [ww][33]: T[c * 33 + rr]
+  C *dinv = T + w * 33;              // 1 / U_cc
   const DevFront f = fr[fl[blockIdx.y]];
   const int k0 = s * w, ww = min(w, f.p - k0);
   const int m = f.m;
   const int r0 = f.p + blockIdx.x * 32;
   if (r0 >= m) return;
   const int nr = min(32, m - r0);
+  const int rr = threadIdx.x & 31, wp = threadIdx.x >> 5;
   C *F = pool + f.off;
   for (int x = threadIdx.x; x < ww * ww; x += blockDim.x) {
     const int r = x % ww, c = x / ww;
-    U[c * w + r] = F[(long long)(k0 + c) * m + k0 + r];
+    const C v = F[(long long)(k0 + c) * m + k0 + r];
+    U[c * w + r] = v;
+    if (r == c) dinv[c] = cinv(v);
   }
-  for (int x = threadIdx.x; x < ww * 32; x += blockDim.x) {
-    const int rr = x & 31, c = x >> 5;
+  for (int c = wp; c < ww; c += 8)
     T[c * 33 + rr] = rr < nr ? F[(long long)(k0 + c) * m + r0 + rr] : czero<C>();
-  }
   __syncthreads();
-  for (int c = 0; c < ww; ++c) {
-    if (threadIdx.x < 32) T[c * 33 + threadIdx.x] = cmul(T[c * 33 + threadIdx.x], cinv(U[c * w + c]));
+  for (int b = 0; b < ww; b += kTB) {
+    const int nb = min(kTB, ww - b);
+    C x[kTB];
+    if (wp == 0) {
+#pragma unroll
+      for (int j = 0; j < kTB; ++j) x[j] = j < nb ? T[(b + j) * 33 + rr] : czero<C>();
+#pragma unroll
+      for (int j = 0; j < kTB; ++j)
+        if (j < nb) {
+          x[j] = cmul(x[j], dinv[b + j]);
+          T[(b + j) * 33 + rr] = x[j];
+#pragma unroll
+          for (int i = j + 1; i < kTB; ++i)
+            if (i < nb) x[i] = cfms(x[i], x[j], U[(b + i) * w + b + j]);
+        }
+    }
     __syncthreads();
-    for (int x = threadIdx.x; x < (ww - 1 - c) * 32; x += blockDim.x) {
-      const int cp = c + 1 + (x >> 5), rr = x & 31;
-      T[cp * 33 + rr] = cfms(T[cp * 33 + rr], T[c * 33 + rr], U[cp * w + c]);
+    if (b + kTB >= ww) break;
+#pragma unroll
+    for (int j = 0; j < kTB; ++j) x[j] = T[(b + j) * 33 + rr];
+    for (int c = b + kTB + wp; c < ww; c += 8) {
+      C v = T[c * 33 + rr];
+#pragma unroll
+      for (int j = 0; j < kTB; ++j) v = cfms(v, x[j], U[c * w + b + j]);
+      T[c * 33 + rr] = v;
     }
     __syncthreads();
   }
-  for (int x = threadIdx.x; x < ww * 32; x += blockDim.x) {
-    const int rr = x & 31, c = x >> 5;
+  for (int c = wp; c < ww; c += 8)
     if (rr < nr) F[(long long)(k0 + c) * m + r0 + rr] = T[c * 33 + rr];
-  }
 }
 
 // U12 = L_kk^-1 F12 for columns k0+ww..m-1 (unit lower L_kk).  CTA = 32
-// columns x all ww rows staged in shared memory; column-oriented forward
-// substitution with all 256 threads: row q final, then t_r -= L_rq t_q for
-// r > q (one barrier per step).
+// columns x all ww rows staged in shared memory; forward substitution in blocks
+// of kTB rows, as in k_trsm_border: t_r -= L_rq t_q for q = 0, 1, ...
 template <class C>
 __global__ void __launch_bounds__(256)
     k_trsm_urow(const int *__restrict__ fl, int s, int w, C *__restrict__ pool,
                 const DevFront *__restrict__ fr) {
+  constexpr int kTB = kTBlock<C>;
   extern __shared__ __align__(16) unsigned char sm[];
   C *Lk = reinterpret_cast<C *>(sm);  // ww x ww, column-major Lk[c * w + r]
   C *T = Lk + w * w;                  // [ww][33]: T[q * 33 + cc]
@@ -597,26 +663,47 @@ __global__ void __launch_bounds__(256)
   const int c0 = k0 + ww + blockIdx.x * 32;
   if (c0 >= m) return;
   const int nc = min(32, m - c0);
+  const int cc = threadIdx.x & 31, wp = threadIdx.x >> 5;
   C *F = pool + f.off;
   for (int x = threadIdx.x; x < ww * ww; x += blockDim.x) {
     const int r = x % ww, c = x / ww;
     Lk[c * w + r] = F[(long long)(k0 + c) * m + k0 + r];
   }
   for (int x = threadIdx.x; x < ww * 32; x += blockDim.x) {
-    const int q = x % ww, cc = x / ww;
-    T[q * 33 + cc] = cc < nc ? F[(long long)(c0 + cc) * m + k0 + q] : czero<C>();
+    const int q = x % ww, c = x / ww;
+    T[q * 33 + c] = c < nc ? F[(long long)(c0 + c) * m + k0 + q] : czero<C>();
   }
   __syncthreads();
-  for (int q = 0; q + 1 < ww; ++q) {
-    for (int x = threadIdx.x; x < (ww - 1 - q) * 32; x += blockDim.x) {
-      const int r = q + 1 + (x >> 5), cc = x & 31;
-      T[r * 33 + cc] = cfms(T[r * 33 + cc], Lk[q * w + r], T[q * 33 + cc]);
+  for (int b = 0; b < ww; b += kTB) {
+    const int nb = min(kTB, ww - b);
+    C x[kTB];
+    if (wp == 0) {
+#pragma unroll
+      for (int j = 0; j < kTB; ++j) x[j] = j < nb ? T[(b + j) * 33 + cc] : czero<C>();
+#pragma unroll
+      for (int j = 0; j < kTB; ++j)
+        if (j < nb) {
+          T[(b + j) * 33 + cc] = x[j];
+#pragma unroll
+          for (int i = j + 1; i < kTB; ++i)
+            if (i < nb) x[i] = cfms(x[i], Lk[(b + j) * w + b + i], x[j]);
+        }
+    }
+    __syncthreads();
+    if (b + kTB >= ww) break;
+#pragma unroll
+    for (int j = 0; j < kTB; ++j) x[j] = T[(b + j) * 33 + cc];
+    for (int r = b + kTB + wp; r < ww; r += 8) {
+      C v = T[r * 33 + cc];
+#pragma unroll
+      for (int j = 0; j < kTB; ++j) v = cfms(v, Lk[(b + j) * w + r], x[j]);
+      T[r * 33 + cc] = v;
     }
     __syncthreads();
   }
   for (int x = threadIdx.x; x < ww * 32; x += blockDim.x) {
-    const int q = x % ww, cc = x / ww;
-    if (cc < nc) F[(long long)(c0 + cc) * m + k0 + q] = T[q * 33 + cc];
+    const int q = x % ww, c = x / ww;
+    if (c < nc) F[(long long)(c0 + c) * m + k0 + q] = T[q * 33 + c];
   }
 }
 
@@ -2656,7 +2743,7 @@ int Factor::factor_impl(tlr_ctx *ctx, double sr, double si, double tiny) {
   C *P = static_cast<C *>(pool);
   TLR_CUDA(ctx, cudaMemsetAsync(d_pert, 0, sizeof(int), st));
   TLR_CUDA(ctx, cudaMemsetAsync(d_tc_err, 0, sizeof(int), st));
-  const size_t tsm = sizeof(C) * (size_t)(w * w + w * 33);
+  const size_t tsm = sizeof(C) * (size_t)(w * w + w * 34);
   TLR_CUDA(ctx, cudaFuncSetAttribute(k_trsm_border<C>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
   TLR_CUDA(ctx, cudaFuncSetAttribute(k_trsm_urow<C>,
