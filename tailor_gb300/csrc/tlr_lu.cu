@@ -176,21 +176,31 @@ __device__ __forceinline__ void column_step(C *a, long long ld, int r0, int r1, 
   }
 }
 
-template <class C>
+template <class C, bool SM>
 __global__ void __launch_bounds__(512)
     k_panel(const int *__restrict__ fl, int s, int w, C *__restrict__ pool,
             const DevFront *__restrict__ fr, int *__restrict__ ipiv,
-            int *__restrict__ pert, double tiny) {
+            int *__restrict__ pert, double tiny, int ldp) {
   using T = typename Real<C>::T;
   __shared__ T sval[2][32];
   __shared__ int sidx[2][32];
   __shared__ C lsub[kSB][kSB];
   __shared__ C sinv;
   const DevFront f = fr[fl[blockIdx.x]];
-  C *F = pool + f.off;
-  const int m = f.m, p = f.p;
-  const int k0 = s * w, ww = min(w, p - k0);
-  const int tid = threadIdx.x, nt = blockDim.x;
+  const int p = f.p, k0 = s * w, ww = min(w, p - k0);
+  const int tid = threadIdx.x, nt = blockDim.x, rows = p - k0;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C *G = pool + f.off + (long long)k0 * f.m + k0;
+  // F[c m + r]: row r, column c of the front, in the staged copy or in place
+  C *F = SM ? reinterpret_cast<C *>(smem_raw) - (long long)k0 * ldp - k0 : pool + f.off;
+  const int m = SM ? ldp : f.m;
+  if (SM) {
+    for (int x = tid; x < rows * ww; x += nt) {
+      const int c = x / rows, r = x - c * rows;
+      F[(long long)(k0 + c) * m + k0 + r] = G[(long long)c * f.m + r];
+    }
+    __syncthreads();
+  }
   for (int jb = 0; jb < ww; jb += kSB) {
     const int nb = min(kSB, ww - jb);
     const int c0 = k0 + jb, c1 = c0 + nb;  // sub-panel columns [c0, c1)
@@ -251,6 +261,11 @@ __global__ void __launch_bounds__(512)
     }
     __syncthreads();
   }
+  if (SM)
+    for (int x = tid; x < rows * ww; x += nt) {
+      const int c = x / rows, r = x - c * rows;
+      G[(long long)c * f.m + r] = F[(long long)(k0 + c) * m + k0 + r];
+    }
 }
 
 // The cluster-wide pivot: the largest candidate value over the KC CTAs,
@@ -2751,6 +2766,8 @@ int Factor::factor_impl(tlr_ctx *ctx, double sr, double si, double tiny) {
   TLR_CUDA(ctx, cudaFuncSetAttribute(k_panel_cluster_sm<C>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)kPanelSmemMax));
+  TLR_CUDA(ctx, cudaFuncSetAttribute(k_panel<C, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)kPanelSmemMax));
   for (size_t h = 0; h < levels.size(); ++h) {
     const Level &L = levels[h];
     TLR_CUDA(ctx, cudaMemsetAsync(P + L.pool_begin, 0,
@@ -2780,8 +2797,10 @@ int Factor::factor_impl(tlr_ctx *ctx, double sr, double si, double tiny) {
         { k_panel_cluster_sm<C><<<S.nf * kPanelCluster, 256, psm, st>>>(fl, s, w, P, d_fronts, d_ipiv, d_pert, tiny, ldp); count_launches(); }
       else if (cluster)
         { k_panel_cluster<C><<<S.nf * kPanelCluster, 256, 0, st>>>(fl, s, w, P, d_fronts, d_ipiv, d_pert, tiny); count_launches(); }
+      else if (const size_t ssm = (size_t)w * (rem | 1) * sizeof(C); ssm <= kPanelSmemMax)
+        { k_panel<C, true><<<S.nf, 512, ssm, st>>>(fl, s, w, P, d_fronts, d_ipiv, d_pert, tiny, rem | 1); count_launches(); }
       else
-        { k_panel<C><<<S.nf, 512, 0, st>>>(fl, s, w, P, d_fronts, d_ipiv, d_pert, tiny); count_launches(); }
+        { k_panel<C, false><<<S.nf, 512, 0, st>>>(fl, s, w, P, d_fronts, d_ipiv, d_pert, tiny, 0); count_launches(); }
       { k_swap<C><<<dim3(blocks_for(S.max_m, 128), S.nf), 128, 0, st>>>(fl, s, w, P, d_fronts,
                                                                        d_ipiv); count_launches(); }
       if (S.max_b > 0)
