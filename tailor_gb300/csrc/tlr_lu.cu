@@ -77,22 +77,31 @@ __global__ void k_extend(const int *__restrict__ kids, const DevFront *__restric
   }
 }
 
-template <class T>
-__device__ __forceinline__ void warp_argmax(T &best, int &bi) {  // result in lane 0
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const T a = __shfl_down_sync(0xffffffffu, best, o);
-    const int ia = __shfl_down_sync(0xffffffffu, bi, o);
-    if (a > best || (a == best && ia < bi)) {
-      best = a;
-      bi = ia;
-    }
-  }
+// Warp-wide argmax of (value, row) pairs, to all lanes: largest value, ties to
+// the smaller row.  By integer reductions of the value's bits (an absolute
+// value, or negative for none): a chain of five shuffles and compares twice per
+// column took a sixth of a panel (60 x 32: 72 -> 62 us per 64 columns on average in
+// k_panel).
+__device__ __forceinline__ void warp_argmax(float &best, int &bi) {
+  const unsigned key = best < 0.f ? 0u : __float_as_uint(best) + 1u;
+  const unsigned top = __reduce_max_sync(0xffffffffu, key);
+  bi = __reduce_min_sync(0xffffffffu, key == top ? bi : 0x7fffffff);
+  best = top ? __uint_as_float(top - 1u) : -1.f;
+}
+
+__device__ __forceinline__ void warp_argmax(double &best, int &bi) {
+  const int hi = best < 0.0 ? -1 : __double2hiint(best);
+  const int top = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned lo = hi == top ? (unsigned)__double2loint(best) : 0u;
+  const unsigned tlo = __reduce_max_sync(0xffffffffu, lo);
+  const bool mine = hi == top && (hi < 0 || lo == tlo);
+  bi = __reduce_min_sync(0xffffffffu, mine ? bi : 0x7fffffff);
+  best = top < 0 ? -1.0 : __hiloint2double(top, (int)tlo);
 }
 
 // Block-wide argmax of (value, row) pairs: largest value, ties to the
 // smaller row; warp shuffles, then every warp over the warp winners, so one
-// barrier is enough.  The result is in lane 0 of every warp (row: all lanes).
+// barrier is enough.
 // wval / widx: 32 entries, alternate ones for successive calls.
 template <class T>
 __device__ __forceinline__ void block_argmax(T &best, int &bi, T *wval, int *widx) {
@@ -106,7 +115,6 @@ __device__ __forceinline__ void block_argmax(T &best, int &bi, T *wval, int *wid
   best = lane < nw ? wval[lane] : T(-2);
   bi = lane < nw ? widx[lane] : 0x7fffffff;
   warp_argmax(best, bi);
-  bi = __shfl_sync(0xffffffffu, bi, 0);
 }
 
 // Panel factorisation of step s for one front per CTA: columns k0..k0+ww,
@@ -117,7 +125,9 @@ __device__ __forceinline__ void block_argmax(T &best, int &bi, T *wval, int *wid
 // update below), so each panel element crosses L2 ww/kSB times instead of
 // ww times.  Bound by the latency of a column; the update of a column looks for
 // the next pivot on the way, and of the eight barriers per column two are left
-// (complex128: four).
+// (complex128: four).  SM: the panel is staged in shared memory (whenever it
+// fits; ldp: its leading dimension), 72 us per 64 columns on average at 60 x 32
+// against 100 us through L1 and L2.
 constexpr int kSB = 8;
 
 // best = the largest |a| (and its row) of one thread's rows in a column
@@ -271,7 +281,7 @@ __global__ void __launch_bounds__(512)
 // The cluster-wide pivot: the largest candidate value over the KC CTAs,
 // ties to the smaller row (the order of a sequential scan over the CTAs).
 // Warp 0 reads one candidate per lane from the other CTAs' shared memory
-// and reduces with shuffles; the winner is broadcast through shared memory.
+// and reduces them; the winner is broadcast through shared memory.
 template <class T, int KC>
 __device__ __forceinline__ int cluster_argmax(cooperative_groups::cluster_group &cluster,
                                               T *cval, int *cidx, int none, int *gsel) {
@@ -283,15 +293,7 @@ __device__ __forceinline__ int cluster_argmax(cooperative_groups::cluster_group 
       a = *cluster.map_shared_rank(cval, lane);
       ia = *cluster.map_shared_rank(cidx, lane);
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const T a2 = __shfl_down_sync(0xffffffffu, a, o);
-      const int i2 = __shfl_down_sync(0xffffffffu, ia, o);
-      if (a2 > a || (a2 == a && i2 < ia)) {
-        a = a2;
-        ia = i2;
-      }
-    }
+    warp_argmax(a, ia);
     if (lane == 0) gsel[0] = ia;
   }
   __syncthreads();
@@ -434,13 +436,18 @@ __global__ void __cluster_dims__(kPanelCluster, 1, 1) __launch_bounds__(256)
 // The cluster panel with the panel held in distributed shared memory: each
 // CTA loads its rows of the ww panel columns once (column-major, leading
 // dimension ldp), factors them in shared memory and writes them back at the
-// end, so a column step costs two cluster barriers and a few shared-memory
-// passes instead of several round trips through L2.  CTA 0 owns the top ww
-// rows (pivot rows land there and the sub-panels' U rows live there);
-// CTAs 1.. own contiguous chunks of the rest.  The pivot row swap is done
-// by CTA 0 alone (its own row and the remote row through DSMEM); the other
-// CTAs read the pivot and the sub-panel's U entries from CTA 0.  Pivots,
-// tie-breaking and every arithmetic operation are those of k_panel.
+// end.  CTA 0 owns the top ww rows (pivot rows land there and the sub-panels' U
+// rows live there); CTAs 1.. own contiguous chunks of the rest.  Bound by the
+// latency of a column step, so it takes one cluster barrier and no remote
+// read on its way: before the barrier every CTA sends its candidate (value, row,
+// and the row's entries in the sub-panel) to all of them, and CTA 0 its row col;
+// after it every CTA picks the same winner, has the pivot row at hand, and the
+// two owners exchange the rows' sub-panel entries.  The rows' other columns,
+// which nobody reads before the sub-panel ends, CTA 0 swaps alone, with its
+// remote reads in flight during the update: 152 -> 119 us per 64 columns on
+// average at 60 x 32, factorisations of 110 instead of 116 ms at 200 x 128 and 306
+// instead of 314 ms at 300 x 192 (with the integer argmax).  Pivots, tie-breaking
+// and every arithmetic operation are those of k_panel.
 template <class C>
 __global__ void __cluster_dims__(kPanelCluster, 1, 1) __launch_bounds__(256)
     k_panel_cluster_sm(const int *__restrict__ fl, int s, int w, C *__restrict__ pool,
@@ -454,12 +461,12 @@ __global__ void __cluster_dims__(kPanelCluster, 1, 1) __launch_bounds__(256)
   C *P = reinterpret_cast<C *>(smem_raw);  // P[(c - k0) * ldp + (r - ra)]
   __shared__ T sval[2][32];
   __shared__ int sidx[2][32];
-  __shared__ T cval;
-  __shared__ int cidx;
-  __shared__ int gsel[1];
+  __shared__ T rval[2][kPanelCluster];  // the CTAs' candidates, alternate columns
+  __shared__ int ridx[2][kPanelCluster];
+  __shared__ C rrow[2][kPanelCluster][kSB];
+  __shared__ C rtop[2][kSB];            // CTA 0's row col in the sub-panel
   __shared__ C lsub[kSB][kSB];
   __shared__ C sinv;
-  __shared__ C urow[2][kSB];            // the pivot and its row in the sub-panel
   __shared__ C ublk[kSB][kPanelW];      // sub-panel U rows for the rank-nb update
   const DevFront f = fr[fl[blockIdx.x / kPanelCluster]];
   C *F = pool + f.off;
@@ -489,41 +496,56 @@ __global__ void __cluster_dims__(kPanelCluster, 1, 1) __launch_bounds__(256)
     for (int col = c0; col < c1; ++col) {
       const int cc = col - k0;
       block_argmax(best, bi, sval[col & 1], sidx[col & 1]);
-      if (tid == 0) {
-        cval = best;
-        cidx = bi;
+      const int par = col & 1;
+      if (tid < 8 * kPanelCluster) {
+        const int d = tid % kPanelCluster, j = tid / kPanelCluster;
+        if (j < nb && bi < p)
+          *cluster.map_shared_rank(&rrow[par][q][j], d) = P[(c0 - k0 + j) * ldp + bi - ra];
+        if (j == 0) {
+          *cluster.map_shared_rank(&rval[par][q], d) = best;
+          *cluster.map_shared_rank(&ridx[par][q], d) = bi;
+        }
+      } else if (q == 0 && tid < 16 * kPanelCluster) {
+        const int d = tid % kPanelCluster, j = tid / kPanelCluster - 8;
+        if (j < nb)
+          *cluster.map_shared_rank(&rtop[par][j], d) = P[(c0 - k0 + j) * ldp + col - k0];
       }
       cluster.sync();
-      if (q == 0) {  // picks the pivot out of the CTAs' candidates
-        const int gi = cluster_argmax<T, kPanelCluster>(cluster, &cval, &cidx, p, gsel);
-        const int pr = gi < p ? gi : col;
-        if (tid == 0) ipiv[f.toff + col] = pr;
-        if (pr != col) {
-          // owner of row pr and its local row (CTA 0 owns [k0, top_end))
-          const int qo = pr < top_end ? 0 : 1 + (pr - top_end) / chunk;
-          const int ro = pr - (qo == 0 ? k0 : top_end + (qo - 1) * chunk);
-          C *Po = cluster.map_shared_rank(P, qo);
-          for (int c = tid; c < ww; c += nt) {
-            const C t = P[c * ldp + col - k0];
-            P[c * ldp + col - k0] = Po[c * ldp + ro];
-            Po[c * ldp + ro] = t;
-          }
+      T gv = (tid & 31) < kPanelCluster ? rval[par][tid & 31] : T(-2);
+      int gi = (tid & 31) < kPanelCluster ? ridx[par][tid & 31] : p;
+      warp_argmax(gv, gi);
+      const int pr = gi < p ? gi : col;
+      // owner of row pr (CTA 0 owns [k0, top_end)) and its local row
+      const int qo = pr < top_end ? 0 : 1 + (pr - top_end) / chunk;
+      const int ro = pr - (qo == 0 ? k0 : top_end + (qo - 1) * chunk);
+      const C *prow = gi < p ? rrow[par][qo] : rtop[par];
+      C pv = prow[col - c0];
+      const bool zero = cabs1(pv) == T(0);
+      if (zero) pv = cmake<C>((T)tiny, 0);
+      if (q == 0) {
+        if (tid == 0) {
+          ipiv[f.toff + col] = pr;
+          if (zero) atomicAdd(pert, 1);
         }
-        __syncthreads();  // the pivot's own column may have been swapped by another thread
-        if (tid == 0 && cabs1(P[cc * ldp + col - k0]) == T(0)) {
-          P[cc * ldp + col - k0] = cmake<C>((T)tiny, 0);
-          atomicAdd(pert, 1);
-        }
+        if (tid < nb) P[(c0 - k0 + tid) * ldp + col - k0] = tid == col - c0 ? pv : prow[tid];
       }
-      cluster.sync();
-      C *ur = urow[col & 1];
-      if (tid < c1 - col) ur[tid] = P0[(cc + tid) * ldp + col - k0];
+      if (q == qo && pr != col && tid >= 32 && tid < 32 + nb)
+        P[(c0 - k0 + tid - 32) * ldp + ro] = rtop[par][tid - 32];
       __syncthreads();
+      const bool other = q == 0 && pr != col && tid < ww - nb;
+      const int oc = (tid < c0 - k0 ? tid : tid + nb) * ldp;  // a column outside the sub-panel
+      C *Po = cluster.map_shared_rank(P, qo);
+      C rem = czero<C>();
+      if (other) rem = Po[oc + ro];
       best = -1;
       bi = p;
       column_step(
-          P + cc * ldp - ra, ldp, max(ra, col + 1), rb, c1 - col - 1, ur[0],
-          [&](int j) { return ur[1 + j]; }, &sinv, best, bi);
+          P + cc * ldp - ra, ldp, max(ra, col + 1), rb, c1 - col - 1, pv,
+          [&](int j) { return prow[col - c0 + 1 + j]; }, &sinv, best, bi);
+      if (other) {
+        Po[oc + ro] = P[oc + col - k0];
+        P[oc + col - k0] = rem;
+      }
     }
     __syncthreads();
     if (c1 >= k0 + ww) break;
