@@ -189,7 +189,13 @@ typedef struct {
   double tol;             /* 0: recipe value                                */
   int max_it;             /* 0: recipe value                                */
   int precision;          /* 0: FP64 factorisation (drop-in form);
-                             1: FP32 factorisation + FP64 refinement       */
+                             1: FP32 factorisation, K^-1 applications
+                             refined against the FP64 operator until ||r||
+                             <= 1e-12 ||y||; consecutive applications are
+                             pipelined (three right-hand sides per
+                             triangular solve) unless block > 1,
+                             refinement or fp64_acceptance asks for the
+                             single ones                                    */
   double sigma_re, sigma_im; /* used when use_sigma != 0                    */
   int use_sigma;          /* 0: sigma = lambda target from omega            */
   const double *start;    /* optional complex [5N] host start vector        */
@@ -203,7 +209,8 @@ typedef struct {
                              the next tile's MMAs); FP64 form with panels of
                              32 columns (its default): tcgen05 on exact
                              integer slices of 56 bits, one FP64 rounding per
-                             entry and panel; other panel widths: CUDA-core
+                             entry and panel, and of 64 bits in the final
+                             rewrite of the factor; other panel widths: CUDA-core
                              FP64 FMA.
                              1: CUDA cores (FP32 / FP64 FMA).  2: mixed form
                              on tcgen05 with every tile staging its own
@@ -235,8 +242,9 @@ typedef struct {
                              summed rows are left (1: always); 0 (default):
                              256; -1: never.  The cluster keeps the
                              panel in distributed shared memory when its
-                             rows fit (up to about 3000 rows at complex64,
-                             64 columns)                                */
+                             rows fit: up to about 2800 rows at 64 columns
+                             of complex64, 6000 on 16 CTAs, which taller
+                             panels use                                     */
   int persistent_solve;   /* 0 (default): each triangular solve replays a
                              CUDA graph of per-step launches; 1: one
                              persistent cooperative launch with grid
@@ -276,8 +284,11 @@ typedef struct {
                              the operator to the next vector.  0: every 4
                              (default); -1: only when the basis is full, as
                              SLEPc                                          */
-  int solve_wave;         /* triangular solves: 0 (default) one launch per
-                             block step; 1 one dependency-driven launch per
+  int solve_wave;         /* block-step triangular solves (the FP64 form;
+                             the mixed form's inverse-form factor takes one
+                             launch per level and direction and ignores
+                             this): 0 (default) one launch per block step;
+                             1 one dependency-driven launch per
                              direction for every level whose fronts have
                              several diagonal blocks (32-row tiles wait only
                              for the blocks they need, bounded waits).  Same
@@ -305,7 +316,9 @@ typedef struct {
   double factor_bytes;    /* bytes of the stored L and U factors            */
   double trisolve_ms;     /* device time of the triangular solves (CUDA
                              events around each solve graph)               */
-  int trisolves;          /* triangular solves timed in trisolve_ms         */
+  int trisolves;          /* triangular solves timed in trisolve_ms (a
+                             pipelined one solves three right-hand sides
+                             and counts once here, three times in solves)   */
   double ortho_ms;        /* Gram-Schmidt of the Arnoldi steps (host clock) */
   double dense_ms;        /* projected Schur problem on the host            */
   double residual_ms;     /* Ritz vectors and explicit residuals            */

@@ -448,8 +448,12 @@ __global__ void __cluster_dims__(kPanelCluster, 1, 1) __launch_bounds__(256)
 // average at 60 x 32, factorisations of 110 instead of 116 ms at 200 x 128 and 306
 // instead of 314 ms at 300 x 192 (with the integer argmax).  Pivots, tie-breaking
 // and every arithmetic operation are those of k_panel.
-template <class C>
-__global__ void __cluster_dims__(kPanelCluster, 1, 1) __launch_bounds__(256)
+// KC = 16 (a cluster size that has to be opted into) for panels whose rows do not
+// fit eight CTAs, 2800 to 6000 rows at 64 columns: through L2 (k_panel_cluster) such
+// a panel took 835 us, the factorisations 306 and 110 ms at 300 x 192 and 200 x 128
+// instead of 286 and 107.
+template <class C, int KC>
+__global__ void __cluster_dims__(KC, 1, 1) __launch_bounds__(256)
     k_panel_cluster_sm(const int *__restrict__ fl, int s, int w, C *__restrict__ pool,
                        const DevFront *__restrict__ fr, int *__restrict__ ipiv,
                        int *__restrict__ pert, double tiny, int ldp) {
@@ -461,21 +465,21 @@ __global__ void __cluster_dims__(kPanelCluster, 1, 1) __launch_bounds__(256)
   C *P = reinterpret_cast<C *>(smem_raw);  // P[(c - k0) * ldp + (r - ra)]
   __shared__ T sval[2][32];
   __shared__ int sidx[2][32];
-  __shared__ T rval[2][kPanelCluster];  // the CTAs' candidates, alternate columns
-  __shared__ int ridx[2][kPanelCluster];
-  __shared__ C rrow[2][kPanelCluster][kSB];
+  __shared__ T rval[2][KC];  // the CTAs' candidates, alternate columns
+  __shared__ int ridx[2][KC];
+  __shared__ C rrow[2][KC][kSB];
   __shared__ C rtop[2][kSB];            // CTA 0's row col in the sub-panel
   __shared__ C lsub[kSB][kSB];
   __shared__ C sinv;
   __shared__ C ublk[kSB][kPanelW];      // sub-panel U rows for the rank-nb update
-  const DevFront f = fr[fl[blockIdx.x / kPanelCluster]];
+  const DevFront f = fr[fl[blockIdx.x / KC]];
   C *F = pool + f.off;
   const int m = f.m, p = f.p;
   const int k0 = s * w, ww = min(w, p - k0);
   const int tid = threadIdx.x, nt = blockDim.x;
   const int top_end = k0 + ww;
   const int rest = p - top_end;
-  const int chunk = (rest + kPanelCluster - 2) / (kPanelCluster - 1);
+  const int chunk = (rest + KC - 2) / (KC - 1);
   const int ra = q == 0 ? k0 : min(p, top_end + (q - 1) * chunk);
   const int rb = q == 0 ? top_end : min(p, ra + chunk);
   const int nown = rb - ra;
@@ -497,22 +501,22 @@ __global__ void __cluster_dims__(kPanelCluster, 1, 1) __launch_bounds__(256)
       const int cc = col - k0;
       block_argmax(best, bi, sval[col & 1], sidx[col & 1]);
       const int par = col & 1;
-      if (tid < 8 * kPanelCluster) {
-        const int d = tid % kPanelCluster, j = tid / kPanelCluster;
+      if (tid < kSB * KC) {
+        const int d = tid % KC, j = tid / KC;
         if (j < nb && bi < p)
           *cluster.map_shared_rank(&rrow[par][q][j], d) = P[(c0 - k0 + j) * ldp + bi - ra];
         if (j == 0) {
           *cluster.map_shared_rank(&rval[par][q], d) = best;
           *cluster.map_shared_rank(&ridx[par][q], d) = bi;
         }
-      } else if (q == 0 && tid < 16 * kPanelCluster) {
-        const int d = tid % kPanelCluster, j = tid / kPanelCluster - 8;
+      } else if (q == 0 && tid < 2 * kSB * KC) {
+        const int d = tid % KC, j = tid / KC - kSB;
         if (j < nb)
           *cluster.map_shared_rank(&rtop[par][j], d) = P[(c0 - k0 + j) * ldp + col - k0];
       }
       cluster.sync();
-      T gv = (tid & 31) < kPanelCluster ? rval[par][tid & 31] : T(-2);
-      int gi = (tid & 31) < kPanelCluster ? ridx[par][tid & 31] : p;
+      T gv = (tid & 31) < KC ? rval[par][tid & 31] : T(-2);
+      int gi = (tid & 31) < KC ? ridx[par][tid & 31] : p;
       warp_argmax(gv, gi);
       const int pr = gi < p ? gi : col;
       // owner of row pr (CTA 0 owns [k0, top_end)) and its local row
@@ -2785,9 +2789,25 @@ int Factor::factor_impl(tlr_ctx *ctx, double sr, double si, double tiny) {
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
   TLR_CUDA(ctx, cudaFuncSetAttribute(k_trsm_urow<C>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
-  TLR_CUDA(ctx, cudaFuncSetAttribute(k_panel_cluster_sm<C>,
+  TLR_CUDA(ctx, cudaFuncSetAttribute(k_panel_cluster_sm<C, kPanelCluster>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)kPanelSmemMax));
+  // clusters of 16 where the device can place them
+  const bool cluster16 = [&]() {
+    auto *k = k_panel_cluster_sm<C, 16>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(16);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = kPanelSmemMax;
+    int n = 0;
+    const bool ok =
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanelSmemMax) ==
+            cudaSuccess &&
+        cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&n, k, &cfg) == cudaSuccess && n > 0;
+    cudaGetLastError();
+    return ok;
+  }();
   TLR_CUDA(ctx, cudaFuncSetAttribute(k_panel<C, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)kPanelSmemMax));
   for (size_t h = 0; h < levels.size(); ++h) {
@@ -2815,8 +2835,12 @@ int Factor::factor_impl(tlr_ctx *ctx, double sr, double si, double tiny) {
       // rows per CTA of the cluster (CTA 0: the top w rows)
       const int ldp = std::max(w, (rem + kPanelCluster - 2) / (kPanelCluster - 1));
       const size_t psm = (size_t)w * ldp * sizeof(C);
+      const int ldp16 = std::max(w, (rem + 14) / 15);
+      const size_t psm16 = (size_t)w * ldp16 * sizeof(C);
       if (cluster && psm <= kPanelSmemMax)
-        { k_panel_cluster_sm<C><<<S.nf * kPanelCluster, 256, psm, st>>>(fl, s, w, P, d_fronts, d_ipiv, d_pert, tiny, ldp); count_launches(); }
+        { k_panel_cluster_sm<C, kPanelCluster><<<S.nf * kPanelCluster, 256, psm, st>>>(fl, s, w, P, d_fronts, d_ipiv, d_pert, tiny, ldp); count_launches(); }
+      else if (cluster && cluster16 && psm16 <= kPanelSmemMax)
+        { k_panel_cluster_sm<C, 16><<<S.nf * 16, 256, psm16, st>>>(fl, s, w, P, d_fronts, d_ipiv, d_pert, tiny, ldp16); count_launches(); }
       else if (cluster)
         { k_panel_cluster<C><<<S.nf * kPanelCluster, 256, 0, st>>>(fl, s, w, P, d_fronts, d_ipiv, d_pert, tiny); count_launches(); }
       else if (const size_t ssm = (size_t)w * (rem | 1) * sizeof(C); ssm <= kPanelSmemMax)
