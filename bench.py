@@ -87,7 +87,7 @@ PLAIN_NCV = 32
 C2 = dict(ny=200, nz=128, amplitude=0.08, alpha=1.8, omega=complex(0.3, 0.01), nev=16)
 C2_NCV = 64
 GOLDEN = ROOT / "tests" / "golden"
-TRISOLVE_TRAFFIC_RATIO = 538.1 / 518.3
+TRISOLVE_TRAFFIC_RATIO = 543.9 / 519.1
 
 
 def c2_case(ny=None, nz=None):
@@ -614,17 +614,19 @@ def main():
     peaks = json.loads((ROOT / "MEASURED_PEAKS.json").read_text()) \
         if (ROOT / "MEASURED_PEAKS.json").exists() else {}
     hbm = peaks.get("hbm_gbs", 6800.0)
-    # dominant kernel: the triangular solves (one CUDA graph per solve of the
-    # block's vectors), CUDA events around every replay
+    # dominant kernel: the triangular solves (the block's vectors at a time, or
+    # the three of a pipelined application), CUDA events around every one
     nvec = last.get("block", 1)
+    nvec = 3 if nvec == 1 else nvec
     tri_bytes = last["factor_bytes"] + 2 * nvec * 5 * case.nodes * 8
     tri_ms = sum(s[3]["trisolve_ms"] for s in rsteps)
     tri_n = sum(s[3]["trisolves"] for s in rsteps)
     tri_avg_ms = tri_ms / max(tri_n, 1)
     achieved = tri_bytes / (tri_avg_ms * 1e-3) / 1e9 if tri_avg_ms > 0 else 0.0
-    # ncu DRAM bytes / algorithmic bytes of the same solve graph, measured on
-    # a 100 x 50 capture (538.1 / 518.3 MB per solve: the factor read once,
-    # plus the D_b blocks), applied to this solve's algorithmic bytes
+    # ncu DRAM bytes / algorithmic bytes of the same solves, measured on a
+    # 100 x 50 capture (543.9 / 519.1 MB per solve of three right-hand sides:
+    # the factor read once, plus indices and partial sums), applied to this
+    # solve's algorithmic bytes
     traffic = TRISOLVE_TRAFFIC_RATIO * tri_bytes
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world,
@@ -648,8 +650,8 @@ def main():
         "clocks": clk,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
                      "frac": achieved / hbm, "traffic": traffic,
-                     "kernel": "triangular solves (solve graph: k_blk_update, k_border_gemv_pf, "
-                               "k_bwd_start, k_sgather; their _m variants for blocks)",
+                     "kernel": "triangular solves (inverse form, three right-hand sides per "
+                               "solve: k_inv_apply, k_inv_gather)",
                      "algorithmic_bytes": tri_bytes, "avg_ms": tri_avg_ms,
                      "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)"},
         "factor": {"flops": last["factor_flops"], "ms": last["factor_ms"],

@@ -242,8 +242,9 @@ class EigenSolver:
         ordering (tlr_solve_opts; 0: the solver's); conv_check: operator
         applications between convergence tests inside an expansion (0: the
         solver's 4; -1: only when the basis is full); solve_wave: one
-        dependency-driven launch per level of the triangular solves instead
-        of one launch per block step (the same bits, measured slower);
+        dependency-driven launch per level of the block-step triangular
+        solves instead of one per block step (the same bits, measured
+        slower; the mixed form's inverse-form factor has no block steps);
         fp64_acceptance: accept each refined application on an FP64
         residual instead of a float-float one (mixed form)."""
         kw = dict(nev=nev, ncv=ncv, tol=tol, max_it=max_it, sigma=sigma, start=start,
