@@ -7,17 +7,20 @@
 // assembles all their K blocks, one launch per child slot extend-adds the
 // children's Schur complements, and each panel step of width w runs five
 // launches over all fronts that still have pivots left:
-//   k_panel        partial pivoting over the fully summed rows (one CTA/front)
+//   k_panel        partial pivoting over the fully summed rows (one CTA per
+//                  front; taller ones on a cluster, k_panel_cluster_sm)
 //   k_swap         the step's row interchanges on the other columns
 //   k_trsm_border  L21 = F21 U_kk^-1 for the front's border rows
 //   k_trsm_urow    U12 = L_kk^-1 F12
-//   k_gemm         trailing update F22 -= L21 U12 (the Schur complement)
+//   k_gemm         trailing update F22 -= L21 U12 (the Schur complement; by
+//                  default on the tensor cores, tlr_tc.cu and tlr_oz.cu)
 // Pivot search is restricted to fully summed rows (no delayed pivots); an
 // exactly zero pivot column is perturbed and counted, and the caller
 // refines.  After the last level every pivot block's SW x SW diagonal
 // blocks are inverted explicitly (k_tri_inv), so each solve step is a
 // parallel GEMV plus one small dense product instead of a serial
-// substitution; the solves walk the same levels.
+// substitution; the solves walk the same levels.  The mixed form goes on to
+// invert whole pivot blocks and solves with those (tlr_inv.cu).
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -2823,7 +2826,7 @@ int Factor::factor_impl(tlr_ctx *ctx, double sr, double si, double tiny) {
             cudaSuccess &&
         cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
         cudaOccupancyMaxActiveClusters(&n, k, &cfg) == cudaSuccess && n > 0;
-    cudaGetLastError();
+    if (!ok) cudaGetLastError();  // not an error of the factorisation
     return ok;
   }();
   TLR_CUDA(ctx, cudaFuncSetAttribute(k_panel<C, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,

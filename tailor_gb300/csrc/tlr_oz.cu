@@ -337,7 +337,8 @@ __device__ __forceinline__ void class_sums(uint32_t taddr, long long (&v)[8]) {
 // (a 64 x 64 tile is 524 K FMAs, 125 us on an SM): complex128 factorisation
 // 123 -> 55 ms at 60 x 32, 1191 -> 272 ms at 150 x 64 with the updates here, 42
 // and 188 ms with the rewrite here too (its CUDA-core kernels took 102 of the
-// 272 ms).  Waits are bounded as in tlr_tc.cu.
+// 272 ms; with faster panels 32 and 167 ms now).  Waits are bounded as in
+// tlr_tc.cu.
 template <class S>
 __global__ void __launch_bounds__(kThreads, 1)
     k_oz_gemm(S src, const int *__restrict__ prefix, const int *__restrict__ pa,

@@ -656,7 +656,8 @@ __global__ void __launch_bounds__(256, MINB)
 // Loads of F22 into registers wait for L1 lines and for the epilogue before
 // (DRAM 52% busy, tensor pipe 32%); with the copies the largest update at 150 x
 // 96 takes 445 instead of 511 us (62%, 36%), a factorisation 334 instead of 350
-// ms at 300 x 192 and 126 instead of 131 ms at 200 x 128.  It is now bound by
+// ms at 300 x 192 and 126 instead of 131 ms at 200 x 128 (283 and 106 ms now,
+// with faster panels).  It is now bound by
 // reading 256 KB of operand images per tile from L2 (11 TB/s over all SMs).
 // Three or five ring stages: 342 ms both; keeping a row tile's A images in
 // shared memory instead: 396 ms, its CTAs work on distant parts of F22.
