@@ -510,7 +510,9 @@ __global__ void __cluster_dims__(KC, 1, 1) __launch_bounds__(256)
     const int rr = x % nown, cc = x / nown;
     P[cc * ldp + rr] = F[(long long)(k0 + cc) * m + ra + rr];
   }
-  __syncthreads();
+  // all CTAs of the cluster run (and have their rows) before any of them writes
+  // into another's shared memory
+  cluster.sync();
   for (int jb = 0; jb < ww; jb += kSB) {
     const int nb = min(kSB, ww - jb);
     const int c0 = k0 + jb, c1 = c0 + nb;
