@@ -531,6 +531,12 @@ int tlr_fdq_rule(int node_count, int q, int periodic, double period, double *nod
  * context stays usable). */
 int tlr_wait_selftest(int which, unsigned limit, int *timed_out);
 
+/* Test hook, no counterpart in the reference: the k-th allocation of device or
+ * pinned memory that a solve on the calling thread makes from here on fails
+ * once, as if memory had run out (0: none does).  Returns the number of such
+ * allocations since the last call of this hook on the thread. */
+int tlr_alloc_fail_at(int k);
+
 /* Kernels of this library launched by the process so far (every kernel
  * node of a replayed CUDA graph counts once per replay; cuBLAS kernels are
  * not counted).  No counterpart in the reference: it lets a caller check

@@ -25,6 +25,14 @@ int cuda_fail(tlr_ctx *ctx, cudaError_t err, const char *what) {
 namespace {
 
 thread_local std::string g_error;
+// tlr_alloc_fail_at: allocations left before the failing one (0: none fails),
+// and the number made since, on this thread
+thread_local int g_fail_in = 0, g_allocs = 0;
+
+cudaError_t fail_now() {
+  ++g_allocs;
+  return g_fail_in > 0 && --g_fail_in == 0 ? cudaErrorMemoryAllocation : cudaSuccess;
+}
 
 int upload_rule(tlr_ctx *ctx, const tlr_rule *r, int expected_nodes,
                 int periodic, DevRule &d, std::vector<int> &h_off,
@@ -136,6 +144,16 @@ int copy_soa(tlr_ctx *ctx, const double *src, int comp, double *dst) {
 
 }  // namespace
 
+cudaError_t dev_malloc(void **p, size_t bytes) {
+  const cudaError_t e = fail_now();
+  return e != cudaSuccess ? e : cudaMalloc(p, bytes);
+}
+
+cudaError_t pin_malloc(void **p, size_t bytes) {
+  const cudaError_t e = fail_now();
+  return e != cudaSuccess ? e : cudaHostAlloc(p, bytes, cudaHostAllocDefault);
+}
+
 void set_global_error(const std::string &msg) { g_error = msg; }
 
 }  // namespace tlr
@@ -143,6 +161,13 @@ void set_global_error(const std::string &msg) { g_error = msg; }
 using namespace tlr;
 
 extern "C" {
+
+int tlr_alloc_fail_at(int k) {
+  const int made = g_allocs;
+  g_allocs = 0;
+  g_fail_in = std::max(k, 0);
+  return made;
+}
 
 const char *tlr_status_string(int status) {
   switch (status) {

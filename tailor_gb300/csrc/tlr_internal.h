@@ -138,6 +138,17 @@ int cuda_fail(tlr_ctx *ctx, cudaError_t err, const char *what);
     if (e_ != cudaSuccess) return tlr::cuda_fail(ctx, e_, #call); \
   } while (0)
 
+// cudaMalloc and pinned cudaHostAlloc of the buffers that a solve makes on first
+// use; the test hook tlr_alloc_fail_at makes one of them fail.
+cudaError_t dev_malloc(void **p, size_t bytes);
+cudaError_t pin_malloc(void **p, size_t bytes);
+template <class T> cudaError_t dev_malloc(T **p, size_t bytes) {
+  return dev_malloc(reinterpret_cast<void **>(p), bytes);
+}
+template <class T> cudaError_t pin_malloc(T **p, size_t bytes) {
+  return pin_malloc(reinterpret_cast<void **>(p), bytes);
+}
+
 // Stage launchers (one .cu file each).
 int run_metrics(tlr_ctx *ctx, tlr_metric_diag *diag);
 int run_derivatives(tlr_ctx *ctx, tlr_deriv_diag *diag);

@@ -402,7 +402,7 @@ int Factor::build_inverse(tlr_ctx *ctx) {
     emit(bw, L.ib_off, L.ib_n, L.ib_small);
   }
   auto up = [&](void **p, const void *src, size_t bytes) -> int {
-    const cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 16));
+    const cudaError_t e = dev_malloc(p, std::max<size_t>(bytes, 16));
     if (e != cudaSuccess) {
       *p = nullptr;
       return fail(ctx, TLR_ERR_NOMEM,

@@ -664,6 +664,48 @@ struct Solver {
 // often converge well before the basis is full) at 2% extra on 200 x 128
 constexpr int kConvCheckDefault = 4;
 
+// every buffer of a workspace for n unknowns, a basis of ncv vectors and, with
+// bsz > 1, blocks
+int alloc_workspace(tlr_ctx *ctx, Workspace *ws, long long n, int ncv, int bsz) {
+  const size_t vb = n * sizeof(double2);
+  ws->n = n;
+  ws->ncv = ncv;
+  // ncv + block columns: the basis and the block of next vectors
+  TLR_CUDA(ctx, dev_malloc(&ws->V, vb * (ncv + Factor::kMaxRhs)));
+  TLR_CUDA(ctx, dev_malloc(&ws->w, vb));
+  TLR_CUDA(ctx, dev_malloc(&ws->y, vb));
+  TLR_CUDA(ctx, dev_malloc(&ws->r, vb));
+  TLR_CUDA(ctx, dev_malloc(&ws->aw, vb));
+  TLR_CUDA(ctx, dev_malloc(&ws->bw, vb));
+  TLR_CUDA(ctx, dev_malloc(&ws->hv, sizeof(double2) * 2 * (kGmresM + 1)));
+  TLR_CUDA(ctx, dev_malloc(&ws->tmp, vb * ncv));
+  TLR_CUDA(ctx, dev_malloc(&ws->x32, n * sizeof(float2)));
+  TLR_CUDA(ctx, dev_malloc(&ws->gv, vb * (2 * kGmresM + 1)));
+  TLR_CUDA(ctx, dev_malloc(&ws->zero, vb));
+  TLR_CUDA(ctx, cudaMemset(ws->zero, 0, vb));
+  TLR_CUDA(ctx, dev_malloc(&ws->nscratch, sizeof(double) * 2 * (ctx->partial_blocks + 1)));
+  TLR_CUDA(ctx, pin_malloc(&ws->hnorm, 4 * sizeof(double)));
+  const size_t hcount = (size_t)2 * ncv * (ncv + Factor::kMaxRhs);
+  TLR_CUDA(ctx, dev_malloc(&ws->kpart,
+                           sizeof(double2) * ctx->partial_blocks * (ncv + Factor::kMaxRhs)));
+  if (bsz > 1) {
+    const size_t bv = (size_t)Factor::kMaxRhs * n;
+    TLR_CUDA(ctx, dev_malloc(&ws->blk, sizeof(double2) * 5 * bv));
+    TLR_CUDA(ctx, dev_malloc(&ws->blk32, sizeof(float2) * bv));
+    TLR_CUDA(ctx, dev_malloc(&ws->bnd, sizeof(double) * 2 * Factor::kMaxRhs));
+    TLR_CUDA(ctx, pin_malloc(&ws->bnh, sizeof(double) * 2 * Factor::kMaxRhs));
+  }
+  TLR_CUDA(ctx, dev_malloc(&ws->npart, sizeof(double) * ctx->partial_blocks));
+  TLR_CUDA(ctx, dev_malloc(&ws->hd, sizeof(double2) * hcount));
+  TLR_CUDA(ctx, dev_malloc(&ws->betad, sizeof(double) * (ncv + 1)));
+  TLR_CUDA(ctx, dev_malloc(&ws->ybuf, sizeof(double2) * ncv * ncv));
+  TLR_CUDA(ctx, dev_malloc(&ws->rnd, sizeof(double) * (ncv + 1)));
+  TLR_CUDA(ctx, pin_malloc(&ws->hpin, sizeof(double2) * hcount + sizeof(double) * (ncv + 1)));
+  TLR_CUDA(ctx, pin_malloc(&ws->ypin, sizeof(double2) * ncv * ncv));
+  TLR_CUDA(ctx, pin_malloc(&ws->rnh, sizeof(double) * (ncv + 1)));
+  return TLR_OK;
+}
+
 void fill_start(std::vector<double2> &v, unsigned long long seed) {
   // deterministic pseudo-random start vector (xorshift64*), entries in (-1, 1)
   unsigned long long s = seed ? seed : 0x9E3779B97F4A7C15ull;
@@ -831,43 +873,10 @@ int run_solve(tlr_ctx *ctx, const tlr_solve_opts *opts, double *lambda,
   if (!ws) {
     ws = new Workspace();
     ctx->kws = ws;
-    ws->n = n;
-    ws->ncv = ncv;
-    // ncv + block columns: the basis and the block of next vectors
-    TLR_CUDA(ctx, cudaMalloc(&ws->V, vb * (ncv + Factor::kMaxRhs)));
-    TLR_CUDA(ctx, cudaMalloc(&ws->w, vb));
-    TLR_CUDA(ctx, cudaMalloc(&ws->y, vb));
-    TLR_CUDA(ctx, cudaMalloc(&ws->r, vb));
-    TLR_CUDA(ctx, cudaMalloc(&ws->aw, vb));
-    TLR_CUDA(ctx, cudaMalloc(&ws->bw, vb));
-    TLR_CUDA(ctx, cudaMalloc(&ws->hv, sizeof(double2) * 2 * (kGmresM + 1)));
-    TLR_CUDA(ctx, cudaMalloc(&ws->tmp, vb * ncv));
-    TLR_CUDA(ctx, cudaMalloc(&ws->x32, n * sizeof(float2)));
-    TLR_CUDA(ctx, cudaMalloc(&ws->gv, vb * (2 * kGmresM + 1)));
-    TLR_CUDA(ctx, cudaMalloc(&ws->zero, vb));
-    TLR_CUDA(ctx, cudaMemset(ws->zero, 0, vb));
-    TLR_CUDA(ctx, cudaMalloc(&ws->nscratch, sizeof(double) * 2 * (ctx->partial_blocks + 1)));
-    TLR_CUDA(ctx, cudaHostAlloc(&ws->hnorm, 4 * sizeof(double), cudaHostAllocDefault));
-    const size_t hcount = (size_t)2 * ncv * (ncv + Factor::kMaxRhs);
-    TLR_CUDA(ctx, cudaMalloc(&ws->kpart,
-                             sizeof(double2) * ctx->partial_blocks * (ncv + Factor::kMaxRhs)));
-    if (bsz > 1) {
-      const size_t bv = (size_t)Factor::kMaxRhs * n;
-      TLR_CUDA(ctx, cudaMalloc(&ws->blk, sizeof(double2) * 5 * bv));
-      TLR_CUDA(ctx, cudaMalloc(&ws->blk32, sizeof(float2) * bv));
-      TLR_CUDA(ctx, cudaMalloc(&ws->bnd, sizeof(double) * 2 * Factor::kMaxRhs));
-      TLR_CUDA(ctx, cudaHostAlloc(&ws->bnh, sizeof(double) * 2 * Factor::kMaxRhs,
-                                  cudaHostAllocDefault));
+    if (const int rc = alloc_workspace(ctx, ws, n, ncv, bsz)) {
+      free_workspace(ctx);  // not left half built for the next call
+      return rc;
     }
-    TLR_CUDA(ctx, cudaMalloc(&ws->npart, sizeof(double) * ctx->partial_blocks));
-    TLR_CUDA(ctx, cudaMalloc(&ws->hd, sizeof(double2) * hcount));
-    TLR_CUDA(ctx, cudaMalloc(&ws->betad, sizeof(double) * (ncv + 1)));
-    TLR_CUDA(ctx, cudaMalloc(&ws->ybuf, sizeof(double2) * ncv * ncv));
-    TLR_CUDA(ctx, cudaMalloc(&ws->rnd, sizeof(double) * (ncv + 1)));
-    TLR_CUDA(ctx, cudaHostAlloc(&ws->hpin, sizeof(double2) * hcount + sizeof(double) * (ncv + 1),
-                                cudaHostAllocDefault));
-    TLR_CUDA(ctx, cudaHostAlloc(&ws->ypin, sizeof(double2) * ncv * ncv, cudaHostAllocDefault));
-    TLR_CUDA(ctx, cudaHostAlloc(&ws->rnh, sizeof(double) * (ncv + 1), cudaHostAllocDefault));
   }
   S.V = ws->V;
   S.w = ws->w;

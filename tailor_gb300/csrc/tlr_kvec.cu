@@ -275,7 +275,7 @@ int arrival_counters(tlr_ctx *ctx, int count) {
   cudaFree(ctx->kv_ctr);
   ctx->kv_ctr = nullptr;
   const int cap = std::max(count, 64);
-  TLR_CUDA(ctx, cudaMalloc(&ctx->kv_ctr, sizeof(int) * cap));
+  TLR_CUDA(ctx, dev_malloc(&ctx->kv_ctr, sizeof(int) * cap));
   TLR_CUDA(ctx, cudaMemsetAsync(ctx->kv_ctr, 0, sizeof(int) * cap, ctx->stream));
   ctx->kv_ctr_n = cap;
   return TLR_OK;
@@ -283,7 +283,7 @@ int arrival_counters(tlr_ctx *ctx, int count) {
 
 int pinned_words(tlr_ctx *ctx) {
   if (!ctx->pin)
-    TLR_CUDA(ctx, cudaHostAlloc(&ctx->pin, sizeof(double) * kPinWords, cudaHostAllocDefault));
+    TLR_CUDA(ctx, pin_malloc(&ctx->pin, sizeof(double) * kPinWords));
   return TLR_OK;
 }
 

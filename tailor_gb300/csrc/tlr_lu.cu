@@ -2517,7 +2517,7 @@ int Factor::setup(tlr_ctx *ctx, int precision, int leaf, int solve_block, int pa
   n_inv_blocks = (int)inv_blocks.size();
   const size_t csize = prec == 0 ? sizeof(double2) : sizeof(float2);
   auto alloc = [&](void **p, size_t bytes) -> int {
-    cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 16));
+    cudaError_t e = dev_malloc(p, std::max<size_t>(bytes, 16));
     if (e != cudaSuccess) {
       *p = nullptr;
       return fail(ctx, TLR_ERR_NOMEM, std::string("factor allocation failed: ") +
@@ -2640,9 +2640,9 @@ int Factor::build_phases(tlr_ctx *ctx) {
   }
   nphases = (int)ph.size();
   cudaError_t e;
-  if ((e = cudaMalloc(&d_phases, std::max<size_t>(ph.size(), 1) * sizeof(Phase))) != cudaSuccess ||
-      (e = cudaMalloc(&d_barrier, sizeof(unsigned))) != cudaSuccess ||
-      (e = cudaMalloc(&d_solve_err, sizeof(int))) != cudaSuccess)
+  if ((e = dev_malloc(&d_phases, std::max<size_t>(ph.size(), 1) * sizeof(Phase))) != cudaSuccess ||
+      (e = dev_malloc(&d_barrier, sizeof(unsigned))) != cudaSuccess ||
+      (e = dev_malloc(&d_solve_err, sizeof(int))) != cudaSuccess)
     return fail(ctx, TLR_ERR_NOMEM, std::string("factor allocation failed: ") + cudaGetErrorString(e));
   TLR_CUDA(ctx, cudaMemcpy(d_phases, ph.data(), ph.size() * sizeof(Phase), cudaMemcpyHostToDevice));
   TLR_CUDA(ctx, cudaMemset(d_solve_err, 0, sizeof(int)));
@@ -3282,10 +3282,17 @@ int Factor::solve_multi_prepare(tlr_ctx *ctx) {
   // buffers for up to kMaxRhs vectors, allocated once per factor
   const size_t cs = sizeof(float2);
   const size_t we = (size_t)std::max<long long>(sym.work_elems, 1);
-  TLR_CUDA(ctx, cudaMalloc(&work_m, (size_t)kMaxRhs * we * cs));
-  TLR_CUDA(ctx, cudaMalloc(&work2_m, (size_t)kMaxRhs * we * cs));
-  TLR_CUDA(ctx, cudaMalloc(&vec_m, (size_t)kMaxRhs * sym.nn * 5 * cs));
-  TLR_CUDA(ctx, cudaMalloc(&partial_m, (size_t)kMaxRhs * partial_stride * sizeof(double2)));
+  cudaError_t e = dev_malloc(&work_m, (size_t)kMaxRhs * we * cs);
+  if (e == cudaSuccess) e = dev_malloc(&work2_m, (size_t)kMaxRhs * we * cs);
+  if (e == cudaSuccess) e = dev_malloc(&vec_m, (size_t)kMaxRhs * sym.nn * 5 * cs);
+  if (e == cudaSuccess)
+    e = dev_malloc(&partial_m, (size_t)kMaxRhs * partial_stride * sizeof(double2));
+  if (e != cudaSuccess) {
+    cudaFree(work_m); cudaFree(work2_m); cudaFree(vec_m); cudaFree(partial_m);
+    work_m = work2_m = vec_m = nullptr;
+    partial_m = nullptr;
+    return cuda_fail(ctx, e, "the multi-vector solve buffers");
+  }
   multi_cap = kMaxRhs;
   return TLR_OK;
 }

@@ -484,9 +484,7 @@ int node_blocks(const Pipe &p) { return blocks_for(p.nn, kNodes); }
 int shift_blocks(const Pipe &p) { return blocks_for(p.nn, kSNodes); }
 int row_blocks(const Pipe &p) { return std::min(p.sms, blocks_for(p.nn, kRWarps)); }
 
-}  // namespace
-
-int pipe_alloc(tlr_ctx *ctx, Pipe &p, int ncv) {
+int alloc_buffers(tlr_ctx *ctx, Pipe &p, int ncv) {
   p.nn = ctx->nn;
   p.n = 5LL * ctx->nn;
   p.ncv = ncv;
@@ -500,23 +498,31 @@ int pipe_alloc(tlr_ctx *ctx, Pipe &p, int ncv) {
   TLR_CUDA(ctx, cudaFuncSetAttribute(k_pipe_residual<3>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRSmem));
   const size_t n = (size_t)p.n;
-  TLR_CUDA(ctx, cudaMalloc(&p.vff, sizeof(float4) * n * (ncv + 1)));
-  TLR_CUDA(ctx, cudaMalloc(&p.xyff, sizeof(float4) * 2 * n));
-  TLR_CUDA(ctx, cudaMalloc(&p.B32, sizeof(float2) * 5 * n));
-  TLR_CUDA(ctx, cudaMalloc(&p.b, sizeof(double2) * n));
-  TLR_CUDA(ctx, cudaMalloc(&p.tx, sizeof(double2) * n));
-  TLR_CUDA(ctx, cudaMalloc(&p.ty, sizeof(double2) * n));
-  TLR_CUDA(ctx, cudaMalloc(&p.by32, sizeof(float2) * n));
-  TLR_CUDA(ctx, cudaMalloc(&p.u32, sizeof(float2) * n));
-  TLR_CUDA(ctx, cudaMalloc(&p.tu32, sizeof(float2) * n));
-  TLR_CUDA(ctx, cudaMalloc(&p.H, sizeof(double2) * p.ldh * ncv));
-  TLR_CUDA(ctx, cudaMalloc(&p.g, sizeof(float4) * 2 * p.ldh));
-  TLR_CUDA(ctx, cudaMalloc(&p.bpart, sizeof(double) * shift_blocks(p)));
-  TLR_CUDA(ctx, cudaMalloc(&p.rpart, sizeof(double) * row_blocks(p)));
-  TLR_CUDA(ctx, cudaMalloc(&p.arrived, sizeof(int)));
+  TLR_CUDA(ctx, dev_malloc(&p.vff, sizeof(float4) * n * (ncv + 1)));
+  TLR_CUDA(ctx, dev_malloc(&p.xyff, sizeof(float4) * 2 * n));
+  TLR_CUDA(ctx, dev_malloc(&p.B32, sizeof(float2) * 5 * n));
+  TLR_CUDA(ctx, dev_malloc(&p.b, sizeof(double2) * n));
+  TLR_CUDA(ctx, dev_malloc(&p.tx, sizeof(double2) * n));
+  TLR_CUDA(ctx, dev_malloc(&p.ty, sizeof(double2) * n));
+  TLR_CUDA(ctx, dev_malloc(&p.by32, sizeof(float2) * n));
+  TLR_CUDA(ctx, dev_malloc(&p.u32, sizeof(float2) * n));
+  TLR_CUDA(ctx, dev_malloc(&p.tu32, sizeof(float2) * n));
+  TLR_CUDA(ctx, dev_malloc(&p.H, sizeof(double2) * p.ldh * ncv));
+  TLR_CUDA(ctx, dev_malloc(&p.g, sizeof(float4) * 2 * p.ldh));
+  TLR_CUDA(ctx, dev_malloc(&p.bpart, sizeof(double) * shift_blocks(p)));
+  TLR_CUDA(ctx, dev_malloc(&p.rpart, sizeof(double) * row_blocks(p)));
+  TLR_CUDA(ctx, dev_malloc(&p.arrived, sizeof(int)));
   TLR_CUDA(ctx, cudaMemsetAsync(p.arrived, 0, sizeof(int), ctx->stream));
-  TLR_CUDA(ctx, cudaHostAlloc(&p.hup, sizeof(double2) * p.ldh * ncv, cudaHostAllocDefault));
+  TLR_CUDA(ctx, pin_malloc(&p.hup, sizeof(double2) * p.ldh * ncv));
   return TLR_OK;
+}
+
+}  // namespace
+
+int pipe_alloc(tlr_ctx *ctx, Pipe &p, int ncv) {
+  const int rc = alloc_buffers(ctx, p, ncv);
+  if (rc) pipe_free(p);  // all of them or none: vff says which
+  return rc;
 }
 
 void pipe_free(Pipe &p) {

@@ -342,9 +342,9 @@ __global__ void __launch_bounds__(32 * kRowsPerCta)
 
 int prepare_ff(tlr_ctx *ctx) {
   const long long nv = ctx->nnzb * 25;
-  if (!ctx->aff) TLR_CUDA(ctx, cudaMalloc(&ctx->aff, (size_t)nv * sizeof(float4)));
+  if (!ctx->aff) TLR_CUDA(ctx, dev_malloc(&ctx->aff, (size_t)nv * sizeof(float4)));
   const long long n = 5LL * ctx->nn;
-  if (!ctx->wff) TLR_CUDA(ctx, cudaMalloc(&ctx->wff, (size_t)n * sizeof(float4)));
+  if (!ctx->wff) TLR_CUDA(ctx, dev_malloc(&ctx->wff, (size_t)n * sizeof(float4)));
   if (!ctx->aff_valid) {
     { k_split_ff<<<blocks_for(nv, 256), 256, 0, ctx->stream>>>(nv, ctx->A, ctx->aff); count_launches(); }
     ctx->aff_valid = true;
@@ -419,7 +419,7 @@ int residual_ff_multi_prepare(tlr_ctx *ctx) {
   int rc = prepare_ff(ctx);
   if (rc) return rc;
   if (!ctx->wff_m)
-    TLR_CUDA(ctx, cudaMalloc(&ctx->wff_m, (size_t)8 * 5 * ctx->nn * sizeof(float4)));
+    TLR_CUDA(ctx, dev_malloc(&ctx->wff_m, (size_t)8 * 5 * ctx->nn * sizeof(float4)));
   return TLR_OK;
 }
 
