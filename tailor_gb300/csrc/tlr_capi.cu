@@ -144,14 +144,24 @@ int copy_soa(tlr_ctx *ctx, const double *src, int comp, double *dst) {
 
 }  // namespace
 
+// A failure leaves a null pointer and no pending error: callers may go on
+// without the buffer.
 cudaError_t dev_malloc(void **p, size_t bytes) {
-  const cudaError_t e = fail_now();
-  return e != cudaSuccess ? e : cudaMalloc(p, bytes);
+  cudaError_t e = fail_now();
+  if (e == cudaSuccess) e = cudaMalloc(p, bytes);
+  if (e == cudaSuccess) return e;
+  cudaGetLastError();
+  *p = nullptr;
+  return e;
 }
 
 cudaError_t pin_malloc(void **p, size_t bytes) {
-  const cudaError_t e = fail_now();
-  return e != cudaSuccess ? e : cudaHostAlloc(p, bytes, cudaHostAllocDefault);
+  cudaError_t e = fail_now();
+  if (e == cudaSuccess) e = cudaHostAlloc(p, bytes, cudaHostAllocDefault);
+  if (e == cudaSuccess) return e;
+  cudaGetLastError();
+  *p = nullptr;
+  return e;
 }
 
 void set_global_error(const std::string &msg) { g_error = msg; }

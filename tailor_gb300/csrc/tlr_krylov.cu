@@ -607,10 +607,9 @@ struct Solver {
     return TLR_OK;
   }
 
-  // allocate what the rounds need (outside any capture) and begin at v
+  // split the operator if it is not (outside any capture) and begin at v
   int pipe_begin(const double2 *v, double2 *x) {
     int rc = prepare_ff(ctx);
-    if (!rc) rc = F->solve_multi_prepare(ctx);
     if (!rc) rc = pipe_start(ctx, *pipe, v, x);
     for (int later = 0; later < 2 && !rc; ++later)
       if (!pipe_exec[later]) rc = build_pipe_graph(x, later);
@@ -955,14 +954,21 @@ int run_solve(tlr_ctx *ctx, const tlr_solve_opts *opts, double *lambda,
   // the mixed form's single-vector applications are pipelined (tlr_pipe.h);
   // GMRES refinement, the cooperative solve, FP64 acceptance and 512-row
   // solve blocks (no multi-vector kernels) refine each application by itself
-  const bool piped = prec == 1 && bsz == 1 && !S.gmres && !S.fp64_accept && !F->persistent &&
-                     sblock != 512;
+  bool piped = prec == 1 && bsz == 1 && !S.gmres && !S.fp64_accept && !F->persistent &&
+               sblock != 512;
   if (piped) {
     int rc = TLR_OK;
     if (!ws->pipe.vff) rc = pipe_alloc(ctx, ws->pipe, ws->ncv);
-    S.pipe = &ws->pipe;
-    if (!rc) rc = S.pipe_begin(S.V, S.w);
-    if (rc) return rc;
+    if (!rc) rc = F->solve_multi_prepare(ctx);
+    if (rc == TLR_ERR_NOMEM) {  // no memory for guesses: single applications need none
+      pipe_free(ws->pipe);
+      ctx->last_error.clear();
+      piped = false;
+    } else {
+      S.pipe = &ws->pipe;
+      if (!rc) rc = S.pipe_begin(S.V, S.w);
+      if (rc) return rc;
+    }
   }
   double maxerr = 0.0;
   const int nout = nev;

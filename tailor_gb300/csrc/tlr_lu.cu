@@ -3291,7 +3291,8 @@ int Factor::solve_multi_prepare(tlr_ctx *ctx) {
     cudaFree(work_m); cudaFree(work2_m); cudaFree(vec_m); cudaFree(partial_m);
     work_m = work2_m = vec_m = nullptr;
     partial_m = nullptr;
-    return cuda_fail(ctx, e, "the multi-vector solve buffers");
+    return fail(ctx, TLR_ERR_NOMEM, std::string("the multi-vector solve buffers: ") +
+                                        cudaGetErrorString(e));
   }
   multi_cap = kMaxRhs;
   return TLR_OK;

@@ -498,22 +498,24 @@ int alloc_buffers(tlr_ctx *ctx, Pipe &p, int ncv) {
   TLR_CUDA(ctx, cudaFuncSetAttribute(k_pipe_residual<3>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRSmem));
   const size_t n = (size_t)p.n;
-  TLR_CUDA(ctx, dev_malloc(&p.vff, sizeof(float4) * n * (ncv + 1)));
-  TLR_CUDA(ctx, dev_malloc(&p.xyff, sizeof(float4) * 2 * n));
-  TLR_CUDA(ctx, dev_malloc(&p.B32, sizeof(float2) * 5 * n));
-  TLR_CUDA(ctx, dev_malloc(&p.b, sizeof(double2) * n));
-  TLR_CUDA(ctx, dev_malloc(&p.tx, sizeof(double2) * n));
-  TLR_CUDA(ctx, dev_malloc(&p.ty, sizeof(double2) * n));
-  TLR_CUDA(ctx, dev_malloc(&p.by32, sizeof(float2) * n));
-  TLR_CUDA(ctx, dev_malloc(&p.u32, sizeof(float2) * n));
-  TLR_CUDA(ctx, dev_malloc(&p.tu32, sizeof(float2) * n));
-  TLR_CUDA(ctx, dev_malloc(&p.H, sizeof(double2) * p.ldh * ncv));
-  TLR_CUDA(ctx, dev_malloc(&p.g, sizeof(float4) * 2 * p.ldh));
-  TLR_CUDA(ctx, dev_malloc(&p.bpart, sizeof(double) * shift_blocks(p)));
-  TLR_CUDA(ctx, dev_malloc(&p.rpart, sizeof(double) * row_blocks(p)));
-  TLR_CUDA(ctx, dev_malloc(&p.arrived, sizeof(int)));
+  auto dev = [](auto **q, size_t bytes) { return dev_malloc(q, bytes) == cudaSuccess; };
+  if (!(dev(&p.vff, sizeof(float4) * n * (ncv + 1)) &&
+        dev(&p.xyff, sizeof(float4) * 2 * n) &&
+        dev(&p.B32, sizeof(float2) * 5 * n) &&
+        dev(&p.b, sizeof(double2) * n) &&
+        dev(&p.tx, sizeof(double2) * n) &&
+        dev(&p.ty, sizeof(double2) * n) &&
+        dev(&p.by32, sizeof(float2) * n) &&
+        dev(&p.u32, sizeof(float2) * n) &&
+        dev(&p.tu32, sizeof(float2) * n) &&
+        dev(&p.H, sizeof(double2) * p.ldh * ncv) &&
+        dev(&p.g, sizeof(float4) * 2 * p.ldh) &&
+        dev(&p.bpart, sizeof(double) * shift_blocks(p)) &&
+        dev(&p.rpart, sizeof(double) * row_blocks(p)) &&
+        dev(&p.arrived, sizeof(int)) &&
+        pin_malloc(&p.hup, sizeof(double2) * p.ldh * ncv) == cudaSuccess))
+    return fail(ctx, TLR_ERR_NOMEM, "no memory for the pipelined applications");
   TLR_CUDA(ctx, cudaMemsetAsync(p.arrived, 0, sizeof(int), ctx->stream));
-  TLR_CUDA(ctx, pin_malloc(&p.hup, sizeof(double2) * p.ldh * ncv));
   return TLR_OK;
 }
 

@@ -45,6 +45,7 @@ struct Pipe {
   double2 *hup = nullptr; // pinned stage of H
 };
 
+// all buffers, or none and TLR_ERR_NOMEM
 int pipe_alloc(tlr_ctx *ctx, Pipe &p, int ncv);
 void pipe_free(Pipe &p);
 // Begin with v (= basis vector 0): x = y = u = 0.
