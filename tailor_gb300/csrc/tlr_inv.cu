@@ -259,8 +259,6 @@ __global__ void __launch_bounds__(32 * kW, NR <= 4 ? 4 : 2)
 }  // namespace
 
 int Factor::build_inverse(tlr_ctx *ctx) {
-  inverse_ok = false;
-  if (prec != 1 || sw != kSW) return TLR_OK;
   const int nf = (int)sym.fronts.size();
   auto blocks_of = [&](int t) { return (sym.fronts[t].p + kSW - 1) / kSW; };
   // inversion batches: step s takes block nblk - 1 - s of every front
@@ -421,12 +419,24 @@ int Factor::build_inverse(tlr_ctx *ctx) {
       (rc = up((void **)&d_items, items.data(), items.size() * sizeof(SvItem))) ||
       (rc = up((void **)&split_part, nullptr, parts * sizeof(float2))) ||
       (rc = up((void **)&split_ctr, nullptr, std::max(1, max_split_tiles) * sizeof(int))) ||
-      (rc = up((void **)&inv_planes, nullptr,
-               (size_t)max_tiles * (kSW / 8) * tc_chunk_image_bytes())))
+      (rc = reserve_planes(ctx, (size_t)max_tiles * (kSW / 8) * tc_chunk_image_bytes()))) {
+    free_inverse();
     return rc;
+  }
   TLR_CUDA(ctx, cudaMemset(split_ctr, 0, std::max(1, max_split_tiles) * sizeof(int)));
   inverse_ok = true;
   return TLR_OK;
+}
+
+void Factor::free_inverse() {
+  cudaFree(d_inv_jobs); cudaFree(d_inv_prefix); cudaFree(d_gtiles); cudaFree(d_items);
+  cudaFree(d_uidx); cudaFree(d_gsrc); cudaFree(split_part); cudaFree(split_ctr);
+  d_inv_jobs = nullptr;
+  d_inv_prefix = d_uidx = d_gsrc = split_ctr = nullptr;
+  d_gtiles = nullptr;
+  d_items = nullptr;
+  split_part = nullptr;
+  inverse_ok = false;
 }
 
 int Factor::invert_pivots(tlr_ctx *ctx) {
@@ -434,7 +444,7 @@ int Factor::invert_pivots(tlr_ctx *ctx) {
   for (const TcBatch &b : inv_batches) {
     const int rc = launch_tc_jobs(ctx, d_inv_jobs + b.job_off, b.jobs, d_inv_prefix + b.prefix_off,
                                   d_inv_prefix + b.pa_off, d_inv_prefix + b.pb_off, b.tiles,
-                                  b.atiles, b.btiles, P, inv_planes, d_tc_err, ctx->stream);
+                                  b.atiles, b.btiles, P, tc_planes, d_tc_err, ctx->stream);
     if (rc) return rc;
   }
   return launch_scale_g(ctx, d_gtiles, n_gtiles, P, d_fronts, d_inv_off,

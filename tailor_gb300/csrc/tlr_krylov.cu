@@ -834,6 +834,7 @@ int run_solve(tlr_ctx *ctx, const tlr_solve_opts *opts, double *lambda,
     if (F->graph_exec) cudaGraphExecDestroy(F->graph_exec);
     F->graph_exec = nullptr;
   }
+  if (const int rc = F->prepare(ctx)) return rc;
   if (F->factored && F->inverse != F->use_inverse()) F->factored = false;
   if (!F->factored) {
     double anorm = 0.0;

@@ -2307,8 +2307,8 @@ int Factor::setup(tlr_ctx *ctx, int precision, int leaf, int solve_block, int pa
   // schedules: per level, fronts sorted by p descending; per step prefix
   std::vector<int> sched;
   long long max_plane_tiles = 0;  // largest atiles + btiles of a panel step
-  size_t oz_bytes = 0;            // largest operand images of a sliced update
-  int oz_fronts = 1;
+  oz_bytes = 0;
+  oz_fronts = 1;
   levels.clear();
   for (size_t h = 0; h < sym.levels.size(); ++h) {
     Level L;
@@ -2493,8 +2493,8 @@ int Factor::setup(tlr_ctx *ctx, int precision, int leaf, int solve_block, int pa
       }
     }
   }
-  std::vector<OzJob> oz_jobs;
-  std::vector<int> oz_prefix;
+  oz_jobs.clear();
+  oz_prefix.clear();
   oz_batches.clear();
   if (prec == 0 && w == kOzPanel && sw == 32 * kOzPasses) {
     std::vector<RewriteFront> rf;
@@ -2562,22 +2562,9 @@ int Factor::setup(tlr_ctx *ctx, int precision, int leaf, int solve_block, int pa
     TLR_CUDA(ctx, cudaMemcpy(d_wave_tiles, wtiles.data(), wtiles.size() * sizeof(int4),
                              cudaMemcpyHostToDevice));
   if (wctr) TLR_CUDA(ctx, cudaMemset(d_wave_ctr, 0, (size_t)wctr * sizeof(int)));
-  if (prec == 1 &&
-      (rc = alloc((void **)&tc_planes, (size_t)max_plane_tiles * ((w + 7) / 8) *
-                                           tc_chunk_image_bytes())))
+  if (prec == 1 && (rc = reserve_planes(ctx, (size_t)max_plane_tiles * ((w + 7) / 8) *
+                                                 tc_chunk_image_bytes())))
     return rc;
-  if (prec == 0 && w == kOzPanel &&
-      ((rc = alloc((void **)&tc_planes, oz_bytes)) ||
-       (rc = alloc((void **)&d_rowexp, sizeof(int) * kOzPanel * oz_fronts)) ||
-       (rc = alloc((void **)&d_oz_jobs, oz_jobs.size() * sizeof(OzJob))) ||
-       (rc = alloc((void **)&d_oz_prefix, oz_prefix.size() * sizeof(int)))))
-    return rc;
-  if (!oz_jobs.empty()) {
-    TLR_CUDA(ctx, cudaMemcpy(d_oz_jobs, oz_jobs.data(), oz_jobs.size() * sizeof(OzJob),
-                             cudaMemcpyHostToDevice));
-    TLR_CUDA(ctx, cudaMemcpy(d_oz_prefix, oz_prefix.data(), oz_prefix.size() * sizeof(int),
-                             cudaMemcpyHostToDevice));
-  }
   if (prec == 0) {
     std::vector<StepFront> sf;
     for (auto &L : levels) {
@@ -2615,8 +2602,47 @@ int Factor::setup(tlr_ctx *ctx, int precision, int leaf, int solve_block, int pa
                            cudaMemcpyHostToDevice));
   TLR_CUDA(ctx, cudaMemcpy(d_sched, sched.data(), sched.size() * sizeof(int),
                            cudaMemcpyHostToDevice));
-  if ((rc = build_inverse(ctx))) return rc;
   return build_phases(ctx);
+}
+
+int Factor::reserve_planes(tlr_ctx *ctx, size_t bytes) {
+  bytes = std::max<size_t>(bytes, 16);
+  if (tc_planes && planes_bytes >= bytes) return TLR_OK;
+  unsigned char *p = nullptr;
+  const cudaError_t e = dev_malloc(&p, bytes);
+  if (e != cudaSuccess)
+    return fail(ctx, TLR_ERR_NOMEM, std::string("factor allocation failed: ") +
+                                        cudaGetErrorString(e));
+  cudaFree(tc_planes);
+  tc_planes = p;
+  planes_bytes = bytes;
+  return TLR_OK;
+}
+
+int Factor::build_oz(tlr_ctx *ctx) {
+  const size_t jb = std::max<size_t>(oz_jobs.size() * sizeof(OzJob), 16);
+  const size_t pb = std::max<size_t>(oz_prefix.size() * sizeof(int), 16);
+  int rc = reserve_planes(ctx, oz_bytes);
+  if (!rc && (dev_malloc(&d_rowexp, sizeof(int) * kOzPanel * oz_fronts) != cudaSuccess ||
+              dev_malloc(&d_oz_jobs, jb) != cudaSuccess ||
+              dev_malloc(&d_oz_prefix, pb) != cudaSuccess))
+    rc = fail(ctx, TLR_ERR_NOMEM, "factor allocation failed: buffers of the sliced products");
+  if (rc) {
+    cudaFree(tc_planes); cudaFree(d_rowexp); cudaFree(d_oz_jobs); cudaFree(d_oz_prefix);
+    tc_planes = nullptr;
+    planes_bytes = 0;
+    d_rowexp = d_oz_prefix = nullptr;
+    d_oz_jobs = nullptr;
+    return rc;
+  }
+  if (!oz_jobs.empty()) {
+    TLR_CUDA(ctx, cudaMemcpy(d_oz_jobs, oz_jobs.data(), oz_jobs.size() * sizeof(OzJob),
+                             cudaMemcpyHostToDevice));
+    TLR_CUDA(ctx, cudaMemcpy(d_oz_prefix, oz_prefix.data(), oz_prefix.size() * sizeof(int),
+                             cudaMemcpyHostToDevice));
+  }
+  oz_ok = true;
+  return TLR_OK;
 }
 
 int Factor::build_phases(tlr_ctx *ctx) {
@@ -2725,19 +2751,13 @@ void Factor::release() {
   d_rowexp = d_oz_prefix = nullptr;
   d_oz_jobs = nullptr;
   d_sfronts = nullptr;
-  cudaFree(d_inv_jobs); cudaFree(d_inv_prefix); cudaFree(inv_planes); cudaFree(d_gtiles);
-  cudaFree(d_items); cudaFree(d_uidx); cudaFree(d_gsrc); cudaFree(split_part); cudaFree(split_ctr);
-  d_inv_jobs = nullptr;
-  d_inv_prefix = d_uidx = d_gsrc = split_ctr = nullptr;
-  inv_planes = nullptr;
-  d_gtiles = nullptr;
-  d_items = nullptr;
-  split_part = nullptr;
-  inverse = inverse_ok = false;
+  free_inverse();
+  inverse = inverse_failed = oz_ok = oz_failed = false;
   d_ltiles_tc = d_utiles_tc = nullptr;
   d_wave_tiles = nullptr;
   d_wave_ctr = nullptr;
   tc_planes = nullptr;
+  planes_bytes = 0;
   d_phases = nullptr;
   d_barrier = nullptr;
   d_solve_err = nullptr;
@@ -2777,7 +2797,7 @@ int Factor::rewrite_factors(tlr_ctx *ctx) {
   }
   long long nu = n_utiles, nl = n_ltiles;
   if constexpr (sizeof(C) == sizeof(double2)) {
-    if (sliced && d_oz_jobs) {  // L' and U' in slices, like the Schur updates
+    if (sliced && oz_ok) {  // L' and U' in slices, like the Schur updates
       for (const OzBatch &b : oz_batches) {
         const int rc = launch_rewrite_oz(ctx, b, d_oz_jobs, d_oz_prefix, P, Li, Ui, tc_planes,
                                          d_rowexp, d_tc_err, st);
@@ -2895,7 +2915,7 @@ int Factor::factor_impl(tlr_ctx *ctx, double sr, double si, double tiny) {
               { k_gemm32<<<S.tiles, 256, 0, st>>>(fl, d_sched + S.prefix_off, S.nf, s, w,
                                                 reinterpret_cast<float2 *>(P), d_fronts); count_launches(); }
           }
-          else if (sliced && w == kOzPanel) {
+          else if (sliced && oz_ok) {
             const int rc = launch_gemm_oz(ctx, fl, d_sched + S.oz_prefix_off, d_sched + S.pa_off,
                                           d_sched + S.pb_off, S.nf, s, w, S.max_ext,
                                           reinterpret_cast<double2 *>(P), d_fronts, S.oz_tiles,
@@ -2925,7 +2945,21 @@ int Factor::factor_impl(tlr_ctx *ctx, double sr, double si, double tiny) {
   return TLR_OK;
 }
 
+int Factor::prepare(tlr_ctx *ctx) {
+  auto optional = [&](int rc, bool &failed) {
+    failed = rc == TLR_ERR_NOMEM;
+    if (failed) ctx->last_error.clear();
+    return failed ? TLR_OK : rc;
+  };
+  if (use_inverse() && !inverse_ok)
+    if (const int rc = optional(build_inverse(ctx), inverse_failed)) return rc;
+  if (sliced && w == kOzPanel && !oz_ok && !oz_failed)
+    if (const int rc = optional(build_oz(ctx), oz_failed)) return rc;
+  return TLR_OK;
+}
+
 int Factor::factor(tlr_ctx *ctx, double sr, double si, double tiny) {
+  if (const int prc = prepare(ctx)) return prc;
   if (inverse != use_inverse()) {  // captured solves are of the other form
     inverse = use_inverse();
     if (graph_exec) cudaGraphExecDestroy(graph_exec);
@@ -3468,7 +3502,7 @@ extern "C" int tlr_rewrite_c128(const double *front, int m, int p, int sliced, d
   tlr_ctx ctx;
   Factor F;
   F.prec = 0;
-  F.sliced = sliced != 0;
+  F.sliced = F.oz_ok = sliced != 0;
   F.oz_batches = batches;
   F.n_inv_blocks = (int)blocks.size();
   F.n_ltiles64 = (long long)l64.size();

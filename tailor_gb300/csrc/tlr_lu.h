@@ -126,14 +126,26 @@ struct Factor {
   // bulk kernel: 2 persistent warp-specialised (default), 0 one tile per CTA
   // with three stages / two CTAs per SM, 1 two stages / three CTAs per SM
   int tc_variant = 2;
+  // scratch, also of the inversion and of the sliced products
   unsigned char *tc_planes = nullptr;
+  size_t planes_bytes = 0;
+  // at least `bytes` of tc_planes (contents are lost); TLR_ERR_NOMEM
+  int reserve_planes(tlr_ctx *ctx, size_t bytes);
   // complex128 Schur updates by exact integer slices on the tensor cores
   // (tlr_oz.cu), with 32-column panels
   bool sliced = false;
   // its products of the factor rewrite, in batches
   std::vector<OzBatch> oz_batches;
+  std::vector<OzJob> oz_jobs;
+  std::vector<int> oz_prefix;
   OzJob *d_oz_jobs = nullptr;
   int *d_oz_prefix = nullptr;
+  size_t oz_bytes = 0;      // operand images of the largest launch
+  int oz_fronts = 1;        // products of the largest launch
+  // whether the buffers of the slices exist; or there is no memory
+  // for them: CUDA cores then
+  bool oz_ok = false, oz_failed = false;
+  int build_oz(tlr_ctx *ctx);
   StepFront *d_sfronts = nullptr;  // complex128: fronts of every level in order
   int *d_rowexp = nullptr;
   int w = 32;    // panel width
@@ -161,11 +173,12 @@ struct Factor {
   // blocks are inverted past the diagonal blocks, so a front needs one
   // product each way (tlr_inv.cu) instead of one step per diagonal block.
   bool inverse = false;            // the form of the present factor
-  bool inverse_ok = false;         // structures of the form exist
+  // whether the structures of the form exist (made by the first factorisation
+  // that uses them), or there is no memory for them: block steps then
+  bool inverse_ok = false, inverse_failed = false;
   std::vector<TcBatch> inv_batches;
   TcJob *d_inv_jobs = nullptr;
   int *d_inv_prefix = nullptr;
-  unsigned char *inv_planes = nullptr;
   int4 *d_gtiles = nullptr;        // 64-column tiles of the D_b row scaling
   long long n_gtiles = 0;
   SvItem *d_items = nullptr;
@@ -175,8 +188,11 @@ struct Factor {
   int max_split_tiles = 0, max_split = 1;
   float2 *split_part = nullptr;    // partial sums of split row tiles
   int *split_ctr = nullptr;
-  bool use_inverse() const { return inverse_ok && tensor_cores && !persistent; }
-  int build_inverse(tlr_ctx *ctx); // host structures, called by setup
+  bool use_inverse() const {
+    return prec == 1 && sw == 256 && tensor_cores && !persistent && !inverse_failed;
+  }
+  int build_inverse(tlr_ctx *ctx);
+  void free_inverse();
   int invert_pivots(tlr_ctx *ctx);
   template <int NR> int solve_inverse(tlr_ctx *ctx, float2 *x, float2 *W, float2 *W2);
   long long inv_elems = 0, n_ltiles = 0, n_utiles = 0;
@@ -236,6 +252,10 @@ struct Factor {
   int setup(tlr_ctx *ctx, int precision, int leaf, int solve_block = 0, int panel_width = 0,
             int ring_slack_percent = 0);
   void release();
+  // What only some forms of the factor need, on the first factorisation in that
+  // form; without the memory for it the factor takes the form that does without.
+  // (factor() does this itself, but not outside a caller's timing.)
+  int prepare(tlr_ctx *ctx);
   int factor(tlr_ctx *ctx, double sr, double si, double tiny);
   // In-place x <- K^-1 x on a device vector in the factor's precision.
   int solve(tlr_ctx *ctx, void *x);

@@ -111,6 +111,7 @@ int autotune(tlr_ctx *ctx, ClassState &cs, int ring_slack) {
     // the 256 block are timed on
     for (int k = bi == 0 ? 1 : 0; k >= 0 && !rc; --k) {
       F->tensor_cores = bi == 0 ? k == 0 : !cs.cuda_core_schur;
+      if ((rc = F->prepare(ctx))) break;
       cudaEventRecord(ctx->ev0, ctx->stream);
       if ((rc = F->factor(ctx, sr, si, tiny))) break;
       cudaEventRecord(ctx->ev1, ctx->stream);
@@ -134,8 +135,9 @@ int autotune(tlr_ctx *ctx, ClassState &cs, int ring_slack) {
       W->tensor_cores = !cs.cuda_core_schur;
       Factor *keep = ctx->factor;
       ctx->factor = W;
+      rc = W->prepare(ctx);
       cudaEventRecord(ctx->ev0, ctx->stream);
-      rc = W->factor(ctx, sr, si, tiny);
+      if (!rc) rc = W->factor(ctx, sr, si, tiny);
       cudaEventRecord(ctx->ev1, ctx->stream);
       cs.wide_factor_ms = rc ? 1e300 : elapsed_ms(ctx);
       cs.panel_width = cs.wide_factor_ms < fbest ? 128 : 64;

@@ -14,8 +14,10 @@ pytestmark = pytest.mark.gpu
 NOMEM = (11, 12)  # TLR_ERR_CUDA with the allocation's message, TLR_ERR_NOMEM
 
 
-# optional: allocations of the pipelined applications (15) and their solves (4)
-@pytest.mark.parametrize("precision,block,optional", [(1, 0, 19), (1, 2, 0), (0, 0, 0)])
+# optional: allocations of the pipelined applications (15) and their solves (4), of
+# the inverse form (8: these fronts have no second diagonal block, so the inversion
+# needs no work space beyond the Schur updates'), of the slices of the FP64 form (4)
+@pytest.mark.parametrize("precision,block,optional", [(1, 0, 27), (1, 2, 8), (0, 0, 4)])
 def test_solve_after_a_failed_allocation(gpu_lib, precision, block, optional):
     ph = Physics(alpha=1.4, reynolds=700.0, nev=2, tol=1e-9)
     kw = dict(nev=2, ncv=12, precision=precision, block=block, fallback=False)
@@ -45,3 +47,25 @@ def test_solve_after_a_failed_allocation(gpu_lib, precision, block, optional):
             again = api.EigenSolver(p).solve(**kw)
         assert np.allclose(again.lam, ref.lam, rtol=1e-7, atol=0)
     assert count - failed == optional
+
+
+@pytest.mark.parametrize("precision,other", [(1, dict(cuda_core_schur=1)),
+                                             (1, dict(persistent_solve=True)),
+                                             (0, dict(cuda_core_schur=1))])
+def test_no_buffers_of_another_form(gpu_lib, precision, other):
+    """A factor makes the inverse form's or the slices' buffers only if it takes that
+    form, on its first factorisation that does."""
+    ph = Physics(alpha=1.4, reynolds=700.0, nev=2, tol=1e-9)
+    kw = dict(nev=2, ncv=12, precision=precision, fallback=False)
+    with api.Problem(make_case(17, 12, physics=ph)) as p:
+        api.run_pipeline(p)
+        lam, made = [], []
+        for opts in (other, {}, other, {}):
+            gpu_lib.tlr_alloc_fail_at(0)
+            lam.append(api.EigenSolver(p).solve(**kw, **opts).lam)
+            made.append(gpu_lib.tlr_alloc_fail_at(0))
+    own = {1: 19 if "persistent_solve" in other else 0, 0: 0}[precision]
+    assert made[1] - own == {1: 8, 0: 4}[precision]
+    assert made[2:] == [0, 0]
+    for a in lam[1:]:
+        assert np.allclose(a, lam[0], rtol=1e-7, atol=0)
