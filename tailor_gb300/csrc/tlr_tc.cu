@@ -820,16 +820,19 @@ __global__ void __launch_bounds__(kPersistThreads, 1)
       consumed_g = g;
       committed_g = committed;
     }
-  } else if (warp == 10) {  // F22 copies
+  } else if (warp == 10) {  // F22 copies, by the whole warp
     int nf22 = 0;
-    for (int t = blockIdx.x; t < tiles && !abort_flag; t += gridDim.x) {
+    bool go = true;
+    for (int t = blockIdx.x; t < tiles && go; t += gridDim.x) {
       const Tile d = decode(t);
       const int rows = min(kTcM, d.r1 - d.R0);
       for (int q = 0; q < kFSlots; ++q, ++nf22) {
-        bool ok = true;
-        if (lane == 0 && nf22 >= kFSlots)
-          ok = wait_bar(&fempty[q], (nf22 / kFSlots - 1) & 1);
-        if (!__shfl_sync(0xffffffffu, ok ? 1 : 0, 0)) break;
+        // the first lane alone looks at the abort word, so that the warp leaves
+        // as one
+        if (lane == 0)
+          go = !abort_flag && (nf22 < kFSlots || wait_bar(&fempty[q], (nf22 / kFSlots - 1) & 1));
+        go = __shfl_sync(0xffffffffu, go ? 1 : 0, 0) != 0;
+        if (!go) break;
         const int c = d.C0 + kFCols * q + lane;
         uint32_t bytes = 0;
         const float2 *src = d.F + (long long)c * d.m + d.R0;
@@ -862,9 +865,9 @@ __global__ void __launch_bounds__(kPersistThreads, 1)
         const int n0 = kFCols * q + 8 * h2;
         TLR_TC_LD8(lane_addr + n0, cr);
         TLR_TC_LD8(lane_addr + 64 + n0, ci);
-        ok = wait_bar(&ffull[q], ti & 1);
+        ok = __all_sync(0xffffffffu, wait_bar(&ffull[q], ti & 1));
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (!__all_sync(0xffffffffu, ok)) break;
+        if (!ok) break;
         if (row_ok) {
           float2 *p = d.F + (long long)(d.C0 + n0) * d.m + d.R0;
           const unsigned char *sp = fbuf + n0 * kFCol + 8 * row;
@@ -883,8 +886,9 @@ __global__ void __launch_bounds__(kPersistThreads, 1)
         if (lane == 0)
           asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(&fempty[q]))
                        : "memory");
+        __syncwarp();  // the next accumulator loads are the whole warp's
       }
-      if (!__all_sync(0xffffffffu, ok)) break;
+      if (!ok) break;
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0)
