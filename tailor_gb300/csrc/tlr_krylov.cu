@@ -616,9 +616,16 @@ struct Solver {
     return rc;
   }
 
-  // x = OP v_j for the current basis vector: rounds until x is accepted
+  // Whether the guesses are of no use: y ~ OP^2 v and u ~ OP^3 v are held in FP32's
+  // range, which the powers of an operator of scale 1e13 or 1e-13 leave.  The
+  // applications that remain are made one at a time then.
+  bool pipe_off = false;
+  int pipe_made = 0, pipe_poor = 0;  // applications; in a row that began no better than at zero
+  double pipe_first = 0.0;           // ||r|| / ||b|| of the first one's first round (from zero)
+
+  // x = OP v for the current basis vector v: rounds until x is accepted
   // (three for the first vector, then mostly one)
-  int pipe_op(double2 *x) {
+  int pipe_op(const double2 *v, double2 *x) {
     double prev = INFINITY;
     for (int round = 0;; ++round) {
       const int later = round > 0;
@@ -636,9 +643,21 @@ struct Solver {
         cudaGetLastError();  // not a failure of the solve: no timing this time
       }
       const double nr = hnorm[0], ny = hnorm[1];
+      if (round == 0) {
+        if (pipe_made == 0) pipe_first = nr / ny;
+        // the third application is the first with a guess from u
+        pipe_poor = pipe_made >= 2 && nr > refine_tol * ny && nr >= 0.1 * pipe_first * ny
+                        ? pipe_poor + 1 : 0;
+        if (pipe_poor >= 3) pipe_off = true;
+        ++pipe_made;
+      }
       if (nr <= refine_tol * ny) {
         refine_res[2] = std::max(refine_res[2], nr / ny);
         return TLR_OK;
+      }
+      if (!std::isfinite(nr)) {  // x went with the guesses: this one from nothing, too
+        pipe_off = true;
+        return op(v, x);
       }
       // no longer contracting (the float-float residual's floor), or not a
       // number: the classic loop with its FP64 residuals decides
@@ -1152,9 +1171,10 @@ int run_solve(tlr_ctx *ctx, const tlr_solve_opts *opts, double *lambda,
           ++checks;
         };
       }
-      int rc = piped      ? S.pipe_op(S.w)
+      int rc = piped      ? S.pipe_op(S.V + (size_t)j0 * n, S.w)
                : bsz == 1 ? S.op(S.V + (size_t)j0 * n, S.w)
                           : S.op_block(S.V + (size_t)j0 * n);
+      if (S.pipe_off) piped = false;
       S.host_work();  // operator paths that did not run it
       if (rc) return rc;
       if (prc) return prc;
