@@ -344,6 +344,9 @@ int tlr_mlp_create(int n_in, int width, int depth, int n_out,
                    unsigned long long seed, tlr_mlp **out);
 void tlr_mlp_destroy(tlr_mlp *m);
 long long tlr_mlp_num_params(const tlr_mlp *m);
+/* Test hook: the side of the square tiles of a layer product with rows x cols
+ * results in so many ranges of its inner index, on a GPU of sms SMs. */
+int tlr_mlp_tile(int rows, int cols, int ranges, int sms);
 /* set != 0 copies params into the network, else out of it */
 int tlr_mlp_params(tlr_mlp *m, float *params, int set);
 /* mean-squared-error loss and its parameter gradient on one batch */

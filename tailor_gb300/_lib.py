@@ -167,6 +167,7 @@ SIGNATURES = {
     "tlr_fdq_rule": ([_I, _I, _I, ctypes.c_double, _P, _P, _P, _P, _P], _I),
     "tlr_symbolic_analyze": ([_P, _P, _I, _I, _P, _P, _P, _P, _I], _I),
     "tlr_frobenius_noalloc": ([_P, ctypes.c_size_t, _P, _P], _I),
+    "tlr_mlp_tile": ([_I, _I, _I, _I], _I),
     "tlr_mlp_create": ([_I, _I, _I, _I, ctypes.c_ulonglong, _P], _I),
     "tlr_mlp_destroy": ([_P], None),
     "tlr_mlp_num_params": ([_P], ctypes.c_longlong),

@@ -30,6 +30,7 @@ struct tlr_mlp {
   float *lpart = nullptr;  // per-CTA partial losses
   int *lctr = nullptr;     // CTAs done with the loss
   long long adam_t = 0;
+  int sms = 1;
   cudaStream_t stream = nullptr;
 };
 
@@ -47,25 +48,35 @@ __device__ __forceinline__ float silu_grad(float z) {
 constexpr int kMaxSplit = 16;   // row ranges of a weight gradient
 constexpr int kLossCtas = 64;
 
-// The three products of a layer in FP32 over 64 x 64 tiles: 256 threads of 4 x
-// 4 results, inner chunks of 16 in shared memory (inner index leading), the
-// next chunk's loads in flight during the present one's FMAs.  32 x 32 tiles
-// with a result per thread were bound by shared-memory reads (two per FMA), and
-// a weight gradient by its 64 CTAs of 2048 serial rows.
+template <int N>
+struct __align__(4 * N) Vec {
+  float v[N];
+};
+
+// The three products of a layer in FP32 over kG x kG tiles: 256 threads of (kG /
+// 16)^2 results, inner chunks of 1024 / kG in shared memory (inner index leading),
+// the next chunk's loads in flight during the present one's FMAs.  64 x 64 tiles
+// are bound by the FMAs; 32 x 32 ones with a result per thread were bound by
+// shared-memory reads (two per FMA), and a weight gradient by its 64 CTAs of 2048
+// serial rows.  Small batches are bound by the latency of the chunks, so they take
+// smaller tiles and longer chunks (layer_tile).  Every result is the sum over the
+// inner index in order, whatever the tile.
 //   kFwd:    Y[r][c] = act(sum_k X[r][k] W[c][k] + b[c]), Z the pre-activation
 //   kData:   dX[r][c] = sum_k dZ[r][k] W[k][c] (times silu'(Z[r][c]) with Z)
 //   kWeight: dW[r][c] = sum_k dZ[k][r] X[k][c], db[r] = sum_k dZ[k][r] over the
 //            rows k of range blockIdx.z
 enum LayerProduct { kFwd, kData, kWeight };
-constexpr int kG = 64, kGK = 16;
+constexpr int kGK(int g) { return 1024 / g; }  // four elements of each operand per thread
 
-template <int MODE>
+template <int MODE, int kG>
 __global__ void __launch_bounds__(256)
     k_layer(int M, int N, int K, const float *__restrict__ A, int lda,
             const float *__restrict__ B, int ldb, const float *__restrict__ bias,
             float *__restrict__ Z, float *__restrict__ C, int ldc, int act, int krange,
             long long zstride, float *__restrict__ db) {
-  __shared__ __align__(16) float as[kGK][kG + 4], bs[kGK][kG + 4];
+  constexpr int kK = kGK(kG), kR = kG / 16;  // inner chunk, results per thread and side
+  constexpr int kQ = kK / 4, kL = kG / 4;    // groups of four along the inner index, of lines
+  __shared__ __align__(16) float as[kK][kG + 4], bs[kK][kG + 4];
   const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
   const int r0 = blockIdx.y * kG, c0 = blockIdx.x * kG;
   const int ka = MODE == kWeight ? blockIdx.z * krange : 0;
@@ -77,42 +88,43 @@ __global__ void __launch_bounds__(256)
   auto load = [&](int k0) {
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const int la = aInner ? tid / 4 : tx * 4 + q, k1 = k0 + (aInner ? (tid % 4) * 4 + q : ty);
+      const int la = aInner ? tid / kQ : tid % kL * 4 + q;
+      const int k1 = k0 + (aInner ? tid % kQ * 4 + q : tid / kL);
       ra[q] = r0 + la < M && k1 < kb
                   ? A[aInner ? (long long)(r0 + la) * lda + k1 : (long long)k1 * lda + r0 + la]
                   : 0.f;
-      const int lb = bInner ? tid / 4 : tx * 4 + q, k2 = k0 + (bInner ? (tid % 4) * 4 + q : ty);
+      const int lb = bInner ? tid / kQ : tid % kL * 4 + q;
+      const int k2 = k0 + (bInner ? tid % kQ * 4 + q : tid / kL);
       rb[q] = c0 + lb < N && k2 < kb
                   ? B[bInner ? (long long)(c0 + lb) * ldb + k2 : (long long)k2 * ldb + c0 + lb]
                   : 0.f;
     }
   };
-  float acc[4][4] = {};
-  float sb = 0.f;  // kWeight: this thread's share of db (64 threads of the first column)
+  float acc[kR][kR] = {};
+  float sb = 0.f;  // kWeight: this thread's share of db (a thread per row, first column)
   load(ka);
-  for (int k0 = ka; k0 < kb; k0 += kGK) {
+  for (int k0 = ka; k0 < kb; k0 += kK) {
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      if (aInner) as[(tid % 4) * 4 + q][tid / 4] = ra[q];
-      else as[ty][tx * 4 + q] = ra[q];
-      if (bInner) bs[(tid % 4) * 4 + q][tid / 4] = rb[q];
-      else bs[ty][tx * 4 + q] = rb[q];
+      if (aInner) as[tid % kQ * 4 + q][tid / kQ] = ra[q];
+      else as[tid / kL][tid % kL * 4 + q] = ra[q];
+      if (bInner) bs[tid % kQ * 4 + q][tid / kQ] = rb[q];
+      else bs[tid / kL][tid % kL * 4 + q] = rb[q];
     }
     __syncthreads();
-    if (k0 + kGK < kb) load(k0 + kGK);
+    if (k0 + kK < kb) load(k0 + kK);
 #pragma unroll
-    for (int k = 0; k < kGK; ++k) {
-      const float4 a = *reinterpret_cast<const float4 *>(&as[k][ty * 4]);
-      const float4 b = *reinterpret_cast<const float4 *>(&bs[k][tx * 4]);
-      const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+    for (int k = 0; k < kK; ++k) {
+      const auto a = *reinterpret_cast<const Vec<kR> *>(&as[k][ty * kR]);
+      const auto b = *reinterpret_cast<const Vec<kR> *>(&bs[k][tx * kR]);
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < kR; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+        for (int j = 0; j < kR; ++j) acc[i][j] = fmaf(a.v[i], b.v[j], acc[i][j]);
     }
     if (MODE == kWeight && blockIdx.x == 0 && tid < kG)
 #pragma unroll
-      for (int k = 0; k < kGK; ++k) sb += as[k][tid];
+      for (int k = 0; k < kK; ++k) sb += as[k][tid];
     __syncthreads();
   }
   if (MODE == kWeight) {
@@ -120,12 +132,12 @@ __global__ void __launch_bounds__(256)
     if (blockIdx.x == 0 && tid < kG && r0 + tid < M) db[blockIdx.z * zstride + r0 + tid] = sb;
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = r0 + ty * 4 + i;
+  for (int i = 0; i < kR; ++i) {
+    const int r = r0 + ty * kR + i;
     if (r >= M) break;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int c = c0 + tx * 4 + j;
+    for (int j = 0; j < kR; ++j) {
+      const int c = c0 + tx * kR + j;
       if (c >= N) break;
       const long long o = (long long)r * ldc + c;
       float v = acc[i][j];
@@ -139,6 +151,32 @@ __global__ void __launch_bounds__(256)
       C[o] = v;
     }
   }
+}
+
+// The tile of a product with m x n results in z ranges: the largest of 64, 32 and 16
+// that gives every other SM a CTA.  Gradients of the 256-wide network, in ms, for
+// batches of 24, 192, 512 and 2048 rows: 0.148, 0.188, 0.198, 0.302, against 0.229,
+// 0.295, 0.286, 0.312 with 64 x 64 tiles everywhere, 0.159, 0.187, 0.198, 0.341 with 32 x
+// 32 and 0.146, 0.188, 0.274, 0.635 with 16 x 16.
+int layer_tile(int m, int n, int z, int sms) {
+  for (int g = 64; g > 16; g /= 2)
+    if (2LL * blocks_for(m, g) * blocks_for(n, g) * z >= sms) return g;
+  return 16;
+}
+
+template <int MODE>
+void launch_layer(const tlr_mlp *m, int M, int N, int K, const float *A, int lda, const float *B,
+                  int ldb, const float *bias, float *Z, float *C, int ldc, int act, int nz = 1,
+                  int krange = 0, float *db = nullptr) {
+  auto go = [&](auto *kernel, int g) {
+    kernel<<<dim3(blocks_for(N, g), blocks_for(M, g), nz), 256, 0, m->stream>>>(
+        M, N, K, A, lda, B, ldb, bias, Z, C, ldc, act, krange, m->n_params, db);
+    count_launches();
+  };
+  const int g = layer_tile(M, N, nz, m->sms);
+  if (g == 64) go(k_layer<MODE, 64>, 64);
+  else if (g == 32) go(k_layer<MODE, 32>, 32);
+  else go(k_layer<MODE, 16>, 16);
 }
 
 // g[x] = the partial gradients of all row ranges, in order
@@ -255,10 +293,8 @@ void forward(tlr_mlp *m, int n) {
   for (int l = 0; l < m->n_layers; ++l) {
     const int in = m->fan_in[l], out = m->fan_out[l];
     float *Z = m->pre + plane * (l + 1), *Y = m->act + plane * (l + 1);
-    const dim3 g(blocks_for(out, kG), blocks_for(n, kG));
-    { k_layer<kFwd><<<g, 256, 0, m->stream>>>(n, out, in, X, ldx, m->params + m->w_off[l], in,
-                                              m->params + m->b_off[l], Z, Y, m->maxw,
-                                              l + 1 < m->n_layers, 0, 0, nullptr); count_launches(); }
+    launch_layer<kFwd>(m, n, out, in, X, ldx, m->params + m->w_off[l], in, m->params + m->b_off[l],
+                       Z, Y, m->maxw, l + 1 < m->n_layers);
     X = Y;
     ldx = m->maxw;
   }
@@ -279,7 +315,7 @@ void loss_gradient(tlr_mlp *m, int n) {
 void backward(tlr_mlp *m, int n) {
   const size_t plane = (size_t)m->cap * m->maxw;
   const int splits = std::min(m->max_split, std::max(1, n / 128));
-  const int krange = ((n + splits - 1) / splits + kGK - 1) / kGK * kGK;
+  const int krange = ((n + splits - 1) / splits + 15) / 16 * 16;
   const int nz = (n + krange - 1) / krange;
   float *dst = nz > 1 ? m->wpart : m->grads;
   for (int l = m->n_layers - 1; l >= 0; --l) {
@@ -287,16 +323,11 @@ void backward(tlr_mlp *m, int n) {
     const float *dZ = m->dact + plane * (l + 1);
     const float *X = l == 0 ? m->xbuf : m->act + plane * l;
     const int ldx = l == 0 ? m->n_in : m->maxw;
-    const dim3 gw(blocks_for(in, kG), blocks_for(out, kG), nz);
-    { k_layer<kWeight><<<gw, 256, 0, m->stream>>>(out, in, n, dZ, m->maxw, X, ldx, nullptr, nullptr,
-                                                  dst + m->w_off[l], in, 0, krange, m->n_params,
-                                                  dst + m->b_off[l]); count_launches(); }
-    if (l > 0) {  // times silu' of the layer below: dZ of that layer
-      const dim3 gd(blocks_for(in, kG), blocks_for(n, kG));
-      { k_layer<kData><<<gd, 256, 0, m->stream>>>(n, in, out, dZ, m->maxw, m->params + m->w_off[l],
-                                                  in, nullptr, m->pre + plane * l,
-                                                  m->dact + plane * l, m->maxw, 0, 0, 0, nullptr); count_launches(); }
-    }
+    launch_layer<kWeight>(m, out, in, n, dZ, m->maxw, X, ldx, nullptr, nullptr, dst + m->w_off[l],
+                          in, 0, nz, krange, dst + m->b_off[l]);
+    if (l > 0)  // times silu' of the layer below: dZ of that layer
+      launch_layer<kData>(m, n, in, out, dZ, m->maxw, m->params + m->w_off[l], in, nullptr,
+                          m->pre + plane * l, m->dact + plane * l, m->maxw, 0);
   }
   if (nz > 1)
     { k_sum_splits<<<blocks_for(m->n_params, 256), 256, 0, m->stream>>>(m->n_params, nz, m->wpart,
@@ -309,6 +340,10 @@ void backward(tlr_mlp *m, int n) {
 using namespace tlr;
 
 extern "C" {
+
+int tlr_mlp_tile(int rows, int cols, int ranges, int sms) {
+  return layer_tile(rows, cols, ranges, sms);
+}
 
 int tlr_mlp_create(int n_in, int width, int depth, int n_out, unsigned long long seed,
                    tlr_mlp **out) {
@@ -340,6 +375,9 @@ int tlr_mlp_create(int n_in, int width, int depth, int n_out, unsigned long long
     for (long long k = 0; k < (long long)m->fan_in[l] * m->fan_out[l]; ++k)
       h[m->w_off[l] + k] = (float)((2.0 * next() - 1.0) * a);
   }
+  int dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess)
+    cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, dev);
   // at most 256 MB of partial gradients
   m->max_split = (int)std::max(1LL, std::min<long long>(kMaxSplit, (64LL << 20) / off));
   if (cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking) ||
