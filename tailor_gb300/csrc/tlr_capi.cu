@@ -436,12 +436,17 @@ int tlr_spmv(tlr_ctx *ctx, int which, const double *x, double *y, int device_poi
     return TLR_OK;
   }
   // the two vectors are kept: the pool's memory went back at every
-  // synchronisation, so each call paid for its allocation again
+  // synchronisation, so each call paid for its allocation again.  Threads that
+  // share the context take turns with them.
+  const std::lock_guard<std::mutex> turn(ctx->spmv_mutex);
   if (!ctx->spmv_xy) TLR_CUDA(ctx, cudaMalloc(&ctx->spmv_xy, 2 * bytes));
   double2 *dx = ctx->spmv_xy, *dy = dx + 5 * (size_t)ctx->nn;
   TLR_CUDA(ctx, cudaMemcpyAsync(dx, x, bytes, cudaMemcpyHostToDevice, ctx->stream));
   const int rc = run_spmv(ctx, which, dx, dy);
-  if (rc) return rc;
+  if (rc) {
+    cudaStreamSynchronize(ctx->stream);  // x is read until then
+    return rc;
+  }
   TLR_CUDA(ctx, cudaMemcpyAsync(y, dy, bytes, cudaMemcpyDeviceToHost, ctx->stream));
   TLR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return TLR_OK;

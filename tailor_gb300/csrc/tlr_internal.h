@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -112,7 +113,8 @@ struct tlr_ctx {
   int kv_ctr_n = 0;
   double *pin = nullptr;     // pinned host words that kernels and copies write
   double *bc_part = nullptr;   // partial sums of the boundary stage's norm
-  double2 *spmv_xy = nullptr;  // operand and result of host-array products
+  double2 *spmv_xy = nullptr;  // operand and result of host-array products, one call at a time
+  std::mutex spmv_mutex;
   int *bc_modes = nullptr;   // [nz][2]: incoming and neutral counts
   double *bc_cond = nullptr; // [nz]: cond(R) per far-field node
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
