@@ -151,6 +151,21 @@ template <class T> cudaError_t pin_malloc(T **p, size_t bytes) {
   return pin_malloc(reinterpret_cast<void **>(p), bytes);
 }
 
+// Let a kernel use all the dynamic shared memory the device has for it.  The limit
+// belongs to the process and may be needed by several threads' launches of different
+// sizes at once, so none sets it to its own size.
+template <class K> cudaError_t allow_dynamic_smem(K *kernel) {
+  cudaFuncAttributes a;
+  int dev = 0, most = 0;
+  cudaError_t e = cudaFuncGetAttributes(&a, kernel);
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  if (e == cudaSuccess)
+    e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              most - (int)a.sharedSizeBytes);
+}
+
 // Stage launchers (one .cu file each).
 int run_metrics(tlr_ctx *ctx, tlr_metric_diag *diag);
 int run_derivatives(tlr_ctx *ctx, tlr_deriv_diag *diag);

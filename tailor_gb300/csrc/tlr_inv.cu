@@ -462,9 +462,7 @@ int Factor::solve_inverse(tlr_ctx *ctx, float2 *x, float2 *W, float2 *W2) {
     if (n <= 0) return TLR_OK;
     auto *kernel = small ? k_inv_apply<NR, true> : k_inv_apply<NR, false>;
     const size_t sm = vec + (small ? 3 * kMaxCols * sizeof(int) : 0);
-    if (sm > 47 * 1024)
-      TLR_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)sm));
+    if (sm > 47 * 1024) TLR_CUDA(ctx, allow_dynamic_smem(kernel));
     TLR_CUDA(ctx, launch_pdl_smem(pdl, kernel, dim3(n), dim3(32 * kW), sm, st,
                                   (const SvItem *)(d_items + off), P, (const int *)d_uidx,
                                   (const int *)d_gsrc, (const int2 *)d_cinv, W, W2, ws, x, xs,

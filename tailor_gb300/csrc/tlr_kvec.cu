@@ -304,9 +304,7 @@ int kv_update(tlr_ctx *ctx, long long n, const double2 *V, long long ldv, int nk
   if (const int rc = arrival_counters(ctx, 1)) return rc;
   const KvColumn c = column ? *column : KvColumn{};
   const size_t sm = sizeof(double2) * std::max({nk, 1, 2 * c.ldh});
-  if (sm > 47 * 1024)
-    TLR_CUDA(ctx, cudaFuncSetAttribute(k_update, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)sm));
+  if (sm > 47 * 1024) TLR_CUDA(ctx, allow_dynamic_smem(k_update));
   { k_update<<<nb, kThreads, sm, ctx->stream>>>(n, V, ldv, nk, h, w, norm ? npart : nullptr, norm,
                                                 ctx->kv_ctr, c); count_launches(); }
   TLR_CUDA(ctx, cudaGetLastError());
@@ -320,9 +318,8 @@ int kv_combine(tlr_ctx *ctx, long long n, const double2 *V, long long ldv, int n
   const dim3 grid(nb, (nl + kChunk - 1) / kChunk);
   const size_t sm = (size_t)nq * kChunk * sizeof(double2);
   if (sm > 48 * 1024) {
-    // more than 192 basis vectors: the shared-memory stage needs opting in
-    TLR_CUDA(ctx, cudaFuncSetAttribute(k_combine, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)sm));
+    // more than 768 basis vectors: the shared-memory stage needs opting in
+    TLR_CUDA(ctx, allow_dynamic_smem(k_combine));
   }
   { k_combine<<<grid, kThreads, sm, ctx->stream>>>(n, V, ldv, nq, Y, ldy, nl, out, ldo); count_launches(); }
   TLR_CUDA(ctx, cudaGetLastError());

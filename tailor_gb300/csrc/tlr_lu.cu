@@ -2828,10 +2828,8 @@ int Factor::factor_impl(tlr_ctx *ctx, double sr, double si, double tiny) {
   TLR_CUDA(ctx, cudaMemsetAsync(d_pert, 0, sizeof(int), st));
   TLR_CUDA(ctx, cudaMemsetAsync(d_tc_err, 0, sizeof(int), st));
   const size_t tsm = sizeof(C) * (size_t)(w * w + w * 34);
-  TLR_CUDA(ctx, cudaFuncSetAttribute(k_trsm_border<C>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
-  TLR_CUDA(ctx, cudaFuncSetAttribute(k_trsm_urow<C>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
+  TLR_CUDA(ctx, allow_dynamic_smem(k_trsm_border<C>));
+  TLR_CUDA(ctx, allow_dynamic_smem(k_trsm_urow<C>));
   TLR_CUDA(ctx, cudaFuncSetAttribute(k_panel_cluster_sm<C, kPanelCluster>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)kPanelSmemMax));

@@ -560,8 +560,7 @@ int pipe_shift(tlr_ctx *ctx, Pipe &p, int j, const double *beta, double sr, doub
                double2 *x, double2 *vnew, const float2 *rhs) {
   const size_t sm = sizeof(float4) * 2 * (j + 2);
   if (sm > 38 * 1024)  // the static arrays take 9 KB of the 48 KB
-    TLR_CUDA(ctx, cudaFuncSetAttribute(k_pipe_shift, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)sm));
+    TLR_CUDA(ctx, allow_dynamic_smem(k_pipe_shift));
   { k_pipe_shift<<<shift_blocks(p), kSThreads, sm, ctx->stream>>>(
       p.n, j + 1, p.ldh, p.vff, p.g, beta, ctx->B, p.B32, make_double2(sr, si), x, vnew,
       p.vff + (size_t)(j + 1) * p.n, p.xyff, p.b, p.tx, p.ty, rhs + 2 * p.n,
