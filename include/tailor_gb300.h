@@ -210,7 +210,10 @@ typedef struct {
                              32 columns (its default): tcgen05 on exact
                              integer slices of 56 bits, one FP64 rounding per
                              entry and panel, and of 64 bits in the final
-                             rewrite of the factor; other panel widths: CUDA-core
+                             rewrite of the factor (bits counted from the
+                             largest entry of an operand's row or column, after
+                             the pivots' scales; subnormal entries count as
+                             zero); other panel widths: CUDA-core
                              FP64 FMA.
                              1: CUDA cores (FP32 / FP64 FMA).  2: mixed form
                              on tcgen05 with every tile staging its own
@@ -450,6 +453,11 @@ int tlr_schur_update_c64(const float *front, int m, int p, int k0, int w, unsign
  * (nvec 2, 4 or 8; every factor tile read once), multi = 0 one at a time;
  * both give the same bits. */
 int tlr_factor_solve(tlr_ctx *ctx, int nvec, const double *rhs, double *out, int multi);
+
+/* Test hook, no counterpart in the reference: the same through the complex128
+ * factor that an FP64 tlr_solve has left, in complex128, one vector after the
+ * other. */
+int tlr_factor_solve_c128(tlr_ctx *ctx, int nvec, const double *rhs, double *out);
 
 /* Test hook, no counterpart in the reference: the same update of a
  * complex128 front (w must be 32) by exact integer slices on the tensor

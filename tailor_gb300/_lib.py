@@ -162,6 +162,7 @@ SIGNATURES = {
     "tlr_schur_update_c64": ([_P, _I, _I, _I, _I, ctypes.c_uint, ctypes.c_uint, _P], _I),
     "tlr_factor_solve": ([_P, _I, _P, _P, _I], _I),
     "tlr_alloc_fail_at": ([_I], _I),
+    "tlr_factor_solve_c128": ([_P, _I, _P, _P], _I),
     "tlr_wait_selftest": ([_I, ctypes.c_uint, _P], _I),
     "tlr_pencil_create": ([_P, _I, _P, _P, _I, _P], _I),
     "tlr_fdq_rule": ([_I, _I, _I, ctypes.c_double, _P, _P, _P, _P, _P], _I),

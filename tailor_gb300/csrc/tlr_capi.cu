@@ -509,6 +509,26 @@ int tlr_solve(tlr_ctx *ctx, const tlr_solve_opts *opts, double *lambda,
   return run_solve(ctx, opts, lambda, residual, modes, diag);
 }
 
+int tlr_factor_solve_c128(tlr_ctx *ctx, int nvec, const double *rhs, double *out) {
+  if (!ctx || !rhs || !out || nvec < 1 || nvec > 8)
+    return ctx ? fail(ctx, TLR_ERR_ARG, "tlr_factor_solve_c128: invalid arguments") : TLR_ERR_ARG;
+  Factor *F = ctx->factor;
+  if (!F || !F->factored || F->prec != 0)
+    return fail(ctx, TLR_ERR_WRONGSTATE,
+                "tlr_factor_solve_c128 needs a complex128 factorisation (an FP64 tlr_solve)");
+  cudaGetLastError();
+  const size_t n = 5 * (size_t)ctx->nn, bytes = n * nvec * sizeof(double2);
+  double2 *d = nullptr;
+  TLR_CUDA(ctx, cudaMalloc(&d, bytes));
+  int rc = cudaMemcpy(d, rhs, bytes, cudaMemcpyHostToDevice) == cudaSuccess ? TLR_OK : TLR_ERR_CUDA;
+  for (int v = 0; v < nvec && !rc; ++v) rc = F->solve(ctx, d + v * n);
+  if (!rc && (cudaStreamSynchronize(ctx->stream) != cudaSuccess ||
+              cudaMemcpy(out, d, bytes, cudaMemcpyDeviceToHost) != cudaSuccess))
+    rc = TLR_ERR_CUDA;
+  cudaFree(d);
+  return rc == TLR_ERR_CUDA ? fail(ctx, rc, "tlr_factor_solve_c128: CUDA error") : rc;
+}
+
 int tlr_factor_solve(tlr_ctx *ctx, int nvec, const double *rhs, double *out, int multi) {
   if (!ctx || !rhs || !out || nvec < 1 || nvec > 8)
     return ctx ? fail(ctx, TLR_ERR_ARG, "tlr_factor_solve: invalid arguments") : TLR_ERR_ARG;

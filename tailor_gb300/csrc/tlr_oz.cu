@@ -1,8 +1,9 @@
 // tlr_oz.cu -- FP64 products of the complex128 factorisation on the tensor
 // cores: the Schur updates F22 -= L21 U12 of the fronts and the products by the
-// inverses of the diagonal blocks that rewrite the finished factor, by exact integer slices (the splitting of Ozaki, Ogita, Oishi
-// and Rump, Numer. Algorithms 59 (2012); tcgen05 has no FP64 kind, and
-// GB300's FP64 pipe runs at about 1.1 TFLOP/s).
+// inverses of the diagonal blocks that rewrite the finished factor, by exact
+// integer slices (the splitting of Ozaki, Ogita, Oishi and Rump, Numer. Algorithms
+// 59 (2012); tcgen05 has no FP64 kind, and GB300's FP64 pipe runs at about 1.1
+// TFLOP/s).
 //
 // For an update C -= A B (A = L21, B = U12) every operand entry becomes a
 // 56-bit fixed-point number relative to its row's (A) or column's (B) largest
@@ -22,6 +23,14 @@
 // such scaling for rows and columns of any scale and stays in FP64, as do the
 // products by blocks of fewer than 32 columns, whose FP64 chains are short and
 // round less.
+//
+// An entry far below the largest of its line keeps fewer bits than FP64 would, and a
+// product of such entries alone loses by it.  A factor does not: pivoting bounds the
+// multipliers, and a line's largest products carry the rounding of either kind.
+// Backward errors of solves in extended precision, sliced / FMA: grids of 30 x 18 to
+// 130 x 60 points 0.37 to 0.91 normwise (0.33 to 1.28 by rows), pencils of order 25 to
+// 600 0.81 to 1.24, with entries spread over 2 to 16 decades without structure 0.70 to
+// 1.26 (by rows 0.66 to 1.44), with rows or columns over 6 and 12 decades 0.67 to 1.92.
 //
 // Complex products as in tlr_tc.cu: A = [Lr | Li] (128 rows), B = [Ur; -Ui]
 // and [Ui; Ur] (32 + 32 "rows"), K chunks of 8 complex columns = 16 real =
