@@ -622,6 +622,11 @@ struct Solver {
   bool pipe_off = false;
   int pipe_made = 0, pipe_poor = 0;  // applications; in a row that began no better than at zero
   double pipe_first = 0.0;           // ||r|| / ||b|| of the first one's first round (from zero)
+  // An application by itself is three solves from zero, accepted at refine_tol: mostly
+  // far below it.  A pipelined one is accepted at twice what three rounds from zero
+  // leave of the first vector, at the residual's rounding floor, or after three
+  // rounds at refine_tol.
+  double pipe_tol = 0.0;
 
   // x = OP v for the current basis vector v: rounds until x is accepted
   // (three for the first vector, then mostly one)
@@ -652,8 +657,14 @@ struct Solver {
         ++pipe_made;
       }
       if (nr <= refine_tol * ny) {
-        refine_res[2] = std::max(refine_res[2], nr / ny);
-        return TLR_OK;
+        const bool floor = round > 0 && nr > 0.25 * prev;
+        if (nr <= pipe_tol * ny || floor || round >= 2) {
+          if (pipe_made == 1 || floor) pipe_tol = std::min(refine_tol, 2.0 * nr / ny);
+          refine_res[2] = std::max(refine_res[2], nr / ny);
+          return TLR_OK;
+        }
+        prev = nr;
+        continue;
       }
       if (!std::isfinite(nr)) {  // x went with the guesses: this one from nothing, too
         pipe_off = true;

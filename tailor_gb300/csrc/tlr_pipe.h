@@ -13,11 +13,15 @@
 // x makes the next x out of y and the next y out of u; the new x usually
 // needs one correction only.  x is accepted on the same residual as before
 // (||B v - K x|| <= 1e-12 ||B v||, A x in float-float), so a poor guess
-// costs another round and no accuracy.  A step's second and later rounds refine
+// costs another round and no accuracy; and not before it is as good as three
+// corrections from nothing are (Solver::pipe_tol), which are mostly far better
+// than that limit: accepted at the limit alone, eigenvalues of pencils of a few
+// rows lost up to two digits for 1 to 3% of the time (60 x 32: 108.9 against 112.1
+// ms, 300 x 192: 898 against 910 ms).  A step's second and later rounds refine
 // u too (against B y + sigma B u in FP32), which makes the next step's y better:
 // 192 -> 175 rounds at 300 x 192, 196 -> 175 at 200 x 128, 353 -> 348 at 60 x 32.
-// Measured rounds per application: 1.12 (60 x 32), 1.16 (100 x 50), 1.32 (300 x
-// 192) and 1.35 (200 x 128, complex target; its factor contracts by 3e-5 only),
+// Measured rounds per application: 1.17 (60 x 32), 1.21 (100 x 50), 1.32 (300 x
+// 192) and 1.34 (200 x 128, complex target; its factor contracts by 3e-5 only),
 // against three dependent solves.  A pass of a point with these applications
 // alone, before and after: 221 -> 161 ms at 60 x 32, 227 -> 173 ms at 100 x 50,
 // 643 -> 594 ms at 200 x 128, 1465 -> 1231 ms at 300 x 192; refining u took
