@@ -340,7 +340,9 @@ int run_bc(tlr_ctx *ctx, tlr_bc_diag *diag) {
   if (!rc) rc = arrival_counters(ctx, 1);
   if (rc) return rc;
   // partial sums of the interior and the boundary rows, in one array
-  const int row_entries = ctx->S * 25, copy_ctas = std::min(ctx->nn, 152 * 8);
+  int sms = 1;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+  const int row_entries = ctx->S * 25, copy_ctas = std::min(ctx->nn, 8 * sms);
   if (!ctx->bc_part)
     TLR_CUDA(ctx, cudaMalloc(&ctx->bc_part, sizeof(double) * (copy_ctas + 2 * ctx->nz)));
   TLR_CUDA(ctx, cudaMemsetAsync(ctx->status, 0, sizeof(int) * ST_COUNT, ctx->stream));

@@ -341,6 +341,8 @@ int Factor::build_inverse(tlr_ctx *ctx) {
   struct Row {
     int t, r0, rows, c0, c1, kind;
   };
+  int sms = 1;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
   auto emit = [&](std::vector<Row> &rows, int &off, int &count, bool &small) {
     // three items per SM where the level has the work for them, of 256 (a
     // shorter share per warp is all start-up: 0.22 ms per solve at 100 x 50
@@ -348,7 +350,7 @@ int Factor::build_inverse(tlr_ctx *ctx) {
     long long total = 0;
     for (const Row &r : rows) total += r.c1 - r.c0;
     const int kc = (int)std::min<long long>(
-        kMaxCols, std::max<long long>(256, (total / 456 + 63) / 64 * 64));
+        kMaxCols, std::max<long long>(256, (total / (3 * sms) + 63) / 64 * 64));
     off = (int)items.size();
     int tile = 0;
     for (const Row &r : rows) {
