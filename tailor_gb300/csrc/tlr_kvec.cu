@@ -120,10 +120,10 @@ __global__ void __launch_bounds__(kThreads)
 // Column j of the projected matrix = the two Gram-Schmidt passes and beta,
 // then g1 = H h and g2 = H g1(0 : j+1), the combinations the pipelined
 // applications need (OP V h = V g1; OP V g1 = V g2 + g1(j+1) OP v_{j+1}).
-// Run by one CTA, four lanes per row; sh: 2 x ldh values.
+// Run by one CTA, four lanes per row; sh: 2 (j + 2) values.
 __device__ void projected_column(const KvColumn &c, double beta, double2 *sh) {
-  double2 *gs = sh + c.ldh;
   const int m = c.j + 2;  // rows of the column
+  double2 *gs = sh + m;
   for (int i = threadIdx.x; i < c.ldh; i += kThreads) {
     double2 v = make_double2(0.0, 0.0);
     if (i <= c.j) {
@@ -303,7 +303,11 @@ int kv_update(tlr_ctx *ctx, long long n, const double2 *V, long long ldv, int nk
   const int nb = row_blocks(ctx, n);
   if (const int rc = arrival_counters(ctx, 1)) return rc;
   const KvColumn c = column ? *column : KvColumn{};
-  const size_t sm = sizeof(double2) * std::max({nk, 1, 2 * c.ldh});
+  // 3072 vectors are the most that the update takes (48 KB of coefficients); the
+  // column's two stages are as long as this basis, whatever the largest one so far
+  if (nk > 3072)
+    return fail(ctx, TLR_ERR_CUDA, "Gram-Schmidt takes at most 3072 basis vectors");
+  const size_t sm = sizeof(double2) * std::max({nk, 1, column ? 2 * (c.j + 2) : 0});
   if (sm > 47 * 1024) TLR_CUDA(ctx, allow_dynamic_smem(k_update));
   { k_update<<<nb, kThreads, sm, ctx->stream>>>(n, V, ldv, nk, h, w, norm ? npart : nullptr, norm,
                                                 ctx->kv_ctr, c); count_launches(); }
