@@ -252,7 +252,9 @@ typedef struct {
                              CUDA graph of per-step launches; 1: one
                              persistent cooperative launch with grid
                              barriers between steps (slower on GB300: 1.82
-                             vs 1.23 ms per solve at 200 x 128)              */
+                             vs 1.23 ms per solve at 200 x 128).  The mixed
+                             form's factor has block steps then, so that a
+                             call which changes this option factors again  */
   int block;              /* Krylov block size: 0 or 1 (default) the single-
                              vector Krylov-Schur of the reference's SLEPc
                              solver; 2, 4 or 8 block Krylov-Schur, every

@@ -121,8 +121,8 @@ __device__ __forceinline__ void warp_argmax(double &best, int &bi) {
 }
 
 // Block-wide argmax of (value, row) pairs: largest value, ties to the
-// smaller row; warp shuffles, then every warp over the warp winners, so one
-// barrier is enough.
+// smaller row; integer reductions within the warps, then in every warp over the
+// warps' winners, so one barrier is enough.
 // wval / widx: 32 entries, alternate ones for successive calls.
 template <class T>
 __device__ __forceinline__ void block_argmax(T &best, int &bi, T *wval, int *widx) {

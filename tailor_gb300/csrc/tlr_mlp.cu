@@ -55,10 +55,11 @@ struct __align__(4 * N) Vec {
 
 // The three products of a layer in FP32 over kG x kG tiles: 256 threads of (kG /
 // 16)^2 results, inner chunks of 1024 / kG in shared memory (inner index leading),
-// the next chunk's loads in flight during the present one's FMAs.  64 x 64 tiles
-// are bound by the FMAs; 32 x 32 ones with a result per thread were bound by
-// shared-memory reads (two per FMA), and a weight gradient by its 64 CTAs of 2048
-// serial rows.  Small batches are bound by the latency of the chunks, so they take
+// the next chunk's loads in flight during the present one's FMAs.  32 x 32 tiles with a
+// result per thread were bound by shared-memory reads (two per FMA), and a weight
+// gradient by its 64 CTAs of 2048 serial rows.  64 x 64 ones are bound by the latency
+// of a chunk on one CTA per SM (2048 rows: 23 us, shared memory 42% and FMAs 22%
+// busy, half of the stalls for global loads).  Small batches are bound by the latency of the chunks, so they take
 // smaller tiles and longer chunks (layer_tile).  Every result is the sum over the
 // inner index in order, whatever the tile.
 //   kFwd:    Y[r][c] = act(sum_k X[r][k] W[c][k] + b[c]), Z the pre-activation

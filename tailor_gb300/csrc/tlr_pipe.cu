@@ -116,10 +116,12 @@ __global__ void k_pipe_split(long long n, const double2 *__restrict__ a, float4 
 
 // v_{j+1} = w / beta, x' = (y - V g1) / beta, y' = (u - V g2 - g1(j+1) x') /
 // beta over the nk = j + 1 old basis vectors and the new one, then B v, the
-// targets of x' and y' and B y'.  Bound by reading the basis: the products
-// run in float-float on the FP32 pipe (they only make the guesses that the
-// refinement corrects; FP64 FMAs would take ten times the reading).  The
-// new basis vector itself is formed in FP64.
+// targets of x' and y' and B y'.  A large basis is bound by reading it: the
+// products run in float-float on the FP32 pipe (they only make the guesses that
+// the refinement corrects; FP64 FMAs would take ten times the reading).  The
+// new basis vector itself is formed in FP64.  A small one is bound by the chain of
+// one CTA: 21 vectors at 100 x 50 take 20 us with DRAM 8%, the FP64 pipe (B's
+// products) 41% and the FP32 pipe 15% busy, a third of the stalls at barriers.
 __global__ void __launch_bounds__(kSThreads, 3)
     k_pipe_shift(long long n, int nk, int ldh, const float4 *__restrict__ vff,
                  const float4 *__restrict__ g, const double *__restrict__ beta,
@@ -296,9 +298,11 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 // A times x (NV = 1), x and y (NV = 2) or x, y and u (NV = 3) in float-float,
-// subtracted from the targets.  Bound by reading the operator (NV = 1) and by
-// the float-float arithmetic on the FP32 pipe (NV = 2, 96 instructions per
-// entry).  A block
+// subtracted from the targets.  Bound by reading the operator (NV = 1: 5.3 TB/s at
+// 300 x 192) and by the float-float arithmetic on the FP32 pipe (NV = 2, 96
+// instructions per entry).  At 100 x 50, two or three block rows per warp, neither is
+// reached: 49 us at 41% of DRAM's rate and 62 us with the FP32 pipe 47% busy, the
+// last rows of a CTA's warps its tail.  A block
 // row's blocks are contiguous, so each warp streams its rows (row gw, gw + W,
 // ...) through its own ring with bulk copies of six blocks, issued by its
 // first lane five stages ahead and across rows.  Lane 5 b + r multiplies row r
